@@ -76,6 +76,98 @@ struct GatherGeom {
     __host__ __device__ size_t cells4() const { return (cells() + 3) & ~size_t(3); }
 };
 
+// One tap column J of a block of Q: window slot (J + Q - 1) % Q receives column k + J + Q - 1, then
+// the Q pixel pairs m accumulate w * column (k + J + m) with the tap operation.  Weights come two taps
+// per float4.
+#define LPAICI_STEP(J)                                                                               \
+    {                                                                                                \
+        if (((J) & 1) == 0) wv = wq[(J) >> 1];                                                       \
+        const float2 w2 = ((J) & 1) ? make_float2(wv.z, wv.w) : make_float2(wv.x, wv.y);             \
+        win[((J) + Q - 1) % Q] = src[(J) + Q - 1];                                                   \
+        _Pragma("unroll") for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[((J) + m) % Q]);  \
+    }
+
+// The last N (< Q) taps of a run: their window columns and weights are loaded before any of them is
+// used, so the tail pays no load latency per tap.  Win: a pointer to the run's first column pair, or a
+// window type with the same indexing (the adjoint's masked field).
+template <int Q, int N, class Win, class Tap>
+__device__ __forceinline__ void conv_tail(float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
+                                          const float4 *__restrict__ wq, const Tap &tap) {
+    float2 tail[N];
+    float4 tw[(N + 1) / 2];
+#pragma unroll
+    for (int J = 0; J < N; J++) tail[J] = src[J + Q - 1];
+#pragma unroll
+    for (int i = 0; i < (N + 1) / 2; i++) tw[i] = wq[i];
+#pragma unroll
+    for (int J = 0; J < N; J++) {
+        const float2 w2 = (J & 1) ? make_float2(tw[J >> 1].z, tw[J >> 1].w) : make_float2(tw[J >> 1].x, tw[J >> 1].y);
+        win[(J + Q - 1) % Q] = tail[J];
+#pragma unroll
+        for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[(J + m) % Q]);
+    }
+}
+
+template <int Q, class Win, class Tap>
+__device__ __forceinline__ void conv_tail_dispatch(int rem, float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
+                                                   const float4 *__restrict__ wq, const Tap &tap) {
+    if constexpr (Q == 4) {
+        switch (rem) {
+            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
+            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
+            default: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
+        }
+    } else {
+        static_assert(Q == 8, "tile configurations use Q = 4 or 8");
+        switch (rem) {
+            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
+            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
+            case 3: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
+            case 4: conv_tail<Q, 4>(acc, win, src, wq, tap); break;
+            case 5: conv_tail<Q, 5>(acc, win, src, wq, tap); break;
+            case 6: conv_tail<Q, 6>(acc, win, src, wq, tap); break;
+            default: conv_tail<Q, 7>(acc, win, src, wq, tap); break;
+        }
+    }
+}
+
+// acc[m] = tap(acc[m], {w_j, w_j}, src[m + j]) for j < len, tap by tap in order, for the Q pixel pairs.
+// src: the run's first column in T8 (row already chosen); wq: the run's duplicated weights as
+// float4 {w_2i, w_2i, w_2i+1, w_2i+1}.
+// The last len % Q taps go to a tail of exactly that many taps (conv_tail): one warp-uniform
+// dispatch, no test per tap.  src and wq advance with the taps, so every load has a constant offset.
+template <int Q, class Win, class Tap>
+__device__ __forceinline__ void conv_run(float2 (&acc)[Q], Win src, const float4 *__restrict__ wq, int len,
+                                         const Tap &tap) {
+    float2 win[Q];
+    float4 wv;
+#pragma unroll
+    for (int i = 0; i < Q - 1; i++) win[i] = src[i];
+    int rem = len;
+    for (; rem >= Q; rem -= Q, src += Q, wq += Q / 2) {
+#pragma unroll
+        for (int J = 0; J < Q; J++) LPAICI_STEP(J)
+    }
+    // rem: 0 .. Q-1, warp-uniform: one dispatch to a tail of exactly rem taps
+    if (rem > 0) conv_tail_dispatch<Q>(rem, acc, win, src, wq, tap);
+}
+#undef LPAICI_STEP
+
+// Copies the adjoint blob to shared memory and rewrites each run (row, col, len, w) on the way into
+// (row * pitch2 + col, len, w / 2, 0): its first input pair as an offset into the tile and its first
+// duplicated weight pair as a float4 index.  Runs occupy words [run_word, weight_word).
+__device__ __forceinline__ void stage_gather_blob(int *dst, const int *__restrict__ src, int words, int run_word,
+                                           int weight_word, int pitch2) {
+    const int4 *s = reinterpret_cast<const int4 *>(src);
+    int4 *d = reinterpret_cast<int4 *>(dst);
+    const int r0 = run_word >> 2, r1 = weight_word >> 2;
+    for (int i = threadIdx.x; i < (words >> 2); i += blockDim.x) {
+        int4 v = __ldg(s + i);
+        if (i >= r0 && i < r1) v = make_int4(v.x * pitch2 + v.y, v.z, v.w >> 1, 0);
+        d[i] = v;
+    }
+}
+
 // Window of a run over a field: column i is the pair {a[i], b[i]} of the lane's two rows (b = a +
 // kGatherPair rows).  Both pointers advance with the taps, so every load has a constant offset.
 struct PairWin {
@@ -180,7 +272,7 @@ __global__ void __launch_bounds__(GatherShape<WY>::kThreads, 1)
     const int4 *s_runs = reinterpret_cast<const int4 *>(s_blob + a.run_word);
     const float4 *s_wq = reinterpret_cast<const float4 *>(s_blob + a.weight_word);
 
-    stage_blob(s_blob, a.blob, a.blob_words, a.run_word, a.weight_word, a.pitch);
+    stage_gather_blob(s_blob, a.blob, a.blob_words, a.run_word, a.weight_word, a.pitch);
     for (int k = threadIdx.x; k < nk; k += blockDim.x) s_rv[k] = rvar_k[k];
     if (threadIdx.x < 4) s_s[cells + threadIdx.x] = 0xff;  // never below a scale: the masking leaves it
 
@@ -241,7 +333,7 @@ __global__ void __launch_bounds__(GatherShape<WY>::kThreads, 1)
             }
             const int r_end = s_blob[k + 1];
             for (int r = s_blob[k] + group; r < r_end; r += G) {
-                const int4 run = s_runs[r];  // (field offset, len, float4 weight index): see stage_blob
+                const int4 run = s_runs[r];  // (field offset, len, float4 weight index): see stage_gather_blob
                 const int o = lane_off + run.x;
                 conv_run<Q>(acc, PairWin{s_f + o, s_f + o + pair_rows}, s_wq + run.z, run.y, tap);
             }

@@ -49,16 +49,13 @@ struct BatchArgs {
     float thr[kMaxKernels];
 };
 
-template <int WX, int WY, int Q>
-__global__ void __launch_bounds__(32 * WX * WY, 1)
+template <int WX, int WY, int Q, int DS>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     lpaici_batched_kernel(const __grid_constant__ BatchArgs a) {
-    using Shape = TileShape<WX, WY, Q>;
+    using Shape = TileShape<WX, WY, Q, DS>;
     extern __shared__ __align__(16) int smem[];
     const int nk = a.D * a.S;
-    int *s_blob = smem;
-    float *s_tab = reinterpret_cast<float *>(smem + a.blob_words);
-    float2 *s_tile = reinterpret_cast<float2 *>(smem + a.blob_words + table_words(nk));
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, a.R, Q);
+    const SweepCta<WX, WY, Q, DS> cta(smem, a.blob_words, nk, a.R);
 
     // the CTA's image arguments live in shared memory: in registers they would stay live across the
     // whole sweep, beside the run loop's (the single-image kernel reads them from its parameters)
@@ -85,17 +82,19 @@ __global__ void __launch_bounds__(32 * WX * WY, 1)
         s_img = img;
         s_xy = make_int2((it.y % tiles_x) * Shape::kTileW, (it.y / tiles_x) * Shape::kTileH);
     }
-    stage_blob(s_blob, a.blob, a.blob_words, a.run_word, a.weight_word, g.pitch2);
-    if (a.shared_tables) stage_tables(s_tab, a.var, a.thr, nk);
     __syncthreads();
-    if (!a.shared_tables) {
-        const float *t = a.tables + a.images[a.items[item].x].tab_offset;
-        stage_tables(s_tab, t, t + nk, nk);
-    }
     const int x0 = s_xy.x, y0 = s_xy.y;
-    load_tile(s_tile, s_img, x0, y0, g);
+    load_tile(cta.tile, s_img, x0, y0, cta.g);
+    stage_blob<Q>(cta.blob, a.blob, a.blob_words, a.run_word, a.weight_word, cta.g.pitch2);
+    if (a.shared_tables) {
+        stage_tables(cta.tab, a.var, a.thr, nk);
+    } else {
+        const float *t = a.tables + a.images[a.items[item].x].tab_offset;
+        stage_tables(cta.tab, t, t + nk, nk);
+    }
+    tile_wait();
     __syncthreads();
-    sweep_tile<WX, Q>(s_img, x0, y0, a.D, a.S, g, s_blob, a.run_word, a.weight_word, s_tab, s_tile, a.neg_zero);
+    sweep_tile<WX, WY, Q, DS, false>(s_img, x0, y0, a.D, a.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch, a.neg_zero);
 }
 
 namespace {
@@ -106,22 +105,20 @@ struct KernelInfo {
     size_t smem;
 };
 
-template <int WX, int WY, int Q>
+template <int WX, int WY, int Q, int DS>
 int batched_info(const KernelTables &tab, KernelInfo *info) {
-    using Shape = TileShape<WX, WY, Q>;
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, tab.R, Q);
-    const int nk = tab.D * tab.S;
-    info->fn = reinterpret_cast<const void *>(lpaici_batched_kernel<WX, WY, Q>);
+    using Shape = TileShape<WX, WY, Q, DS>;
+    info->fn = reinterpret_cast<const void *>(lpaici_batched_kernel<WX, WY, Q, DS>);
     info->tile_w = Shape::kTileW;
     info->tile_h = Shape::kTileH;
     info->threads = Shape::kThreads;
-    info->smem = sizeof(int) * (tab.blob_words + table_words(nk)) + g.tile_bytes();
+    info->smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
     return LPAICI_OK;
 }
 
 int get_info(int config, const KernelTables &tab, KernelInfo *info) {
-#define LPAICI_BATCH_CASE(idx, WX, WY, Q) \
-    case idx: return batched_info<WX, WY, Q>(tab, info);
+#define LPAICI_BATCH_CASE(idx, WX, WY, Q, DS) \
+    case idx: return batched_info<WX, WY, Q, DS>(tab, info);
     switch (config) {
         LPAICI_TILE_CONFIGS(LPAICI_BATCH_CASE)
         default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);
@@ -194,7 +191,8 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     KernelTables tab;
     fill_tables(ks, nullptr, 1.0f, 1.0f, &tab);
     tab.blob = blob;
-    rc = get_info(config, tab, &b->info);
+    rc = check_forward_limit(tab);
+    if (rc == LPAICI_OK) rc = get_info(config, tab, &b->info);
     if (rc != LPAICI_OK) {
         batch_plan_free(b);
         return rc;

@@ -29,11 +29,34 @@ int default_config(const lpaici_kernelset *ks) {
     return LPAICI_DEFAULT_TILE_CONFIG;  // nothing fits: the launch reports LPAICI_ERR_UNSUPPORTED
 }
 
-// ms one B200 SM (1,965 MHz) spends on one tile of each configuration, measured on the 4096^2
-// benchmark image with the 16x7 symmetric kernels (launch time / waves): the estimate for kernel sets
-// that were not tuned.
-static const float kTileMs[LPAICI_NUM_TILE_CONFIGS] = {0.349f, 0.350f, 0.357f, 0.426f, 0.427f, 0.442f,
-                                                0.261f, 0.412f, 0.412f, 0.485f, 0.479f};
+// Time of one tile of configuration c on one SM of a B200 (1,965 MHz), for kernel sets that were not tuned:
+//   base + per_work * W * (directions a round takes, rounded up) / D,   W = taps + 1.4 runs + 5 kernels,
+// fitted to 4096^2 launches (time / waves) of the 16 x 7 symmetric set (W = 8,041) and the 8 x 4 set
+// (W = 545); the tapered set (W = 14,552) is 4 % above its estimate.  A run costs about 1.4 taps beside its
+// taps, a kernel's interval update about 5 (measured with synthetic kernel sets of one run length).
+struct TileCost {
+    float base_us, ns_per_work;
+};
+static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{7.8f, 61.5f}, {8.0f, 34.1f}, {7.5f, 26.3f}, {4.2f, 17.3f},
+                                                            {2.7f, 9.11f}, {1.0f, 4.95f}, {1.2f, 2.64f}, {1.0f, 25.0f},
+                                                            {7.9f, 47.3f}, {8.7f, 36.0f}, {1.4f, 2.81f}, {5.5f, 19.5f}};
+
+static int groups_of(int c) {
+#define LPAICI_GROUPS_CASE(idx, WX, WY, Q, DS) \
+    case idx: return DS;
+    switch (c) {
+        LPAICI_TILE_CONFIGS(LPAICI_GROUPS_CASE)
+        default: return 1;
+    }
+#undef LPAICI_GROUPS_CASE
+}
+
+static float estimated_tile_ms(const lpaici_kernelset *ks, int c) {
+    const int nk = ks->D * ks->S, ds = groups_of(c);
+    const float work = static_cast<float>(ks->run_w.size()) + 1.4f * ks->layout.n_runs + 5.0f * nk;
+    const float rounded = static_cast<float>((ks->D + ds - 1) / ds * ds) / ks->D;
+    return 1e-3f * kTileCost[c].base_us + 1e-6f * kTileCost[c].ns_per_work * work * rounded;
+}
 
 // CTAs per SM of configuration c for ks on device dev (cached; 0 when it does not fit).
 static int cached_bps(const lpaici_kernelset *ks, int dev, int c, int max_optin) {
@@ -75,7 +98,7 @@ int config_for_images(const lpaici_kernelset *ks, const int *widths, const int *
     double best_ms = 0.0;
     for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
         const int bps = cached_bps(ks, dev, c, max_optin);
-        const float tile_ms = tuned.empty() ? kTileMs[c] : tuned[c];
+        const float tile_ms = tuned.empty() ? estimated_tile_ms(ks, c) : tuned[c];
         if (bps <= 0 || !(tile_ms > 0.0f)) continue;
         long tiles = 0;
         for (int i = 0; i < n; i++) tiles += tiles_of(c, widths[i], rows[i]);
@@ -198,11 +221,11 @@ int lpaici_forward_channels(const lpaici_kernelset *ks, const float *d_noisy, in
 int lpaici_num_tile_configs(void) { return LPAICI_NUM_TILE_CONFIGS; }
 
 int lpaici_tile_config_desc(int index, int *tile_w, int *tile_h, int *threads, int *pixels_per_thread) {
-#define LPAICI_DESC_CASE(idx, WX, WY, Q)                  \
+#define LPAICI_DESC_CASE(idx, WX, WY, Q, DS)              \
     case idx:                                             \
         if (tile_w) *tile_w = (WX) * 4 * (Q);             \
         if (tile_h) *tile_h = (WY) * 16;                  \
-        if (threads) *threads = 32 * (WX) * (WY);         \
+        if (threads) *threads = 32 * (WX) * (WY) * (DS);  \
         if (pixels_per_thread) *pixels_per_thread = 2 * (Q); \
         return LPAICI_OK;
     switch (index) {

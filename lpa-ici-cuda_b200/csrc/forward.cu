@@ -13,40 +13,34 @@ namespace lpaici {
 
 // Fused = false: every tap's product and sum rounded on their own (bit-exact with the reference);
 // true: each tap one fused multiply-add (lpaici_forward_ffma).
-template <int WX, int WY, int Q, bool Fused>
-__global__ void __launch_bounds__(32 * WX * WY, 1)
+template <int WX, int WY, int Q, int DS, bool Fused>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     lpaici_forward_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
-    using Shape = TileShape<WX, WY, Q>;
     extern __shared__ __align__(16) int smem[];
     const int nk = tab.D * tab.S;
-    int *s_blob = smem;
-    float *s_tab = reinterpret_cast<float *>(smem + tab.blob_words);
-    float2 *s_tile = reinterpret_cast<float2 *>(smem + tab.blob_words + table_words(nk));
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, tab.R, Q);
+    const SweepCta<WX, WY, Q, DS> cta(smem, tab.blob_words, nk, tab.R);
+    using Shape = TileShape<WX, WY, Q, DS>;
     const int x0 = blockIdx.x * Shape::kTileW, y0 = blockIdx.y * Shape::kTileH;
 
-    stage_blob(s_blob, tab.blob, tab.blob_words, tab.run_word, tab.weight_word, g.pitch2);
-    stage_tables(s_tab, tab.var, tab.thr, nk);
-    load_tile(s_tile, img, x0, y0, g);
+    load_tile(cta.tile, img, x0, y0, cta.g);
+    stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.run_word, tab.weight_word, cta.g.pitch2);
+    stage_tables(cta.tab, tab.var, tab.thr, nk);
+    tile_wait();
     __syncthreads();
-    sweep_tile<WX, Q, Fused>(img, x0, y0, tab.D, tab.S, g, s_blob, tab.run_word, tab.weight_word, s_tab, s_tile,
-                             tab.neg_zero);
+    sweep_tile<WX, WY, Q, DS, Fused>(img, x0, y0, tab.D, tab.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch, tab.neg_zero);
 }
 
 // Several images of one size, pitch, sigma and gamma in one launch (a batched plan of such images):
 // grid layer z is image z, whose buffers replace img's; everything else is the single-image kernel.  The
 // CTAs of image z + 1 fill the SMs image z's last wave leaves idle.  No counterpart in the reference.
-template <int WX, int WY, int Q>
-__global__ void __launch_bounds__(32 * WX * WY, 1)
+template <int WX, int WY, int Q, int DS>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     lpaici_forward_multi_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab,
                                 const __grid_constant__ MultiImages mi) {
-    using Shape = TileShape<WX, WY, Q>;
     extern __shared__ __align__(16) int smem[];
     const int nk = tab.D * tab.S;
-    int *s_blob = smem;
-    float *s_tab = reinterpret_cast<float *>(smem + tab.blob_words);
-    float2 *s_tile = reinterpret_cast<float2 *>(smem + tab.blob_words + table_words(nk));
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, tab.R, Q);
+    const SweepCta<WX, WY, Q, DS> cta(smem, tab.blob_words, nk, tab.R);
+    using Shape = TileShape<WX, WY, Q, DS>;
     const int x0 = blockIdx.x * Shape::kTileW, y0 = blockIdx.y * Shape::kTileH;
     ImageArgs im = img;
     im.in = mi.in[blockIdx.z];
@@ -54,24 +48,22 @@ __global__ void __launch_bounds__(32 * WX * WY, 1)
     im.smap = mi.smap[blockIdx.z];
     im.rden = mi.rden[blockIdx.z];
 
-    stage_blob(s_blob, tab.blob, tab.blob_words, tab.run_word, tab.weight_word, g.pitch2);
-    stage_tables(s_tab, tab.var, tab.thr, nk);
-    load_tile(s_tile, im, x0, y0, g);
+    load_tile(cta.tile, im, x0, y0, cta.g);
+    stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.run_word, tab.weight_word, cta.g.pitch2);
+    stage_tables(cta.tab, tab.var, tab.thr, nk);
+    tile_wait();
     __syncthreads();
-    sweep_tile<WX, Q, false>(im, x0, y0, tab.D, tab.S, g, s_blob, tab.run_word, tab.weight_word, s_tab, s_tile,
-                             tab.neg_zero);
+    sweep_tile<WX, WY, Q, DS, false>(im, x0, y0, tab.D, tab.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch, tab.neg_zero);
 }
 
 namespace {
 
-template <int WX, int WY, int Q>
+template <int WX, int WY, int Q, int DS>
 int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n,
                      cudaStream_t stream) {
-    using Shape = TileShape<WX, WY, Q>;
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, tab.R, Q);
-    const int nk = tab.D * tab.S;
-    const size_t smem = sizeof(int) * (tab.blob_words + table_words(nk)) + g.tile_bytes();
-    auto kern = lpaici_forward_multi_kernel<WX, WY, Q>;
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
+    auto kern = lpaici_forward_multi_kernel<WX, WY, Q, DS>;
     int dev = 0, max_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -89,13 +81,11 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
     return LPAICI_OK;
 }
 
-template <int WX, int WY, int Q, bool Fused>
+template <int WX, int WY, int Q, int DS, bool Fused>
 int launch_cfg(const ImageArgs &img, const KernelTables &tab, cudaStream_t stream) {
-    using Shape = TileShape<WX, WY, Q>;
-    const TileGeom g = TileGeom::make(Shape::kTileW, Shape::kTileH, tab.R, Q);
-    const int nk = tab.D * tab.S;
-    const size_t smem = sizeof(int) * (tab.blob_words + table_words(nk)) + g.tile_bytes();
-    auto kern = lpaici_forward_kernel<WX, WY, Q, Fused>;
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
+    auto kern = lpaici_forward_kernel<WX, WY, Q, DS, Fused>;
     int dev = 0, max_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -114,18 +104,18 @@ int launch_cfg(const ImageArgs &img, const KernelTables &tab, cudaStream_t strea
 
 }  // namespace
 
-#define LPAICI_FWD_CASE(idx, WX, WY, Q) \
-    case idx: return fused ? launch_cfg<WX, WY, Q, true>(img, tab, stream) : launch_cfg<WX, WY, Q, false>(img, tab, stream);
+#define LPAICI_FWD_CASE(idx, WX, WY, Q, DS) \
+    case idx: return fused ? launch_cfg<WX, WY, Q, DS, true>(img, tab, stream) : launch_cfg<WX, WY, Q, DS, false>(img, tab, stream);
 
-template <int WX, int WY, int Q>
+template <int WX, int WY, int Q, int DS>
 int blocks_per_sm(size_t smem) {
-    auto kern = lpaici_forward_kernel<WX, WY, Q, false>;
+    auto kern = lpaici_forward_kernel<WX, WY, Q, DS, false>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, TileShape<WX, WY, Q>::kThreads, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, TileShape<WX, WY, Q, DS>::kThreads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -133,8 +123,8 @@ int blocks_per_sm(size_t smem) {
 }
 
 int config_blocks_per_sm(int config, size_t smem) {
-#define LPAICI_BPS_CASE(idx, WX, WY, Q) \
-    case idx: return blocks_per_sm<WX, WY, Q>(smem);
+#define LPAICI_BPS_CASE(idx, WX, WY, Q, DS) \
+    case idx: return blocks_per_sm<WX, WY, Q, DS>(smem);
     switch (config) {
         LPAICI_TILE_CONFIGS(LPAICI_BPS_CASE)
         default: return 0;
@@ -143,7 +133,7 @@ int config_blocks_per_sm(int config, size_t smem) {
 }
 
 void config_tile(int config, int *tile_w, int *tile_h) {
-#define LPAICI_TILE_CASE(idx, WX, WY, Q) \
+#define LPAICI_TILE_CASE(idx, WX, WY, Q, DS) \
     case idx:                            \
         *tile_w = 4 * (Q) * (WX);        \
         *tile_h = 16 * (WY);             \
@@ -157,10 +147,9 @@ void config_tile(int config, int *tile_w, int *tile_h) {
 
 // Shared memory a tile configuration needs for a kernel set: blob + tables + the T8 tile.
 size_t config_smem(int config, int blob_words, int nk, int R) {
-#define LPAICI_SMEM_CASE(idx, WX, WY, Q)                                                   \
-    case idx:                                                                              \
-        return sizeof(int) * (blob_words + table_words(nk)) +                              \
-               TileGeom::make(4 * (Q) * (WX), 16 * (WY), R, Q).tile_bytes();
+#define LPAICI_SMEM_CASE(idx, WX, WY, Q, DS)                                                   \
+    case idx:                                             \
+        return sweep_smem<TileShape<WX, WY, Q, DS>, Q>(blob_words, nk, R);
     switch (config) {
         LPAICI_TILE_CONFIGS(LPAICI_SMEM_CASE)
         default: return ~size_t(0);
@@ -168,15 +157,27 @@ size_t config_smem(int config, int blob_words, int nk, int R) {
 #undef LPAICI_SMEM_CASE
 }
 
+int check_forward_limit(const KernelTables &tab) {
+    int dev = 0, max_optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const size_t need = sizeof(int) * (tab.limit_words + table_words(tab.D * tab.S)) +
+                        sizeof(float2) * static_cast<size_t>(tile_pitch2(64 + 2 * tab.R + 4)) * (24 + 2 * tab.R);
+    if (need <= static_cast<size_t>(max_optin)) return LPAICI_OK;
+    return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d", need, max_optin);
+}
+
 int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, int config,
                          cudaStream_t stream) {
     if (tab.S > kMaxScales)
         return set_error(LPAICI_ERR_UNSUPPORTED, "%d scales per direction; the kernels support at most %d", tab.S,
                          kMaxScales);
+    const int rc = check_forward_limit(tab);
+    if (rc != LPAICI_OK) return rc;
     if (n < 1 || n > kMaxMultiImages)
         return set_error(LPAICI_ERR_INVALID_ARG, "%d images in one launch; at most %d", n, kMaxMultiImages);
-#define LPAICI_MULTI_CASE(idx, WX, WY, Q) \
-    case idx: return launch_multi_cfg<WX, WY, Q>(img, tab, mi, n, stream);
+#define LPAICI_MULTI_CASE(idx, WX, WY, Q, DS) \
+    case idx: return launch_multi_cfg<WX, WY, Q, DS>(img, tab, mi, n, stream);
     switch (config) {
         LPAICI_TILE_CONFIGS(LPAICI_MULTI_CASE)
         default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);
@@ -190,6 +191,8 @@ int launch_forward(const lpaici_kernelset *ks, const ImageArgs &img, const Kerne
     if (tab.S > kMaxScales)
         return set_error(LPAICI_ERR_UNSUPPORTED, "%d scales per direction; the kernels support at most %d", tab.S,
                          kMaxScales);
+    const int rc = check_forward_limit(tab);
+    if (rc != LPAICI_OK) return rc;
     switch (config) {
         LPAICI_TILE_CONFIGS(LPAICI_FWD_CASE)
         default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);

@@ -19,20 +19,23 @@ constexpr int kMaxRadius = 127;
 // The sweeps keep each pixel's selected scale in 4 bits.
 constexpr int kMaxScales = 16;
 
-// One row run of a kernel, as the device reads it: the taps (dy, dx0 + j), j < len, whose weights
-// are wdup[wofs + j] = {w_j, w_j}.  dy/dx0 are offsets from the output pixel
-// (row - rows/2, col - cols/2); wofs is even, so two taps' duplicated weights are one 16-byte load.
-struct Run {
-    int dy, dx0, len, wofs;
-};
-
-// Device image of a kernel set, one contiguous block of 32-bit words:
+// Device image of a kernel set, one contiguous block of 32-bit words, every part 16-byte aligned.
+// A row run of a kernel is the taps (dy, dx0 + j), j < L, offsets from the output pixel (row - rows/2,
+// col - cols/2), in row-major order.  The forward's blob:
+//   [0, 2*(nk+1))           per kernel k {its first run, its first weight's byte offset in the weights};
+//                           kernel k's runs end where kernel k + 1's begin
+//   [run_word, +4*n_runs)   per run {dy, dx0, L % 4, L / 4}
+//   [weight_word, ...)      weights: per run its first L % 4 taps padded to a group of 4, then the other
+//                           taps, so that every load of a group is one aligned 16-byte load
+// The adjoint's blob (adj_layout):
 //   [0, nk+1)               first run of kernel k (kernel k's runs are [begin[k], begin[k+1]))
-//   [run_word, +4*n_runs)   Run records, 16-byte aligned
+//   [run_word, +4*n_runs)   per run {dy, dx0, L, wofs}: its weights are wdup[wofs + j] = {w_j, w_j}
 //   [weight_word, ...)      float2 {w, w} per tap, every run padded to an even number of taps
 struct BlobLayout {
-    int nk = 0, n_runs = 0, n_wdup = 0;
-    int run_word = 0, weight_word = 0, total_words = 0;  // total padded to a multiple of 4
+    int nk = 0, n_runs = 0;
+    int run_word = 0, weight_word = 0, total_words = 0;  // total a multiple of 4
+    // the forward's support limit (check_forward_limit): words of the set with every weight stored twice
+    int limit_words = 0;
 };
 
 // Per-launch arguments shared by the forward and backward kernels (passed by value as a
@@ -53,6 +56,7 @@ struct KernelTables {
     float neg_zero;  // -0.0f, read at run time (see prod2 in tile_core.cuh)
     const int *blob;  // device blob (BlobLayout)
     int blob_words, run_word, weight_word;
+    int limit_words;
     float var[kMaxKernels];
     float thr[kMaxKernels];
 };
@@ -135,6 +139,10 @@ int default_config(const lpaici_kernelset *ks);
 int config_for(const lpaici_kernelset *ks, int width, int rows);
 // The same for one launch over n images (a batched plan's tile queue): the images' tiles add up.
 int config_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n);
+// Kernel sets are supported up to what a 64 x 32 tile with 24 + 2R pair rows takes in shared memory beside
+// the set with duplicated weights: the bound on radius and taps that callers have always met, kept as it is
+// (LPAICI_ERR_UNSUPPORTED beyond it) although today's tiles and weights take less.
+int check_forward_limit(const KernelTables &tab);
 // CTAs of the forward kernel of `config` that fit on one SM with `smem` bytes of shared memory.
 int config_blocks_per_sm(int config, size_t smem);
 // Tile width and height of a configuration.

@@ -95,7 +95,6 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         wofs[r] = n2;
         n2 += (rlen[r] + 1) & ~1;
     }
-    L.n_wdup = n2;
     L.total_words = (L.weight_word + 2 * (n2 + 16) + 3) & ~3;
     ks->adj_layout = L;
     ks->adj_blob.assign(L.total_words, 0);
@@ -160,40 +159,42 @@ static int finish_kernelset(lpaici_kernelset *ks) {
     if (ks->radius > kMaxRadius)
         return set_error(LPAICI_ERR_UNSUPPORTED, "kernel radius %d exceeds the supported %d", ks->radius, kMaxRadius);
 
-    // device blob: [run begin per kernel (nk+1)] [Run records] [{w, w} per tap, runs padded to even]
+    // device blob (BlobLayout): [{first run, weight byte} per kernel (nk+1)] [{dy, dx0, L % 4, L / 4} per run]
+    // [weights: per run its first L % 4 taps padded to 4, then the other taps]
     BlobLayout &L = ks->layout;
     L.nk = nk;
     L.n_runs = static_cast<int>(ks->run_row.size());
-    L.run_word = (nk + 1 + 3) & ~3;
+    L.run_word = (2 * (nk + 1) + 3) & ~3;
     L.weight_word = L.run_word + 4 * L.n_runs;
-    std::vector<int> wofs(L.n_runs);
-    int n2 = 0;
+    int n_w = 0, n_dup = 16;
     for (int r = 0; r < L.n_runs; r++) {
-        wofs[r] = n2;
-        n2 += (ks->run_len[r] + 1) & ~1;
+        n_w += (ks->run_len[r] + 3) & ~3;
+        n_dup += (ks->run_len[r] + 1) & ~1;
     }
-    L.n_wdup = n2;
-    // 16 spare {0, 0} taps after the last run, a margin: the kernels' weight loads stay within each
-    // run's taps and its even-length padding
-    L.total_words = (L.weight_word + 2 * (n2 + 16) + 3) & ~3;
+    L.limit_words = (((nk + 1 + 3) & ~3) + 4 * L.n_runs + 2 * n_dup + 3) & ~3;
+    L.total_words = L.weight_word + n_w;
     ks->blob.assign(L.total_words, 0);
-    for (int k = 0; k < nk; k++) ks->blob[k] = ks->k_first_run[k];
-    ks->blob[nk] = L.n_runs;
     float *wd = reinterpret_cast<float *>(ks->blob.data() + L.weight_word);
+    int at = 0;
     for (int k = 0; k < nk; k++) {
+        ks->blob[2 * k] = ks->k_first_run[k];
+        ks->blob[2 * k + 1] = static_cast<int>(sizeof(float)) * at;
         int w = ks->k_first_weight[k];
         for (int r = ks->k_first_run[k]; r < ks->k_first_run[k] + ks->k_num_runs[k]; r++) {
-            ks->blob[L.run_word + 4 * r + 0] = ks->run_row[r];
-            ks->blob[L.run_word + 4 * r + 1] = ks->run_col[r];
-            ks->blob[L.run_word + 4 * r + 2] = ks->run_len[r];
-            ks->blob[L.run_word + 4 * r + 3] = wofs[r];
-            for (int j = 0; j < ks->run_len[r]; j++) {
-                wd[2 * (wofs[r] + j)] = ks->run_w[w + j];
-                wd[2 * (wofs[r] + j) + 1] = ks->run_w[w + j];
-            }
-            w += ks->run_len[r];
+            const int len = ks->run_len[r], head = len % 4;
+            int32_t *run = &ks->blob[L.run_word + 4 * r];
+            run[0] = ks->run_row[r];
+            run[1] = ks->run_col[r];
+            run[2] = head;
+            run[3] = len / 4;
+            for (int j = 0; j < head; j++) wd[at + j] = ks->run_w[w + j];
+            at += head ? 4 : 0;
+            for (int j = head; j < len; j++) wd[at++] = ks->run_w[w + j];
+            w += len;
         }
     }
+    ks->blob[2 * nk] = L.n_runs;
+    ks->blob[2 * nk + 1] = static_cast<int>(sizeof(float)) * at;
 
     return build_adjoint_blob(ks);
 }
@@ -252,6 +253,7 @@ void fill_tables(const lpaici_kernelset *ks, const float *var_or_null, float sig
     t->blob_words = ks->layout.total_words;
     t->run_word = ks->layout.run_word;
     t->weight_word = ks->layout.weight_word;
+    t->limit_words = ks->layout.limit_words;
     const float s2 = sigma * sigma;
     for (int k = 0; k < nk; k++) {
         const float v = var_or_null ? var_or_null[k] : s2 * ks->norm2[k];

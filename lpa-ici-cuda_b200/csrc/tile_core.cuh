@@ -1,19 +1,40 @@
 // tile_core.cuh -- the per-tile LPA-ICI sweep shared by the single-image, batched and adjoint kernels.
 //
 // Shared memory of one CTA:
-//   blob   the packed kernel set (BlobLayout): run ranges, Run records, duplicated weights {w, w}
+//   blob   the packed kernel set (BlobLayout): kernel table, runs, weights
 //   tab    var[nk], thr[nk], rvar[nk] = 1/var of the image being processed
-//   tile   T8[j][c] = {x(j, c), x(j + 8, c)}: the input window of the output tile as pairs of rows
-//          8 apart, j < TH - 8 + 2R, c < pitch2 (odd); input row j is output row j - R of the tile,
+//   tile   T[j][c] = {x(j, c), x(j + TH/2, c)}: the input window of the TW x TH output tile as pairs of
+//          rows TH/2 apart, j < TH/2 + 2R, c < pitch2 (odd); input row j is output row j - R of the tile,
 //          input column c is output column c - R; zero outside the input
+//   xch    (direction groups only) the groups' estimates of one round, see sweep_tile
 //
-// Thread mapping (Q = column pairs per thread, 4 or 8): a warp covers 16 rows x 4Q columns; the lane
-// with row index a (0..7) and column group b (0..3) owns the 2Q pixels of rows (a, a + 8) and columns
-// Qb .. Qb + Q - 1, held as Q float2 pairs {row a, row a + 8}.  Every window value is then a natural
-// register pair, so one packed product and one packed add do two pixels' taps.  The 16 lanes of a
-// half-warp hit 16 different bank pairs with 8-byte loads (pitch2 odd): Q = 4 puts 4 rows x 4 groups
-// in a half-warp (rows give the residues mod 4, groups the multiples of 4), Q = 8 puts 8 rows x 2
-// groups (rows give 8 distinct values mod 16 that never differ by 8, groups add 0 or 8).
+// Thread mapping (Q = column pairs per thread, 4 or 8): a region warp covers 8 + 8 rows x 4Q columns; the
+// lane with row index a (0..7) and column group b (0..3) owns the 2Q pixels of rows (a, a + TH/2) and
+// columns Qb .. Qb + Q - 1, held as Q float2 pairs {row a, row a + TH/2}.  Every window value is then a
+// natural register pair, so one packed product and one packed add do two pixels' taps.  The 16 lanes of a
+// half-warp hit 16 different bank pairs with 8-byte loads (pitch2 odd): Q = 4 puts 4 rows x 4 groups in a
+// half-warp (rows give the residues mod 4, groups the multiples of 4), Q = 8 puts 8 rows x 2 groups (rows
+// give 8 distinct values mod 16 that never differ by 8, groups add 0 or 8).  Pairing rows half a tile
+// apart instead of 8 stores TH/2 + 2R pair rows instead of TH - 8 + 2R (128 x 64 tiles at R = 31: 146 KB
+// instead of 184 KB).
+//
+// What bounds the sweep, and why it looks as it does.  The work is FP32 arithmetic, two packed
+// instructions per tap and pixel pair; on sm_100a each takes two cycles of its SM quarter's FP32 pipe, and
+// an ALU instruction beside them costs 0.2 to 0.9 cycles more (its register reads compete with the packed
+// instructions' 64-bit operands; measured with chains of packed instructions and one other instruction
+// type), a shared load next to nothing.  So:
+//   - 16 pixels per thread (Q = 8) where the image fills the chip: a run's descriptor, branches and
+//     addresses serve twice the pixels of Q = 4;
+//   - weights are single floats, four taps per 16-byte load: the packed product takes the weight as one
+//     broadcast register, a {w, w} pair costs a second operand read and twice the shared memory;
+//   - a run of L taps is a head of L % 4 taps (one dispatch to straight-line code) followed by L / 4
+//     blocks of 4 taps over a sliding register window, with the four descriptor words ready to use;
+//   - shared memory is read by 32-bit shared addresses (ld.shared in PTX): generic pointers cost a third
+//     of the uniform instructions per run.
+// 4096^2, 16 x 7 symmetric kernels: 8.15 ms before (Q = 4, 64 x 96 tiles, 103 warp instructions per run of
+// a 256-pixel warp), 7.04 ms now (128 x 64 tiles, 142 per run of a 512-pixel warp); the packed arithmetic
+// alone would take 5.3 ms.  Per tile of 8,192 pixels and 16 warps: 32 cycles a tap (the packed arithmetic's
+// own), about 45 a run and 150 an interval update.
 //
 // Arithmetic (bit-identical to src/v1_0_lpa_ici_2D_fused.cpp:803-930 for finite inputs):
 //   conv  = sum over the kernel's taps in row-major order of w*x (rounded), added one by one with
@@ -23,8 +44,6 @@
 //   lb/ub = conv -+ thr;  lo = max(lo, lb); hi = min(hi, ub); accept while hi >= lo, else stop;
 //   num  += est * (1/var); den += 1/var (in direction order, 1/var correctly rounded);  out = num / den.
 #pragma once
-
-#include <type_traits>
 
 #include "internal.h"
 
@@ -84,129 +103,181 @@ struct FmaTap {
     __device__ __forceinline__ float2 operator()(float2 acc, float2 w, float2 x) const { return fma2(w, x, acc); }
 };
 
+// Shared loads by 32-bit shared address.  Volatile keeps them behind the barrier that publishes the data.
+__device__ __forceinline__ unsigned smem_addr(const void *p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ float lds1(unsigned a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float2 lds2(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float4 lds4(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds_u2(unsigned a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ int4 lds_i4(unsigned a) {
+    int4 v;
+    asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+
+// 4 bytes from global to shared memory, asynchronously; zero (and no read) unless ok.
+__device__ __forceinline__ void copy_or_zero(unsigned dst, const float *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+
 // Smallest odd pitch (in float2) >= need.
 __host__ __device__ inline int tile_pitch2(int need) { return need | 1; }
 
-template <int WX, int WY, int Q>
+// A tile configuration: WX x WY region warps of Q column pairs per thread, times DS direction groups.
+template <int WX, int WY, int Q, int DS>
 struct TileShape {
-    static constexpr int kThreads = 32 * WX * WY;
+    static_assert(Q == 4 || Q == 8, "the lane mapping and the run loop know Q = 4 and Q = 8");
+    static constexpr int kRegion = 32 * WX * WY;  // threads of one direction group
+    static constexpr int kThreads = kRegion * DS;
     static constexpr int kTileW = WX * 4 * Q;
     static constexpr int kTileH = WY * 16;
+    // the exchange of a round: estimate * 1/var and 1/var of every group and pixel
+    static constexpr size_t kXchBytes = DS > 1 ? sizeof(float) * 2 * DS * 2 * Q * kRegion : 0;
 };
 
 // Shared-memory geometry of a tile for radius R and Q column pairs per thread: tile_w + 2R columns
 // of halo'd input plus Q spare columns, a margin no load reaches (the last column a run's window
 // reads is tile_w + 2R - 1).
 struct TileGeom {
-    int R, pitch2, pairs;  // pairs: number of T8 rows
+    int R, pitch2, pairs, half;  // pairs: number of T rows; half: rows between the two halves of a pair
     __host__ __device__ static TileGeom make(int tile_w, int tile_h, int R, int Q) {
         TileGeom g;
         g.R = R;
+        g.half = tile_h / 2;
         g.pitch2 = tile_pitch2(tile_w + 2 * R + Q);
-        g.pairs = tile_h - 8 + 2 * R;
+        g.pairs = g.half + 2 * R;
         return g;
     }
-    __host__ __device__ size_t tile_bytes() const { return sizeof(float2) * static_cast<size_t>(pitch2) * pairs; }
+    // rounded to 16 bytes: the exchange area follows
+    __host__ __device__ size_t tile_bytes() const {
+        return (sizeof(float2) * static_cast<size_t>(pitch2) * pairs + 15) & ~size_t(15);
+    }
 };
 
 // Words of shared memory before the tile: the blob, then var/thr/rvar (padded to 16 bytes).
 __host__ __device__ inline int table_words(int nk) { return (3 * nk + 3) & ~3; }
 
-// One tap column J of a block of Q: window slot (J + Q - 1) % Q receives column k + J + Q - 1, then
-// the Q pixel pairs m accumulate w * column (k + J + m) with the tap operation.  Weights come two taps
-// per float4.
-#define LPAICI_STEP(J)                                                                               \
-    {                                                                                                \
-        if (((J) & 1) == 0) wv = wq[(J) >> 1];                                                       \
-        const float2 w2 = ((J) & 1) ? make_float2(wv.z, wv.w) : make_float2(wv.x, wv.y);             \
-        win[((J) + Q - 1) % Q] = src[(J) + Q - 1];                                                   \
-        _Pragma("unroll") for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[((J) + m) % Q]);  \
-    }
+template <class Shape, int Q>
+__host__ __device__ inline size_t sweep_smem(int blob_words, int nk, int R) {
+    return sizeof(int) * (blob_words + table_words(nk)) + TileGeom::make(Shape::kTileW, Shape::kTileH, R, Q).tile_bytes() +
+           Shape::kXchBytes;
+}
 
-// The last N (< Q) taps of a run: their window columns and weights are loaded before any of them is
-// used, so the tail pays no load latency per tap.  Win: a pointer to the run's first column pair, or a
-// window type with the same indexing (the adjoint's masked field).
-template <int Q, int N, class Win, class Tap>
-__device__ __forceinline__ void conv_tail(float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
-                                          const float4 *__restrict__ wq, const Tap &tap) {
-    float2 tail[N];
-    float4 tw[(N + 1) / 2];
+// The first H = L % 4 taps of a run of L: straight-line code that loads the H + Q - 1 window columns and
+// the H weights (one 16-byte group) and leaves the window of the next tap in win[0 .. Q - 2].
+template <int Q, int H, class Tap>
+__device__ __forceinline__ void run_head(float2 (&acc)[Q], float2 (&win)[Q], unsigned src, unsigned &wp, const Tap &tap) {
+    float2 t[H + Q - 1];
+    float w[4] = {};
+    if constexpr (H == 1) {
+        w[0] = lds1(wp);
+    } else if constexpr (H == 2) {
+        const float2 v = lds2(wp);
+        w[0] = v.x, w[1] = v.y;
+    } else if constexpr (H == 3) {
+        const float4 v = lds4(wp);
+        w[0] = v.x, w[1] = v.y, w[2] = v.z;
+    }
 #pragma unroll
-    for (int J = 0; J < N; J++) tail[J] = src[J + Q - 1];
+    for (int i = 0; i < H + Q - 1; i++) t[i] = lds2(src + 8 * i);
 #pragma unroll
-    for (int i = 0; i < (N + 1) / 2; i++) tw[i] = wq[i];
+    for (int j = 0; j < H; j++)
 #pragma unroll
-    for (int J = 0; J < N; J++) {
-        const float2 w2 = (J & 1) ? make_float2(tw[J >> 1].z, tw[J >> 1].w) : make_float2(tw[J >> 1].x, tw[J >> 1].y);
-        win[(J + Q - 1) % Q] = tail[J];
+        for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], make_float2(w[j], w[j]), t[j + m]);
 #pragma unroll
-        for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[(J + m) % Q]);
+    for (int i = 0; i < Q - 1; i++) win[i] = t[H + i];
+    if constexpr (H > 0) wp += 16;
+}
+
+// Four taps; the window slots have been rotated by 4 * P taps (Q = 8 alternates P = 0, 1).  src: column
+// Q - 1 of the first of them.
+template <int Q, int P, class Tap>
+__device__ __forceinline__ void run_block(float2 (&acc)[Q], float2 (&win)[Q], unsigned src, unsigned wp, const Tap &tap) {
+    const float4 v = lds4(wp);
+    const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        win[(4 * P + j + Q - 1) % Q] = lds2(src + 8 * j);
+#pragma unroll
+        for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], make_float2(w[j], w[j]), win[(4 * P + j + m) % Q]);
     }
 }
 
-template <int Q, class Win, class Tap>
-__device__ __forceinline__ void conv_tail_dispatch(int rem, float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
-                                                   const float4 *__restrict__ wq, const Tap &tap) {
-    if constexpr (Q == 4) {
-        switch (rem) {
-            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
-            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
-            default: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
-        }
-    } else {
-        static_assert(Q == 8, "tile configurations use Q = 4 or 8");
-        switch (rem) {
-            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
-            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
-            case 3: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
-            case 4: conv_tail<Q, 4>(acc, win, src, wq, tap); break;
-            case 5: conv_tail<Q, 5>(acc, win, src, wq, tap); break;
-            case 6: conv_tail<Q, 6>(acc, win, src, wq, tap); break;
-            default: conv_tail<Q, 7>(acc, win, src, wq, tap); break;
-        }
-    }
-}
-
-// acc[m] = tap(acc[m], {w_j, w_j}, src[m + j]) for j < len, tap by tap in order, for the Q pixel pairs.
-// src: the run's first column in T8 (row already chosen); wq: the run's duplicated weights as
-// float4 {w_2i, w_2i, w_2i+1, w_2i+1}.
-// The last len % Q taps go to a tail of exactly that many taps (conv_tail): one warp-uniform
-// dispatch, no test per tap.  src and wq advance with the taps, so every load has a constant offset.
-template <int Q, class Win, class Tap>
-__device__ __forceinline__ void conv_run(float2 (&acc)[Q], Win src, const float4 *__restrict__ wq, int len,
-                                         const Tap &tap) {
+// acc[m] = tap(acc[m], w_j, T[.][col + m + j]) for j < L, tap by tap in order, for the thread's Q pixel
+// pairs.  run: {byte offset of the run's first column from the lane's pixel, L % 4, 16 * (L / 4), byte
+// offset of column L % 4 + Q - 1}; wp advances over the run's weights.
+template <int Q, class Tap>
+__device__ __forceinline__ void conv_taps(float2 (&acc)[Q], unsigned lane_base, const int4 run, unsigned &wp, const Tap &tap) {
     float2 win[Q];
-    float4 wv;
-#pragma unroll
-    for (int i = 0; i < Q - 1; i++) win[i] = src[i];
-    int rem = len;
-    for (; rem >= Q; rem -= Q, src += Q, wq += Q / 2) {
-#pragma unroll
-        for (int J = 0; J < Q; J++) LPAICI_STEP(J)
+    unsigned src = lane_base + run.x;
+    const int h = run.y;
+    if (h < 2) {
+        if (h == 0)
+            run_head<Q, 0>(acc, win, src, wp, tap);
+        else
+            run_head<Q, 1>(acc, win, src, wp, tap);
+    } else {
+        if (h == 2)
+            run_head<Q, 2>(acc, win, src, wp, tap);
+        else
+            run_head<Q, 3>(acc, win, src, wp, tap);
     }
-    // rem: 0 .. Q-1, warp-uniform: one dispatch to a tail of exactly rem taps
-    if (rem > 0) conv_tail_dispatch<Q>(rem, acc, win, src, wq, tap);
+    int n = run.z;
+    if (n == 0) return;
+    src = lane_base + run.w;
+#pragma unroll 1
+    while (true) {
+        run_block<Q, 0>(acc, win, src, wp, tap);
+        wp += 16;
+        n -= 16;
+        if constexpr (Q == 8) {
+            if (n == 0) break;
+            run_block<Q, 1>(acc, win, src + 32, wp, tap);
+            wp += 16;
+            n -= 16;
+        }
+        if (n == 0) break;
+        src += 8 * Q;
+    }
 }
-#undef LPAICI_STEP
 
-// Copies `words` 32-bit words (a multiple of 4, 16-byte aligned) from global to shared memory.
-__device__ __forceinline__ void stage_words(int *dst, const int *__restrict__ src, int words) {
-    const int4 *s = reinterpret_cast<const int4 *>(src);
-    int4 *d = reinterpret_cast<int4 *>(dst);
-    for (int i = threadIdx.x; i < (words >> 2); i += blockDim.x) d[i] = __ldg(s + i);
-}
-
-// Copies the forward blob like stage_words and rewrites each run (row, col, len, w) on the way into
-// (row * pitch2 + col, len, w / 2, 0): its first input pair as an offset into the tile and its first
-// duplicated weight pair as a float4 index.  Runs occupy words [run_word, weight_word).
-__device__ __forceinline__ void stage_blob(int *dst, const int *__restrict__ src, int words, int run_word,
-                                           int weight_word, int pitch2) {
+// Copies the forward blob to shared memory and resolves it for this tile: kernel table entries become
+// shared addresses {first run, first weight}, runs {dy, dx0, L % 4, L / 4} become the byte offsets that
+// conv_taps reads.
+template <int Q>
+__device__ __forceinline__ void stage_blob(int *dst, const int *__restrict__ src, int words, int run_word, int weight_word,
+                                           int pitch2) {
     const int4 *s = reinterpret_cast<const int4 *>(src);
     int4 *d = reinterpret_cast<int4 *>(dst);
     const int r0 = run_word >> 2, r1 = weight_word >> 2;
+    const int runs = static_cast<int>(smem_addr(dst + run_word)), weights = static_cast<int>(smem_addr(dst + weight_word));
+#pragma unroll 4
     for (int i = threadIdx.x; i < (words >> 2); i += blockDim.x) {
         int4 v = __ldg(s + i);
-        if (i >= r0 && i < r1) v = make_int4(v.x * pitch2 + v.y, v.z, v.w >> 1, 0);
+        if (i < r0) {
+            v = make_int4(runs + 16 * v.x, weights + v.y, runs + 16 * v.z, weights + v.w);
+        } else if (i < r1) {
+            const int o = 8 * (v.x * pitch2 + v.y);
+            v = make_int4(o, v.z, 16 * v.w, o + 8 * (v.z + Q - 1));
+        }
         d[i] = v;
     }
 }
@@ -220,162 +291,239 @@ __device__ __forceinline__ void stage_tables(float *s_tab, const float *var, con
     }
 }
 
-// Builds T8 for the output tile whose top-left output pixel is (x0, y0): input pixel
-// (gy0 + j, gx0 + c) and (gy0 + j + 8, gx0 + c), gy0 = y0 + row_begin - R, gx0 = x0 - R.
+// Builds T for the output tile whose top-left output pixel is (x0, y0): input pixel (gy0 + j, gx0 + c) and
+// (gy0 + j + TH/2, gx0 + c), gy0 = y0 + row_begin - R, gx0 = x0 - R.  Asynchronous 4-byte copies straight
+// into the interleaved pairs (no alignment asked of the image, zeros where it ends): no load latency is
+// waited for until tile_wait, and the kernel set is staged meanwhile (16 x 16 tiles: 24.0 us a tile, 25.7
+// with plain loads; 128 x 64: 503 us, 508).
 __device__ __forceinline__ void load_tile(float2 *s_tile, const ImageArgs &img, int x0, int y0, const TileGeom &g) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int gy0 = y0 + img.row_begin - g.R, gx0 = x0 - g.R;
     for (int j = warp; j < g.pairs; j += nwarps) {
-        const int ga = gy0 + j, gb = ga + 8;
+        const int ga = gy0 + j, gb = ga + g.half;
         const bool ok_a = ga >= 0 && ga < img.in_h, ok_b = gb >= 0 && gb < img.in_h;
         const float *ra = img.in + static_cast<size_t>(ok_a ? ga : 0) * img.in_pitch;
         const float *rb = img.in + static_cast<size_t>(ok_b ? gb : 0) * img.in_pitch;
-        float2 *dst = s_tile + j * g.pitch2;
+        const unsigned dst = smem_addr(s_tile + j * g.pitch2);
         for (int c = lane; c < g.pitch2; c += 32) {
             const int gx = gx0 + c;
             const bool ok_x = gx >= 0 && gx < img.W;
-            const size_t at = static_cast<size_t>(gx) * img.step;
-            dst[c] = make_float2(ok_a && ok_x ? __ldg(ra + at) : 0.0f, ok_b && ok_x ? __ldg(rb + at) : 0.0f);
+            const size_t at = static_cast<size_t>(ok_x ? gx : 0) * img.step;
+            copy_or_zero(dst + 8 * c, ra + at, ok_a && ok_x);
+            copy_or_zero(dst + 8 * c + 4, rb + at, ok_b && ok_x);
         }
     }
 }
+// This thread's copies have landed (the barrier after it publishes everyone's).
+__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Lane geometry inside the tile: rows ty and ty + 8, columns tx .. tx + Q - 1 (tile-local output).
-template <int WX, int Q>
-struct LaneGeom {
-    int ty, tx;
-    __device__ __forceinline__ LaneGeom() {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int a = Q == 4 ? (lane >> 2) : (lane & 7), b = Q == 4 ? (lane & 3) : (lane >> 3);
-        ty = (warp / WX) * 16 + a;
-        tx = (warp % WX) * 4 * Q + Q * b;
-    }
-};
-
-// Pixel i = 2m + h of a thread: column tx + m, row ty + 8h.
+// Pixel i = 2m + h of a thread: column tx + m, row ty + h * TH/2.
 template <int Q>
 __device__ __forceinline__ float pick(const float2 (&v)[Q], int i) { return (i & 1) ? v[i >> 1].y : v[i >> 1].x; }
 
-// Per-thread selected-scale indices, 4 bits per pixel.
-template <int Q>
-using ScaleBits = typename std::conditional<(8 * Q <= 32), unsigned, unsigned long long>::type;
-
 // The ICI scale sweep of direction d for the thread's 2Q pixels (mask `valid`): per pixel the estimate
-// of the last accepted scale (best) and that scale's index (sidx, 4 bits per pixel).  The intersection
-// [lo, hi] only shrinks, so once it is empty no later scale can be accepted: a stopped pixel needs no
-// mask, its updates simply never accept again.  Scale 0 is always accepted (lo = -inf, hi = +inf), so
-// the index is the count of accepted scales after it.  Warp-uniform scale loop; it ends when every
-// valid pixel of the warp has stopped.
-template <int Q, bool Fused>
-__device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, const float2 *lane_tile,
-                                                const int *s_blob, const int4 *s_runs, const float4 *s_wq,
-                                                const float *s_thr, float2 nz, float2 (&best)[Q], ScaleBits<Q> &sidx) {
+// of the last accepted scale (best) and that scale's index (4 bits per pixel in sidx, 8 pixels a word).
+// The intersection [lo, hi] only shrinks, so once it is empty no later scale can be accepted: a stopped
+// pixel needs no mask, its updates simply never accept again; a pixel outside the image starts with an
+// empty intersection.  Scale 0 is always accepted (lo = -inf, hi = +inf before it), so the index is the
+// count of accepted scales after it.  Warp-uniform scale loop; it ends when no pixel of the warp accepts.
+template <int Q, class Tap>
+__device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, unsigned lane_base, unsigned kernel_table,
+                                                unsigned thr_addr, const Tap &tap, float2 (&best)[Q],
+                                                unsigned (&sidx)[Q / 4]) {
     float lo[2 * Q], hi[2 * Q];
+    unsigned next = kernel_table + 8 * d * S;
+    unsigned thr_at = thr_addr + 4 * d * S;
+    const uint2 first = lds_u2(next);
+    unsigned rp = first.x, wp = first.y;
 #pragma unroll
-    for (int i = 0; i < 2 * Q; i++) {
-        lo[i] = -INFINITY;
-        hi[i] = INFINITY;
-    }
-#pragma unroll
-    for (int m = 0; m < Q; m++) best[m] = make_float2(0.0f, 0.0f);
-    sidx = 0;
-    bool alive = valid != 0;
+    for (int i = 0; i < Q / 4; i++) sidx[i] = 0;
+#pragma unroll 1
     for (int s = 0; s < S; s++) {
-        if (!__any_sync(0xffffffffu, alive)) break;  // every valid pixel of the warp has stopped
-        const int k = d * S + s;
         float2 acc[Q];
 #pragma unroll
         for (int m = 0; m < Q; m++) acc[m] = make_float2(0.0f, 0.0f);
-        const int rb = s_blob[k], re = s_blob[k + 1];
-        // two runs per iteration for Q = 4: the compiler then keeps the 768-thread tiles within 80
-        // registers without spilling (measured: 24 warps per SM beat 20)
-#pragma unroll(Q == 4 ? 2 : 1)
-        for (int r = rb; r < re; r++) {
-            const int4 run = s_runs[r];  // (tile offset, len, float4 weight index): see stage_blob
-            if constexpr (Fused)
-                conv_run<Q>(acc, lane_tile + run.x, s_wq + run.z, run.y, FmaTap{});
-            else
-                conv_run<Q>(acc, lane_tile + run.x, s_wq + run.z, run.y, ExactTap{nz});
+        next += 8;
+        const unsigned end = lds_u2(next).x;
+        if (rp != end) {
+#pragma unroll 1
+            do {
+                const int4 run = lds_i4(rp);
+                rp += 16;
+                conv_taps<Q>(acc, lane_base, run, wp, tap);
+            } while (rp != end);
         }
-        const float thr = s_thr[k];
-        const ScaleBits<Q> step = s > 0 ? 1 : 0;
-        float2 lb[Q], ub[Q];
+        const float thr = lds1(thr_at);
+        thr_at += 4;
+        if (s == 0) {
+#pragma unroll
+            for (int m = 0; m < Q; m++) {
+                const float2 lb = add2(acc[m], make_float2(-thr, -thr));  // conv - thr, exactly
+                const float2 ub = add2(acc[m], make_float2(thr, thr));
+                best[m] = acc[m];
+                lo[2 * m] = (valid >> (2 * m)) & 1u ? fmaxf(-INFINITY, lb.x) : INFINITY;
+                hi[2 * m] = (valid >> (2 * m)) & 1u ? fminf(INFINITY, ub.x) : -INFINITY;
+                lo[2 * m + 1] = (valid >> (2 * m + 1)) & 1u ? fmaxf(-INFINITY, lb.y) : INFINITY;
+                hi[2 * m + 1] = (valid >> (2 * m + 1)) & 1u ? fminf(INFINITY, ub.y) : -INFINITY;
+            }
+            continue;
+        }
+        unsigned was[Q / 4], changed = 0;
+#pragma unroll
+        for (int i = 0; i < Q / 4; i++) was[i] = sidx[i];
 #pragma unroll
         for (int m = 0; m < Q; m++) {
-            lb[m] = add2(acc[m], make_float2(-thr, -thr));  // conv - thr, exactly
-            ub[m] = add2(acc[m], make_float2(thr, thr));
+            const float2 lb = add2(acc[m], make_float2(-thr, -thr));
+            const float2 ub = add2(acc[m], make_float2(thr, thr));
+            lo[2 * m] = fmaxf(lo[2 * m], lb.x);
+            hi[2 * m] = fminf(hi[2 * m], ub.x);
+            lo[2 * m + 1] = fmaxf(lo[2 * m + 1], lb.y);
+            hi[2 * m + 1] = fminf(hi[2 * m + 1], ub.y);
+            if (hi[2 * m] >= lo[2 * m]) {
+                best[m].x = acc[m].x;
+                sidx[m / 4] += 1u << (8 * (m % 4));
+            }
+            if (hi[2 * m + 1] >= lo[2 * m + 1]) {
+                best[m].y = acc[m].y;
+                sidx[m / 4] += 16u << (8 * (m % 4));
+            }
         }
-        alive = false;
 #pragma unroll
-        for (int i = 0; i < 2 * Q; i++) {
-            lo[i] = fmaxf(lo[i], pick<Q>(lb, i));
-            hi[i] = fminf(hi[i], pick<Q>(ub, i));
-            const bool ok = hi[i] >= lo[i];
-            if (i & 1)
-                best[i >> 1].y = ok ? acc[i >> 1].y : best[i >> 1].y;
-            else
-                best[i >> 1].x = ok ? acc[i >> 1].x : best[i >> 1].x;
-            sidx += ok ? static_cast<ScaleBits<Q>>(step << (4 * i)) : ScaleBits<Q>(0);
-            alive |= ok && ((valid >> i) & 1u);
-        }
+        for (int i = 0; i < Q / 4; i++) changed |= was[i] ^ sidx[i];
+        if (!__any_sync(0xffffffffu, changed != 0)) break;  // every pixel of the warp has stopped
     }
 }
 
-// The forward sweep of one tile (tile in shared memory, block-synchronised).
-template <int WX, int Q, bool Fused = false>
+// The forward sweep of one tile (blob, tables and tile in shared memory, block-synchronised).
+//
+// DS = 1: every thread sweeps all directions of its pixels and sums num and den in registers.  DS > 1:
+// DS groups of threads cover the same pixels and take the directions in rounds, group g direction
+// round * DS + g; after each round the groups' estimates meet in shared memory (xch) and each group adds
+// them, in direction order, to the num and den of its share of the pixels -- the same additions in the same
+// order as DS = 1, so the results are equal bit for bit.  A tile then takes 1/DS of the time: images with
+// fewer pixels than the chip has room for (148 SMs x 8,192 pixels) are cut into smaller tiles (97 x 64: 257
+// us before, 27 us as 16 x 16 tiles of 16 groups; 512^2: 268 us before, 147 us as 64 x 32 tiles of 4).  It
+// costs halo and a barrier per round: at 4096^2 the tiles of 2, 4, 8 and 16 groups take 7.9, 8.0, 8.4 and
+// 9.0 ms against 7.04 ms.
+template <int WX, int WY, int Q, int DS, bool Fused>
 __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0, int D, int S, const TileGeom &g,
-                                           const int *s_blob, int run_word, int weight_word, const float *s_tab,
-                                           const float2 *s_tile, float neg_zero) {
-    const LaneGeom<WX, Q> lg;
+                                           const int *s_blob, const float *s_tab, const float2 *s_tile, float *s_xch,
+                                           float neg_zero) {
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const int group = DS == 1 ? 0 : static_cast<int>(threadIdx.x) / Shape::kRegion;
+    const int rt = threadIdx.x - group * Shape::kRegion;  // thread of the region
+    const int warp = rt >> 5, lane = rt & 31;
+    const int a = Q == 4 ? (lane >> 2) : (lane & 7), b = Q == 4 ? (lane & 3) : (lane >> 3);
+    const int ty = (warp / WX) * 8 + a, tx = (warp % WX) * 4 * Q + Q * b;
     const int nk = D * S;
-    const int oy = y0 + lg.ty, ox = x0 + lg.tx;
+    const int oy = y0 + ty, ox = x0 + tx;
     unsigned valid = 0;
 #pragma unroll
     for (int i = 0; i < 2 * Q; i++)
-        if (oy + 8 * (i & 1) < img.rows_out && ox + (i >> 1) < img.W) valid |= 1u << i;
-    const float2 *lane_tile = s_tile + (lg.ty + g.R) * g.pitch2 + lg.tx + g.R;
-    const int4 *s_runs = reinterpret_cast<const int4 *>(s_blob + run_word);
-    const float4 *s_wq = reinterpret_cast<const float4 *>(s_blob + weight_word);
-    const float *s_thr = s_tab + nk, *s_rvar = s_tab + 2 * nk;
+        if (oy + g.half * (i & 1) < img.rows_out && ox + (i >> 1) < img.W) valid |= 1u << i;
+    const bool work = __any_sync(0xffffffffu, valid != 0);  // a warp outside the image only joins the barriers
+    if (DS == 1 && !work) return;
+    const unsigned lane_base = smem_addr(s_tile + (ty + g.R) * g.pitch2 + tx + g.R);
+    const unsigned kernel_table = smem_addr(s_blob);
+    const unsigned thr_addr = smem_addr(s_tab + nk), rvar_addr = smem_addr(s_tab + 2 * nk);
+    // opaque, so that the compiler keeps it in a register instead of reading it again in every run
+    asm volatile("mov.b32 %0, %0;" : "+f"(neg_zero));
     const float2 nz = make_float2(neg_zero, neg_zero);
 
+    // the pixels whose num and den this thread sums: all 2Q (DS = 1), else kOwn of them
+    constexpr int kOwn = DS == 1 ? 2 * Q : (2 * Q >= DS ? 2 * Q / DS : 1);
     float2 num[Q], den[Q];
+    float onum[kOwn], oden[kOwn];
+    if constexpr (DS == 1) {
 #pragma unroll
-    for (int m = 0; m < Q; m++) num[m] = den[m] = make_float2(0.0f, 0.0f);
+        for (int m = 0; m < Q; m++) num[m] = den[m] = make_float2(0.0f, 0.0f);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kOwn; i++) onum[i] = oden[i] = 0.0f;
+    }
 
-    for (int d = 0; d < D; d++) {
-        float2 best[Q];
-        ScaleBits<Q> sidx;
-        direction_sweep<Q, Fused>(d, S, valid, lane_tile, s_blob, s_runs, s_wq, s_thr, nz, best, sidx);
+#pragma unroll 1
+    for (int d0 = 0; d0 < D; d0 += DS) {
+        const int d = d0 + group;
+        if (DS > 1 && d0 > 0) __syncthreads();  // the previous round's estimates have been added
+        if (d < D && work) {
+            float2 best[Q];
+            unsigned sidx[Q / 4];
+            if constexpr (Fused)
+                direction_sweep<Q>(d, S, valid, lane_base, kernel_table, thr_addr, FmaTap{}, best, sidx);
+            else
+                direction_sweep<Q>(d, S, valid, lane_base, kernel_table, thr_addr, ExactTap{nz}, best, sidx);
+            const unsigned rd = rvar_addr + 4 * d * S;
 #pragma unroll
-        for (int m = 0; m < Q; m++) {
-            const float2 r = make_float2(s_rvar[d * S + static_cast<int>((sidx >> (8 * m)) & 15)],
-                                         s_rvar[d * S + static_cast<int>((sidx >> (8 * m + 4)) & 15)]);
-            num[m] = add2(num[m], prod2(best[m], r, nz));
-            den[m] = add2(den[m], r);
+            for (int m = 0; m < Q; m++) {
+                const unsigned bits = sidx[m / 4] >> (8 * (m % 4));
+                const float2 r = make_float2(lds1(rd + 4 * (bits & 15)), lds1(rd + 4 * ((bits >> 4) & 15)));
+                const float2 e = prod2(best[m], r, nz);
+                if constexpr (DS == 1) {
+                    num[m] = add2(num[m], e);
+                    den[m] = add2(den[m], r);
+                } else {
+                    float *x = s_xch + (group * 2 * Q + 2 * m) * Shape::kRegion + rt;
+                    x[0] = e.x;
+                    x[Shape::kRegion] = e.y;
+                    x += DS * 2 * Q * Shape::kRegion;
+                    x[0] = r.x;
+                    x[Shape::kRegion] = r.y;
+                }
+            }
+            if (img.smap) {
+#pragma unroll
+                for (int i = 0; i < 2 * Q; i++)
+                    if (valid & (1u << i))
+                        img.smap[(static_cast<size_t>(d) * img.rows_out + oy + g.half * (i & 1)) * img.W + ox + (i >> 1)] =
+                            static_cast<uint8_t>((sidx[i / 8] >> (4 * (i % 8))) & 15);
+            }
         }
-        if (img.smap) {
+        if constexpr (DS > 1) {
+            __syncthreads();
+            if (group * kOwn < 2 * Q && work) {
+                const float *x = s_xch + group * kOwn * Shape::kRegion + rt;
 #pragma unroll
-            for (int i = 0; i < 2 * Q; i++)
-                if (valid & (1u << i))
-                    img.smap[(static_cast<size_t>(d) * img.rows_out + oy + 8 * (i & 1)) * img.W + ox + (i >> 1)] =
-                        static_cast<uint8_t>((sidx >> (4 * i)) & 15);
+                for (int e = 0; e < DS; e++) {
+                    if (d0 + e >= D) break;
+#pragma unroll
+                    for (int i = 0; i < kOwn; i++) {
+                        const float *p = x + (e * 2 * Q + i) * Shape::kRegion;
+                        onum[i] = __fadd_rn(onum[i], p[0]);
+                        oden[i] = __fadd_rn(oden[i], p[DS * 2 * Q * Shape::kRegion]);
+                    }
+                }
+            }
         }
     }
-    if (img.out) {
+    if (DS > 1 && group * kOwn >= 2 * Q) return;
 #pragma unroll
-        for (int i = 0; i < 2 * Q; i++)
-            if (valid & (1u << i))
-                img.out[static_cast<size_t>(oy + 8 * (i & 1)) * img.out_pitch +
-                        static_cast<size_t>(ox + (i >> 1)) * img.step] =
-                    __fdiv_rn(pick<Q>(num, i), pick<Q>(den, i));
-    }
-    if (img.rden) {
-#pragma unroll
-        for (int i = 0; i < 2 * Q; i++)
-            if (valid & (1u << i))
-                img.rden[static_cast<size_t>(oy + 8 * (i & 1)) * img.W + ox + (i >> 1)] = __frcp_rn(pick<Q>(den, i));
+    for (int j = 0; j < kOwn; j++) {
+        const int i = DS == 1 ? j : group * kOwn + j;
+        if (!(valid & (1u << i))) continue;
+        const float nu = DS == 1 ? pick<Q>(num, j) : onum[j], de = DS == 1 ? pick<Q>(den, j) : oden[j];
+        const int y = oy + g.half * (i & 1), x = ox + (i >> 1);
+        if (img.out)
+            img.out[static_cast<size_t>(y) * img.out_pitch + static_cast<size_t>(x) * img.step] = __fdiv_rn(nu, de);
+        if (img.rden) img.rden[static_cast<size_t>(y) * img.W + x] = __frcp_rn(de);
     }
 }
+
+// One CTA's work on the tile at (x0, y0) of img: stages the kernel set, the tables and the tile, and sweeps.
+template <int WX, int WY, int Q, int DS>
+struct SweepCta {
+    using Shape = TileShape<WX, WY, Q, DS>;
+    int *blob;
+    float *tab;
+    float2 *tile;
+    float *xch;
+    TileGeom g;
+    __device__ __forceinline__ SweepCta(int *smem, int blob_words, int nk, int R)
+        : blob(smem), g(TileGeom::make(Shape::kTileW, Shape::kTileH, R, Q)) {
+        tab = reinterpret_cast<float *>(smem + blob_words);
+        tile = reinterpret_cast<float2 *>(smem + blob_words + table_words(nk));
+        xch = reinterpret_cast<float *>(reinterpret_cast<char *>(tile) + g.tile_bytes());
+    }
+};
 
 }  // namespace lpaici

@@ -1,0 +1,80 @@
+"""The tile sweep's run loop and direction groups at their edges, bit for bit against the oracle: direction
+counts below, at and beside the groups of a tile configuration, run lengths with every remainder of the
+four-tap blocks (1 to 9 taps), one to sixteen scales, images at and beside the tiles' edges."""
+import numpy as np
+import pytest
+
+import lpaici
+import oracle_bind as ob
+
+pytestmark = pytest.mark.gpu
+
+
+def random_set(D, S, seed):
+    """Dense kernels of D x S: rows of 1 .. 9 taps at random offsets, some rows empty."""
+    rng = np.random.default_rng(seed)
+    w, off, rows, cols = [], [], [], []
+    at = 0
+    shapes = [(int(rng.integers(1, 8)), int(rng.integers(9, 14))) for _ in range(S)]
+    for _ in range(D):
+        for s in range(S):
+            r, c = shapes[s]
+            h = np.zeros((r, c), np.float32)
+            for y in range(r):
+                if y != r // 2 and rng.random() < 0.25:
+                    continue
+                n = int(rng.integers(1, 10))
+                x = int(rng.integers(0, c - n + 1))
+                h[y, x:x + n] = rng.uniform(0.05, 1.0, n).astype(np.float32)
+            h /= h.sum()
+            w.append(h.ravel())
+            off.append(at)
+            rows.append(r)
+            cols.append(c)
+            at += r * c
+    w = np.concatenate(w).astype(np.float32)
+    off, rows, cols = (np.array(v, np.int32) for v in (off, rows, cols))
+    return (lpaici.KernelSet.from_dense(w, off, rows, cols, D, S), ob.DenseKernels(D, S, w, off, rows, cols))
+
+
+@pytest.mark.parametrize("config", range(lpaici.lib().lpaici_num_tile_configs()))
+@pytest.mark.parametrize("D,S", [(1, 1), (2, 16), (3, 4), (5, 2), (16, 3), (17, 2)])
+def test_sweep_edges(config, D, S):
+    import torch
+
+    ks, ko = random_set(D, S, 100 * D + S)
+    tw, th, _, _ = lpaici.tile_configs()[config]
+    ks.set_tile_config(config)
+    sigma, gamma = 0.1, 1.7
+    var = ks.variances(sigma)
+    for W, H in ((1, 1), (tw, th), (tw + 1, th // 2 + 1), (2 * tw - 1, th + 3)):
+        rng = np.random.default_rng(W * 1000 + H)
+        x = rng.uniform(0.0, 1.0, (H, W)).astype(np.float32)
+        out, smap = lpaici.forward(ks, torch.from_numpy(x).cuda(), sigma, gamma, scale_map=True)
+        ref, rmap, _ = ob.oracle_forward_f32(x, ko, var, gamma, want_map=True)
+        assert np.array_equal(smap.cpu().numpy(), rmap), (W, H)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32)), (W, H)
+
+
+def test_non_finite_pixels_reach_the_same_outputs():
+    """Infinities and NaNs in the input: every tile configuration gives the same bits (no configuration
+    multiplies a pixel by a padding weight)."""
+    import torch
+
+    ks, _ = random_set(5, 3, 7)
+    rng = np.random.default_rng(3)
+    x = rng.uniform(0.0, 1.0, (70, 90)).astype(np.float32)
+    for v in (np.inf, -np.inf, np.nan):
+        x[rng.integers(0, 70), rng.integers(0, 90)] = v
+    t = torch.from_numpy(x).cuda()
+    ref = None
+    for config in range(lpaici.lib().lpaici_num_tile_configs()):
+        ks.set_tile_config(config)
+        out, smap = (v.cpu().numpy() for v in lpaici.forward(ks, t, 0.1, 1.7, scale_map=True))
+        if ref is None:
+            ref = (out, smap)
+            reach = ~np.isfinite(out)
+            assert reach.any() and not reach.all()
+        assert np.array_equal(np.nan_to_num(out, nan=7.5).view(np.uint32),
+                              np.nan_to_num(ref[0], nan=7.5).view(np.uint32)), config
+        assert np.array_equal(smap, ref[1]), config
