@@ -39,7 +39,7 @@ struct TileCost {
 };
 static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{7.8f, 61.5f}, {8.0f, 34.1f}, {7.5f, 26.3f}, {4.2f, 17.3f},
                                                             {2.7f, 9.11f}, {1.0f, 4.95f}, {1.2f, 2.64f}, {1.0f, 25.0f},
-                                                            {7.9f, 47.3f}, {8.7f, 36.0f}, {1.4f, 2.81f}, {5.5f, 19.5f}};
+                                                            {7.9f, 47.3f}, {8.7f, 36.0f}, {5.5f, 19.5f}};
 
 static int groups_of(int c) {
 #define LPAICI_GROUPS_CASE(idx, WX, WY, Q, DS) \
@@ -103,7 +103,10 @@ int config_for_images(const lpaici_kernelset *ks, const int *widths, const int *
         long tiles = 0;
         for (int i = 0; i < n; i++) tiles += tiles_of(c, widths[i], rows[i]);
         const long slots = static_cast<long>(sms) * bps;
-        const double est = tile_ms * bps * static_cast<double>((tiles + slots - 1) / slots);
+        // a lone CTA of a configuration that two fit on an SM takes 1.5 tile times, not 2 (97 x 64 as 28
+        // tiles of 16 x 16: 36.9 us against 24 us for one more tile per SM at full occupancy)
+        const double waves = tiles <= sms ? 0.5 * (1 + bps) / bps : static_cast<double>((tiles + slots - 1) / slots);
+        const double est = tile_ms * bps * waves;
         if (best < 0 || est < best_ms) {
             best = c;
             best_ms = est;
@@ -226,7 +229,7 @@ int lpaici_tile_config_desc(int index, int *tile_w, int *tile_h, int *threads, i
         if (tile_w) *tile_w = (WX) * 4 * (Q);             \
         if (tile_h) *tile_h = (WY) * 16;                  \
         if (threads) *threads = 32 * (WX) * (WY) * (DS);  \
-        if (pixels_per_thread) *pixels_per_thread = 2 * (Q); \
+        if (pixels_per_thread) *pixels_per_thread = 2 * (Q) / (DS); \
         return LPAICI_OK;
     switch (index) {
         LPAICI_TILE_CONFIGS(LPAICI_DESC_CASE)

@@ -19,12 +19,11 @@
     X(7, 4, 2, 4, 1)           \
     X(8, 3, 4, 8, 1)           \
     X(9, 2, 4, 8, 1)           \
-    X(10, 1, 1, 4, 16)         \
-    X(11, 2, 4, 4, 2)
+    X(10, 2, 4, 4, 2)
 
-#define LPAICI_NUM_TILE_CONFIGS 12
+#define LPAICI_NUM_TILE_CONFIGS 11
 #define LPAICI_DEFAULT_TILE_CONFIG 0
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.
-#define LPAICI_TILE_PREFERENCE {0, 8, 1, 2, 9, 3, 4, 5, 11, 7, 6, 10}
+#define LPAICI_TILE_PREFERENCE {0, 8, 1, 3, 2, 4, 9, 5, 10, 6, 7}

@@ -294,7 +294,7 @@ __device__ __forceinline__ void stage_tables(float *s_tab, const float *var, con
 // Builds T for the output tile whose top-left output pixel is (x0, y0): input pixel (gy0 + j, gx0 + c) and
 // (gy0 + j + TH/2, gx0 + c), gy0 = y0 + row_begin - R, gx0 = x0 - R.  Asynchronous 4-byte copies straight
 // into the interleaved pairs (no alignment asked of the image, zeros where it ends): no load latency is
-// waited for until tile_wait, and the kernel set is staged meanwhile (16 x 16 tiles: 24.0 us a tile, 25.7
+// waited for until tile_wait, and the kernel set is staged meanwhile (16 x 16 tiles: 22.4 us a tile, 24.0
 // with plain loads; 128 x 64: 503 us, 508).
 __device__ __forceinline__ void load_tile(float2 *s_tile, const ImageArgs &img, int x0, int y0, const TileGeom &g) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -402,7 +402,7 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
 // them, in direction order, to the num and den of its share of the pixels -- the same additions in the same
 // order as DS = 1, so the results are equal bit for bit.  A tile then takes 1/DS of the time: images with
 // fewer pixels than the chip has room for (148 SMs x 8,192 pixels) are cut into smaller tiles (97 x 64: 257
-// us before, 27 us as 16 x 16 tiles of 16 groups; 512^2: 268 us before, 147 us as 64 x 32 tiles of 4).  It
+// us before, 37 us as 16 x 16 tiles of 8 groups; 512^2: 268 us before, 147 us as 64 x 32 tiles of 4).  It
 // costs halo and a barrier per round: at 4096^2 the tiles of 2, 4, 8 and 16 groups take 7.9, 8.0, 8.4 and
 // 9.0 ms against 7.04 ms.
 template <int WX, int WY, int Q, int DS, bool Fused>
