@@ -11,19 +11,23 @@
 //      pixel) and 1/den(p) into a transient workspace -- the forward stores nothing for the adjoint;
 //   u: u = g / den over the workspace's 1/den (an elementwise pass; from a kept state the gather forms
 //      the product itself);
-//   B. gather: one CTA per 128 x 64 output tile.  Per direction it reads s*(d,.) and u on the tile plus
-//      its R-pixel halo (from L2) and forms the field c_d = u / v_{d,s*} in shared memory.
+//   B. gather: 128 x 64 output tiles.  Per direction it reads s*(d,.) and u on the tile plus its R-pixel
+//      halo (from L2) and forms the field c_d = u / v_{d,s*} in shared memory.
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
 //      turns the sum over scales into
 //          sum_s D_s (*) (c_d [s* >= s]):
 //      the field is zeroed in place where s* < s, scale after scale (only where the next kernel
-//      reaches), and never rebuilt.  The runs are the forward's run loop (register sliding window over
-//      Q columns, exact-length tails) with packed FMAs over two output rows -- the adjoint is checked
-//      against FP64 finite differences, not bit patterns.  Groups of warps take every G-th run of each
-//      kernel over the same outputs and add their sums in group order at the end.  Every output is
-//      written once: no atomics, deterministic.
+//      reaches), and never rebuilt.  Two groups of warps take every other run of each kernel over the same
+//      outputs.  Every output is written once: no atomics, deterministic.
+//
+// Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
+// zero (its runs in order), the chunks' sums are added in order, and group 1's total is added to group 0's.
+// A tile is gathered by one CTA or by a cluster of kGatherChunks or half as many CTAs that share the chunks
+// and add the same sums in the same order through distributed shared memory, so the gradient does not depend on
+// how many CTAs a tile gets (single images, plans and kept states agree bit for bit).
 // No counterpart in the reference.
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -36,148 +40,30 @@ namespace lpaici {
 
 namespace {
 
-// Gather tile geometry.  A lane owns output rows ty and ty + 8 at Q = 8 consecutive columns and keeps
-// them as the two halves of packed FMAs; a warp covers 16 rows x 32 columns: lane l has row index
-// a = l & 7 and column group b = l >> 3.  The fields are plain row-major float arrays whose pitch p is
-// 1 mod 8, so the 32 lanes' scalar loads of one row hit 32 different banks (a*p gives the residues
-// mod 8, 8b the multiples of 8).  kGatherWX warps across and WY down make one group; G groups cover
-// the same outputs, each with every G-th run of a kernel: four groups of up to 256 threads, else as
-// many as make 1,024 threads.  Eight columns per lane spread each run's loop, window preload and tail
-// over 16 outputs.
-constexpr int kGatherQ = 8;
-constexpr int kGatherPair = 8;  // rows between a lane's two output rows
-constexpr int kGatherWX = 4;
-constexpr int kGatherWarpCols = 32 / kGatherPair * kGatherQ;  // columns one warp covers
-template <int WY>
+// Gather tile geometry.  A lane owns output rows ty, ty + 1 (ty even) at Q = 16 consecutive columns; a warp
+// covers 32 rows x 32 columns (lane l: row pair l & 15, column group l >> 4), WX x WY warps make a group,
+// two groups a CTA.
+//
+// Why row pairs one row apart: field row j meets output row y in kernel row j - y and output row y + 1 in
+// kernel row j - y - 1, so one window of field values serves both output rows, and the packed FMA takes
+// {D(dy, t), D(dy - 1, t)} times one broadcast value.  Against rows 8 apart with one weight and a pair of
+// values per tap (the design before), that halves the shared loads, which the gather was limited by (29
+// wavefronts a run of 5.7 taps against 8 x 5.7 packed FMAs at 16 outputs a lane), and the packed FMA itself
+// issues faster: 2.0 to 2.2 cycles with one 64-bit operand reused, one broadcast and the accumulator,
+// against 2.4 to 3.4 with three register pairs (measured in chains).  It costs the taps where only one of
+// two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.
+// Q = 16 spreads a run's descriptor, branches and window over 32 outputs.
+// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 475 us now (313 us of it the runs: 254 cycles
+// a run of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 47 us, masking 60 us); tapered
+// set 964 and 705 us; 384 x 320 (15 tiles) 571 and 70 us.
+constexpr int kGatherQ = 16;
+constexpr int kGatherGroups = 2;
+constexpr int kGatherChunks = 8;
+template <int WX, int WY>
 struct GatherShape {
-    static constexpr int kTW = kGatherWarpCols * kGatherWX;
-    static constexpr int kTH = 2 * kGatherPair * WY;
-    static constexpr int kGroupThreads = 32 * kGatherWX * WY;
-    static constexpr int kG = kGroupThreads > 256 ? 1024 / kGroupThreads : 4;
-    static constexpr int kThreads = kG * kGroupThreads;
-};
-// Tile heights the host can choose (the tallest whose field and kernels fit in shared memory): 128 x 64
-// output tiles (two groups of 16 warps) for the 16 x 7 sets with radius 31.
-constexpr int kGatherNWY = 4;
-constexpr int kGatherWYs[kGatherNWY] = {4, 3, 2, 1};
-
-// Field geometry: rows th + 2R, pitch 1 mod 8 and >= tw + 2R + Q (a margin no load reaches).
-struct GatherGeom {
-    int rows, pitch;
-    __host__ __device__ static GatherGeom make(int tw, int th, int R) {
-        GatherGeom g;
-        g.rows = th + 2 * R;
-        g.pitch = ((tw + 2 * R + kGatherQ + 6) & ~7) + 1;
-        return g;
-    }
-    __host__ __device__ size_t cells() const { return static_cast<size_t>(rows) * pitch; }
-    // cells rounded up to whole 4-cell words: the field and the scale map start 16-byte aligned, as the
-    // masking's 16-byte accesses need
-    __host__ __device__ size_t cells4() const { return (cells() + 3) & ~size_t(3); }
-};
-
-// One tap column J of a block of Q: window slot (J + Q - 1) % Q receives column k + J + Q - 1, then
-// the Q pixel pairs m accumulate w * column (k + J + m) with the tap operation.  Weights come two taps
-// per float4.
-#define LPAICI_STEP(J)                                                                               \
-    {                                                                                                \
-        if (((J) & 1) == 0) wv = wq[(J) >> 1];                                                       \
-        const float2 w2 = ((J) & 1) ? make_float2(wv.z, wv.w) : make_float2(wv.x, wv.y);             \
-        win[((J) + Q - 1) % Q] = src[(J) + Q - 1];                                                   \
-        _Pragma("unroll") for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[((J) + m) % Q]);  \
-    }
-
-// The last N (< Q) taps of a run: their window columns and weights are loaded before any of them is
-// used, so the tail pays no load latency per tap.  Win: a pointer to the run's first column pair, or a
-// window type with the same indexing (the adjoint's masked field).
-template <int Q, int N, class Win, class Tap>
-__device__ __forceinline__ void conv_tail(float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
-                                          const float4 *__restrict__ wq, const Tap &tap) {
-    float2 tail[N];
-    float4 tw[(N + 1) / 2];
-#pragma unroll
-    for (int J = 0; J < N; J++) tail[J] = src[J + Q - 1];
-#pragma unroll
-    for (int i = 0; i < (N + 1) / 2; i++) tw[i] = wq[i];
-#pragma unroll
-    for (int J = 0; J < N; J++) {
-        const float2 w2 = (J & 1) ? make_float2(tw[J >> 1].z, tw[J >> 1].w) : make_float2(tw[J >> 1].x, tw[J >> 1].y);
-        win[(J + Q - 1) % Q] = tail[J];
-#pragma unroll
-        for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], w2, win[(J + m) % Q]);
-    }
-}
-
-template <int Q, class Win, class Tap>
-__device__ __forceinline__ void conv_tail_dispatch(int rem, float2 (&acc)[Q], float2 (&win)[Q], const Win &src,
-                                                   const float4 *__restrict__ wq, const Tap &tap) {
-    if constexpr (Q == 4) {
-        switch (rem) {
-            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
-            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
-            default: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
-        }
-    } else {
-        static_assert(Q == 8, "tile configurations use Q = 4 or 8");
-        switch (rem) {
-            case 1: conv_tail<Q, 1>(acc, win, src, wq, tap); break;
-            case 2: conv_tail<Q, 2>(acc, win, src, wq, tap); break;
-            case 3: conv_tail<Q, 3>(acc, win, src, wq, tap); break;
-            case 4: conv_tail<Q, 4>(acc, win, src, wq, tap); break;
-            case 5: conv_tail<Q, 5>(acc, win, src, wq, tap); break;
-            case 6: conv_tail<Q, 6>(acc, win, src, wq, tap); break;
-            default: conv_tail<Q, 7>(acc, win, src, wq, tap); break;
-        }
-    }
-}
-
-// acc[m] = tap(acc[m], {w_j, w_j}, src[m + j]) for j < len, tap by tap in order, for the Q pixel pairs.
-// src: the run's first column in T8 (row already chosen); wq: the run's duplicated weights as
-// float4 {w_2i, w_2i, w_2i+1, w_2i+1}.
-// The last len % Q taps go to a tail of exactly that many taps (conv_tail): one warp-uniform
-// dispatch, no test per tap.  src and wq advance with the taps, so every load has a constant offset.
-template <int Q, class Win, class Tap>
-__device__ __forceinline__ void conv_run(float2 (&acc)[Q], Win src, const float4 *__restrict__ wq, int len,
-                                         const Tap &tap) {
-    float2 win[Q];
-    float4 wv;
-#pragma unroll
-    for (int i = 0; i < Q - 1; i++) win[i] = src[i];
-    int rem = len;
-    for (; rem >= Q; rem -= Q, src += Q, wq += Q / 2) {
-#pragma unroll
-        for (int J = 0; J < Q; J++) LPAICI_STEP(J)
-    }
-    // rem: 0 .. Q-1, warp-uniform: one dispatch to a tail of exactly rem taps
-    if (rem > 0) conv_tail_dispatch<Q>(rem, acc, win, src, wq, tap);
-}
-#undef LPAICI_STEP
-
-// Copies the adjoint blob to shared memory and rewrites each run (row, col, len, w) on the way into
-// (row * pitch2 + col, len, w / 2, 0): its first input pair as an offset into the tile and its first
-// duplicated weight pair as a float4 index.  Runs occupy words [run_word, weight_word).
-__device__ __forceinline__ void stage_gather_blob(int *dst, const int *__restrict__ src, int words, int run_word,
-                                           int weight_word, int pitch2) {
-    const int4 *s = reinterpret_cast<const int4 *>(src);
-    int4 *d = reinterpret_cast<int4 *>(dst);
-    const int r0 = run_word >> 2, r1 = weight_word >> 2;
-    for (int i = threadIdx.x; i < (words >> 2); i += blockDim.x) {
-        int4 v = __ldg(s + i);
-        if (i >= r0 && i < r1) v = make_int4(v.x * pitch2 + v.y, v.z, v.w >> 1, 0);
-        d[i] = v;
-    }
-}
-
-// Window of a run over a field: column i is the pair {a[i], b[i]} of the lane's two rows (b = a +
-// kGatherPair rows).  Both pointers advance with the taps, so every load has a constant offset.
-struct PairWin {
-    const float *a, *b;
-    __device__ __forceinline__ float2 operator[](int i) const { return make_float2(a[i], b[i]); }
-    __device__ __forceinline__ PairWin &operator+=(int n) {
-        a += n;
-        b += n;
-        return *this;
-    }
+    static constexpr int kTW = 32 * WX, kTH = 32 * WY;
+    static constexpr int kRegion = 32 * WX * WY;
+    static constexpr int kThreads = kGatherGroups * kRegion;
 };
 
 // One image of the gather: pass A's outputs and the caller's buffers.
@@ -195,12 +81,12 @@ struct GatherImage {
 struct GatherArgs {
     GatherImage single;          // the image of a one-image launch (images == null)
     const GatherImage *images;   // batched: per-image descriptors in device memory
-    const int2 *items;           // batched: (image, tile) of every CTA
+    const int2 *items;           // batched: (image, tile) of every tile
     int D, S, R;
-    const int *blob;       // mirrored kernels (lpaici_kernelset::adj_blob, BlobLayout)
-    int blob_words, run_word, weight_word;
-    int pitch, rows;       // field geometry (GatherGeom of the tile)
-    int th;                // output rows per tile
+    const int *blob;       // mirrored kernels (lpaici_kernelset::adj_blob, AdjointLayout)
+    int block_bytes;       // shared memory for one kernel's block
+    int pitch, plane;      // field geometry (AdjointLayout)
+    int cluster;           // CTAs per tile: 1, kGatherChunks / 2 or kGatherChunks
     float rvar[kMaxKernels];  // 1 / v_k of the one image
     // per kernel: the field cells its correlation reads, rows [x, y), columns [z, w); per direction: the
     // union over its scales (the cells its field needs)
@@ -208,49 +94,265 @@ struct GatherArgs {
     int4 drect[kMaxKernels];
 };
 
-// Shared memory: blob (runs as field offsets) | 1/v table | field | selected scales.
-__host__ __device__ inline int rv_words(int nk) { return (nk + 3) & ~3; }
-// The scale map carries 4 bytes past its last cell, set to 0xff: the masking reads it in whole words.
-__host__ __device__ inline size_t gather_smem(int blob_words, int nk, const GatherGeom &g) {
-    return sizeof(int) * (blob_words + rv_words(nk)) + sizeof(float) * g.cells4() + ((g.cells4() + 4 + 15) & ~size_t(15));
+// Shared memory: kernel table | 1/v table | non-finite flags | two kernel blocks | field | selected scales |
+// the groups' sums over the chunks (touched once per chunk: in registers they would cost the run loop its own).
+// The field is stored as two planes of even and odd rows (field row r: plane r & 1, row r >> 1): the 16 row
+// pairs of a warp start on rows of one parity, so with an odd pitch its 32 scalar loads hit 32 banks.
+struct GatherSmem {
+    int rv, flag, block, field, smap, sums, total;  // byte offsets
+    __host__ __device__ static GatherSmem make(int nk, int block_bytes, int plane, int region) {
+        GatherSmem m;
+        m.rv = (8 * (nk + 1) + 15) & ~15;
+        m.flag = m.rv + ((4 * nk + 15) & ~15);
+        m.block = m.flag + 16;
+        m.field = m.block + 2 * block_bytes;
+        m.smap = m.field + 4 * 2 * plane;
+        m.sums = m.smap + ((2 * plane + 15) & ~15);
+        m.total = m.sums + static_cast<int>(sizeof(float2)) * kGatherQ * region * kGatherGroups;
+        return m;
+    }
+};
+
+// The first H = L % 4 taps of a run: H + 15 field values, H weight pairs; leaves the next tap's window.
+template <int H>
+__device__ __forceinline__ void gather_head(float2 (&acc)[kGatherQ], float (&win)[kGatherQ], unsigned &src, unsigned &wp) {
+    constexpr int Q = kGatherQ;
+    float lead[H > 0 ? H : 1];  // the H columns before the next tap's window
+    float2 w[H > 0 ? H : 1];
+#pragma unroll
+    for (int j = 0; j < H; j++) w[j] = lds2(wp + 8 * j);
+#pragma unroll
+    for (int j = 0; j < H; j++) lead[j] = lds1(src + 4 * j);
+#pragma unroll
+    for (int i = 0; i < Q - 1; i++) win[i] = lds1(src + 4 * (H + i));
+#pragma unroll
+    for (int j = 0; j < H; j++)
+#pragma unroll
+        for (int m = 0; m < Q; m++) {
+            const float x = j + m < H ? lead[j + m < H ? j + m : 0] : win[j + m < H ? 0 : j + m - H];
+            acc[m] = fma2(w[j], make_float2(x, x), acc[m]);
+        }
+    src += 4 * (H + Q - 1);
+    wp += 8 * H;
 }
 
-// Columns [c0, c1) of field row i0 / pitch of a direction's field build, lanes along the row: s*(d, .)
-// into s_s and c_d = u / v_{d,s*} into s_f.  u is read from drow (UReady: u = g / den already) or formed
-// as g * (1/den); cells outside the image get s* = 0 and u = 0.
-template <bool UReady>
-__device__ __forceinline__ void build_field_row(uint8_t *s_s, float *s_f, const float *rv_d, const uint8_t *prow,
-                                                const float *grow, const float *drow, int i0, int c0, int c1, int gx0,
-                                                int W, bool row_ok, int lane) {
-    for (int c = c0 + lane; c < c1; c += 32) {
-        const int gx = gx0 + c;
-        unsigned sc = 0u;
-        float u = 0.0f;
-        if (row_ok && gx >= 0 && gx < W) {
-            sc = __ldg(prow + gx);
-            u = UReady ? __ldg(drow + gx) : __ldg(grow + gx) * __ldg(drow + gx);
+// Four taps; the window slots have been rotated by 4 * P taps.
+template <int P>
+__device__ __forceinline__ void gather_block(float2 (&acc)[kGatherQ], float (&win)[kGatherQ], unsigned src, unsigned wp) {
+    constexpr int Q = kGatherQ;
+    float2 w[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) w[j] = lds2(wp + 8 * j);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        win[(4 * P + j + Q - 1) % Q] = lds1(src + 4 * j);
+#pragma unroll
+        for (int m = 0; m < Q; m++) {
+            const float x = win[(4 * P + j + m) % Q];
+            acc[m] = fma2(w[j], make_float2(x, x), acc[m]);
         }
-        s_s[i0 + c] = static_cast<uint8_t>(sc);
-        s_f[i0 + c] = u * rv_d[sc];
     }
 }
 
-template <int WY>
-__global__ void __launch_bounds__(GatherShape<WY>::kThreads, 1)
+// acc[m] += {w0_t, w1_t} * field[src + m + t] over a run of 4n + h taps.
+__device__ __forceinline__ void gather_run(float2 (&acc)[kGatherQ], unsigned src, unsigned wp, int h, int n) {
+    float win[kGatherQ];
+    if (h < 2) {
+        if (h == 0)
+            gather_head<0>(acc, win, src, wp);
+        else
+            gather_head<1>(acc, win, src, wp);
+    } else {
+        if (h == 2)
+            gather_head<2>(acc, win, src, wp);
+        else
+            gather_head<3>(acc, win, src, wp);
+    }
+    if (n == 0) return;
+#pragma unroll 1
+    while (true) {
+        gather_block<0>(acc, win, src, wp);
+        src += 16; wp += 32;
+        if (--n == 0) break;
+        gather_block<1>(acc, win, src, wp);
+        src += 16; wp += 32;
+        if (--n == 0) break;
+        gather_block<2>(acc, win, src, wp);
+        src += 16; wp += 32;
+        if (--n == 0) break;
+        gather_block<3>(acc, win, src, wp);
+        src += 16; wp += 32;
+        if (--n == 0) break;
+    }
+}
+
+// The same for a field with infinities or NaNs: the padding weights (-0, where only the other output row has
+// a tap) are skipped, so that only the pixels whose kernels reach such a value see it.
+__device__ __noinline__ void gather_run_skipping(float2 *acc, unsigned src, unsigned wp, int len) {
+    for (int t = 0; t < len; t++) {
+        const float2 w = lds2(wp + 8 * t);
+        const bool first = __float_as_uint(w.x) != 0x80000000u, second = __float_as_uint(w.y) != 0x80000000u;
+        for (int m = 0; m < kGatherQ; m++) {
+            const float x = lds1(src + 4 * (t + m));
+            if (first) acc[m].x = fmaf(w.x, x, acc[m].x);
+            if (second) acc[m].y = fmaf(w.y, x, acc[m].y);
+        }
+    }
+}
+
+// A byte or a float from global memory, 0 (and no read) unless ok: predicated, no branch around every load.
+__device__ __forceinline__ unsigned ldg_u8_if(const uint8_t *p, bool ok) {
+    unsigned v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.nc.u8 %0, [%1];\n\t}"
+                 : "=r"(v)
+                 : "l"(p), "r"(static_cast<int>(ok)));
+    return v;
+}
+__device__ __forceinline__ float ldg_if(const float *p, bool ok) {
+    float v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+                 : "=f"(v)
+                 : "l"(p), "r"(static_cast<int>(ok)));
+    return v;
+}
+
+// s*(d, .) and c_d = u / v_{d, s*}, u = g / den (0 outside the image), for the field rows [dr.x, dr.y) and
+// columns [dr.z, dr.w) that the direction's kernels reach; the other cells keep stale values that no
+// correlation of this direction reads.  u is read again for every direction (from L2): kept in shared memory
+// it would not leave room for 128 x 64 tiles.  A warp takes kRows rows of kAcross x 32 columns at a time, all
+// loads in flight: between the barriers around it the build is bound by the loads' latency and the index
+// arithmetic, not by the bytes.  Returns whether a value of this thread is infinite or NaN.
+template <bool UReady, bool Inside>
+__device__ __forceinline__ bool build_field(float *s_f, uint8_t *s_s, const float *rv_d, const GatherImage &im,
+                                            const uint8_t *map, const int4 dr, int gx0, int gy0, int pitch, int plane,
+                                            int warp, int nwarps, int lane) {
+    constexpr int kRows = 2, kAcross = 5;
+    bool bad = false;
+    const unsigned rv = smem_addr(rv_d);
+    for (int c0 = dr.z; c0 < dr.w; c0 += 32 * kAcross) {
+        const int c = c0 + lane, gx = gx0 + c;
+        // columns c + 32 i: stored for i < stored, read from the image for first <= i < past
+        const int stored = (dr.w - c + 31) >> 5, first = gx >= 0 ? 0 : (-gx + 31) >> 5, past = min(stored, (im.W - gx + 31) >> 5);
+        for (int r0 = dr.x + warp; r0 < dr.y; r0 += kRows * nwarps) {
+            float u[kRows][kAcross];
+            unsigned sc[kRows][kAcross];
+#pragma unroll
+            for (int j = 0; j < kRows; j++) {
+                const int r = r0 + j * nwarps, gy = gy0 + r;
+                const bool ok = r < dr.y && (Inside || (gy >= 0 && gy < im.H));
+                const ptrdiff_t px = static_cast<ptrdiff_t>(ok ? gy : 0) * im.W + gx;
+                const uint8_t *pm = map + px;
+                const float *pd = im.rden + px, *pg = im.g + static_cast<ptrdiff_t>(ok ? gy : 0) * im.g_pitch + gx;
+                const int f = Inside ? 0 : first, e = ok ? (Inside ? stored : past) : 0;
+#pragma unroll
+                for (int i = 0; i < kAcross; i++) {
+                    const bool in = (Inside || i >= f) && i < e;
+                    sc[j][i] = ldg_u8_if(pm + 32 * i, in);
+                    u[j][i] = ldg_if(pd + 32 * i, in);
+                    if (!UReady) u[j][i] = ldg_if(pg + 32 * i, in) * u[j][i];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kRows; j++) {
+                const int r = r0 + j * nwarps;
+                if (r >= dr.y) break;
+                const int at = (r & 1) * plane + (r >> 1) * pitch + c;
+                float *pf = s_f + at;
+                uint8_t *ps = s_s + at;
+#pragma unroll
+                for (int i = 0; i < kAcross; i++) {
+                    const float v = u[j][i] * lds1(rv + 4 * sc[j][i]);
+                    bad |= !(fabsf(v) <= FLT_MAX);
+                    if (i < stored) {
+                        ps[32 * i] = static_cast<uint8_t>(sc[j][i]);
+                        pf[32 * i] = v;
+                    }
+                }
+            }
+        }
+    }
+    return bad;
+}
+
+// All ones where the top bit of byte B is set, else 0 (prmt's sign replication).
+template <int B>
+__device__ __forceinline__ unsigned spread_top_bit(unsigned v) {
+    unsigned r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(0x8888 + 0x1111 * B));
+    return r;
+}
+
+// Zeroes the field where s* < s, in the rows and columns of rc: every 4-cell word from the rectangle's first
+// cell to its last in each row plane, as one flat range over all threads (the cells beside the rectangle in
+// those rows are masked too: zeroing a cell with s* < s anywhere keeps the field c_d [s* >= s]).  Per byte,
+// (s* | 0x80) - s keeps its top bit exactly where s* >= s (scales are below 0x80) and borrows from no other
+// byte; cells outside this direction's region hold stale bytes, which no correlation reads.
+__device__ __forceinline__ void mask_words(float *s_f, const uint8_t *s_s, int first, int end, unsigned below, int nthreads) {
+    constexpr int kWords = 4;  // loaded before the first is used
+    const unsigned *sw = reinterpret_cast<const unsigned *>(s_s);
+    float4 *f4 = reinterpret_cast<float4 *>(s_f);
+    for (int w = first; w < end; w += kWords * nthreads) {
+        unsigned v[kWords];
+#pragma unroll
+        for (int j = 0; j < kWords; j++) v[j] = w + j * nthreads < end ? sw[w + j * nthreads] : 0xffffffffu;
+#pragma unroll
+        for (int j = 0; j < kWords; j++) {
+            const unsigned ge = ((v[j] | 0x80808080u) - below) & 0x80808080u;
+            if (ge != 0x80808080u) {  // a cell of the word has s* < s: keep the others
+                float4 f = f4[w + j * nthreads];
+                f.x = __uint_as_float(__float_as_uint(f.x) & spread_top_bit<0>(ge));
+                f.y = __uint_as_float(__float_as_uint(f.y) & spread_top_bit<1>(ge));
+                f.z = __uint_as_float(__float_as_uint(f.z) & spread_top_bit<2>(ge));
+                f.w = __uint_as_float(__float_as_uint(f.w) & spread_top_bit<3>(ge));
+                f4[w + j * nthreads] = f;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void mask_field(float *s_f, const uint8_t *s_s, const int4 rc, unsigned s, int pitch, int plane,
+                                           int tid, int nthreads) {
+    const unsigned below = 0x01010101u * s;
+    // even rows (rc.x + 1) / 2 .. (rc.y + 1) / 2 of plane 0, odd rows rc.x / 2 .. rc.y / 2 of plane 1; the odd
+    // rows go to the threads from the last one on, which the even rows' last step leaves idle
+    const int e0 = (rc.x + 1) >> 1, e1 = (rc.y + 1) >> 1, o0 = rc.x >> 1, o1 = rc.y >> 1;
+    if (e1 > e0)
+        mask_words(s_f, s_s, ((e0 * pitch + rc.z) >> 2) + tid, ((e1 - 1) * pitch + rc.w + 3) >> 2, below, nthreads);
+    if (o1 > o0)
+        mask_words(s_f, s_s, ((plane + o0 * pitch + rc.z) >> 2) + (nthreads - 1 - tid), (plane + (o1 - 1) * pitch + rc.w + 3) >> 2,
+                   below, nthreads);
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The float2 at shared address a of CTA `rank` of the cluster.
+__device__ __forceinline__ float2 cluster_lds2(unsigned a, unsigned rank) {
+    unsigned remote;
+    float2 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+    return v;
+}
+
+template <int WX, int WY>
+__global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     lpaici_adjoint_gather_kernel(const __grid_constant__ GatherArgs a) {
-    using Shape = GatherShape<WY>;
-    constexpr int Q = kGatherQ, G = Shape::kG;
+    using Shape = GatherShape<WX, WY>;
+    constexpr int Q = kGatherQ, nthreads = Shape::kThreads;
     extern __shared__ __align__(16) int smem[];
     const int nk = a.D * a.S;
-    const int cells = a.rows * a.pitch, cells4 = (cells + 3) & ~3;
-    int *s_blob = smem;
-    float *s_rv = reinterpret_cast<float *>(smem + a.blob_words);
-    float *s_f = s_rv + rv_words(nk);  // the field of the current direction
-    uint8_t *s_s = reinterpret_cast<uint8_t *>(s_f + cells4);  // s*(d, .) on the halo'd tile
+    const GatherSmem lay = GatherSmem::make(nk, a.block_bytes, a.plane, Shape::kRegion);
+    char *base = reinterpret_cast<char *>(smem);
+    uint2 *s_tab = reinterpret_cast<uint2 *>(base);
+    float *s_rv = reinterpret_cast<float *>(base + lay.rv);
+    int *s_flag = reinterpret_cast<int *>(base + lay.flag);
+    float *s_f = reinterpret_cast<float *>(base + lay.field);  // the field of the current direction
+    uint8_t *s_s = reinterpret_cast<uint8_t *>(base + lay.smap);  // s*(d, .) on the halo'd tile
+    const int rank = a.cluster > 1 ? static_cast<int>(blockIdx.x % a.cluster) : 0;
+    int tile = blockIdx.x / a.cluster;
     GatherImage im;
-    int tile = blockIdx.x;
     if (a.images) {
-        const int2 it = a.items[blockIdx.x];
+        const int2 it = a.items[tile];
         im = a.images[it.x];
         tile = it.y;
     } else {
@@ -259,115 +361,160 @@ __global__ void __launch_bounds__(GatherShape<WY>::kThreads, 1)
     const float *rvar_k = a.images ? im.rvar : a.rvar;
     const int x0 = (tile % im.tiles_x) * Shape::kTW, y0 = (tile / im.tiles_x) * Shape::kTH;
     const int gx0 = x0 - a.R, gy0 = y0 - a.R;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = Shape::kThreads >> 5;
-    // the group is the same in every lane of a warp: reduced, the compiler knows it warp-uniform, so the
-    // run loops and the tails' dispatch branch without reconvergence bookkeeping
-    const int group = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(threadIdx.x / Shape::kGroupThreads));
-    const int gtid = threadIdx.x % Shape::kGroupThreads;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
+    // the same in every lane of a warp: reduced, the compiler knows it warp-uniform
+    const int group = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(tid / Shape::kRegion));
+    const int gtid = tid % Shape::kRegion;
     const int gwarp = gtid >> 5;
-    const int ty = (gwarp / kGatherWX) * 2 * kGatherPair + (lane & (kGatherPair - 1));  // and ty + kGatherPair
-    const int tx = (gwarp % kGatherWX) * kGatherWarpCols + (lane / kGatherPair) * Q;
-    const int lane_off = (ty + a.R) * a.pitch + tx + a.R;
-    const int pair_rows = kGatherPair * a.pitch;
-    const int4 *s_runs = reinterpret_cast<const int4 *>(s_blob + a.run_word);
-    const float4 *s_wq = reinterpret_cast<const float4 *>(s_blob + a.weight_word);
+    const int ty = (gwarp / WX) * 32 + 2 * (lane & 15), tx = (gwarp % WX) * 32 + (lane >> 4) * Q;
+    const unsigned lane_base = smem_addr(s_f + (ty >> 1) * a.pitch + tx);
+    const unsigned blocks = smem_addr(base + lay.block);
 
-    stage_gather_blob(s_blob, a.blob, a.blob_words, a.run_word, a.weight_word, a.pitch);
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) s_rv[k] = rvar_k[k];
-    if (threadIdx.x < 4) s_s[cells + threadIdx.x] = 0xff;  // never below a scale: the masking leaves it
+    for (int i = tid; i <= nk; i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
+    for (int k = tid; k < nk; k += nthreads) s_rv[k] = rvar_k[k];
+    if (tid < 2) s_flag[tid] = 0;
+    __syncthreads();
+    // kernel k's block to shared memory, asynchronously, into block buffer k & 1
+    auto stage = [&](int k) {
+        const unsigned from = s_tab[k].x, bytes = s_tab[k + 1].x - from;
+        const unsigned dst = blocks + (k & 1) * a.block_bytes;
+        const char *src = reinterpret_cast<const char *>(a.blob) + from;
+        for (unsigned o = 16 * tid; o < bytes; o += 16 * nthreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + o), "l"(src + o) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    const int per_chunk = (a.D + kGatherChunks - 1) / kGatherChunks;
+    const int chunks = kGatherChunks / a.cluster;  // of this CTA
+    const int d_begin = min(a.D, rank * chunks * per_chunk), d_end = min(a.D, (rank + 1) * chunks * per_chunk);
+    const int k_end = d_end * a.S;
+    if (d_begin < d_end) stage(d_begin * a.S);
 
     float2 acc[Q];
+    // sums of this thread's outputs, pair i at [i * kRegion]: over all chunks (one CTA per tile), else the
+    // sums of this CTA's first chunk
+    constexpr int slot = Q * Shape::kRegion;  // float2 of one group's sums
+    float2 *s_sum = reinterpret_cast<float2 *>(base + lay.sums) + group * slot + gtid;
 #pragma unroll
-    for (int i = 0; i < Q; i++) acc[i] = make_float2(0.0f, 0.0f);
-    const FmaTap tap;
+    for (int i = 0; i < Q; i++) {
+        acc[i] = make_float2(0.0f, 0.0f);
+        s_sum[i * Shape::kRegion] = acc[i];
+    }
 
-    for (int d = 0; d < a.D; d++) {
-        __syncthreads();  // the tables staged; the previous direction's correlations are done
-        // s*(d, .) and c_d = u / v_{d, s*}, u = g / den (0 outside the image), where the direction's
-        // kernels reach; the other cells keep stale values that no correlation of this direction reads.
-        // u is read again for every direction (from L2) instead of being kept in shared memory, which
-        // leaves room for 128 x 64 tiles
-        const uint8_t *plane = im.smap + static_cast<size_t>(d) * im.H * im.W;
-        const float *rv_d = s_rv + d * a.S;
-        const int4 dr = a.drect[d];
-        for (int r = dr.x + warp; r < dr.y; r += nwarps) {
-            const int gy = gy0 + r;
-            const bool row_ok = gy >= 0 && gy < im.H;
-            const size_t row = static_cast<size_t>(row_ok ? gy : 0);
-            const uint8_t *prow = plane + row * im.W;
-            const float *grow = im.g + row * im.g_pitch, *drow = im.rden + row * im.W;
+    int d = d_begin;
+#pragma unroll 1
+    for (int c = 0; c < chunks; c++) {
+        const int d_stop = min(d_end, d_begin + (c + 1) * per_chunk);
+#pragma unroll 1
+        for (; d < d_stop; d++) {
+            __syncthreads();  // the previous direction's correlations are done with the field
+            const uint8_t *map = im.smap + static_cast<size_t>(d) * im.H * im.W;
+            const float *rv_d = s_rv + d * a.S;
+            const int4 dr = a.drect[d];
+            const bool inside = gx0 + dr.z >= 0 && gx0 + dr.w <= im.W && gy0 + dr.x >= 0 && gy0 + dr.y <= im.H;
+            bool bad;
             if (im.u_ready)
-                build_field_row<true>(s_s, s_f, rv_d, prow, grow, drow, r * a.pitch, dr.z, dr.w, gx0, im.W, row_ok, lane);
+                bad = inside ? build_field<true, true>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane)
+                             : build_field<true, false>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane);
             else
-                build_field_row<false>(s_s, s_f, rv_d, prow, grow, drow, r * a.pitch, dr.z, dr.w, gx0, im.W, row_ok, lane);
-        }
-        __syncthreads();
-        // telescoped scales: zero the field where s* < s, as far as D_s reaches, then correlate
-        for (int s = 0; s < a.S; s++) {
-            const int k = d * a.S + s;
-            if (s > 0) {
-                const int4 rc = a.rect[k];
-                const unsigned below = 0x01010101u * static_cast<unsigned>(s);
-                __syncthreads();  // every correlation of the previous scale is done with the field
-                // every 4-cell word from the rectangle's first cell to its last, as one flat range over all
-                // threads (the cells beside the rectangle in those rows are masked too: zeroing a cell with
-                // s* < s anywhere keeps the field c_d [s* >= s]).  Per byte, (s* | 0x80) - s keeps its top
-                // bit exactly where s* >= s (scales are below 0x80) and borrows from no other byte; cells
-                // outside this direction's region hold stale bytes, which no correlation reads.
-                const int w0 = (rc.x * a.pitch + rc.z) >> 2, w1 = ((rc.y - 1) * a.pitch + rc.w + 3) >> 2;
-                const unsigned *sw = reinterpret_cast<const unsigned *>(s_s);
-                for (int wi = w0 + static_cast<int>(threadIdx.x); wi < w1; wi += Shape::kThreads) {
-                    const unsigned ge = ((sw[wi] | 0x80808080u) - below) & 0x80808080u;
-                    if (ge != 0x80808080u) {  // a cell of the word has s* < s: keep the others
-                        const unsigned keep = (ge >> 7) * 0xffu;  // 0xff per kept cell
-                        float4 *f4 = reinterpret_cast<float4 *>(s_f) + wi;
-                        float4 v = *f4;
-                        v.x = __uint_as_float(__float_as_uint(v.x) & __byte_perm(keep, 0u, 0x0000));
-                        v.y = __uint_as_float(__float_as_uint(v.y) & __byte_perm(keep, 0u, 0x1111));
-                        v.z = __uint_as_float(__float_as_uint(v.z) & __byte_perm(keep, 0u, 0x2222));
-                        v.w = __uint_as_float(__float_as_uint(v.w) & __byte_perm(keep, 0u, 0x3333));
-                        *f4 = v;
-                    }
-                }
+                bad = build_field<false, false>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane);
+            if (bad) s_flag[d & 1] = 1;
+#pragma unroll 1
+            for (int s = 0; s < a.S; s++) {
+                const int k = d * a.S + s;
+                if (s > 0) __syncthreads();  // every correlation of the previous scale is done with the field
+                if (k + 1 < k_end)
+                    stage(k + 1);
+                else
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                if (s > 0) mask_field(s_f, s_s, a.rect[k], static_cast<unsigned>(s), a.pitch, a.plane, tid, nthreads);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");  // this kernel's block has landed
                 __syncthreads();
+                const bool finite = s_flag[d & 1] == 0;
+                if (s == 0 && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
+                const unsigned block = blocks + (k & 1) * a.block_bytes;
+                const unsigned n_units = s_tab[k].y;
+                // units group, group + 2, ... of the kernel: {field byte offset | taps % 4, taps / 4 | weights << 8}
+                unsigned up = block + 8 * group;
+                const unsigned uend = block + 8 * n_units;
+                if (finite) {
+#pragma unroll 1
+                    for (; up < uend; up += 8 * kGatherGroups) {
+                        const uint2 u = lds_u2(up);
+                        gather_run(acc, lane_base + (u.x & ~3u), block + 8 * (u.y >> 8), u.x & 3, u.y & 255);
+                    }
+                } else {
+                    float2 tmp[Q];
+#pragma unroll
+                    for (int i = 0; i < Q; i++) tmp[i] = acc[i];
+#pragma unroll 1
+                    for (; up < uend; up += 8 * kGatherGroups) {
+                        const uint2 u = lds_u2(up);
+                        gather_run_skipping(tmp, lane_base + (u.x & ~3u), block + 8 * (u.y >> 8), 4 * (u.y & 255) + (u.x & 3));
+                    }
+#pragma unroll
+                    for (int i = 0; i < Q; i++) acc[i] = tmp[i];
+                }
             }
-            const int r_end = s_blob[k + 1];
-            for (int r = s_blob[k] + group; r < r_end; r += G) {
-                const int4 run = s_runs[r];  // (field offset, len, float4 weight index): see stage_gather_blob
-                const int o = lane_off + run.x;
-                conv_run<Q>(acc, PairWin{s_f + o, s_f + o + pair_rows}, s_wq + run.z, run.y, tap);
+        }
+        if (a.cluster == 1 || c == 0) {
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                const float2 t = s_sum[i * Shape::kRegion];
+                s_sum[i * Shape::kRegion] = make_float2(t.x + acc[i].x, t.y + acc[i].y);
+                if (c + 1 < chunks) acc[i] = make_float2(0.0f, 0.0f);
             }
         }
     }
-    // groups 1, 2, ... hand their partial sums to group 0 in turn through the field (free after the
-    // barrier); group 0 adds them in group order
-    float2 *s_h = reinterpret_cast<float2 *>(s_f);
-    for (int g = 1; g < G; g++) {
-        __syncthreads();
-        if (group == g) {
-#pragma unroll
-            for (int i = 0; i < Q; i++) s_h[i * Shape::kGroupThreads + gtid] = acc[i];
-        }
-        __syncthreads();
+    __syncthreads();  // every sum is there, and the field is free
+    if (a.cluster == 1) {
         if (group == 0) {
 #pragma unroll
             for (int i = 0; i < Q; i++) {
-                const float2 other = s_h[i * Shape::kGroupThreads + gtid];
-                acc[i] = make_float2(acc[i].x + other.x, acc[i].y + other.y);
+                const float2 t = s_sum[i * Shape::kRegion], other = s_sum[slot + i * Shape::kRegion];
+                acc[i] = make_float2(t.x + other.x, t.y + other.y);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int oy = y0 + ty + h;
+                if (oy >= im.H) break;
+                float *o = im.grad + static_cast<size_t>(oy) * im.grad_pitch + x0 + tx;
+#pragma unroll
+                for (int i = 0; i < Q; i++)
+                    if (x0 + tx + i < im.W) o[i] = h == 0 ? acc[i].x : acc[i].y;
             }
         }
+        return;
     }
-    if (group == 0) {
+    // a cluster: the second chunk's sums go over the field; every CTA adds its share of the tile's outputs
+    // over all CTAs
+    float2 *s_second = reinterpret_cast<float2 *>(smem);
+    if (chunks == 2) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int oy = y0 + ty + kGatherPair * h;
-            if (oy >= im.H) break;
-            float *o = im.grad + static_cast<size_t>(oy) * im.grad_pitch + x0 + tx;
+        for (int i = 0; i < Q; i++) s_second[group * slot + i * Shape::kRegion + gtid] = acc[i];
+    }
+    cluster_barrier();
+    const int share = slot / a.cluster;
+    const unsigned part[2] = {smem_addr(base + lay.sums), smem_addr(s_second)};
+    for (int e = rank * share + tid; e < (rank + 1) * share; e += nthreads) {
+        float2 sum[kGatherGroups];
 #pragma unroll
-            for (int i = 0; i < Q; i++)
-                if (x0 + tx + i < im.W) o[i] = h == 0 ? acc[i].x : acc[i].y;
+        for (int g = 0; g < kGatherGroups; g++) {
+            sum[g] = make_float2(0.0f, 0.0f);
+            for (int c = 0; c < kGatherChunks; c++) {
+                const float2 v = cluster_lds2(part[c % chunks] + 8 * (g * slot + e), c / chunks);
+                sum[g] = make_float2(sum[g].x + v.x, sum[g].y + v.y);
+            }
+        }
+        const int t = e % Shape::kRegion, m = e / Shape::kRegion, w = t >> 5, l = t & 31;
+        const int ox = x0 + (w % WX) * 32 + (l >> 4) * Q + m, oy = y0 + (w / WX) * 32 + 2 * (l & 15);
+        if (ox < im.W && oy < im.H) {
+            float *o = im.grad + static_cast<size_t>(oy) * im.grad_pitch + ox;
+            o[0] = sum[0].x + sum[1].x;
+            if (oy + 1 < im.H) o[im.grad_pitch] = sum[0].y + sum[1].y;
         }
     }
+    cluster_barrier();  // a CTA's shared memory stays until every other one has read it
 }
 
 // u = g * (1 / den) written over 1 / den, once per image between the two passes of the recomputing
@@ -397,92 +544,63 @@ int u_launch(const GatherImage *images, const GatherImage &single, int n, int ma
 
 namespace {
 
-// The gather kernel of tile height index I .. kGatherNWY - 1 whose WY is wy (null when none is).
-template <int I>
-const void *gather_fn(int wy) {
-    if constexpr (I < kGatherNWY) {
-        if (wy == kGatherWYs[I]) return reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<kGatherWYs[I]>);
-        return gather_fn<I + 1>(wy);
-    } else {
-        return nullptr;
-    }
+const void *gather_fn(const AdjointLayout &L) {
+    return L.wx == 4 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2>)
+                     : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1>);
 }
 
-template <int I>
-bool gather_launch_at(const GatherArgs &ga, int wy, unsigned grid, size_t smem, cudaStream_t stream) {
-    if constexpr (I < kGatherNWY) {
-        constexpr int WY = kGatherWYs[I];
-        if (wy != WY) return gather_launch_at<I + 1>(ga, wy, grid, smem, stream);
-        lpaici_adjoint_gather_kernel<WY><<<grid, GatherShape<WY>::kThreads, smem, stream>>>(ga);
-        return true;
-    } else {
-        return false;
-    }
-}
+int gather_threads(const AdjointLayout &L) { return kGatherGroups * 32 * L.wx * L.wy; }
 
-int gather_launch(const GatherArgs &ga, int wy, unsigned grid, size_t smem, cudaStream_t stream) {
-    if (!gather_launch_at<0>(ga, wy, grid, smem, stream))
-        return set_error(LPAICI_ERR_INVALID_ARG, "adjoint gather: no kernel for tile height %d", wy);
-    const cudaError_t e = cudaGetLastError();
+int gather_launch(const AdjointLayout &L, const GatherArgs &ga, long tiles, size_t smem, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles * ga.cluster));
+    cfg.blockDim = dim3(gather_threads(L));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ga.cluster);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ga.cluster > 1 ? 1 : 0;
+    void *params[] = {const_cast<GatherArgs *>(&ga)};
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, gather_fn(L), params);
     return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "adjoint gather launch");
 }
 
-// Chooses the tile height (*wy: 16 * wy output rows), fills the geometry and the per-kernel rectangles of
-// the in-place masking; smem receives the dynamic shared memory, checked against the device.
-int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga, size_t *smem, int *wy) {
-    const BlobLayout &L = ks->adj_layout;
-    const int nk = ks->D * ks->S;
-    ga->R = ks->radius;
-    ga->blob_words = L.total_words;
+// Fills the geometry and the per-kernel rectangles of the in-place masking; smem receives the dynamic shared
+// memory of one CTA per tile, checked against the device.
+int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga, size_t *smem) {
+    const AdjointLayout &L = ks->adj_layout;
+    const int nk = ks->D * ks->S, tw = 32 * L.wx, th = 32 * L.wy;
     int dev = 0, max_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    *wy = 0;
-    GatherGeom geo{};
-    constexpr int kTW = GatherShape<1>::kTW;
-    for (const int w : kGatherWYs) {
-        geo = GatherGeom::make(kTW, GatherShape<1>::kTH * w, ga->R);
-        *smem = gather_smem(L.total_words, nk, geo);
-        if (*smem <= static_cast<size_t>(max_optin)) {
-            *wy = w;
-            break;
-        }
-    }
-    if (*wy == 0)
-        return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d", *smem,
-                         max_optin);
-    ga->th = GatherShape<1>::kTH * *wy;
-    ga->pitch = geo.pitch;
-    ga->rows = geo.rows;
+    if (L.limit_bytes > static_cast<size_t>(max_optin))
+        return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d",
+                         L.limit_bytes, max_optin);
     ga->D = ks->D;
     ga->S = ks->S;
+    ga->R = ks->radius;
     ga->blob = adj_blob;
-    ga->run_word = L.run_word;
-    ga->weight_word = L.weight_word;
+    ga->block_bytes = L.block_bytes;
+    ga->pitch = L.pitch;
+    ga->plane = L.plane;
+    ga->cluster = 1;
+    const GatherSmem m = GatherSmem::make(nk, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    *smem = m.total;
+    if (*smem > static_cast<size_t>(max_optin))
+        return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d", *smem,
+                         max_optin);
+    const int rows = th + 2 * ga->R;
     for (int k = 0; k < nk; k++) {
-        // a lane reads rows ty + R + dy and ty + 8 + R + dy (ty + 8 < th) and columns
-        // tx + R + dx0 + [0, len + Q - 1) (tx + Q <= tile width): rows [R + dy_min, R + th + dy_max),
-        // columns [R + dx_min, R + tile width + dx_max)
-        int ylo = 0, yhi = -1, xlo = 0, xhi = -1;
-        for (int r = ks->adj_blob[k]; r < ks->adj_blob[k + 1]; r++) {
-            const int *run = &ks->adj_blob[L.run_word + 4 * r];
-            const int dy = run[0], c0 = run[1], c1 = run[1] + run[2] - 1;
-            if (yhi < ylo) {
-                ylo = yhi = dy;
-                xlo = c0;
-                xhi = c1;
-            } else {
-                ylo = std::min(ylo, dy);
-                yhi = std::max(yhi, dy);
-                xlo = std::min(xlo, c0);
-                xhi = std::max(xhi, c1);
-            }
-        }
-        if (yhi < ylo)
-            ga->rect[k] = make_int4(0, 0, 0, 0);  // no taps
-        else
-            ga->rect[k] = make_int4(std::max(0, ga->R + ylo), std::min(geo.rows, ga->R + ga->th + yhi),
-                                    std::max(0, ga->R + xlo), std::min(geo.pitch, ga->R + kTW + xhi));
+        // a lane reads rows ty + R + j for field rows j of its two output rows (ty + 1 < th) and columns
+        // tx + R + dx + [0, Q) (tx + Q <= tile width): rows [R + dy_min, R + th + dy_max), columns
+        // [R + dx_min, R + tile width + dx_max)
+        const int4 box = make_int4(L.box[4 * k], L.box[4 * k + 1], L.box[4 * k + 2], L.box[4 * k + 3]);
+        ga->rect[k] = box.y < box.x ? make_int4(0, 0, 0, 0)
+                                    : make_int4(std::max(0, ga->R + box.x), std::min(rows, ga->R + th + box.y),
+                                                std::max(0, ga->R + box.z), std::min(ga->pitch, ga->R + tw + box.w));
     }
     for (int d = 0; d < ks->D; d++) {
         int4 u = make_int4(0, 0, 0, 0);
@@ -497,14 +615,39 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
         }
         ga->drect[d] = u;
     }
-    cudaError_t e = cudaFuncSetAttribute(gather_fn<0>(*wy), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(*smem));
+    return LPAICI_OK;
+}
+
+// CTAs per tile: one when the tiles fill the SMs, else as many as shorten the launch.  A tile's time goes
+// with its share of the directions, plus 1.8 % of it for the cluster's exchange and staging; a cluster needs
+// its CTAs free at once in one GPC, which leaves about three clusters fewer than SMs / CTAs running together.
+// Measured (16 x 7 symmetric set, us for 1 / 4 / 8 CTAs per tile): 15 tiles 473 / 129 / 70, 32 tiles
+// 475 / 130 / 201, 40 tiles 475 / 254 / 203, 128 tiles 475 / 505 / 599, 160 tiles 947 / 629 / 732.
+int gather_cluster(const lpaici_kernelset *ks, GatherArgs *ga, long tiles, size_t smem) {
+    const AdjointLayout &L = ks->adj_layout;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    double best = static_cast<double>((tiles + sms - 1) / sms);
+    const GatherSmem m = GatherSmem::make(ks->D * ks->S, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    for (const int c : {kGatherChunks / 2, kGatherChunks}) {
+        // the second chunk's sums of half as many CTAs lie over everything before the first one's
+        if (c < kGatherChunks && m.sums < m.total - m.sums) continue;
+        if (ks->D < c || tiles * c > 0x7fffffffL) continue;
+        const long slots = std::max(1, sms / c - 3);
+        const double t = (1.0 / c + 0.018) * static_cast<double>((tiles + slots - 1) / slots);
+        if (t < best) {
+            best = t;
+            ga->cluster = c;
+        }
+    }
+    const cudaError_t e = cudaFuncSetAttribute(gather_fn(L), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "adjoint gather attributes");
 }
 
-long gather_tiles(int width, int height, int th, int *tiles_x) {
-    *tiles_x = (width + GatherShape<1>::kTW - 1) / GatherShape<1>::kTW;
-    return static_cast<long>(*tiles_x) * ((height + th - 1) / th);
+long gather_tiles(const AdjointLayout &L, int width, int height, int *tiles_x) {
+    *tiles_x = (width + 32 * L.wx - 1) / (32 * L.wx);
+    return static_cast<long>(*tiles_x) * ((height + 32 * L.wy - 1) / (32 * L.wy));
 }
 
 }  // namespace
@@ -518,7 +661,7 @@ int adjoint_passes(const lpaici_kernelset *ks, const int *blob, const int *adj_b
                    const float *d_noisy, int noisy_pitch, const float *d_grad_out, int gout_pitch, float *d_grad_in,
                    int gin_pitch, int width, int height, float sigma, float gamma, cudaStream_t stream) {
     int tiles_x = 0;
-    if (gather_tiles(width, height, 16, &tiles_x) > 0x7fffffffL)  // the shortest tile the gather may use
+    if (gather_tiles(ks->adj_layout, width, height, &tiles_x) > 0x7fffffffL)
         return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", width, height);
 
     // A. selection
@@ -555,18 +698,19 @@ int gather_pass(const lpaici_kernelset *ks, const int *adj_blob, const uint8_t *
                 float sigma, bool u_ready, cudaStream_t stream) {
     GatherArgs ga{};
     size_t smem = 0;
-    int wy = 0;
-    int rc = gather_setup(ks, adj_blob, &ga, &smem, &wy);
+    int rc = gather_setup(ks, adj_blob, &ga, &smem);
     if (rc != LPAICI_OK) return rc;
     int tiles_x = 0;
-    const long tiles = gather_tiles(width, height, ga.th, &tiles_x);
+    const long tiles = gather_tiles(ks->adj_layout, width, height, &tiles_x);
     if (tiles > 0x7fffffffL) return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", width, height);
+    rc = gather_cluster(ks, &ga, tiles, smem);
+    if (rc != LPAICI_OK) return rc;
     KernelTables tab;
     fill_tables(ks, nullptr, sigma, 1.0f, &tab);
     ga.single = GatherImage{d_grad_out, smap, rden, d_grad_in, nullptr, gout_pitch, gin_pitch, width, height, tiles_x,
                             u_ready ? 1 : 0};
     for (int k = 0; k < ks->D * ks->S; k++) ga.rvar[k] = 1.0f / tab.var[k];
-    return gather_launch(ga, wy, static_cast<unsigned>(tiles), smem, stream);
+    return gather_launch(ks->adj_layout, ga, tiles, smem, stream);
 }
 
 namespace {
@@ -682,8 +826,8 @@ struct lpaici_backward_batch {
     void *dev_mem = nullptr;         // s* planes | 1/den maps | GatherImage[n] | 1/v tables | items
     GatherArgs ga{};
     size_t smem = 0;
-    int wy = 0;
-    unsigned grid = 0;
+    AdjointLayout layout;
+    long tiles = 0;
     int n = 0, max_h = 0;  // images; the tallest one's rows (the u launch)
     bool use_graph = false;
     cudaGraph_t graph = nullptr;
@@ -697,7 +841,7 @@ int backward_batch_enqueue(lpaici_backward_batch *b, cudaStream_t stream) {
     if (rc != LPAICI_OK) return rc;
     rc = u_launch(b->ga.images, GatherImage{}, b->n, b->max_h, stream);
     if (rc != LPAICI_OK) return rc;
-    return gather_launch(b->ga, b->wy, b->grid, b->smem, stream);
+    return gather_launch(b->layout, b->ga, b->tiles, b->smem, stream);
 }
 
 void backward_batch_free(lpaici_backward_batch *b) {
@@ -733,7 +877,8 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
     if (rc != LPAICI_OK) return rc;
     auto *b = new lpaici_backward_batch();
     cudaGetDevice(&b->device);
-    rc = gather_setup(ks, adj, &b->ga, &b->smem, &b->wy);
+    b->layout = ks->adj_layout;
+    rc = gather_setup(ks, adj, &b->ga, &b->smem);
     if (rc != LPAICI_OK) {
         backward_batch_free(b);
         return rc;
@@ -751,7 +896,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
         off = align256(off + static_cast<size_t>(ks->D) * npx);
         rden_off[i] = off;
         off = align256(off + sizeof(float) * npx);
-        total_tiles += gather_tiles(images[i].width, images[i].height, b->ga.th, &tiles_x[i]);
+        total_tiles += gather_tiles(ks->adj_layout, images[i].width, images[i].height, &tiles_x[i]);
     }
     if (total_tiles > 0x7fffffffL) {
         backward_batch_free(b);
@@ -787,7 +932,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
                               im.gout_pitch, im.gin_pitch, im.width, im.height, tiles_x[i], 1};
         b->max_h = std::max(b->max_h, im.height);
         int tx = 0;
-        const long t = gather_tiles(im.width, im.height, b->ga.th, &tx);
+        const long t = gather_tiles(ks->adj_layout, im.width, im.height, &tx);
         for (long j = 0; j < t; j++) items.push_back(make_int2(i, static_cast<int>(j)));
         specs[i] = BatchSpec{im.noisy, nullptr, smap, rden, im.width, im.height, im.noisy_pitch, im.width, im.sigma,
                              im.gamma};
@@ -801,7 +946,12 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
     }
     b->ga.images = reinterpret_cast<const GatherImage *>(base + desc_off);
     b->ga.items = reinterpret_cast<const int2 *>(base + item_off);
-    b->grid = static_cast<unsigned>(total_tiles);
+    b->tiles = total_tiles;
+    rc = gather_cluster(ks, &b->ga, total_tiles, b->smem);
+    if (rc != LPAICI_OK) {
+        backward_batch_free(b);
+        return rc;
+    }
     b->n = n;
 
     int config = opts ? opts->tile_config : -1;

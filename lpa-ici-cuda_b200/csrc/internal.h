@@ -27,15 +27,27 @@ constexpr int kMaxScales = 16;
 //   [run_word, +4*n_runs)   per run {dy, dx0, L % 4, L / 4}
 //   [weight_word, ...)      weights: per run its first L % 4 taps padded to a group of 4, then the other
 //                           taps, so that every load of a group is one aligned 16-byte load
-// The adjoint's blob (adj_layout):
-//   [0, nk+1)               first run of kernel k (kernel k's runs are [begin[k], begin[k+1]))
-//   [run_word, +4*n_runs)   per run {dy, dx0, L, wofs}: its weights are wdup[wofs + j] = {w_j, w_j}
-//   [weight_word, ...)      float2 {w, w} per tap, every run padded to an even number of taps
 struct BlobLayout {
     int nk = 0, n_runs = 0;
     int run_word = 0, weight_word = 0, total_words = 0;  // total a multiple of 4
     // the forward's support limit (check_forward_limit): words of the set with every weight stored twice
     int limit_words = 0;
+};
+
+// Device image of the adjoint's kernels (mirrored and telescoped, kernelset.cpp) for the gather's tile of
+// 32*wx x 32*wy outputs and its field of two row planes (backward.cu), in bytes:
+//   [0, 8*(nk+1))  per kernel {its block's byte offset, its units}; kernel k's block ends where k + 1's begins
+//   blocks, 16-byte aligned: units {field byte offset | L % 4, L / 4 | weights << 8}, weights
+// A unit is a field row j of a kernel and the columns [a, a + L) where kernel row j (the tap of the lane's first
+// output row) or kernel row j - 1 (of its second) has taps.  The field offset is that of (row R + j, column
+// R + a); `weights` counts 8-byte pairs from the block's start to the L pairs {D(j, t), D(j - 1, t)}, -0 where
+// a row has no tap.
+struct AdjointLayout {
+    int wx = 0, wy = 0;       // warps of one group across and down a tile
+    int pitch = 0, plane = 0; // floats of a field row and of a row plane
+    int block_bytes = 0;      // the largest block
+    size_t limit_bytes = 0;   // shared memory the support limit counts (gather_setup)
+    std::vector<int> box;     // per kernel: first and last row, first and last column of its taps (empty: 0, -1)
 };
 
 // Per-launch arguments shared by the forward and backward kernels (passed by value as a
@@ -96,10 +108,9 @@ struct lpaici_kernelset {
     int radius = 0;
     lpaici::BlobLayout layout;
     std::vector<int32_t> blob;  // host copy of the device blob
-    // the adjoint gather's kernels, mirrored through their centre (taps (-dy, -dx)), in the forward
-    // blob's layout (adj_layout): scale 0 as it is, every later scale as the difference from the scale
-    // before it (kernelset.cpp, build_adjoint_blob)
-    lpaici::BlobLayout adj_layout;
+    // the adjoint gather's kernels, mirrored through their centre (taps (-dy, -dx)): scale 0 as it is, every
+    // later scale as the difference from the scale before it (kernelset.cpp, build_adjoint_blob)
+    lpaici::AdjointLayout adj_layout;
     std::vector<int32_t> adj_blob;
     // device copies, one per CUDA device, created on first use
     mutable std::mutex mu;

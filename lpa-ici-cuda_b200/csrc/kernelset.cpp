@@ -41,8 +41,8 @@ int cuda_error(cudaError_t e, const char *what) {
 //     sum_s h_s * (c [s* = s]) = sum_s D_s * (c [s* >= s]),
 // so the gather masks one field in place, scale after scale, instead of building a field per scale.
 // The difference is formed in double over the union of the two kernels' boxes (centres aligned) and
-// rounded once.  Same device layout as the forward blob (BlobLayout): run ranges, runs
-// {dy, dx0, len, wofs}, weights as {w, w} pairs with every run padded to an even length, 16 spare taps.
+// rounded once.  A lane of the gather owns two neighbouring output rows, so every field row of a kernel
+// becomes a unit of weight pairs {D(j, t), D(j - 1, t)} over the columns of either row (AdjointLayout).
 // ---------------------------------------------------------------------------------------------
 static int build_adjoint_blob(lpaici_kernelset *ks) {
     const int D = ks->D, S = ks->S, nk = D * S;
@@ -83,34 +83,91 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
             }
         }
     begin[nk] = static_cast<int>(rdy.size());
-    const int n_runs = begin[nk];
-    BlobLayout L;
-    L.nk = nk;
-    L.n_runs = n_runs;
-    L.run_word = (nk + 1 + 3) & ~3;
-    L.weight_word = L.run_word + 4 * n_runs;
-    std::vector<int> wofs(n_runs);
-    int n2 = 0;
-    for (int r = 0; r < n_runs; r++) {
-        wofs[r] = n2;
-        n2 += (rlen[r] + 1) & ~1;
-    }
-    L.total_words = (L.weight_word + 2 * (n2 + 16) + 3) & ~3;
-    ks->adj_layout = L;
-    ks->adj_blob.assign(L.total_words, 0);
-    for (int k = 0; k <= nk; k++) ks->adj_blob[k] = begin[k];
-    float *wd = reinterpret_cast<float *>(ks->adj_blob.data() + L.weight_word);
-    int wi = 0;
-    for (int r = 0; r < n_runs; r++) {
-        ks->adj_blob[L.run_word + 4 * r + 0] = rdy[r];
-        ks->adj_blob[L.run_word + 4 * r + 1] = rdx[r];
-        ks->adj_blob[L.run_word + 4 * r + 2] = rlen[r];
-        ks->adj_blob[L.run_word + 4 * r + 3] = wofs[r];
-        for (int j = 0; j < rlen[r]; j++, wi++) {
-            wd[2 * (wofs[r] + j)] = w[wi];
-            wd[2 * (wofs[r] + j) + 1] = w[wi];
+    const int n_runs = begin[nk], R = ks->radius;
+
+    // the support limit, kept where it has always been: a 128 x 16 tile's field and selected scales beside the
+    // runs and the weights stored twice (also the least size of the blob, which lpaici_kernelset_info reports
+    // and the no-allocation adjoint's scratch counts)
+    int n2 = 16;
+    for (int r = 0; r < n_runs; r++) n2 += (rlen[r] + 1) & ~1;
+    const int limit_words = (((nk + 1 + 3) & ~3) + 4 * n_runs + 2 * n2 + 3) & ~3;
+    const size_t limit_cells = (static_cast<size_t>(16 + 2 * R) * (((128 + 2 * R + 14) & ~7) + 1) + 3) & ~size_t(3);
+    AdjointLayout &L = ks->adj_layout;
+    L.limit_bytes = 4 * (static_cast<size_t>(limit_words) + ((nk + 3) & ~3)) + 4 * limit_cells + ((limit_cells + 4 + 15) & ~size_t(15));
+
+    // units and weights of every kernel; the offsets of a unit's field rows need the tile's geometry, and the
+    // tile needs the largest block: 128 x 64 outputs if that fits on an SM, else 64 x 32
+    struct Unit {
+        int row, col, len;
+    };
+    std::vector<std::vector<Unit>> units(nk);
+    std::vector<std::vector<float>> pairs(nk);
+    L.box.assign(4 * static_cast<size_t>(nk), 0);
+    L.block_bytes = 0;
+    for (int k = 0, w0 = 0; k < nk; k++) {
+        int *box = &L.box[4 * static_cast<size_t>(k)];
+        box[1] = -1;
+        std::vector<int> first_w(static_cast<size_t>(begin[k + 1] - begin[k]));
+        for (int r = begin[k]; r < begin[k + 1]; r++) {
+            first_w[r - begin[k]] = w0;
+            w0 += rlen[r];
+            const bool none = box[1] < box[0];
+            box[0] = none ? rdy[r] : std::min(box[0], rdy[r]);
+            box[1] = none ? rdy[r] : std::max(box[1], rdy[r]);
+            box[2] = none ? rdx[r] : std::min(box[2], rdx[r]);
+            box[3] = none ? rdx[r] + rlen[r] - 1 : std::max(box[3], rdx[r] + rlen[r] - 1);
         }
+        // rows ascend; `r` is the first run whose row is not above j - 1
+        int r = begin[k];
+        for (int j = box[0]; box[1] >= box[0] && j <= box[1] + 1; j++) {
+            while (r < begin[k + 1] && rdy[r] < j - 1) r++;
+            int row_of[2] = {-1, -1};  // the runs of rows j and j - 1
+            for (int q = r; q < begin[k + 1] && rdy[q] <= j; q++) row_of[rdy[q] == j ? 0 : 1] = q;
+            if (row_of[0] < 0 && row_of[1] < 0) continue;
+            int c0 = 1 << 30, c1 = -(1 << 30);
+            for (const int q : row_of)
+                if (q >= 0) {
+                    c0 = std::min(c0, rdx[q]);
+                    c1 = std::max(c1, rdx[q] + rlen[q]);
+                }
+            units[k].push_back({j, c0, c1 - c0});
+            for (int c = c0; c < c1; c++)
+                for (const int q : row_of) {
+                    const bool tap = q >= 0 && c >= rdx[q] && c < rdx[q] + rlen[q];
+                    const float v = tap ? w[first_w[q - begin[k]] + c - rdx[q]] : 0.0f;
+                    pairs[k].push_back(tap ? (v == 0.0f ? 0.0f : v) : -0.0f);  // -0 marks padding only
+                }
+        }
+        const int bytes = static_cast<int>(8 * units[k].size() + 4 * pairs[k].size());
+        L.block_bytes = std::max(L.block_bytes, (bytes + 15) & ~15);
     }
+    constexpr size_t kSharedPerCta = 232448;  // sm_100a
+    for (const int wide : {1, 0}) {
+        L.wx = wide ? 4 : 2;
+        L.wy = wide ? 2 : 1;
+        L.pitch = (32 * L.wx + 2 * R) | 1;
+        L.plane = ((32 * L.wy + 2 * R + 1) / 2 * L.pitch + 3) & ~3;
+        const size_t sums = 8 * 16 * 2 * static_cast<size_t>(32 * L.wx * L.wy);
+        if (10 * static_cast<size_t>(L.plane) + 2 * L.block_bytes + 12 * (nk + 1) + 64 + sums <= kSharedPerCta) break;
+    }
+    std::vector<int32_t> &blob = ks->adj_blob;
+    blob.assign((2 * (static_cast<size_t>(nk) + 1) + 3) & ~size_t(3), 0);
+    for (int k = 0; k < nk; k++) {
+        blob[2 * k] = static_cast<int>(4 * blob.size());
+        blob[2 * k + 1] = static_cast<int>(units[k].size());
+        int at = static_cast<int>(units[k].size());  // in 8-byte pairs from the block's start
+        for (const Unit &u : units[k]) {
+            const int row = R + u.row;
+            blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col) | (u.len % 4));
+            blob.push_back(u.len / 4 | at << 8);
+            at += u.len;
+        }
+        const size_t n = blob.size();
+        blob.resize((n + pairs[k].size() + 3) & ~size_t(3), 0);
+        std::memcpy(blob.data() + n, pairs[k].data(), 4 * pairs[k].size());
+    }
+    blob[2 * nk] = static_cast<int>(4 * blob.size());
+    blob.resize(std::max<size_t>(blob.size(), limit_words), 0);
     return LPAICI_OK;
 }
 
@@ -131,7 +188,9 @@ static int finish_kernelset(lpaici_kernelset *ks) {
         const float *h = ks->dense_w.data() + ks->off[k];
         const int R = ks->rows[k], Cc = ks->cols[k];
         float nsq = 0.0f;
-        for (int i = 0; i < R * Cc; i++) nsq += h[i] * h[i];  // compute_kernel_variances order
+        // compute_kernel_variances order; a zero tap would add +0 to a sum that is never -0
+        for (int i = 0; i < R * Cc; i++)
+            if (h[i] != 0.0f) nsq += h[i] * h[i];
         ks->norm2[k] = nsq;
         ks->k_first_run.push_back(static_cast<int>(ks->run_row.size()));
         ks->k_first_weight.push_back(static_cast<int>(ks->run_w.size()));
@@ -173,7 +232,8 @@ static int finish_kernelset(lpaici_kernelset *ks) {
     }
     L.limit_words = (((nk + 1 + 3) & ~3) + 4 * L.n_runs + 2 * n_dup + 3) & ~3;
     L.total_words = L.weight_word + n_w;
-    ks->blob.assign(L.total_words, 0);
+    // (at least limit_words: the size that lpaici_kernelset_info reports and scratch limits count)
+    ks->blob.assign(std::max(L.total_words, L.limit_words), 0);
     float *wd = reinterpret_cast<float *>(ks->blob.data() + L.weight_word);
     int at = 0;
     for (int k = 0; k < nk; k++) {
