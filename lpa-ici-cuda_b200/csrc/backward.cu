@@ -679,7 +679,7 @@ int adjoint_passes(const lpaici_kernelset *ks, const int *blob, const int *adj_b
     KernelTables tab;
     fill_tables(ks, nullptr, sigma, gamma, &tab);
     tab.blob = blob;
-    int rc = launch_forward(ks, img, tab, config_for(ks, width, height), stream);
+    int rc = launch_forward(img, tab, plan_for(ks, width, height), stream);
     if (rc != LPAICI_OK) return rc;
     // u = g / den over the workspace's 1/den
     rc = u_launch(nullptr, GatherImage{d_grad_out, smap, rden, d_grad_in, nullptr, gout_pitch, gin_pitch, width, height, 0, 0},
@@ -954,15 +954,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
     }
     b->n = n;
 
-    int config = opts ? opts->tile_config : -1;
-    if (config < 0) {
-        std::vector<int> w(n), h(n);
-        for (int i = 0; i < n; i++) {
-            w[i] = specs[i].width;
-            h[i] = specs[i].height;
-        }
-        config = config_for_images(ks, w.data(), h.data(), n);
-    }
+    const int config = opts ? opts->tile_config : -1;
     rc = batch_plan_create(ks, specs.data(), n, config, false, stream, &b->select);
     if (rc != LPAICI_OK) {
         backward_batch_free(b);
@@ -1073,7 +1065,7 @@ extern "C" int lpaici_forward_state(const lpaici_kernelset *ks, const float *d_n
     KernelTables tab;
     fill_tables(ks, nullptr, sigma, gamma, &tab);
     tab.blob = blob;
-    return launch_forward(ks, img, tab, config_for(ks, width, height), reinterpret_cast<cudaStream_t>(stream_));
+    return launch_forward(img, tab, plan_for(ks, width, height), reinterpret_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int lpaici_backward_state(const lpaici_kernelset *ks, const void *d_state, const float *d_grad_out,

@@ -36,7 +36,7 @@ struct BatchImage {
 struct BatchArgs {
     const BatchImage *images;
     const float *tables;    // per image var[nk], thr[nk]
-    const int2 *items;      // (image, tile index within the image)
+    const int4 *items;      // (image, x0, y0, 1 for a small tile of a mix)
     int n_items;
     int D, S, R;
     const int *blob;
@@ -49,25 +49,29 @@ struct BatchArgs {
     float thr[kMaxKernels];
 };
 
+// One tile: stages the kernel set, the image's tables and the tile, and sweeps it.
 template <int WX, int WY, int Q, int DS>
-__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
-    lpaici_batched_kernel(const __grid_constant__ BatchArgs a) {
-    using Shape = TileShape<WX, WY, Q, DS>;
-    extern __shared__ __align__(16) int smem[];
+__device__ __forceinline__ void batched_tile(int *smem, const BatchArgs &a, const ImageArgs &img, int image, int x0, int y0) {
     const int nk = a.D * a.S;
     const SweepCta<WX, WY, Q, DS> cta(smem, a.blob_words, nk, a.R);
+    load_tile(cta.tile, img, x0, y0, cta.g);
+    stage_blob<Q>(cta.blob, a.blob, a.blob_words, a.run_word, a.weight_word, cta.g.pitch2);
+    if (a.shared_tables) {
+        stage_tables(cta.tab, a.var, a.thr, nk);
+    } else {
+        const float *t = a.tables + a.images[image].tab_offset;
+        stage_tables(cta.tab, t, t + nk, nk);
+    }
+    tile_wait();
+    __syncthreads();
+    sweep_tile<WX, WY, Q, DS, false>(img, x0, y0, a.D, a.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch, a.neg_zero);
+}
 
-    // the CTA's image arguments live in shared memory: in registers they would stay live across the
-    // whole sweep, beside the run loop's (the single-image kernel reads them from its parameters)
-    __shared__ __align__(16) unsigned char s_img_raw[sizeof(ImageArgs)];
-    __shared__ int2 s_xy;
-    ImageArgs &s_img = *reinterpret_cast<ImageArgs *>(s_img_raw);
-    const int item = blockIdx.x;  // one CTA per queue item, dispatched in queue order
-    if (item >= a.n_items) return;
+// The CTA's image arguments live in shared memory: in registers they would stay live across the whole sweep,
+// beside the run loop's (the single-image kernel reads them from its parameters).
+__device__ __forceinline__ void batched_image(const BatchArgs &a, int image, ImageArgs *out) {
     if (threadIdx.x == 0) {
-        const int2 it = a.items[item];
-        const BatchImage bi = a.images[it.x];
-        const int tiles_x = (bi.W + Shape::kTileW - 1) / Shape::kTileW;
+        const BatchImage bi = a.images[image];
         ImageArgs img{};
         img.in = bi.in;
         img.out = bi.out;
@@ -79,22 +83,36 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
         img.out_pitch = bi.out_pitch;
         img.row_begin = 0;
         img.rows_out = bi.H;
-        s_img = img;
-        s_xy = make_int2((it.y % tiles_x) * Shape::kTileW, (it.y / tiles_x) * Shape::kTileH);
+        *out = img;
     }
     __syncthreads();
-    const int x0 = s_xy.x, y0 = s_xy.y;
-    load_tile(cta.tile, s_img, x0, y0, cta.g);
-    stage_blob<Q>(cta.blob, a.blob, a.blob_words, a.run_word, a.weight_word, cta.g.pitch2);
-    if (a.shared_tables) {
-        stage_tables(cta.tab, a.var, a.thr, nk);
-    } else {
-        const float *t = a.tables + a.images[a.items[item].x].tab_offset;
-        stage_tables(cta.tab, t, t + nk, nk);
-    }
-    tile_wait();
-    __syncthreads();
-    sweep_tile<WX, WY, Q, DS, false>(s_img, x0, y0, a.D, a.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch, a.neg_zero);
+}
+
+// One CTA per queue item, dispatched in queue order.
+template <int WX, int WY, int Q, int DS>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
+    lpaici_batched_kernel(const __grid_constant__ BatchArgs a) {
+    extern __shared__ __align__(16) int smem[];
+    __shared__ __align__(16) unsigned char s_img[sizeof(ImageArgs)];
+    ImageArgs &img = *reinterpret_cast<ImageArgs *>(s_img);
+    const int4 item = __ldg(a.items + blockIdx.x);
+    batched_image(a, item.x, &img);
+    batched_tile<WX, WY, Q, DS>(smem, a, img, item.x, item.y, item.z);
+}
+
+// The same with two kinds of tiles (see lpaici_forward_mixed_kernel): the queue's big tiles come first.
+template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD>
+__global__ void __launch_bounds__(32 * AX * AY * AD, 1)
+    lpaici_batched_mixed_kernel(const __grid_constant__ BatchArgs a) {
+    extern __shared__ __align__(16) int smem[];
+    __shared__ __align__(16) unsigned char s_img[sizeof(ImageArgs)];
+    ImageArgs &img = *reinterpret_cast<ImageArgs *>(s_img);
+    const int4 item = __ldg(a.items + blockIdx.x);
+    batched_image(a, item.x, &img);
+    if (item.w == 0)
+        batched_tile<AX, AY, AQ, AD>(smem, a, img, item.x, item.y, item.z);
+    else
+        batched_tile<BX, BY, BQ, BD>(smem, a, img, item.x, item.y, item.z);
 }
 
 namespace {
@@ -103,6 +121,7 @@ struct KernelInfo {
     const void *fn;
     int tile_w, tile_h, threads;
     size_t smem;
+    int small_w = 0, small_h = 0;  // of a mix's small tiles
 };
 
 template <int WX, int WY, int Q, int DS>
@@ -124,6 +143,32 @@ int get_info(int config, const KernelTables &tab, KernelInfo *info) {
         default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);
     }
 #undef LPAICI_BATCH_CASE
+}
+
+template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD>
+void mixed_info(const KernelTables &tab, KernelInfo *info) {
+    using Big = TileShape<AX, AY, AQ, AD>;
+    using Small = TileShape<BX, BY, BQ, BD>;
+    info->fn = reinterpret_cast<const void *>(lpaici_batched_mixed_kernel<AX, AY, AQ, AD, BX, BY, BQ, BD>);
+    info->tile_w = Big::kTileW;
+    info->tile_h = Big::kTileH;
+    info->threads = Big::kThreads;
+    info->smem = std::max(sweep_smem<Big, AQ>(tab.blob_words, tab.D * tab.S, tab.R),
+                          sweep_smem<Small, BQ>(tab.blob_words, tab.D * tab.S, tab.R));
+    info->small_w = Small::kTileW;
+    info->small_h = Small::kTileH;
+}
+
+int get_mix_info(int mix, const KernelTables &tab, KernelInfo *info) {
+#define LPAICI_MIX_CASE(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD)           \
+    case idx:                                                                \
+        mixed_info<AX, AY, AQ, AD, BX, BY, BQ, BD>(tab, info);               \
+        return LPAICI_OK;
+    switch (mix) {
+        LPAICI_TILE_MIXES(LPAICI_MIX_CASE)
+        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile mix %d out of range", mix);
+    }
+#undef LPAICI_MIX_CASE
 }
 
 }  // namespace
@@ -151,14 +196,14 @@ struct lpaici_batch {
     MultiImages mi{};
     ImageArgs img{};
     KernelTables tab{};
-    int config = 0;
+    TilePlan plan;
 };
 
 namespace lpaici {
 
 int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream) {
-    if (b->single) return launch_forward(nullptr, b->img, b->tab, b->config, stream);
-    if (b->multi) return launch_forward_multi(b->img, b->tab, b->mi, b->n_multi, b->config, stream);
+    if (b->single) return launch_forward(b->img, b->tab, b->plan, stream);
+    if (b->multi) return launch_forward_multi(b->img, b->tab, b->mi, b->n_multi, b->plan, stream);
     void *params[] = {&b->args};
     const cudaError_t e = cudaLaunchKernel(b->info.fn, dim3(b->grid), dim3(b->info.threads), params, b->info.smem, stream);
     if (e != cudaSuccess) return cuda_error(e, "batched launch");
@@ -191,8 +236,29 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     KernelTables tab;
     fill_tables(ks, nullptr, 1.0f, 1.0f, &tab);
     tab.blob = blob;
+    bool one_size = n >= 2 && n <= kMaxMultiImages;
+    for (int i = 1; one_size && i < n; i++) {
+        const BatchSpec &a0 = specs[0], &ai = specs[i];
+        one_size = ai.width == a0.width && ai.height == a0.height && ai.noisy_pitch == a0.noisy_pitch &&
+                   ai.out_pitch == a0.out_pitch && ai.sigma == a0.sigma && ai.gamma == a0.gamma &&
+                   (ai.out == nullptr) == (a0.out == nullptr) && (ai.smap == nullptr) == (a0.smap == nullptr) &&
+                   (ai.rden == nullptr) == (a0.rden == nullptr);
+    }
+    if (config >= 0) {
+        b->plan.config = config;
+    } else if (n == 1 || one_size) {
+        b->plan = plan_for(ks, specs[0].width, specs[0].height, n);
+    } else {
+        std::vector<int> w(n), h(n);
+        for (int i = 0; i < n; i++) {
+            w[i] = specs[i].width;
+            h[i] = specs[i].height;
+        }
+        b->plan = plan_for_images(ks, w.data(), h.data(), n);
+    }
+    const bool mixed = b->plan.mix >= 0;
     rc = check_forward_limit(tab);
-    if (rc == LPAICI_OK) rc = get_info(config, tab, &b->info);
+    if (rc == LPAICI_OK) rc = mixed ? get_mix_info(b->plan.mix, tab, &b->info) : get_info(b->plan.config, tab, &b->info);
     if (rc != LPAICI_OK) {
         batch_plan_free(b);
         return rc;
@@ -202,10 +268,16 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     std::vector<BatchImage> imgs(n);
     std::vector<float> tables(static_cast<size_t>(n) * 2 * nk);
     struct Item {
-        int image, tile;
+        int image, x, y;
         long key;
     };
-    std::vector<Item> items;
+    std::vector<Item> items, small;
+    auto push = [&](std::vector<Item> &to, int i, int x, int y, int tw, int th) {
+        const int w = std::min(tw, specs[i].width - x), h = std::min(th, specs[i].height - y);
+        // full tiles first, then by image size (largest first), then raster order
+        const long area = static_cast<long>(specs[i].width) * specs[i].height;
+        if (w > 0 && h > 0) to.push_back({i, x, y, static_cast<long>(w) * h * (1L << 40) + area});
+    };
     for (int i = 0; i < n; i++) {
         const BatchSpec &im = specs[i];
         KernelTables t;
@@ -214,26 +286,30 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk + nk], t.thr, sizeof(float) * nk);
         imgs[i] = BatchImage{im.noisy, im.out, im.smap, im.rden, im.width, im.height, im.noisy_pitch, im.out_pitch,
                              i * 2 * nk, 0};
-        const int tx = (im.width + b->info.tile_w - 1) / b->info.tile_w;
-        const int ty = (im.height + b->info.tile_h - 1) / b->info.tile_h;
-        const long area = static_cast<long>(im.width) * im.height;
-        for (int y = 0; y < ty; y++)
-            for (int x = 0; x < tx; x++) {
-                const int w = std::min(b->info.tile_w, im.width - x * b->info.tile_w);
-                const int h = std::min(b->info.tile_h, im.height - y * b->info.tile_h);
-                // full tiles first, then by image size (largest first), then raster order
-                items.push_back({i, y * tx + x, static_cast<long>(w) * h * (1L << 40) + area});
-            }
+        for (int y = 0; y < im.height; y += b->info.tile_h)
+            for (int x = 0; x < im.width; x += b->info.tile_w) push(items, i, x, y, b->info.tile_w, b->info.tile_h);
     }
-    std::stable_sort(items.begin(), items.end(), [](const Item &p, const Item &q) { return p.key > q.key; });
-    std::vector<int2> qitems(items.size());
-    for (size_t j = 0; j < items.size(); j++) qitems[j] = make_int2(items[j].image, items[j].tile);
+    const auto by_key = [](const Item &p, const Item &q) { return p.key > q.key; };
+    std::stable_sort(items.begin(), items.end(), by_key);
+    if (mixed && !(n == 1 || one_size)) {  // all tiles past the plan's big ones are cut small
+        const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_rows));
+        for (size_t j = big; j < items.size(); j++)
+            for (int y = 0; y < b->info.tile_h; y += b->info.small_h)
+                for (int x = 0; x < b->info.tile_w; x += b->info.small_w)
+                    push(small, items[j].image, items[j].x + x, items[j].y + y, b->info.small_w, b->info.small_h);
+        items.resize(big);
+        std::stable_sort(small.begin(), small.end(), by_key);
+    }
+    std::vector<int4> qitems;
+    qitems.reserve(items.size() + small.size());
+    for (const Item &it : items) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
+    for (const Item &it : small) qitems.push_back(make_int4(it.image, it.x, it.y, 1));
 
     const size_t img_bytes = sizeof(BatchImage) * n;
     const size_t tab_off = (img_bytes + 255) & ~size_t(255);
     const size_t tab_bytes = sizeof(float) * tables.size();
     const size_t item_off = (tab_off + tab_bytes + 255) & ~size_t(255);
-    const size_t item_bytes = sizeof(int2) * qitems.size();
+    const size_t item_bytes = sizeof(int4) * qitems.size();
     const size_t total = item_off + item_bytes;
     cudaError_t e = cudaMalloc(&b->dev_mem, total);
     if (e != cudaSuccess) {
@@ -250,7 +326,7 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     }
     b->args.images = reinterpret_cast<const BatchImage *>(base);
     b->args.tables = reinterpret_cast<const float *>(base + tab_off);
-    b->args.items = reinterpret_cast<const int2 *>(base + item_off);
+    b->args.items = reinterpret_cast<const int4 *>(base + item_off);
     b->args.n_items = static_cast<int>(qitems.size());
     b->args.D = ks->D;
     b->args.S = ks->S;
@@ -284,14 +360,6 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
                                 : set_error(LPAICI_ERR_UNSUPPORTED, "batched kernel does not fit on an SM");
     }
     b->grid = b->args.n_items;  // one CTA per queue item
-    bool one_size = n >= 2 && n <= kMaxMultiImages;
-    for (int i = 1; one_size && i < n; i++) {
-        const BatchSpec &a0 = specs[0], &ai = specs[i];
-        one_size = ai.width == a0.width && ai.height == a0.height && ai.noisy_pitch == a0.noisy_pitch &&
-                   ai.out_pitch == a0.out_pitch && ai.sigma == a0.sigma && ai.gamma == a0.gamma &&
-                   (ai.out == nullptr) == (a0.out == nullptr) && (ai.smap == nullptr) == (a0.smap == nullptr) &&
-                   (ai.rden == nullptr) == (a0.rden == nullptr);
-    }
     if (n == 1 || one_size) {
         const BatchSpec &im = specs[0];
         b->single = n == 1;
@@ -303,7 +371,6 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
             b->mi.smap[i] = specs[i].smap;
             b->mi.rden[i] = specs[i].rden;
         }
-        b->config = config;
         b->img.in = im.noisy;
         b->img.out = im.out;
         b->img.smap = im.smap;
@@ -368,15 +435,7 @@ int lpaici_batch_create(const lpaici_kernelset *ks, const lpaici_image *images, 
         specs[i] = BatchSpec{im.noisy, im.denoised, im.scale_map, nullptr, im.width, im.height, im.noisy_pitch,
                              im.out_pitch, im.sigma, im.gamma};
     }
-    int config = opts ? opts->tile_config : -1;
-    if (config < 0) {
-        std::vector<int> w(n), h(n);
-        for (int i = 0; i < n; i++) {
-            w[i] = specs[i].width;
-            h[i] = specs[i].height;
-        }
-        config = config_for_images(ks, w.data(), h.data(), n);
-    }
+    const int config = opts ? opts->tile_config : -1;
     return batch_plan_create(ks, specs.data(), n, config, opts && opts->use_graph,
                              reinterpret_cast<cudaStream_t>(stream_), out);
 }

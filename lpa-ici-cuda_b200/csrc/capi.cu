@@ -81,41 +81,135 @@ static long tiles_of(int c, int width, int rows) {
     return static_cast<long>((width + tw - 1) / tw) * ((rows + th - 1) / th);
 }
 
-int config_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n) {
-    int dev = 0, sms = 0, max_optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return default_config(ks);
+// Time until the last of n_small tiles of t is done, handed out as SMs get free after n_big tiles of big_t.
+static double mixed_makespan(long n_big, double big_t, long n_small, double t, int sms) {
+    const long waves = n_big / sms, rem = n_big % sms;
+    const double early = waves * big_t, late = early + (rem > 0 ? big_t : 0.0);
+    // the first j for which sms - rem SMs from `early` and rem SMs from `late` take n_small tiles by early + j t
+    const long gap = rem > 0 ? static_cast<long>(std::ceil(big_t / t)) : 0;
+    const long before = std::min(n_small, gap * (sms - rem));  // done before the late SMs join
+    if (before == n_small) return std::max(late, early + t * ((n_small + sms - rem - 1) / (sms - rem)));
+    return early + t * (gap + (n_small - before + sms - 1) / sms);
+}
+
+// What a plan is chosen with: the tile times of a kernel set on the current device.
+struct PlanCosts {
+    int sms = 0;
+    bool forced = false;
+    int forced_config = 0;
+    float tile_ms[LPAICI_NUM_TILE_CONFIGS];  // <= 0: does not fit
+    int bps[LPAICI_NUM_TILE_CONFIGS];
+};
+
+static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
+    int dev = 0, max_optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
     std::vector<float> tuned;
     {
         std::lock_guard<std::mutex> lock(ks->mu);
         const bool have = dev < static_cast<int>(ks->tuned_config.size()) && ks->tuned_config[dev] >= 0;
         const bool timed = dev < static_cast<int>(ks->tuned_tile_ms.size()) && !ks->tuned_tile_ms[dev].empty();
-        if (have && !timed) return ks->tuned_config[dev];  // forced by lpaici_set_tile_config
+        if (have && !timed) {  // forced by lpaici_set_tile_config
+            pc->forced = true;
+            pc->forced_config = ks->tuned_config[dev];
+            return true;
+        }
         if (timed) tuned = ks->tuned_tile_ms[dev];
     }
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&pc->sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    int best = -1;
-    double best_ms = 0.0;
     for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        const int bps = cached_bps(ks, dev, c, max_optin);
-        const float tile_ms = tuned.empty() ? estimated_tile_ms(ks, c) : tuned[c];
-        if (bps <= 0 || !(tile_ms > 0.0f)) continue;
+        pc->bps[c] = cached_bps(ks, dev, c, max_optin);
+        pc->tile_ms[c] = pc->bps[c] <= 0 ? 0.0f : tuned.empty() ? estimated_tile_ms(ks, c) : tuned[c];
+    }
+    return true;
+}
+
+static constexpr int kMixFirst[] = {
+#define LPAICI_MIX_FIRST(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD) A,
+    LPAICI_TILE_MIXES(LPAICI_MIX_FIRST)
+#undef LPAICI_MIX_FIRST
+};
+static constexpr int kMixSecond[] = {
+#define LPAICI_MIX_SECOND(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD) B,
+    LPAICI_TILE_MIXES(LPAICI_MIX_SECOND)
+#undef LPAICI_MIX_SECOND
+};
+
+// by_rows: the images are one size and a mix's big tiles are whole tile rows of every image.
+static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const int *rows, int n, bool by_rows) {
+    TilePlan plan;
+    PlanCosts pc;
+    if (!plan_costs(ks, &pc)) {
+        plan.config = default_config(ks);
+        return plan;
+    }
+    if (pc.forced) {
+        plan.config = pc.forced_config;
+        return plan;
+    }
+    double best_ms = -1.0;
+    for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
+        const float tile_ms = pc.tile_ms[c];
+        const int bps = pc.bps[c];
+        if (!(tile_ms > 0.0f)) continue;
         long tiles = 0;
         for (int i = 0; i < n; i++) tiles += tiles_of(c, widths[i], rows[i]);
-        const long slots = static_cast<long>(sms) * bps;
+        const long slots = static_cast<long>(pc.sms) * bps;
         // a lone CTA of a configuration that two fit on an SM takes 1.5 tile times, not 2 (97 x 64 as 28
         // tiles of 16 x 16: 36.9 us against 24 us for one more tile per SM at full occupancy)
-        const double waves = tiles <= sms ? 0.5 * (1 + bps) / bps : static_cast<double>((tiles + slots - 1) / slots);
+        const double waves = tiles <= pc.sms ? 0.5 * (1 + bps) / bps : static_cast<double>((tiles + slots - 1) / slots);
         const double est = tile_ms * bps * waves;
-        if (best < 0 || est < best_ms) {
-            best = c;
+        if (best_ms < 0.0 || est < best_ms) {
+            plan.config = c;
             best_ms = est;
         }
     }
-    return best >= 0 ? best : default_config(ks);
+    if (best_ms < 0.0) {
+        plan.config = default_config(ks);
+        return plan;
+    }
+    // a mix: whole waves of big tiles, or one wave fewer, the rest in small ones
+    for (int m = 0; m < LPAICI_NUM_TILE_MIXES; m++) {
+        const int a = kMixFirst[m], b = kMixSecond[m];
+        if (!(pc.tile_ms[a] > 0.0f) || !(pc.tile_ms[b] > 0.0f)) continue;
+        int aw = 1, ah = 1, bw = 1, bh = 1;
+        config_tile(a, &aw, &ah);
+        config_tile(b, &bw, &bh);
+        long whole = 0, all = 0;  // whole big tiles; small tiles if everything were cut small
+        for (int i = 0; i < n; i++) {
+            whole += static_cast<long>(widths[i] / aw) * (rows[i] / ah);
+            all += static_cast<long>((widths[i] + bw - 1) / bw) * ((rows[i] + bh - 1) / bh);
+        }
+        const long per = static_cast<long>(aw / bw) * (ah / bh);
+        auto consider = [&](long big, int big_rows) {
+            const long small = all - big * per;
+            if (big <= 0 || small <= 0) return;
+            const double est = mixed_makespan(big, pc.tile_ms[a], small, pc.tile_ms[b], pc.sms);
+            if (est < best_ms) {
+                best_ms = est;
+                plan = TilePlan{a, m, big_rows};
+            }
+        };
+        const long row = by_rows ? static_cast<long>(widths[0] / aw) * n : 1;  // big tiles of one tile row
+        if (row <= 0 || whole <= 0) continue;
+        const long full = whole / row, w0 = whole / pc.sms;
+        for (long r : {full, std::min(full, w0 * pc.sms / row), std::min(full, (w0 - 1) * pc.sms / row)})
+            consider(r * row, static_cast<int>(r));
+    }
+    return plan;
 }
 
-int config_for(const lpaici_kernelset *ks, int width, int rows) { return config_for_images(ks, &width, &rows, 1); }
+static int mix_second(int mix) { return kMixSecond[mix]; }
+
+TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n) {
+    const std::vector<int> w(n, width), h(n, rows);
+    return choose_plan(ks, w.data(), h.data(), n, true);
+}
+
+TilePlan plan_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n) {
+    return choose_plan(ks, widths, rows, n, false);
+}
 
 static int check_params(float sigma_or_one, float gamma) {
     if (!(sigma_or_one > 0.0f) || !std::isfinite(sigma_or_one))
@@ -125,11 +219,10 @@ static int check_params(float sigma_or_one, float gamma) {
     return LPAICI_OK;
 }
 
-// Shared body of the forward entry points.
-static int forward_common(const lpaici_kernelset *ks, const float *d_in, int in_pitch, int width, int in_height,
-                          int row_begin, int row_count, float *d_out, int out_pitch, const float *host_var,
-                          float sigma, float gamma, uint8_t *d_smap, cudaStream_t stream, int step = 1,
-                          int config = -1, bool fused = false) {
+// Checks a forward call and fills its launch arguments.
+static int forward_args(const lpaici_kernelset *ks, const float *d_in, int in_pitch, int width, int in_height,
+                        int row_begin, int row_count, float *d_out, int out_pitch, const float *host_var, float sigma,
+                        float gamma, uint8_t *d_smap, int step, ImageArgs *args, KernelTables *tables) {
     if (!ks || !d_in || !d_out) return set_error(LPAICI_ERR_INVALID_ARG, "forward: null kernel set or image pointer");
     if (width <= 0 || in_height <= 0 || row_count <= 0)
         return set_error(LPAICI_ERR_INVALID_ARG, "forward: non-positive size %d x %d", width, row_count);
@@ -148,7 +241,8 @@ static int forward_common(const lpaici_kernelset *ks, const float *d_in, int in_
     const int *blob = nullptr;
     rc = device_blob(ks, &blob);
     if (rc != LPAICI_OK) return rc;
-    ImageArgs img{};
+    ImageArgs &img = *args;
+    img = ImageArgs{};
     img.in = d_in;
     img.out = d_out;
     img.smap = d_smap;
@@ -159,26 +253,43 @@ static int forward_common(const lpaici_kernelset *ks, const float *d_in, int in_
     img.row_begin = row_begin;
     img.rows_out = row_count;
     img.step = step;
+    fill_tables(ks, host_var, sigma, gamma, tables);
+    tables->blob = blob;
+    return LPAICI_OK;
+}
+
+// Shared body of the forward entry points.
+static int forward_common(const lpaici_kernelset *ks, const float *d_in, int in_pitch, int width, int in_height,
+                          int row_begin, int row_count, float *d_out, int out_pitch, const float *host_var,
+                          float sigma, float gamma, uint8_t *d_smap, cudaStream_t stream,
+                          const TilePlan *plan = nullptr, bool fused = false) {
+    ImageArgs img{};
     KernelTables tab;
-    fill_tables(ks, host_var, sigma, gamma, &tab);
-    tab.blob = blob;
-    return launch_forward(ks, img, tab, config >= 0 ? config : config_for(ks, width, row_count), stream, fused);
+    const int rc = forward_args(ks, d_in, in_pitch, width, in_height, row_begin, row_count, d_out, out_pitch, host_var,
+                                sigma, gamma, d_smap, 1, &img, &tab);
+    if (rc != LPAICI_OK) return rc;
+    return launch_forward(img, tab, plan ? *plan : plan_for(ks, width, row_count), stream, fused);
 }
 
 // Every channel of an interleaved image (pixel (x, y), channel c at row y, float x * channels + c) as
-// its own image, in place: one launch per channel with element stride `channels`.
+// its own image, in place with element stride `channels`: one launch over all of them.
 static int forward_channels(const lpaici_kernelset *ks, const float *d_in, int in_pitch, float *d_out, int out_pitch,
                             int width, int height, int channels, const float *host_var, float sigma, float gamma,
                             cudaStream_t stream) {
-    if (channels <= 0 || channels > 64)
-        return set_error(LPAICI_ERR_INVALID_ARG, "channels must be 1 .. 64, got %d", channels);
+    if (channels <= 0 || channels > kMaxMultiImages)
+        return set_error(LPAICI_ERR_INVALID_ARG, "channels must be 1 .. %d, got %d", kMaxMultiImages, channels);
+    ImageArgs img{};
+    KernelTables tab;
+    const int rc = forward_args(ks, d_in, in_pitch, width, height, 0, height, d_out, out_pitch, host_var, sigma, gamma,
+                                nullptr, channels, &img, &tab);
+    if (rc != LPAICI_OK) return rc;
+    if (channels == 1) return launch_forward(img, tab, plan_for(ks, width, height), stream);
+    MultiImages mi{};
     for (int c = 0; c < channels; c++) {
-        const int rc = forward_common(ks, d_in ? d_in + c : nullptr, in_pitch, width, height, 0, height,
-                                      d_out ? d_out + c : nullptr, out_pitch, host_var, sigma, gamma, nullptr, stream,
-                                      channels);
-        if (rc != LPAICI_OK) return rc;
+        mi.in[c] = d_in + c;
+        mi.out[c] = d_out + c;
     }
-    return LPAICI_OK;
+    return launch_forward_multi(img, tab, mi, channels, plan_for(ks, width, height, channels), stream);
 }
 
 }  // namespace lpaici
@@ -196,7 +307,7 @@ int lpaici_forward_ffma(const lpaici_kernelset *ks, const float *d_noisy, int no
                         int out_pitch, int width, int height, float sigma, float gamma, uint8_t *d_scale_map,
                         lpaici_stream_t stream) {
     return forward_common(ks, d_noisy, noisy_pitch, width, height, 0, height, d_denoised, out_pitch, nullptr, sigma,
-                          gamma, d_scale_map, reinterpret_cast<cudaStream_t>(stream), 1, -1, true);
+                          gamma, d_scale_map, reinterpret_cast<cudaStream_t>(stream), nullptr, true);
 }
 
 int lpaici_forward_var(const lpaici_kernelset *ks, const float *d_noisy, int noisy_pitch, float *d_denoised,
@@ -244,11 +355,13 @@ namespace {
 // Device buffers of lpaici_denoise_host, per thread and device.
 // Device buffers and the copy/compute pipeline of lpaici_denoise_host, per host thread and device.
 constexpr int kMaxBands = 64;
+// Bands in flight: one of fewer tiles than SMs would otherwise hold back the next one on its stream for a tile's time.
+constexpr int kBandStreams = 8;
 struct HostBuffers {
     int dev = -1;
     float *in = nullptr, *out = nullptr;
     size_t cap = 0;
-    cudaStream_t s_in = nullptr, s_out = nullptr, s_comp[2] = {nullptr, nullptr};
+    cudaStream_t s_in = nullptr, s_out = nullptr, s_comp[kBandStreams] = {};
     cudaEvent_t ev_start = nullptr, ev_done = nullptr, ev_in[kMaxBands] = {}, ev_comp[kMaxBands] = {};
     ~HostBuffers() { release(); }
     void release() {
@@ -258,7 +371,9 @@ struct HostBuffers {
             cudaSetDevice(dev);
             cudaFree(in);
             cudaFree(out);
-            for (cudaStream_t st : {s_in, s_out, s_comp[0], s_comp[1]})
+            for (cudaStream_t st : {s_in, s_out})
+                if (st) cudaStreamDestroy(st);
+            for (cudaStream_t st : s_comp)
                 if (st) cudaStreamDestroy(st);
             for (cudaEvent_t ev : {ev_start, ev_done})
                 if (ev) cudaEventDestroy(ev);
@@ -270,15 +385,18 @@ struct HostBuffers {
             if (cur >= 0) cudaSetDevice(cur);
         }
         in = out = nullptr;
-        s_in = s_out = s_comp[0] = s_comp[1] = nullptr;
+        s_in = s_out = nullptr;
+        for (cudaStream_t &st : s_comp) st = nullptr;
         ev_start = ev_done = nullptr;
         cap = 0;
         dev = -1;
     }
     cudaError_t make_pipeline() {
         cudaError_t e = cudaSuccess;
-        for (cudaStream_t *st : {&s_in, &s_out, &s_comp[0], &s_comp[1]})
+        for (cudaStream_t *st : {&s_in, &s_out})
             if (e == cudaSuccess) e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+        for (cudaStream_t &st : s_comp)
+            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         for (cudaEvent_t *ev : {&ev_start, &ev_done})
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
         for (int i = 0; i < kMaxBands && e == cudaSuccess; i++) {
@@ -315,37 +433,51 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
         t_bufs.cap = n;
     }
     // Row bands, pipelined: the upload of the rows band b needs (its rows + R below) on s_in, its
-    // forward on one of two compute streams (the next band's CTAs fill the SMs while this band's last
-    // wave drains), its download on s_out.  With pinned host buffers the copies overlap the kernels.
-    // one configuration for all bands, chosen for the whole image: the bands' launches overlap on two
-    // streams, so the GPU sees one stream of tiles, not separate short launches
-    const int config = config_for(ks, width, height);
-    int tile_h = 64;
-    lpaici_tile_config_desc(config, nullptr, &tile_h, nullptr, nullptr);
+    // forward on one of the compute streams (the next bands' CTAs fill the SMs that this band leaves
+    // idle), its download on s_out.  With pinned host buffers the copies overlap the kernels.
+    // The bands' launches overlap, so the GPU sees one stream of tiles: they take the whole
+    // image's plan, big tiles in the upper bands and the plan's small ones in the lower (2048^2: 2.45 ms with
+    // one configuration in ten bands on two streams, 1.95 ms so).  The first band is one tile row, so that the first forward
+    // starts after a short upload, the last one at most two rows of small tiles, so that the download after the
+    // last forward is short; the bands between are about a sixth of the image.
+    const TilePlan plan = plan_for(ks, width, height);
+    const bool mixed = plan.mix >= 0;
+    int big_h = 64, low_h = 64;
+    lpaici_tile_config_desc(plan.config, nullptr, &big_h, nullptr, nullptr);
+    const int low_config = mixed ? mix_second(plan.mix) : plan.config;
+    lpaici_tile_config_desc(low_config, nullptr, &low_h, nullptr, nullptr);
     const int R = ks->radius;
-    // band i covers rows [edge[i], edge[i + 1]): the first is one tile row high and the last one or two,
-    // so the upload before the first forward and the download after the last one are short; the
-    // bands between are about an eighth of the image
+    // band i covers rows [edge[i], edge[i + 1]); bands from `low` on use low_config
     int edge[kMaxBands + 1];
-    int nb = 0;
-    if (height <= 3 * tile_h) {
-        edge[0] = 0;
-        edge[1] = height;
-        nb = 1;
-    } else {
-        const int last = tile_h + (height - 2 * tile_h) % tile_h;  // the middle bands stay whole tile rows
-        const int mid = height - tile_h - last;
-        int band = ((height + 7) / 8 + tile_h - 1) / tile_h * tile_h;
-        while (2 + (mid + band - 1) / band > kMaxBands) band += tile_h;
-        edge[0] = 0;
-        edge[1] = tile_h;
-        nb = 1;
-        for (int r = tile_h; r < tile_h + mid; r += band) edge[++nb] = std::min(tile_h + mid, r + band);
+    int nb = 0, low = 0;
+    edge[0] = 0;
+    if (height <= 3 * big_h) {
         edge[++nb] = height;
+        low = nb;
+    } else {
+        const int upper = mixed ? std::min(plan.big_rows * big_h, height) : 0;
+        auto cut = [&](int to, int tile, int rows) {  // bands of about `rows` rows, whole tile rows, up to row `to`
+            int band = std::max(1, (rows + tile - 1) / tile) * tile;
+            while (edge[nb] < to && nb < kMaxBands - 8) {
+                edge[nb + 1] = std::min(to, edge[nb] + band);
+                nb++;
+            }
+            if (edge[nb] < to) edge[++nb] = to;
+        };
+        if (upper > 0) {
+            cut(big_h, big_h, big_h);
+            cut(upper, big_h, (height + 5) / 6);
+        }
+        low = nb;
+        if (nb == 0) cut(low_h, low_h, low_h);
+        const int last = std::max(edge[nb], height - 2 * low_h - (height - edge[nb]) % low_h);
+        cut(last, low_h, (height + 5) / 6);
+        cut(height, height, height);
+        if (!mixed) low = 0;
     }
     HostBuffers &b = t_bufs;
     e = cudaEventRecord(b.ev_start, stream);
-    for (cudaStream_t st : {b.s_in, b.s_out, b.s_comp[0], b.s_comp[1]})
+    for (cudaStream_t st : {b.s_in, b.s_out})
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b.ev_start, 0);
     if (e != cudaSuccess) return cuda_error(e, "lpaici_denoise_host: stream order");
     int copied = 0;  // input rows [0, copied) uploaded
@@ -357,14 +489,15 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
             copied = need;
         }
         if (e == cudaSuccess) e = cudaEventRecord(b.ev_in[i], b.s_in);
-        cudaStream_t sc = b.s_comp[i & 1];
+        cudaStream_t sc = b.s_comp[i % kBandStreams];
         if (e == cudaSuccess) e = cudaStreamWaitEvent(sc, b.ev_in[i], 0);
         if (e != cudaSuccess) {
             rc = cuda_error(e, "lpaici_denoise_host: upload");
             break;
         }
+        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.mix, (r1 - r0) / big_h} : TilePlan{low_config, -1, 0};
         rc = forward_common(ks, b.in, width, width, height, r0, r1 - r0, b.out + static_cast<size_t>(r0) * width, width,
-                            nullptr, sigma, gamma, nullptr, sc, 1, config);
+                            nullptr, sigma, gamma, nullptr, sc, &band);
         if (rc != LPAICI_OK) break;
         e = cudaEventRecord(b.ev_comp[i], sc);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b.s_out, b.ev_comp[i], 0);
@@ -499,7 +632,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
     int best = -1;
     std::vector<float> config_ms(LPAICI_NUM_TILE_CONFIGS, -1.0f);
     for (int c = 0; rc == LPAICI_OK && c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        int crc = launch_forward(ks, img, tab, c, stream);  // warm-up
+        int crc = launch_forward(img, tab, TilePlan{c, -1, 0}, stream);  // warm-up
         if (crc != LPAICI_OK) {
             if (ms_out) ms_out[c] = -1.0f;
             if (crc == LPAICI_ERR_UNSUPPORTED) continue;  // this tile does not fit for this kernel set
@@ -507,7 +640,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
             break;
         }
         cudaEventRecord(e0, stream);
-        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(ks, img, tab, c, stream);
+        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(img, tab, TilePlan{c, -1, 0}, stream);
         cudaEventRecord(e1, stream);
         e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) {
@@ -533,7 +666,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
     if (best_config) *best_config = best;
     rc = lpaici_set_tile_config(ks, best);
     if (rc != LPAICI_OK) return rc;
-    // per-tile times, for picking the configuration of other image sizes (config_for)
+    // per-tile times, for picking the plan of other image sizes (plan_for)
     int dev = 0, sms = 0, max_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

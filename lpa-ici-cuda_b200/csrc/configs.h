@@ -2,7 +2,7 @@
 // column pairs per thread Q (4 or 8), direction groups DS.  A region warp covers 16 rows x 4Q columns (2Q
 // pixels per thread), so a CTA covers (4Q*WX) x (16*WY) pixels with 32*WX*WY*DS threads: DS groups of warps
 // share the tile and split the directions (sweep_tile in tile_core.cuh).  Each launch takes the
-// configuration with the least estimated time for its image (config_for in capi.cu); configurations whose
+// configuration with the least estimated time for its image (plan_for in capi.cu); configurations whose
 // shared memory does not fit a kernel set are skipped.  The adjoint's selection pass runs the configuration
 // the forward uses.
 #pragma once
@@ -23,6 +23,15 @@
 
 #define LPAICI_NUM_TILE_CONFIGS 11
 #define LPAICI_DEFAULT_TILE_CONFIG 0
+
+// Two configurations in one launch (forward_mixed in forward.cu): tiles of the first over most of the image,
+// tiles of the second over what they leave.  Both have 512 threads.
+// X(index, first, WX, WY, Q, DS, second, WX, WY, Q, DS)
+#define LPAICI_TILE_MIXES(X)                \
+    X(0, 0, 4, 4, 8, 1, 4, 1, 2, 8, 8)      \
+    X(1, 0, 4, 4, 8, 1, 5, 1, 1, 8, 16)     \
+    X(2, 3, 2, 2, 8, 4, 5, 1, 1, 8, 16)
+#define LPAICI_NUM_TILE_MIXES 3
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.

@@ -73,6 +73,14 @@ struct KernelTables {
     float thr[kMaxKernels];
 };
 
+// How a launch cuts its images into tiles: configuration `config` everywhere, or (mix >= 0) the first
+// configuration of LPAICI_TILE_MIXES entry `mix` over the whole tile columns of the first big_rows tile rows
+// and the second one over the rest.
+struct TilePlan {
+    int config = 0;
+    int mix = -1, big_rows = 0;
+};
+
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
 // output, scale maps and 1/den (the last three may be null, as in ImageArgs).
 constexpr int kMaxMultiImages = 64;
@@ -136,20 +144,21 @@ void fill_tables(const lpaici_kernelset *ks, const float *var_or_null, float sig
 // Forward / backward launchers (forward.cu, backward.cu).
 // fused: each tap one fused multiply-add instead of a rounded product and a rounded sum (faster, not
 // bit-exact with the reference: lpaici_forward_ffma).
-int launch_forward(const lpaici_kernelset *ks, const ImageArgs &img, const KernelTables &tab, int config,
-                   cudaStream_t stream, bool fused = false);
+int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan &plan, cudaStream_t stream,
+                   bool fused = false);
 // n images of img's size, pitches and tables (tab) in one launch, their buffers in mi.
-int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, int config,
+int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, const TilePlan &plan,
                          cudaStream_t stream);
 // Bytes of shared memory tile configuration `config` needs for a kernel set.
 size_t config_smem(int config, int blob_words, int nk, int R);
 // The autotuned configuration of ks on the current device, else the first one that fits.
 int default_config(const lpaici_kernelset *ks);
-// The configuration expected to be fastest for one launch over width x rows pixels: per-tile time
-// (tuned, else a B200 table) times the waves of CTAs the image needs.  A forced configuration wins.
-int config_for(const lpaici_kernelset *ks, int width, int rows);
-// The same for one launch over n images (a batched plan's tile queue): the images' tiles add up.
-int config_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n);
+// The plan expected to be fastest for one launch over n images of width x rows pixels: per-tile time (tuned,
+// else a B200 cost model) times the waves of CTAs the images need.  A forced configuration wins.
+TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n = 1);
+// The same for one launch over n images of any sizes (a batched plan's tile queue): the images' tiles add up.
+// A mix's big_rows stands for the number of big tiles.
+TilePlan plan_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n);
 // Kernel sets are supported up to what a 64 x 32 tile with 24 + 2R pair rows takes in shared memory beside
 // the set with duplicated weights: the bound on radius and taps that callers have always met, kept as it is
 // (LPAICI_ERR_UNSUPPORTED beyond it) although today's tiles and weights take less.
@@ -167,6 +176,7 @@ struct BatchSpec {
     int width, height, noisy_pitch, out_pitch;
     float sigma, gamma;
 };
+// config < 0: chosen for the images (plan_for, plan_for_images).
 int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n, int config, bool use_graph,
                       cudaStream_t stream, lpaici_batch **out);
 int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream);  // queue reset + persistent launch
