@@ -36,11 +36,11 @@ struct BatchImage {
 struct BatchArgs {
     const BatchImage *images;
     const float *tables;    // per image var[nk], thr[nk]
-    const int4 *items;      // (image, x0, y0, 1 for a small tile of a mix)
-    int n_items;
+    const int4 *items;      // (image, x0, y0, unused)
+    int rest_follows;       // a launch over the plan's small tiles follows
     int D, S, R;
     const int *blob;
-    int blob_words, run_word, weight_word;
+    int blob_words, mask_word, stream_word;
     float neg_zero;  // -0.0f, read at run time (see prod2 in tile_core.cuh)
     // every image of the plan has the same sigma and gamma (always so for one image): its var and thr
     // travel here, as in the single-image launch, instead of being read per CTA from `tables`
@@ -55,7 +55,7 @@ __device__ __forceinline__ void batched_tile(int *smem, const BatchArgs &a, cons
     const int nk = a.D * a.S;
     const SweepCta<WX, WY, Q, DS> cta(smem, a.blob_words, nk, a.R);
     load_tile(cta.tile, img, x0, y0, cta.g);
-    stage_blob<Q>(cta.blob, a.blob, a.blob_words, a.run_word, a.weight_word, cta.g.pitch2);
+    stage_blob<Q>(cta.blob, a.blob, a.blob_words, a.mask_word, a.stream_word, cta.g.pitch2);
     if (a.shared_tables) {
         stage_tables(cta.tab, a.var, a.thr, nk);
     } else {
@@ -95,24 +95,13 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     extern __shared__ __align__(16) int smem[];
     __shared__ __align__(16) unsigned char s_img[sizeof(ImageArgs)];
     ImageArgs &img = *reinterpret_cast<ImageArgs *>(s_img);
+    // a plan's big tiles let the launch over its small ones start as they end; the last small tile waits for the
+    // big ones, so that what follows in the stream follows both (lpaici_forward_rest_kernel)
+    if (a.rest_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int4 item = __ldg(a.items + blockIdx.x);
     batched_image(a, item.x, &img);
     batched_tile<WX, WY, Q, DS>(smem, a, img, item.x, item.y, item.z);
-}
-
-// The same with two kinds of tiles (see lpaici_forward_mixed_kernel): the queue's big tiles come first.
-template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD>
-__global__ void __launch_bounds__(32 * AX * AY * AD, 1)
-    lpaici_batched_mixed_kernel(const __grid_constant__ BatchArgs a) {
-    extern __shared__ __align__(16) int smem[];
-    __shared__ __align__(16) unsigned char s_img[sizeof(ImageArgs)];
-    ImageArgs &img = *reinterpret_cast<ImageArgs *>(s_img);
-    const int4 item = __ldg(a.items + blockIdx.x);
-    batched_image(a, item.x, &img);
-    if (item.w == 0)
-        batched_tile<AX, AY, AQ, AD>(smem, a, img, item.x, item.y, item.z);
-    else
-        batched_tile<BX, BY, BQ, BD>(smem, a, img, item.x, item.y, item.z);
+    if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 namespace {
@@ -121,7 +110,6 @@ struct KernelInfo {
     const void *fn;
     int tile_w, tile_h, threads;
     size_t smem;
-    int small_w = 0, small_h = 0;  // of a mix's small tiles
 };
 
 template <int WX, int WY, int Q, int DS>
@@ -145,32 +133,6 @@ int get_info(int config, const KernelTables &tab, KernelInfo *info) {
 #undef LPAICI_BATCH_CASE
 }
 
-template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD>
-void mixed_info(const KernelTables &tab, KernelInfo *info) {
-    using Big = TileShape<AX, AY, AQ, AD>;
-    using Small = TileShape<BX, BY, BQ, BD>;
-    info->fn = reinterpret_cast<const void *>(lpaici_batched_mixed_kernel<AX, AY, AQ, AD, BX, BY, BQ, BD>);
-    info->tile_w = Big::kTileW;
-    info->tile_h = Big::kTileH;
-    info->threads = Big::kThreads;
-    info->smem = std::max(sweep_smem<Big, AQ>(tab.blob_words, tab.D * tab.S, tab.R),
-                          sweep_smem<Small, BQ>(tab.blob_words, tab.D * tab.S, tab.R));
-    info->small_w = Small::kTileW;
-    info->small_h = Small::kTileH;
-}
-
-int get_mix_info(int mix, const KernelTables &tab, KernelInfo *info) {
-#define LPAICI_MIX_CASE(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD)           \
-    case idx:                                                                \
-        mixed_info<AX, AY, AQ, AD, BX, BY, BQ, BD>(tab, info);               \
-        return LPAICI_OK;
-    switch (mix) {
-        LPAICI_TILE_MIXES(LPAICI_MIX_CASE)
-        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile mix %d out of range", mix);
-    }
-#undef LPAICI_MIX_CASE
-}
-
 }  // namespace
 }  // namespace lpaici
 
@@ -178,9 +140,9 @@ using namespace lpaici;
 
 struct lpaici_batch {
     int device = -1;
-    KernelInfo info{};
+    KernelInfo info{}, rest{};  // rest: of a plan's small tiles
     BatchArgs args{};
-    int grid = 0;
+    int grid = 0, rest_grid = 0;
     void *dev_mem = nullptr;  // images | tables | items
     bool use_graph = false;
     cudaGraph_t graph = nullptr;
@@ -205,8 +167,28 @@ int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream) {
     if (b->single) return launch_forward(b->img, b->tab, b->plan, stream);
     if (b->multi) return launch_forward_multi(b->img, b->tab, b->mi, b->n_multi, b->plan, stream);
     void *params[] = {&b->args};
-    const cudaError_t e = cudaLaunchKernel(b->info.fn, dim3(b->grid), dim3(b->info.threads), params, b->info.smem, stream);
+    cudaError_t e = b->grid > 0
+                        ? cudaLaunchKernel(b->info.fn, dim3(b->grid), dim3(b->info.threads), params, b->info.smem, stream)
+                        : cudaSuccess;
     if (e != cudaSuccess) return cuda_error(e, "batched launch");
+    if (b->rest_grid > 0) {
+        BatchArgs rest = b->args;
+        rest.items += b->grid;
+        rest.rest_follows = 0;
+        void *rest_params[] = {&rest};
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(b->rest_grid);
+        cfg.blockDim = dim3(b->rest.threads);
+        cfg.dynamicSmemBytes = b->rest.smem;
+        cfg.stream = stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelExC(&cfg, b->rest.fn, rest_params);
+        if (e != cudaSuccess) return cuda_error(e, "batched launch (small tiles)");
+    }
     return LPAICI_OK;
 }
 
@@ -256,9 +238,10 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         }
         b->plan = plan_for_images(ks, w.data(), h.data(), n);
     }
-    const bool mixed = b->plan.mix >= 0;
+    const bool mixed = b->plan.rest >= 0;
     rc = check_forward_limit(tab);
-    if (rc == LPAICI_OK) rc = mixed ? get_mix_info(b->plan.mix, tab, &b->info) : get_info(b->plan.config, tab, &b->info);
+    if (rc == LPAICI_OK) rc = get_info(b->plan.config, tab, &b->info);
+    if (rc == LPAICI_OK && mixed) rc = get_info(b->plan.rest, tab, &b->rest);
     if (rc != LPAICI_OK) {
         batch_plan_free(b);
         return rc;
@@ -294,16 +277,16 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     if (mixed && !(n == 1 || one_size)) {  // all tiles past the plan's big ones are cut small
         const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_rows));
         for (size_t j = big; j < items.size(); j++)
-            for (int y = 0; y < b->info.tile_h; y += b->info.small_h)
-                for (int x = 0; x < b->info.tile_w; x += b->info.small_w)
-                    push(small, items[j].image, items[j].x + x, items[j].y + y, b->info.small_w, b->info.small_h);
+            for (int y = 0; y < b->info.tile_h; y += b->rest.tile_h)
+                for (int x = 0; x < b->info.tile_w; x += b->rest.tile_w)
+                    push(small, items[j].image, items[j].x + x, items[j].y + y, b->rest.tile_w, b->rest.tile_h);
         items.resize(big);
         std::stable_sort(small.begin(), small.end(), by_key);
     }
     std::vector<int4> qitems;
     qitems.reserve(items.size() + small.size());
     for (const Item &it : items) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
-    for (const Item &it : small) qitems.push_back(make_int4(it.image, it.x, it.y, 1));
+    for (const Item &it : small) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
 
     const size_t img_bytes = sizeof(BatchImage) * n;
     const size_t tab_off = (img_bytes + 255) & ~size_t(255);
@@ -327,14 +310,13 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     b->args.images = reinterpret_cast<const BatchImage *>(base);
     b->args.tables = reinterpret_cast<const float *>(base + tab_off);
     b->args.items = reinterpret_cast<const int4 *>(base + item_off);
-    b->args.n_items = static_cast<int>(qitems.size());
     b->args.D = ks->D;
     b->args.S = ks->S;
     b->args.R = ks->radius;
     b->args.blob = blob;
     b->args.blob_words = tab.blob_words;
-    b->args.run_word = tab.run_word;
-    b->args.weight_word = tab.weight_word;
+    b->args.mask_word = tab.mask_word;
+    b->args.stream_word = tab.stream_word;
     b->args.neg_zero = -0.0f;
     bool same = true;
     for (int i = 1; i < n; i++) same = same && specs[i].sigma == specs[0].sigma && specs[i].gamma == specs[0].gamma;
@@ -359,7 +341,15 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         return e != cudaSuccess ? cuda_error(e, "batched occupancy")
                                 : set_error(LPAICI_ERR_UNSUPPORTED, "batched kernel does not fit on an SM");
     }
-    b->grid = b->args.n_items;  // one CTA per queue item
+    b->grid = static_cast<int>(items.size());  // one CTA per queue item
+    b->rest_grid = static_cast<int>(small.size());
+    b->args.rest_follows = b->rest_grid > 0 ? 1 : 0;
+    if (e == cudaSuccess && b->rest_grid > 0)
+        e = cudaFuncSetAttribute(b->rest.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->rest.smem));
+    if (e != cudaSuccess) {
+        batch_plan_free(b);
+        return cuda_error(e, "batched attributes");
+    }
     if (n == 1 || one_size) {
         const BatchSpec &im = specs[0];
         b->single = n == 1;

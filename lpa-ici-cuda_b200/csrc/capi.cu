@@ -37,9 +37,9 @@ int default_config(const lpaici_kernelset *ks) {
 struct TileCost {
     float base_us, ns_per_work;
 };
-static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{7.8f, 61.5f}, {8.0f, 34.1f}, {7.5f, 26.3f}, {4.2f, 17.3f},
-                                                            {2.7f, 9.11f}, {1.0f, 4.95f}, {1.2f, 2.64f}, {1.0f, 25.0f},
-                                                            {7.9f, 47.3f}, {8.7f, 36.0f}, {5.5f, 19.5f}};
+static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{8.7f, 59.7f}, {8.1f, 31.2f}, {7.3f, 25.0f}, {4.2f, 15.8f},
+                                                            {2.9f, 8.35f}, {0.6f, 4.58f}, {1.2f, 2.60f}, {0.5f, 26.1f},
+                                                            {9.0f, 47.3f}, {9.8f, 36.9f}, {4.8f, 19.5f}};
 
 static int groups_of(int c) {
 #define LPAICI_GROUPS_CASE(idx, WX, WY, Q, DS) \
@@ -83,13 +83,17 @@ static long tiles_of(int c, int width, int rows) {
 
 // Time until the last of n_small tiles of t is done, handed out as SMs get free after n_big tiles of big_t.
 static double mixed_makespan(long n_big, double big_t, long n_small, double t, int sms) {
-    const long waves = n_big / sms, rem = n_big % sms;
+    const long waves = n_big / sms, rem = n_big % sms;  // rem SMs sweep one big tile more
     const double early = waves * big_t, late = early + (rem > 0 ? big_t : 0.0);
-    // the first j for which sms - rem SMs from `early` and rem SMs from `late` take n_small tiles by early + j t
-    const long gap = rem > 0 ? static_cast<long>(std::ceil(big_t / t)) : 0;
-    const long before = std::min(n_small, gap * (sms - rem));  // done before the late SMs join
-    if (before == n_small) return std::max(late, early + t * ((n_small + sms - rem - 1) / (sms - rem)));
-    return early + t * (gap + (n_small - before + sms - 1) / sms);
+    const auto done = [&](double at) {  // small tiles finished by then
+        const long a = static_cast<long>((at - early) / t + 1e-6), b = at > late ? static_cast<long>((at - late) / t + 1e-6) : 0;
+        return a * (sms - rem) + b * rem;
+    };
+    const long before = done(late);  // the SMs of the last wave's gap
+    if (before >= n_small) return std::max(late, early + t * ((n_small + sms - rem - 1) / (sms - rem)));
+    const double by_late = late + t * ((n_small - before + sms - 1) / sms);
+    const double by_early = early + t * static_cast<long>((by_late - early) / t + 1e-6);  // the early SMs' last end before it
+    return by_early > late && done(by_early) >= n_small ? by_early : by_late;
 }
 
 // What a plan is chosen with: the tile times of a kernel set on the current device.
@@ -125,16 +129,7 @@ static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
     return true;
 }
 
-static constexpr int kMixFirst[] = {
-#define LPAICI_MIX_FIRST(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD) A,
-    LPAICI_TILE_MIXES(LPAICI_MIX_FIRST)
-#undef LPAICI_MIX_FIRST
-};
-static constexpr int kMixSecond[] = {
-#define LPAICI_MIX_SECOND(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD) B,
-    LPAICI_TILE_MIXES(LPAICI_MIX_SECOND)
-#undef LPAICI_MIX_SECOND
-};
+static constexpr int kMixes[][2] = LPAICI_TILE_MIXES;
 
 // by_rows: the images are one size and a mix's big tiles are whole tile rows of every image.
 static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const int *rows, int n, bool by_rows) {
@@ -170,8 +165,8 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
         return plan;
     }
     // a mix: whole waves of big tiles, or one wave fewer, the rest in small ones
-    for (int m = 0; m < LPAICI_NUM_TILE_MIXES; m++) {
-        const int a = kMixFirst[m], b = kMixSecond[m];
+    for (const auto &mix : kMixes) {
+        const int a = mix[0], b = mix[1];
         if (!(pc.tile_ms[a] > 0.0f) || !(pc.tile_ms[b] > 0.0f)) continue;
         int aw = 1, ah = 1, bw = 1, bh = 1;
         config_tile(a, &aw, &ah);
@@ -188,7 +183,7 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
             const double est = mixed_makespan(big, pc.tile_ms[a], small, pc.tile_ms[b], pc.sms);
             if (est < best_ms) {
                 best_ms = est;
-                plan = TilePlan{a, m, big_rows};
+                plan = TilePlan{a, b, big_rows};
             }
         };
         const long row = by_rows ? static_cast<long>(widths[0] / aw) * n : 1;  // big tiles of one tile row
@@ -199,8 +194,6 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
     }
     return plan;
 }
-
-static int mix_second(int mix) { return kMixSecond[mix]; }
 
 TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n) {
     const std::vector<int> w(n, width), h(n, rows);
@@ -441,10 +434,10 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
     // starts after a short upload, the last one at most two rows of small tiles, so that the download after the
     // last forward is short; the bands between are about a sixth of the image.
     const TilePlan plan = plan_for(ks, width, height);
-    const bool mixed = plan.mix >= 0;
+    const bool mixed = plan.rest >= 0;
     int big_h = 64, low_h = 64;
     lpaici_tile_config_desc(plan.config, nullptr, &big_h, nullptr, nullptr);
-    const int low_config = mixed ? mix_second(plan.mix) : plan.config;
+    const int low_config = mixed ? plan.rest : plan.config;
     lpaici_tile_config_desc(low_config, nullptr, &low_h, nullptr, nullptr);
     const int R = ks->radius;
     // band i covers rows [edge[i], edge[i + 1]); bands from `low` on use low_config
@@ -495,7 +488,7 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
             rc = cuda_error(e, "lpaici_denoise_host: upload");
             break;
         }
-        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.mix, (r1 - r0) / big_h} : TilePlan{low_config, -1, 0};
+        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.rest, (r1 - r0) / big_h} : TilePlan{low_config, -1, 0};
         rc = forward_common(ks, b.in, width, width, height, r0, r1 - r0, b.out + static_cast<size_t>(r0) * width, width,
                             nullptr, sigma, gamma, nullptr, sc, &band);
         if (rc != LPAICI_OK) break;

@@ -24,14 +24,12 @@
 #define LPAICI_NUM_TILE_CONFIGS 11
 #define LPAICI_DEFAULT_TILE_CONFIG 0
 
-// Two configurations in one launch (forward_mixed in forward.cu): tiles of the first over most of the image,
-// tiles of the second over what they leave.  Both have 512 threads.
-// X(index, first, WX, WY, Q, DS, second, WX, WY, Q, DS)
-#define LPAICI_TILE_MIXES(X)                \
-    X(0, 0, 4, 4, 8, 1, 4, 1, 2, 8, 8)      \
-    X(1, 0, 4, 4, 8, 1, 5, 1, 1, 8, 16)     \
-    X(2, 3, 2, 2, 8, 4, 5, 1, 1, 8, 16)
-#define LPAICI_NUM_TILE_MIXES 3
+// The configurations that can take what whole waves of bigger tiles leave of an image (launch_rest in
+// forward.cu), and the mixes {big, rest} that a plan considers.
+#define LPAICI_REST_CONFIGS(X) \
+    X(4, 1, 2, 8, 8)           \
+    X(5, 1, 1, 8, 16)
+#define LPAICI_TILE_MIXES {{0, 4}, {0, 5}, {1, 5}, {3, 5}}
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.

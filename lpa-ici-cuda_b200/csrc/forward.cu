@@ -11,6 +11,12 @@
 
 namespace lpaici {
 
+// A launch over part of the tiles may be followed by one over the rest (launch_rest), whose CTAs the hardware
+// hands out once every CTA of this one has started.
+__device__ __forceinline__ void let_rest_start(const KernelTables &tab) {
+    if (tab.rest_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Stages the kernel set, the tables and the tile at (x0, y0) of img, and sweeps it.
 // Fused = false: every tap's product and sum rounded on their own (bit-exact with the reference);
 // true: each tap one fused multiply-add (lpaici_forward_ffma).
@@ -19,7 +25,7 @@ __device__ __forceinline__ void forward_tile(int *smem, const ImageArgs &img, co
     const int nk = tab.D * tab.S;
     const SweepCta<WX, WY, Q, DS> cta(smem, tab.blob_words, nk, tab.R);
     load_tile(cta.tile, img, x0, y0, cta.g);
-    stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.run_word, tab.weight_word, cta.g.pitch2);
+    stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.mask_word, tab.stream_word, cta.g.pitch2);
     stage_tables(cta.tab, tab.var, tab.thr, nk);
     tile_wait();
     __syncthreads();
@@ -31,17 +37,29 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     lpaici_forward_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
     extern __shared__ __align__(16) int smem[];
     using Shape = TileShape<WX, WY, Q, DS>;
+    let_rest_start(tab);
     forward_tile<WX, WY, Q, DS, Fused>(smem, img, tab, blockIdx.x * Shape::kTileW, blockIdx.y * Shape::kTileH);
 }
 
-__device__ __forceinline__ ImageArgs image_of(const ImageArgs &img, const MultiImages &mi, int z) {
-    ImageArgs im = img;
-    im.in = mi.in[z];
-    im.out = mi.out[z];
-    im.smap = mi.smap[z];
-    im.rden = mi.rden[z];
-    return im;
-}
+// Image z of a launch over several images (mi; img itself of a launch over one), in shared memory: kept in
+// registers its pointers would stay live across the sweep (the single-image kernel reads its parameters).
+struct SharedImage {
+    __align__(16) unsigned char raw[sizeof(ImageArgs)];
+    __device__ __forceinline__ const ImageArgs &fill(const ImageArgs &img, const MultiImages &mi, int images, int z) {
+        ImageArgs &im = *reinterpret_cast<ImageArgs *>(raw);
+        if (threadIdx.x == 0) {
+            im = img;
+            if (images > 1) {
+                im.in = mi.in[z];
+                im.out = mi.out[z];
+                im.smap = mi.smap[z];
+                im.rden = mi.rden[z];
+            }
+        }
+        __syncthreads();
+        return im;
+    }
+};
 
 // Several images of one size, pitch, sigma and gamma in one launch (a batched plan of such images, the channels
 // of an interleaved image): grid layer z is image z, whose buffers replace img's; everything else is the
@@ -52,66 +70,55 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     lpaici_forward_multi_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab,
                                 const __grid_constant__ MultiImages mi) {
     extern __shared__ __align__(16) int smem[];
+    __shared__ SharedImage s_img;
     using Shape = TileShape<WX, WY, Q, DS>;
-    forward_tile<WX, WY, Q, DS, false>(smem, image_of(img, mi, blockIdx.z), tab, blockIdx.x * Shape::kTileW,
+    let_rest_start(tab);
+    forward_tile<WX, WY, Q, DS, false>(smem, s_img.fill(img, mi, 2, blockIdx.z), tab, blockIdx.x * Shape::kTileW,
                                        blockIdx.y * Shape::kTileH);
 }
 
-// How a mixed launch cuts each image: big tiles over [0, wb) x [0, hb), small ones over the strip to their right
-// and over the rows below.  CTAs: the big tiles of all images, then the small ones.
+// How a mix cuts each image: big tiles over [0, wb) x [0, hb), small ones over the strip to their right and over
+// the rows below.
 struct MixGrid {
     int images;
-    int wb, hb, big_x, n_big;
+    int wb, hb;
     int right_x, n_right, bottom_x, n_small;  // n_small: both strips
 };
 
-// Big tiles sweep a pixel in the least time, but an image of a few waves of them leaves SMs idle in the last
-// one: the launch takes whole waves of big tiles and cuts the rest into tiles of 8 or 16 direction groups, an
-// eighth or a sixteenth of a big one's time, which fill the SMs as the big tiles end.  1535 x 1021 (192 big
-// tiles are 1.3 waves): 817 us with one configuration, 736 us mixed; 1600 x 1200 contracted 738 and 641 us; a
-// 10-image plan 2506 and 2173 us.
-template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD, bool Fused>
-__global__ void __launch_bounds__(32 * AX * AY * AD, 1)
-    lpaici_forward_mixed_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab,
-                                const __grid_constant__ MultiImages mi, const __grid_constant__ MixGrid g) {
-    static_assert(AX * AY * AD == BX * BY * BD, "both tiles have the CTA's threads");
-    static_assert(AY % BY == 0 && AX * AQ % (BX * BQ) == 0, "a big tile is whole small ones");
+// The small tiles of a mix.  Big tiles sweep a pixel in the least time, but an image of a few waves of them
+// leaves SMs idle in the last one: the first launch takes whole waves of big tiles, this one cuts the rest into
+// tiles of 8 or 16 direction groups, an eighth or a sixteenth of a big one's time, which fill the SMs as the big
+// tiles end (programmatic dependent launch).  It depends on nothing of the first launch; its last CTA waits for
+// that one, so that what follows in the stream follows both.
+// us, gaussian 16 x 7 set with scale maps, 1535 x 1021 (192 big tiles are 1.3 waves): 787 with one configuration,
+// 698 so; 768 x 513 x 3 channels 642 and 526.  (Both kinds of tiles in one kernel cost the big ones 2 to 5 %: the
+// compiler allocates registers for both sweeps together.)
+template <int WX, int WY, int Q, int DS, bool Fused>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
+    lpaici_forward_rest_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab,
+                               const __grid_constant__ MultiImages mi, const __grid_constant__ MixGrid g) {
     extern __shared__ __align__(16) int smem[];
-    using Big = TileShape<AX, AY, AQ, AD>;
-    using Small = TileShape<BX, BY, BQ, BD>;
-    int b = blockIdx.x;
-    const int all_big = g.images * g.n_big;
-    if (b < all_big) {
-        const int z = b / g.n_big, t = b - z * g.n_big;
-        const int x0 = (t % g.big_x) * Big::kTileW, y0 = (t / g.big_x) * Big::kTileH;
-        if (g.images == 1)
-            forward_tile<AX, AY, AQ, AD, Fused>(smem, img, tab, x0, y0);
-        else
-            forward_tile<AX, AY, AQ, AD, Fused>(smem, image_of(img, mi, z), tab, x0, y0);
-        return;
-    }
-    b -= all_big;
-    const int z = b / g.n_small;
-    int t = b - z * g.n_small, x0, y0;
-    if (t < g.n_right) {
-        x0 = g.wb + (t % g.right_x) * Small::kTileW;
-        y0 = (t / g.right_x) * Small::kTileH;
-    } else {
-        t -= g.n_right;
-        x0 = (t % g.bottom_x) * Small::kTileW;
-        y0 = g.hb + (t / g.bottom_x) * Small::kTileH;
-    }
+    __shared__ SharedImage s_img;
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const int z = blockIdx.x / g.n_small, t = blockIdx.x - z * g.n_small;
     // (the strips' tiles end where the big tiles do: a big tile is whole small ones high and wide)
-    if (g.images == 1)
-        forward_tile<BX, BY, BQ, BD, Fused>(smem, img, tab, x0, y0);
-    else
-        forward_tile<BX, BY, BQ, BD, Fused>(smem, image_of(img, mi, z), tab, x0, y0);
+    int x0, y0;
+    if (t < g.n_right) {
+        x0 = g.wb + (t % g.right_x) * Shape::kTileW;
+        y0 = (t / g.right_x) * Shape::kTileH;
+    } else {
+        x0 = ((t - g.n_right) % g.bottom_x) * Shape::kTileW;
+        y0 = g.hb + ((t - g.n_right) / g.bottom_x) * Shape::kTileH;
+    }
+    forward_tile<WX, WY, Q, DS, Fused>(smem, s_img.fill(img, mi, g.images, z), tab, x0, y0);
+    if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 namespace {
 
+// across x down tiles from the image's origin (0: as many as cover it)
 template <int WX, int WY, int Q, int DS>
-int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n,
+int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, int across, int down,
                      cudaStream_t stream) {
     using Shape = TileShape<WX, WY, Q, DS>;
     const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
@@ -124,8 +131,8 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
                          max_optin);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, several images)");
-    const dim3 grid((img.W + Shape::kTileW - 1) / Shape::kTileW, (img.rows_out + Shape::kTileH - 1) / Shape::kTileH,
-                    n);
+    const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
+                    across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH, n);
     if (grid.y > 65535u) return set_error(LPAICI_ERR_UNSUPPORTED, "image too tall: %d rows", img.rows_out);
     kern<<<grid, Shape::kThreads, smem, stream>>>(img, tab, mi);
     e = cudaGetLastError();
@@ -134,7 +141,7 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
 }
 
 template <int WX, int WY, int Q, int DS, bool Fused>
-int launch_cfg(const ImageArgs &img, const KernelTables &tab, cudaStream_t stream) {
+int launch_cfg(const ImageArgs &img, const KernelTables &tab, int across, int down, cudaStream_t stream) {
     using Shape = TileShape<WX, WY, Q, DS>;
     const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
     auto kern = lpaici_forward_kernel<WX, WY, Q, DS, Fused>;
@@ -146,7 +153,8 @@ int launch_cfg(const ImageArgs &img, const KernelTables &tab, cudaStream_t strea
                          max_optin);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward)");
-    const dim3 grid((img.W + Shape::kTileW - 1) / Shape::kTileW, (img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
+    const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
+                    across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
     if (grid.y > 65535u) return set_error(LPAICI_ERR_UNSUPPORTED, "image too tall: %d rows", img.rows_out);
     kern<<<grid, Shape::kThreads, smem, stream>>>(img, tab);
     e = cudaGetLastError();
@@ -154,51 +162,41 @@ int launch_cfg(const ImageArgs &img, const KernelTables &tab, cudaStream_t strea
     return LPAICI_OK;
 }
 
-template <int AX, int AY, int AQ, int AD, int BX, int BY, int BQ, int BD, bool Fused>
-int launch_mixed(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, int big_rows,
-                 cudaStream_t stream) {
-    using Big = TileShape<AX, AY, AQ, AD>;
-    using Small = TileShape<BX, BY, BQ, BD>;
-    const size_t sa = sweep_smem<Big, AQ>(tab.blob_words, tab.D * tab.S, tab.R);
-    const size_t sb = sweep_smem<Small, BQ>(tab.blob_words, tab.D * tab.S, tab.R);
-    const size_t smem = sa > sb ? sa : sb;
-    auto kern = lpaici_forward_mixed_kernel<AX, AY, AQ, AD, BX, BY, BQ, BD, Fused>;
+template <int WX, int WY, int Q, int DS, bool Fused>
+int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, const MixGrid &grid, cudaStream_t stream) {
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
+    auto kern = lpaici_forward_rest_kernel<WX, WY, Q, DS, Fused>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, mixed tiles)");
-    MixGrid g{};
-    g.images = n;
-    g.big_x = img.W / Big::kTileW;
-    g.wb = g.big_x * Big::kTileW;
-    g.hb = big_rows * Big::kTileH;
-    g.n_big = g.big_x * big_rows;
-    g.right_x = (img.W - g.wb + Small::kTileW - 1) / Small::kTileW;
-    g.n_right = g.right_x * ((g.hb + Small::kTileH - 1) / Small::kTileH);
-    g.bottom_x = (img.W + Small::kTileW - 1) / Small::kTileW;
-    g.n_small = g.n_right + g.bottom_x * ((img.rows_out - g.hb + Small::kTileH - 1) / Small::kTileH);
-    const long ctas = static_cast<long>(n) * (g.n_big + g.n_small);
+    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, rest)");
+    MixGrid g = grid;
+    g.right_x = (img.W - g.wb + Shape::kTileW - 1) / Shape::kTileW;
+    g.n_right = g.right_x * ((g.hb + Shape::kTileH - 1) / Shape::kTileH);
+    g.bottom_x = (img.W + Shape::kTileW - 1) / Shape::kTileW;
+    g.n_small = g.n_right + g.bottom_x * ((img.rows_out - g.hb + Shape::kTileH - 1) / Shape::kTileH);
+    const long ctas = static_cast<long>(g.images) * g.n_small;
     if (ctas > 0x7fffffffL) return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", img.W, img.rows_out);
-    kern<<<static_cast<unsigned>(ctas), Big::kThreads, smem, stream>>>(img, tab, mi, g);
-    e = cudaGetLastError();
-    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "forward launch (mixed tiles)");
-}
-
-int forward_mixed(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, const TilePlan &plan,
-                  bool fused, cudaStream_t stream) {
-#define LPAICI_MIX_CASE(idx, A, AX, AY, AQ, AD, B, BX, BY, BQ, BD)                                                     \
-    case idx:                                                                                                          \
-        return fused ? launch_mixed<AX, AY, AQ, AD, BX, BY, BQ, BD, true>(img, tab, mi, n, plan.big_rows, stream)     \
-                     : launch_mixed<AX, AY, AQ, AD, BX, BY, BQ, BD, false>(img, tab, mi, n, plan.big_rows, stream);
-    switch (plan.mix) {
-        LPAICI_TILE_MIXES(LPAICI_MIX_CASE)
-        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile mix %d out of range", plan.mix);
-    }
-#undef LPAICI_MIX_CASE
+    if (ctas == 0) return LPAICI_OK;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(Shape::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, img, tab, mi, g);
+    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "forward launch (rest)");
 }
 
 }  // namespace
 
-#define LPAICI_FWD_CASE(idx, WX, WY, Q, DS) \
-    case idx: return fused ? launch_cfg<WX, WY, Q, DS, true>(img, tab, stream) : launch_cfg<WX, WY, Q, DS, false>(img, tab, stream);
+#define LPAICI_FWD_CASE(idx, WX, WY, Q, DS)                                      \
+    case idx:                                                                    \
+        return fused ? launch_cfg<WX, WY, Q, DS, true>(img, tab, across, down, stream) \
+                     : launch_cfg<WX, WY, Q, DS, false>(img, tab, across, down, stream);
 
 template <int WX, int WY, int Q, int DS>
 int blocks_per_sm(size_t smem) {
@@ -260,36 +258,81 @@ int check_forward_limit(const KernelTables &tab) {
     return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d", need, max_optin);
 }
 
+static int launch_config(const ImageArgs &img, const KernelTables &tab, int config, int across, int down, bool fused,
+                         cudaStream_t stream) {
+    switch (config) {
+        LPAICI_TILE_CONFIGS(LPAICI_FWD_CASE)
+        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);
+    }
+}
+
+static int launch_multi_config(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, int config,
+                               int across, int down, cudaStream_t stream) {
+#define LPAICI_MULTI_CASE(idx, WX, WY, Q, DS) \
+    case idx: return launch_multi_cfg<WX, WY, Q, DS>(img, tab, mi, n, across, down, stream);
+    switch (config) {
+        LPAICI_TILE_CONFIGS(LPAICI_MULTI_CASE)
+        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", config);
+    }
+#undef LPAICI_MULTI_CASE
+}
+
+static int launch_rest_config(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, const MixGrid &g,
+                              int config, bool fused, cudaStream_t stream) {
+#define LPAICI_REST_CASE(idx, WX, WY, Q, DS)                                          \
+    case idx:                                                                         \
+        return fused ? launch_rest<WX, WY, Q, DS, true>(img, tab, mi, g, stream)      \
+                     : launch_rest<WX, WY, Q, DS, false>(img, tab, mi, g, stream);
+    switch (config) {
+        LPAICI_REST_CONFIGS(LPAICI_REST_CASE)
+        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d takes no rest", config);
+    }
+#undef LPAICI_REST_CASE
+}
+
+// The strips of a plan's mix, for images of img's size.
+static MixGrid mix_grid(const ImageArgs &img, const TilePlan &plan, int n, int *across) {
+    int tw = 1, th = 1;
+    config_tile(plan.config, &tw, &th);
+    *across = img.W / tw;
+    MixGrid g{};
+    g.images = n;
+    g.wb = *across * tw;
+    g.hb = plan.big_rows * th;
+    return g;
+}
+
 int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n,
                          const TilePlan &plan, cudaStream_t stream) {
     if (tab.S > kMaxScales)
         return set_error(LPAICI_ERR_UNSUPPORTED, "%d scales per direction; the kernels support at most %d", tab.S,
                          kMaxScales);
-    const int rc = check_forward_limit(tab);
+    int rc = check_forward_limit(tab);
     if (rc != LPAICI_OK) return rc;
     if (n < 1 || n > kMaxMultiImages)
         return set_error(LPAICI_ERR_INVALID_ARG, "%d images in one launch; at most %d", n, kMaxMultiImages);
-    if (plan.mix >= 0) return forward_mixed(img, tab, mi, n, plan, false, stream);
-#define LPAICI_MULTI_CASE(idx, WX, WY, Q, DS) \
-    case idx: return launch_multi_cfg<WX, WY, Q, DS>(img, tab, mi, n, stream);
-    switch (plan.config) {
-        LPAICI_TILE_CONFIGS(LPAICI_MULTI_CASE)
-        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", plan.config);
-    }
-#undef LPAICI_MULTI_CASE
+    if (plan.rest < 0) return launch_multi_config(img, tab, mi, n, plan.config, 0, 0, stream);
+    int across = 0;
+    const MixGrid g = mix_grid(img, plan, n, &across);
+    KernelTables first = tab;
+    first.rest_follows = 1;
+    rc = launch_multi_config(img, first, mi, n, plan.config, across, plan.big_rows, stream);
+    return rc == LPAICI_OK ? launch_rest_config(img, tab, mi, g, plan.rest, false, stream) : rc;
 }
 
 int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan &plan, cudaStream_t stream, bool fused) {
     if (tab.S > kMaxScales)
         return set_error(LPAICI_ERR_UNSUPPORTED, "%d scales per direction; the kernels support at most %d", tab.S,
                          kMaxScales);
-    const int rc = check_forward_limit(tab);
+    int rc = check_forward_limit(tab);
     if (rc != LPAICI_OK) return rc;
-    if (plan.mix >= 0) return forward_mixed(img, tab, MultiImages{}, 1, plan, fused, stream);
-    switch (plan.config) {
-        LPAICI_TILE_CONFIGS(LPAICI_FWD_CASE)
-        default: return set_error(LPAICI_ERR_INVALID_ARG, "tile config %d out of range", plan.config);
-    }
+    if (plan.rest < 0) return launch_config(img, tab, plan.config, 0, 0, fused, stream);
+    int across = 0;
+    const MixGrid g = mix_grid(img, plan, 1, &across);
+    KernelTables first = tab;
+    first.rest_follows = 1;
+    rc = launch_config(img, first, plan.config, across, plan.big_rows, fused, stream);
+    return rc == LPAICI_OK ? launch_rest_config(img, tab, MultiImages{}, g, plan.rest, fused, stream) : rc;
 }
 
 }  // namespace lpaici

@@ -22,14 +22,14 @@ constexpr int kMaxScales = 16;
 // Device image of a kernel set, one contiguous block of 32-bit words, every part 16-byte aligned.
 // A row run of a kernel is the taps (dy, dx0 + j), j < L, offsets from the output pixel (row - rows/2,
 // col - cols/2), in row-major order.  The forward's blob:
-//   [0, 2*(nk+1))           per kernel k {its first run, its first weight's byte offset in the weights};
-//                           kernel k's runs end where kernel k + 1's begin
-//   [run_word, +4*n_runs)   per run {dy, dx0, L % 4, L / 4}
-//   [weight_word, ...)      weights: per run its first L % 4 taps padded to a group of 4, then the other
-//                           taps, so that every load of a group is one aligned 16-byte load
+//   [0, nk+1)               per kernel k the byte offset of its runs in the stream; they end where kernel
+//                           k + 1's begin
+//   [mask_word, ...)        one bit per 16-byte group of the stream: set for a run's first group
+//   [stream_word, ...)      the stream: per run {dy, dx0, L % 4, L / 4}, its first L % 4 weights padded to a
+//                           group of 4 (none if L % 4 is 0), the other weights in groups of 4
 struct BlobLayout {
     int nk = 0, n_runs = 0;
-    int run_word = 0, weight_word = 0, total_words = 0;  // total a multiple of 4
+    int mask_word = 0, stream_word = 0, total_words = 0;  // total a multiple of 4
     // the forward's support limit (check_forward_limit): words of the set with every weight stored twice
     int limit_words = 0;
 };
@@ -67,18 +67,18 @@ struct KernelTables {
     int D, S, R;
     float neg_zero;  // -0.0f, read at run time (see prod2 in tile_core.cuh)
     const int *blob;  // device blob (BlobLayout)
-    int blob_words, run_word, weight_word;
+    int blob_words, mask_word, stream_word;
     int limit_words;
+    int rest_follows = 0;  // a launch over the tiles that this one leaves follows (TilePlan::rest)
     float var[kMaxKernels];
     float thr[kMaxKernels];
 };
 
-// How a launch cuts its images into tiles: configuration `config` everywhere, or (mix >= 0) the first
-// configuration of LPAICI_TILE_MIXES entry `mix` over the whole tile columns of the first big_rows tile rows
-// and the second one over the rest.
+// How a launch cuts its images into tiles: configuration `config` everywhere, or (rest >= 0) `config` over the
+// whole tile columns of the first big_rows tile rows and configuration `rest` over what they leave.
 struct TilePlan {
     int config = 0;
-    int mix = -1, big_rows = 0;
+    int rest = -1, big_rows = 0;
 };
 
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
@@ -157,7 +157,7 @@ int default_config(const lpaici_kernelset *ks);
 // else a B200 cost model) times the waves of CTAs the images need.  A forced configuration wins.
 TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n = 1);
 // The same for one launch over n images of any sizes (a batched plan's tile queue): the images' tiles add up.
-// A mix's big_rows stands for the number of big tiles.
+// big_rows stands for the number of big tiles.
 TilePlan plan_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n);
 // Kernel sets are supported up to what a 64 x 32 tile with 24 + 2R pair rows takes in shared memory beside
 // the set with duplicated weights: the bound on radius and taps that callers have always met, kept as it is

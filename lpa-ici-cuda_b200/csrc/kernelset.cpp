@@ -46,40 +46,48 @@ int cuda_error(cudaError_t e, const char *what) {
 // ---------------------------------------------------------------------------------------------
 static int build_adjoint_blob(lpaici_kernelset *ks) {
     const int D = ks->D, S = ks->S, nk = D * S;
-    std::vector<int> begin(nk + 1), rdy, rdx, rlen;
+    std::vector<int> begin(nk + 1), rdy, rdx, rlen, run_first_w(ks->run_row.size());
     std::vector<float> w;
+    std::vector<double> row;
+    for (int k = 0; k < nk; k++) {
+        int at = ks->k_first_weight[k];
+        for (int r = ks->k_first_run[k]; r < ks->k_first_run[k] + ks->k_num_runs[k]; r++) {
+            run_first_w[r] = at;
+            at += ks->run_len[r];
+        }
+    }
+    for (auto *v : {&rdy, &rdx, &rlen}) v->reserve(2 * ks->run_row.size());
+    w.reserve(2 * ks->run_w.size());
     for (int d = 0; d < D; d++)
         for (int s = 0; s < S; s++) {
             const int k = d * S + s;
             begin[k] = static_cast<int>(rdy.size());
             const int kp = s > 0 ? k - 1 : -1;  // the kernel subtracted: h_{s-1}
-            const int hy = std::max(ks->rows[k] / 2, kp >= 0 ? ks->rows[kp] / 2 : 0);
-            const int hx = std::max(ks->cols[k] / 2, kp >= 0 ? ks->cols[kp] / 2 : 0);
-            const int bw = 2 * hx + 1;
-            std::vector<double> box(static_cast<size_t>(2 * hy + 1) * bw, 0.0);  // offset (dy, dx) at (dy+hy, dx+hx)
-            auto add = [&](int kk, double sign) {
-                const float *h = ks->dense_w.data() + ks->off[kk];
-                const int R = ks->rows[kk], Cc = ks->cols[kk];
-                for (int r = 0; r < R; r++)
-                    for (int c = 0; c < Cc; c++)
-                        box[static_cast<size_t>(r - R / 2 + hy) * bw + (c - Cc / 2 + hx)] += sign * h[r * Cc + c];
-            };
-            add(k, 1.0);
-            if (kp >= 0) add(kp, -1.0);
-            // mirrored: tap (my, mx) of the gather kernel is box(-my, -mx)
-            for (int my = -hy; my <= hy; my++) {
-                const double *row = box.data() + static_cast<size_t>(-my + hy) * bw;
-                int first = 1 << 30, last = -(1 << 30);
-                for (int mx = -hx; mx <= hx; mx++)
-                    if (static_cast<float>(row[-mx + hx]) != 0.0f) {
-                        first = std::min(first, mx);
-                        last = std::max(last, mx);
+            // rows of D descend with the mirrored rows: my = -dy, and columns mx = -dx likewise
+            const int i0 = ks->k_first_run[k], j0 = kp >= 0 ? ks->k_first_run[kp] : 0;
+            int i = i0 + ks->k_num_runs[k] - 1, j = kp >= 0 ? j0 + ks->k_num_runs[kp] - 1 : j0 - 1;
+            while (i >= i0 || j >= j0) {
+                const int dy = i >= i0 && (j < j0 || ks->run_row[i] >= ks->run_row[j]) ? ks->run_row[i] : ks->run_row[j];
+                const int ri = i >= i0 && ks->run_row[i] == dy ? i-- : -1, rj = j >= j0 && ks->run_row[j] == dy ? j-- : -1;
+                int c0 = 1 << 30, c1 = -(1 << 30);  // columns of either kernel's run
+                for (const int r : {ri, rj})
+                    if (r >= 0) {
+                        c0 = std::min(c0, ks->run_col[r]);
+                        c1 = std::max(c1, ks->run_col[r] + ks->run_len[r] - 1);
                     }
+                row.assign(c1 - c0 + 1, 0.0);
+                if (ri >= 0)
+                    for (int t = 0; t < ks->run_len[ri]; t++) row[ks->run_col[ri] + t - c0] += ks->run_w[run_first_w[ri] + t];
+                if (rj >= 0)
+                    for (int t = 0; t < ks->run_len[rj]; t++) row[ks->run_col[rj] + t - c0] -= ks->run_w[run_first_w[rj] + t];
+                int first = c0, last = c1;  // trimmed to the nonzero taps
+                while (first <= last && static_cast<float>(row[first - c0]) == 0.0f) first++;
+                while (last >= first && static_cast<float>(row[last - c0]) == 0.0f) last--;
                 if (first > last) continue;
-                rdy.push_back(my);
-                rdx.push_back(first);
+                rdy.push_back(-dy);
+                rdx.push_back(-last);
                 rlen.push_back(last - first + 1);
-                for (int mx = first; mx <= last; mx++) w.push_back(static_cast<float>(row[-mx + hx]));
+                for (int dx = last; dx >= first; dx--) w.push_back(static_cast<float>(row[dx - c0]));
             }
         }
     begin[nk] = static_cast<int>(rdy.size());
@@ -117,6 +125,8 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
             box[2] = none ? rdx[r] : std::min(box[2], rdx[r]);
             box[3] = none ? rdx[r] + rlen[r] - 1 : std::max(box[3], rdx[r] + rlen[r] - 1);
         }
+        units[k].reserve(begin[k + 1] - begin[k] + 1);
+        pairs[k].reserve(6 * static_cast<size_t>(w0 - (begin[k + 1] > begin[k] ? first_w[0] : w0)));
         // rows ascend; `r` is the first run whose row is not above j - 1
         int r = begin[k];
         for (int j = box[0]; box[1] >= box[0] && j <= box[1] + 1; j++) {
@@ -151,6 +161,7 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         if (10 * static_cast<size_t>(L.plane) + 2 * L.block_bytes + 12 * (nk + 1) + 64 + sums <= kSharedPerCta) break;
     }
     std::vector<int32_t> &blob = ks->adj_blob;
+    blob.reserve(limit_words + limit_words / 4);
     blob.assign((2 * (static_cast<size_t>(nk) + 1) + 3) & ~size_t(3), 0);
     for (int k = 0; k < nk; k++) {
         blob[2 * k] = static_cast<int>(4 * blob.size());
@@ -188,73 +199,74 @@ static int finish_kernelset(lpaici_kernelset *ks) {
         const float *h = ks->dense_w.data() + ks->off[k];
         const int R = ks->rows[k], Cc = ks->cols[k];
         float nsq = 0.0f;
-        // compute_kernel_variances order; a zero tap would add +0 to a sum that is never -0
-        for (int i = 0; i < R * Cc; i++)
-            if (h[i] != 0.0f) nsq += h[i] * h[i];
-        ks->norm2[k] = nsq;
         ks->k_first_run.push_back(static_cast<int>(ks->run_row.size()));
         ks->k_first_weight.push_back(static_cast<int>(ks->run_w.size()));
         for (int r = 0; r < R; r++) {
-            int first = -1, last = -1;
-            for (int c = 0; c < Cc; c++)
-                if (h[r * Cc + c] != 0.0f) {
-                    if (first < 0) first = c;
-                    last = c;
-                    ks->nnz[k]++;
-                }
-            if (first < 0) continue;
+            const float *row = h + static_cast<size_t>(r) * Cc;
+            uint32_t any = 0;  // of either sign, zero
+            for (int c = 0; c < Cc; c++) {
+                uint32_t bits;
+                std::memcpy(&bits, row + c, sizeof(bits));
+                any |= bits << 1;
+            }
+            if (any == 0) continue;
+            int first = 0, last = Cc - 1;
+            while (row[first] == 0.0f) first++;
+            while (row[last] == 0.0f) last--;
+            for (int c = first; c <= last; c++) {
+                nsq += row[c] * row[c];  // compute_kernel_variances order; the zero taps left out would add +0
+                ks->nnz[k] += row[c] != 0.0f;
+            }
             const int dy = r - R / 2, dx0 = first - Cc / 2, len = last - first + 1;
             ks->run_row.push_back(dy);
             ks->run_col.push_back(dx0);
             ks->run_len.push_back(len);
-            for (int c = first; c <= last; c++) ks->run_w.push_back(h[r * Cc + c]);
+            ks->run_w.insert(ks->run_w.end(), row + first, row + last + 1);
             int reach = std::abs(dy);
             if (std::abs(dx0) > reach) reach = std::abs(dx0);
             if (std::abs(dx0 + len - 1) > reach) reach = std::abs(dx0 + len - 1);
             if (reach > ks->radius) ks->radius = reach;
         }
+        ks->norm2[k] = nsq;
         ks->k_num_runs.push_back(static_cast<int>(ks->run_row.size()) - ks->k_first_run[k]);
     }
     if (ks->radius > kMaxRadius)
         return set_error(LPAICI_ERR_UNSUPPORTED, "kernel radius %d exceeds the supported %d", ks->radius, kMaxRadius);
 
-    // device blob (BlobLayout): [{first run, weight byte} per kernel (nk+1)] [{dy, dx0, L % 4, L / 4} per run]
-    // [weights: per run its first L % 4 taps padded to 4, then the other taps]
+    // device blob (BlobLayout): [stream offset per kernel (nk+1)] [a bit per stream group] [the stream]
     BlobLayout &L = ks->layout;
     L.nk = nk;
     L.n_runs = static_cast<int>(ks->run_row.size());
-    L.run_word = (2 * (nk + 1) + 3) & ~3;
-    L.weight_word = L.run_word + 4 * L.n_runs;
-    int n_w = 0, n_dup = 16;
+    int groups = 0, n_dup = 16;
     for (int r = 0; r < L.n_runs; r++) {
-        n_w += (ks->run_len[r] + 3) & ~3;
+        groups += 1 + (ks->run_len[r] + 3) / 4;
         n_dup += (ks->run_len[r] + 1) & ~1;
     }
+    L.mask_word = (nk + 1 + 3) & ~3;
+    L.stream_word = L.mask_word + (((groups + 31) / 32 + 3) & ~3);
+    L.total_words = L.stream_word + 4 * groups;
     L.limit_words = (((nk + 1 + 3) & ~3) + 4 * L.n_runs + 2 * n_dup + 3) & ~3;
-    L.total_words = L.weight_word + n_w;
     // (at least limit_words: the size that lpaici_kernelset_info reports and scratch limits count)
     ks->blob.assign(std::max(L.total_words, L.limit_words), 0);
-    float *wd = reinterpret_cast<float *>(ks->blob.data() + L.weight_word);
-    int at = 0;
+    int32_t *stream = &ks->blob[L.stream_word];
+    int at = 0;  // group
     for (int k = 0; k < nk; k++) {
-        ks->blob[2 * k] = ks->k_first_run[k];
-        ks->blob[2 * k + 1] = static_cast<int>(sizeof(float)) * at;
+        ks->blob[k] = 16 * at;
         int w = ks->k_first_weight[k];
         for (int r = ks->k_first_run[k]; r < ks->k_first_run[k] + ks->k_num_runs[k]; r++) {
             const int len = ks->run_len[r], head = len % 4;
-            int32_t *run = &ks->blob[L.run_word + 4 * r];
-            run[0] = ks->run_row[r];
-            run[1] = ks->run_col[r];
-            run[2] = head;
-            run[3] = len / 4;
-            for (int j = 0; j < head; j++) wd[at + j] = ks->run_w[w + j];
-            at += head ? 4 : 0;
-            for (int j = head; j < len; j++) wd[at++] = ks->run_w[w + j];
+            ks->blob[L.mask_word + (at >> 5)] |= static_cast<int32_t>(1u << (at & 31));
+            const int32_t desc[4] = {ks->run_row[r], ks->run_col[r], head, len / 4};
+            std::memcpy(stream + 4 * at, desc, sizeof(desc));
+            at++;
+            std::memcpy(stream + 4 * at, &ks->run_w[w], sizeof(float) * head);
+            at += head ? 1 : 0;
+            std::memcpy(stream + 4 * at, ks->run_w.data() + w + head, sizeof(float) * (len - head));
+            at += len / 4;
             w += len;
         }
     }
-    ks->blob[2 * nk] = L.n_runs;
-    ks->blob[2 * nk + 1] = static_cast<int>(sizeof(float)) * at;
+    ks->blob[nk] = 16 * at;
 
     return build_adjoint_blob(ks);
 }
@@ -311,8 +323,8 @@ void fill_tables(const lpaici_kernelset *ks, const float *var_or_null, float sig
     t->neg_zero = -0.0f;
     t->R = ks->radius;
     t->blob_words = ks->layout.total_words;
-    t->run_word = ks->layout.run_word;
-    t->weight_word = ks->layout.weight_word;
+    t->mask_word = ks->layout.mask_word;
+    t->stream_word = ks->layout.stream_word;
     t->limit_words = ks->layout.limit_words;
     const float s2 = sigma * sigma;
     for (int k = 0; k < nk; k++) {

@@ -28,12 +28,13 @@
 //   - weights are single floats, four taps per 16-byte load: the packed product takes the weight as one
 //     broadcast register, a {w, w} pair costs a second operand read and twice the shared memory;
 //   - a run of L taps is a head of L % 4 taps (one dispatch to straight-line code) followed by L / 4
-//     blocks of 4 taps over a sliding register window, with the four descriptor words ready to use;
+//     blocks of 4 taps over a sliding register window, with the four descriptor words ready to use; descriptor
+//     and weights lie in one stream, so one pointer walks a direction's runs and ends every loop;
 //   - shared memory is read by 32-bit shared addresses (ld.shared in PTX): generic pointers cost a third
 //     of the uniform instructions per run.
 // 4096^2, 16 x 7 symmetric kernels: 8.15 ms before (Q = 4, 64 x 96 tiles, 103 warp instructions per run of
-// a 256-pixel warp), 7.04 ms now (128 x 64 tiles, 142 per run of a 512-pixel warp); the packed arithmetic
-// alone would take 5.3 ms.  Per tile of 8,192 pixels and 16 warps: 32 cycles a tap (the packed arithmetic's
+// a 256-pixel warp), 6.84 ms now (128 x 64 tiles, 144 per run of a 512-pixel warp; with descriptors and weights
+// behind pointers of their own 7.04 ms); the packed arithmetic alone would take 5.3 ms.  Per tile of 8,192 pixels and 16 warps: 32 cycles a tap (the packed arithmetic's
 // own), about 45 a run and 150 an interval update.
 //
 // Arithmetic (bit-identical to src/v1_0_lpa_ici_2D_fused.cpp:803-930 for finite inputs):
@@ -122,6 +123,11 @@ __device__ __forceinline__ float4 lds4(unsigned a) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
+__device__ __forceinline__ unsigned lds_u1(unsigned a) {
+    unsigned v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ uint2 lds_u2(unsigned a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
@@ -182,18 +188,19 @@ __host__ __device__ inline size_t sweep_smem(int blob_words, int nk, int R) {
 }
 
 // The first H = L % 4 taps of a run of L: straight-line code that loads the H + Q - 1 window columns and
-// the H weights (one 16-byte group) and leaves the window of the next tap in win[0 .. Q - 2].
+// the H weights (one 16-byte group after the descriptor at `at`) and leaves the window of the next tap in
+// win[0 .. Q - 2] and `at` behind the head.
 template <int Q, int H, class Tap>
-__device__ __forceinline__ void run_head(float2 (&acc)[Q], float2 (&win)[Q], unsigned src, unsigned &wp, const Tap &tap) {
+__device__ __forceinline__ void run_head(float2 (&acc)[Q], float2 (&win)[Q], unsigned src, unsigned &at, const Tap &tap) {
     float2 t[H + Q - 1];
     float w[4] = {};
     if constexpr (H == 1) {
-        w[0] = lds1(wp);
+        w[0] = lds1(at + 16);
     } else if constexpr (H == 2) {
-        const float2 v = lds2(wp);
+        const float2 v = lds2(at + 16);
         w[0] = v.x, w[1] = v.y;
     } else if constexpr (H == 3) {
-        const float4 v = lds4(wp);
+        const float4 v = lds4(at + 16);
         w[0] = v.x, w[1] = v.y, w[2] = v.z;
     }
 #pragma unroll
@@ -204,7 +211,7 @@ __device__ __forceinline__ void run_head(float2 (&acc)[Q], float2 (&win)[Q], uns
         for (int m = 0; m < Q; m++) acc[m] = tap(acc[m], make_float2(w[j], w[j]), t[j + m]);
 #pragma unroll
     for (int i = 0; i < Q - 1; i++) win[i] = t[H + i];
-    if constexpr (H > 0) wp += 16;
+    at += H > 0 ? 32 : 16;
 }
 
 // Four taps; the window slots have been rotated by 4 * P taps (Q = 8 alternates P = 0, 1).  src: column
@@ -222,63 +229,75 @@ __device__ __forceinline__ void run_block(float2 (&acc)[Q], float2 (&win)[Q], un
 }
 
 // acc[m] = tap(acc[m], w_j, T[.][col + m + j]) for j < L, tap by tap in order, for the thread's Q pixel
-// pairs.  run: {byte offset of the run's first column from the lane's pixel, L % 4, 16 * (L / 4), byte
-// offset of column L % 4 + Q - 1}; wp advances over the run's weights.
+// pairs.  The run's descriptor is at `at`, its weights follow, the next run's descriptor follows them: {byte
+// offset of the run's first column from the lane's pixel, L % 4, address of the run's end, byte offset of
+// column L % 4 + Q - 1}.
 template <int Q, class Tap>
-__device__ __forceinline__ void conv_taps(float2 (&acc)[Q], unsigned lane_base, const int4 run, unsigned &wp, const Tap &tap) {
+__device__ __forceinline__ void conv_taps(float2 (&acc)[Q], unsigned lane_base, unsigned &at, const Tap &tap) {
     float2 win[Q];
+    const int4 run = lds_i4(at);
     unsigned src = lane_base + run.x;
+    const unsigned end = run.z;
     const int h = run.y;
     if (h < 2) {
         if (h == 0)
-            run_head<Q, 0>(acc, win, src, wp, tap);
+            run_head<Q, 0>(acc, win, src, at, tap);
         else
-            run_head<Q, 1>(acc, win, src, wp, tap);
+            run_head<Q, 1>(acc, win, src, at, tap);
     } else {
         if (h == 2)
-            run_head<Q, 2>(acc, win, src, wp, tap);
+            run_head<Q, 2>(acc, win, src, at, tap);
         else
-            run_head<Q, 3>(acc, win, src, wp, tap);
+            run_head<Q, 3>(acc, win, src, at, tap);
     }
-    int n = run.z;
-    if (n == 0) return;
+    if (at == end) return;
     src = lane_base + run.w;
 #pragma unroll 1
     while (true) {
-        run_block<Q, 0>(acc, win, src, wp, tap);
-        wp += 16;
-        n -= 16;
+        run_block<Q, 0>(acc, win, src, at, tap);
+        at += 16;
         if constexpr (Q == 8) {
-            if (n == 0) break;
-            run_block<Q, 1>(acc, win, src + 32, wp, tap);
-            wp += 16;
-            n -= 16;
+            if (at == end) break;
+            run_block<Q, 1>(acc, win, src + 32, at, tap);
+            at += 16;
         }
-        if (n == 0) break;
+        if (at == end) break;
         src += 8 * Q;
     }
 }
 
 // Copies the forward blob to shared memory and resolves it for this tile: kernel table entries become
-// shared addresses {first run, first weight}, runs {dy, dx0, L % 4, L / 4} become the byte offsets that
-// conv_taps reads.
+// shared addresses, run descriptors {dy, dx0, L % 4, L / 4} the offsets and addresses that conv_taps reads.
 template <int Q>
-__device__ __forceinline__ void stage_blob(int *dst, const int *__restrict__ src, int words, int run_word, int weight_word,
+__device__ __forceinline__ void stage_blob(int *dst, const int *__restrict__ src, int words, int mask_word, int stream_word,
                                            int pitch2) {
     const int4 *s = reinterpret_cast<const int4 *>(src);
     int4 *d = reinterpret_cast<int4 *>(dst);
-    const int r0 = run_word >> 2, r1 = weight_word >> 2;
-    const int runs = static_cast<int>(smem_addr(dst + run_word)), weights = static_cast<int>(smem_addr(dst + weight_word));
-#pragma unroll 4
-    for (int i = threadIdx.x; i < (words >> 2); i += blockDim.x) {
-        int4 v = __ldg(s + i);
-        if (i < r0) {
-            v = make_int4(runs + 16 * v.x, weights + v.y, runs + 16 * v.z, weights + v.w);
-        } else if (i < r1) {
-            const int o = 8 * (v.x * pitch2 + v.y);
-            v = make_int4(o, v.z, 16 * v.w, o + 8 * (v.z + Q - 1));
+    const int m0 = mask_word >> 2, s0 = stream_word >> 2;
+    const int stream = static_cast<int>(smem_addr(dst + stream_word));
+    constexpr int kAhead = 4;  // groups and mask words loaded before the first is used
+    const int n = words >> 2, step = blockDim.x;
+    for (int i0 = threadIdx.x; i0 < n; i0 += kAhead * step) {
+        int4 v[kAhead];
+        int m[kAhead];
+#pragma unroll
+        for (int e = 0; e < kAhead; e++) {
+            const int i = i0 + e * step, j = i - s0;
+            v[e] = i < n ? __ldg(s + i) : make_int4(0, 0, 0, 0);
+            m[e] = i < n && j >= 0 ? __ldg(src + mask_word + (j >> 5)) >> (j & 31) : 0;
         }
-        d[i] = v;
+#pragma unroll
+        for (int e = 0; e < kAhead; e++) {
+            const int i = i0 + e * step, j = i - s0;
+            int4 r = v[e];
+            if (i < m0) {
+                r = make_int4(stream + r.x, stream + r.y, stream + r.z, stream + r.w);
+            } else if (m[e] & 1) {
+                const int o = 8 * (r.x * pitch2 + r.y);
+                r = make_int4(o, r.z, stream + 16 * (j + 1 + (r.z > 0) + r.w), o + 8 * (r.z + Q - 1));
+            }
+            if (i < n) d[i] = r;
+        }
     }
 }
 
@@ -332,10 +351,9 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
                                                 unsigned thr_addr, const Tap &tap, float2 (&best)[Q],
                                                 unsigned (&sidx)[Q / 4]) {
     float lo[2 * Q], hi[2 * Q];
-    unsigned next = kernel_table + 8 * d * S;
+    unsigned next = kernel_table + 4 * d * S;
     unsigned thr_at = thr_addr + 4 * d * S;
-    const uint2 first = lds_u2(next);
-    unsigned rp = first.x, wp = first.y;
+    unsigned at = lds_u1(next);
 #pragma unroll
     for (int i = 0; i < Q / 4; i++) sidx[i] = 0;
 #pragma unroll 1
@@ -343,15 +361,12 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
         float2 acc[Q];
 #pragma unroll
         for (int m = 0; m < Q; m++) acc[m] = make_float2(0.0f, 0.0f);
-        next += 8;
-        const unsigned end = lds_u2(next).x;
-        if (rp != end) {
+        next += 4;
+        const unsigned end = lds_u1(next);
+        if (at != end) {
 #pragma unroll 1
-            do {
-                const int4 run = lds_i4(rp);
-                rp += 16;
-                conv_taps<Q>(acc, lane_base, run, wp, tap);
-            } while (rp != end);
+            do conv_taps<Q>(acc, lane_base, at, tap);
+            while (at != end);
         }
         const float thr = lds1(thr_at);
         thr_at += 4;
@@ -402,28 +417,42 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
 // them, in direction order, to the num and den of its share of the pixels -- the same additions in the same
 // order as DS = 1, so the results are equal bit for bit.  A tile then takes 1/DS of the time: images with
 // fewer pixels than the chip has room for (148 SMs x 8,192 pixels) are cut into smaller tiles (97 x 64: 257
-// us before, 37 us as 16 x 16 tiles of 8 groups; 512^2: 268 us before, 147 us as 64 x 32 tiles of 4).  It
-// costs halo and a barrier per round: at 4096^2 the tiles of 2, 4, 8 and 16 groups take 7.9, 8.0, 8.4 and
-// 9.0 ms against 7.04 ms.
+// us before, 36 us as 16 x 16 tiles of 8 groups; 512^2: 268 us before, 135 us as 64 x 32 tiles of 4).  It
+// costs halo and a barrier per round: at 4096^2 the tiles of 2, 4, 8 and 16 groups take 7.3, 7.3, 7.8 and
+// 8.3 ms against 6.84 ms.
 template <int WX, int WY, int Q, int DS, bool Fused>
 __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0, int D, int S, const TileGeom &g,
                                            const int *s_blob, const float *s_tab, const float2 *s_tile, float *s_xch,
                                            float neg_zero) {
     using Shape = TileShape<WX, WY, Q, DS>;
-    const int group = DS == 1 ? 0 : static_cast<int>(threadIdx.x) / Shape::kRegion;
-    const int rt = threadIdx.x - group * Shape::kRegion;  // thread of the region
-    const int warp = rt >> 5, lane = rt & 31;
-    const int a = Q == 4 ? (lane >> 2) : (lane & 7), b = Q == 4 ? (lane & 3) : (lane >> 3);
-    const int ty = (warp / WX) * 8 + a, tx = (warp % WX) * 4 * Q + Q * b;
+    // first output row and column of a thread's pixels (see the thread mapping above), from its index: formed
+    // again where results are written (`again` is opaque), so that the sweep does not carry them
+    auto place = [&](int t, int *oy, int *ox) {
+        const int rt = DS == 1 ? t : t % Shape::kRegion, warp = rt >> 5, lane = rt & 31;
+        const int a = Q == 4 ? (lane >> 2) : (lane & 7), b = Q == 4 ? (lane & 3) : (lane >> 3);
+        *oy = y0 + (warp / WX) * 8 + a;
+        *ox = x0 + (warp % WX) * 4 * Q + Q * b;
+    };
+    auto again = [] {
+        int t;
+        asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+        return t;
+    };
+    // the group is the same in every lane of a warp: reduced, the compiler knows it warp-uniform, so the run
+    // loops branch without reconvergence bookkeeping
+    const int group = DS == 1 ? 0 : static_cast<int>(__reduce_max_sync(0xffffffffu, threadIdx.x / Shape::kRegion));
     const int nk = D * S;
-    const int oy = y0 + ty, ox = x0 + tx;
-    unsigned valid = 0;
+    unsigned valid = 0, lane_base;
+    {
+        int oy, ox;
+        place(threadIdx.x, &oy, &ox);
 #pragma unroll
-    for (int i = 0; i < 2 * Q; i++)
-        if (oy + g.half * (i & 1) < img.rows_out && ox + (i >> 1) < img.W) valid |= 1u << i;
+        for (int i = 0; i < 2 * Q; i++)
+            if (oy + g.half * (i & 1) < img.rows_out && ox + (i >> 1) < img.W) valid |= 1u << i;
+        lane_base = smem_addr(s_tile + (oy - y0 + g.R) * g.pitch2 + ox - x0 + g.R);
+    }
     const bool work = __any_sync(0xffffffffu, valid != 0);  // a warp outside the image only joins the barriers
     if (DS == 1 && !work) return;
-    const unsigned lane_base = smem_addr(s_tile + (ty + g.R) * g.pitch2 + tx + g.R);
     const unsigned kernel_table = smem_addr(s_blob);
     const unsigned thr_addr = smem_addr(s_tab + nk), rvar_addr = smem_addr(s_tab + 2 * nk);
     // opaque, so that the compiler keeps it in a register instead of reading it again in every run
@@ -463,7 +492,7 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
                     num[m] = add2(num[m], e);
                     den[m] = add2(den[m], r);
                 } else {
-                    float *x = s_xch + (group * 2 * Q + 2 * m) * Shape::kRegion + rt;
+                    float *x = s_xch + (group * 2 * Q + 2 * m) * Shape::kRegion + threadIdx.x % Shape::kRegion;
                     x[0] = e.x;
                     x[Shape::kRegion] = e.y;
                     x += DS * 2 * Q * Shape::kRegion;
@@ -472,17 +501,30 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
                 }
             }
             if (img.smap) {
+                int oy, ox;
+                place(again(), &oy, &ox);
 #pragma unroll
-                for (int i = 0; i < 2 * Q; i++)
-                    if (valid & (1u << i))
-                        img.smap[(static_cast<size_t>(d) * img.rows_out + oy + g.half * (i & 1)) * img.W + ox + (i >> 1)] =
-                            static_cast<uint8_t>((sidx[i / 8] >> (4 * (i % 8))) & 15);
+                for (int h = 0; h < 2; h++) {
+                    uint8_t *row = img.smap + (static_cast<size_t>(d) * img.rows_out + oy + g.half * h) * img.W + ox;
+                    constexpr unsigned kRow = Q == 8 ? 0x5555u : 0x55u;  // this half's pixels in `valid`
+                    if (((valid >> h) & kRow) == kRow && (reinterpret_cast<size_t>(row) & 3) == 0) {
+                        // the index words hold four pixels of either row as bytes of 4 + 4 bits
+#pragma unroll
+                        for (int w = 0; w < Q / 4; w++)
+                            reinterpret_cast<unsigned *>(row)[w] = (sidx[w] >> (4 * h)) & 0x0f0f0f0fu;
+                    } else {
+#pragma unroll
+                        for (int m = 0; m < Q; m++)
+                            if (valid & (1u << (2 * m + h)))
+                                row[m] = static_cast<uint8_t>((sidx[m / 4] >> (8 * (m % 4) + 4 * h)) & 15);
+                    }
+                }
             }
         }
         if constexpr (DS > 1) {
             __syncthreads();
             if (group * kOwn < 2 * Q && work) {
-                const float *x = s_xch + group * kOwn * Shape::kRegion + rt;
+                const float *x = s_xch + group * kOwn * Shape::kRegion + threadIdx.x % Shape::kRegion;
 #pragma unroll
                 for (int e = 0; e < DS; e++) {
                     if (d0 + e >= D) break;
@@ -497,6 +539,8 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
         }
     }
     if (DS > 1 && group * kOwn >= 2 * Q) return;
+    int oy, ox;
+    place(again(), &oy, &ox);
 #pragma unroll
     for (int j = 0; j < kOwn; j++) {
         const int i = DS == 1 ? j : group * kOwn + j;
