@@ -22,7 +22,8 @@
 //
 // Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
 // zero (its runs in order), the chunks' sums are added in order, and group 1's total is added to group 0's.
-// A tile is gathered by one CTA or by a cluster of kGatherChunks or half as many CTAs that share the chunks
+// A tile is gathered by one CTA or by a cluster of kGatherChunks or half as many CTAs (the tiles after the last
+// whole wave, gather_plan) that share the chunks
 // and add the same sums in the same order through distributed shared memory, so the gradient does not depend on
 // how many CTAs a tile gets (single images, plans and kept states agree bit for bit).
 // No counterpart in the reference.
@@ -87,6 +88,8 @@ struct GatherArgs {
     int block_bytes;       // shared memory for one kernel's block
     int pitch, plane;      // field geometry (AdjointLayout)
     int cluster;           // CTAs per tile: 1, kGatherChunks / 2 or kGatherChunks
+    int first_tile;        // this launch's tiles start here
+    int rest_follows;      // a launch over the tiles after this one's follows
     float rvar[kMaxKernels];  // 1 / v_k of the one image
     // per kernel: the field cells its correlation reads, rows [x, y), columns [z, w); per direction: the
     // union over its scales (the cells its field needs)
@@ -348,8 +351,10 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     int *s_flag = reinterpret_cast<int *>(base + lay.flag);
     float *s_f = reinterpret_cast<float *>(base + lay.field);  // the field of the current direction
     uint8_t *s_s = reinterpret_cast<uint8_t *>(base + lay.smap);  // s*(d, .) on the halo'd tile
+    // the rest's CTAs may start once every CTA of this launch has (they depend on nothing of it)
+    if (a.rest_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int rank = a.cluster > 1 ? static_cast<int>(blockIdx.x % a.cluster) : 0;
-    int tile = blockIdx.x / a.cluster;
+    int tile = a.first_tile + blockIdx.x / a.cluster;
     GatherImage im;
     if (a.images) {
         const int2 it = a.items[tile];
@@ -515,6 +520,8 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
         }
     }
     cluster_barrier();  // a CTA's shared memory stays until every other one has read it
+    // what follows in the stream follows the launch before this one too
+    if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // u = g * (1 / den) written over 1 / den, once per image between the two passes of the recomputing
@@ -551,21 +558,45 @@ const void *gather_fn(const AdjointLayout &L) {
 
 int gather_threads(const AdjointLayout &L) { return kGatherGroups * 32 * L.wx * L.wy; }
 
-int gather_launch(const AdjointLayout &L, const GatherArgs &ga, long tiles, size_t smem, cudaStream_t stream) {
+// How a launch's tiles are gathered: the first n_single by one CTA each, the others by clusters of `cluster`.
+struct GatherPlan {
+    long tiles = 0, n_single = 0;
+    int cluster = 1;
+};
+
+int gather_launch(const AdjointLayout &L, const GatherArgs &args, const GatherPlan &plan, size_t smem, cudaStream_t stream) {
+    GatherArgs ga = args;
+    void *params[] = {&ga};
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(tiles * ga.cluster));
     cfg.blockDim = dim3(gather_threads(L));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(ga.cluster);
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = ga.cluster > 1 ? 1 : 0;
-    void *params[] = {const_cast<GatherArgs *>(&ga)};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, gather_fn(L), params);
-    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "adjoint gather launch");
+    const long rest = plan.tiles - plan.n_single;
+    if (plan.n_single > 0) {
+        ga.cluster = 1;
+        ga.first_tile = 0;
+        ga.rest_follows = rest > 0 ? 1 : 0;
+        cfg.gridDim = dim3(static_cast<unsigned>(plan.n_single));
+        const cudaError_t e = cudaLaunchKernelExC(&cfg, gather_fn(L), params);
+        if (e != cudaSuccess) return cuda_error(e, "adjoint gather launch");
+    }
+    if (rest > 0) {
+        ga.cluster = plan.cluster;
+        ga.first_tile = static_cast<int>(plan.n_single);
+        ga.rest_follows = 0;
+        cfg.gridDim = dim3(static_cast<unsigned>(rest * plan.cluster));
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(plan.cluster);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = plan.n_single > 0 ? 2 : 1;
+        const cudaError_t e = cudaLaunchKernelExC(&cfg, gather_fn(L), params);
+        if (e != cudaSuccess) return cuda_error(e, "adjoint gather launch (clusters)");
+    }
+    return LPAICI_OK;
 }
 
 // Fills the geometry and the per-kernel rectangles of the in-place masking; smem receives the dynamic shared
@@ -586,7 +617,6 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
     ga->block_bytes = L.block_bytes;
     ga->pitch = L.pitch;
     ga->plane = L.plane;
-    ga->cluster = 1;
     const GatherSmem m = GatherSmem::make(nk, L.block_bytes, L.plane, 32 * L.wx * L.wy);
     *smem = m.total;
     if (*smem > static_cast<size_t>(max_optin))
@@ -618,27 +648,33 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
     return LPAICI_OK;
 }
 
-// CTAs per tile: one when the tiles fill the SMs, else as many as shorten the launch.  A tile's time goes
-// with its share of the directions, plus 1.8 % of it for the cluster's exchange and staging; a cluster needs
-// its CTAs free at once in one GPC, which leaves about three clusters fewer than SMs / CTAs running together.
+// CTAs per tile: one for whole waves of tiles, for the rest as many as shorten the launch.  A tile's time goes
+// with its share of the directions, plus about 8.5 us for the cluster's exchange and staging; a cluster needs its
+// CTAs free at once in one GPC: 33 clusters of four or 15 of eight run together on 148 SMs.  The tile's time is
+// fitted to the symmetric (475 us), tapered (706 us) and 8 x 4 (74 us) sets.
 // Measured (16 x 7 symmetric set, us for 1 / 4 / 8 CTAs per tile): 15 tiles 473 / 129 / 70, 32 tiles
 // 475 / 130 / 201, 40 tiles 475 / 254 / 203, 128 tiles 475 / 505 / 599, 160 tiles 947 / 629 / 732.
-int gather_cluster(const lpaici_kernelset *ks, GatherArgs *ga, long tiles, size_t smem) {
+int gather_plan(const lpaici_kernelset *ks, long tiles, size_t smem, GatherPlan *plan) {
     const AdjointLayout &L = ks->adj_layout;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    *plan = GatherPlan{tiles, tiles, 1};
+    const double tile_us = ks->D * (1.8 + 1.27 * ks->S) + 0.0354 * L.taps + 0.046 * L.units;
     double best = static_cast<double>((tiles + sms - 1) / sms);
     const GatherSmem m = GatherSmem::make(ks->D * ks->S, L.block_bytes, L.plane, 32 * L.wx * L.wy);
     for (const int c : {kGatherChunks / 2, kGatherChunks}) {
         // the second chunk's sums of half as many CTAs lie over everything before the first one's
         if (c < kGatherChunks && m.sums < m.total - m.sums) continue;
         if (ks->D < c || tiles * c > 0x7fffffffL) continue;
-        const long slots = std::max(1, sms / c - 3);
-        const double t = (1.0 / c + 0.018) * static_cast<double>((tiles + slots - 1) / slots);
-        if (t < best) {
-            best = t;
-            ga->cluster = c;
+        const long slots = std::max(1, (sms - 4 - 3 * c) / c);
+        for (const long waves : {0L, tiles / sms}) {
+            const long rest = tiles - waves * sms;
+            const double t = waves + (1.0 / c + 8.5 / tile_us) * static_cast<double>((rest + slots - 1) / slots);
+            if (rest > 0 && t < best) {
+                best = t;
+                *plan = GatherPlan{tiles, waves * sms, c};
+            }
         }
     }
     const cudaError_t e = cudaFuncSetAttribute(gather_fn(L), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -703,14 +739,15 @@ int gather_pass(const lpaici_kernelset *ks, const int *adj_blob, const uint8_t *
     int tiles_x = 0;
     const long tiles = gather_tiles(ks->adj_layout, width, height, &tiles_x);
     if (tiles > 0x7fffffffL) return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", width, height);
-    rc = gather_cluster(ks, &ga, tiles, smem);
+    GatherPlan plan;
+    rc = gather_plan(ks, tiles, smem, &plan);
     if (rc != LPAICI_OK) return rc;
     KernelTables tab;
     fill_tables(ks, nullptr, sigma, 1.0f, &tab);
     ga.single = GatherImage{d_grad_out, smap, rden, d_grad_in, nullptr, gout_pitch, gin_pitch, width, height, tiles_x,
                             u_ready ? 1 : 0};
     for (int k = 0; k < ks->D * ks->S; k++) ga.rvar[k] = 1.0f / tab.var[k];
-    return gather_launch(ks->adj_layout, ga, tiles, smem, stream);
+    return gather_launch(ks->adj_layout, ga, plan, smem, stream);
 }
 
 namespace {
@@ -827,7 +864,7 @@ struct lpaici_backward_batch {
     GatherArgs ga{};
     size_t smem = 0;
     AdjointLayout layout;
-    long tiles = 0;
+    GatherPlan plan;
     int n = 0, max_h = 0;  // images; the tallest one's rows (the u launch)
     bool use_graph = false;
     cudaGraph_t graph = nullptr;
@@ -841,7 +878,7 @@ int backward_batch_enqueue(lpaici_backward_batch *b, cudaStream_t stream) {
     if (rc != LPAICI_OK) return rc;
     rc = u_launch(b->ga.images, GatherImage{}, b->n, b->max_h, stream);
     if (rc != LPAICI_OK) return rc;
-    return gather_launch(b->layout, b->ga, b->tiles, b->smem, stream);
+    return gather_launch(b->layout, b->ga, b->plan, b->smem, stream);
 }
 
 void backward_batch_free(lpaici_backward_batch *b) {
@@ -946,8 +983,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
     }
     b->ga.images = reinterpret_cast<const GatherImage *>(base + desc_off);
     b->ga.items = reinterpret_cast<const int2 *>(base + item_off);
-    b->tiles = total_tiles;
-    rc = gather_cluster(ks, &b->ga, total_tiles, b->smem);
+    rc = gather_plan(ks, total_tiles, b->smem, &b->plan);
     if (rc != LPAICI_OK) {
         backward_batch_free(b);
         return rc;

@@ -46,6 +46,7 @@ struct AdjointLayout {
     int wx = 0, wy = 0;       // warps of one group across and down a tile
     int pitch = 0, plane = 0; // floats of a field row and of a row plane
     int block_bytes = 0;      // the largest block
+    int units = 0, taps = 0;  // of all kernels (weight pairs)
     size_t limit_bytes = 0;   // shared memory the support limit counts (gather_setup)
     std::vector<int> box;     // per kernel: first and last row, first and last column of its taps (empty: 0, -1)
 };

@@ -150,6 +150,8 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         }
         const int bytes = static_cast<int>(8 * units[k].size() + 4 * pairs[k].size());
         L.block_bytes = std::max(L.block_bytes, (bytes + 15) & ~15);
+        L.units += static_cast<int>(units[k].size());
+        L.taps += static_cast<int>(pairs[k].size() / 2);
     }
     constexpr size_t kSharedPerCta = 232448;  // sm_100a
     for (const int wide : {1, 0}) {
