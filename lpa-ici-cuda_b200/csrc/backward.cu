@@ -325,15 +325,10 @@ __device__ __forceinline__ void mask_field(float *s_f, const uint8_t *s_s, const
                    below, nthreads);
 }
 
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // The float2 at shared address a of CTA `rank` of the cluster.
 __device__ __forceinline__ float2 cluster_lds2(unsigned a, unsigned rank) {
-    unsigned remote;
     float2 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(a), "r"(rank));
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr(a, rank)) : "memory");
     return v;
 }
 

@@ -51,12 +51,18 @@ static int groups_of(int c) {
 #undef LPAICI_GROUPS_CASE
 }
 
-static float estimated_tile_ms(const lpaici_kernelset *ks, int c) {
-    const int nk = ks->D * ks->S, ds = groups_of(c);
+// The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; 97 x 64 takes 22.6 us with the
+// symmetric set and 28.7 us with the tapered one, 128 x 128 28.7 and 36.9 us, of which a launch is 3.6 us).
+static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{10.0f, 1.05f}, {14.0f, 1.30f}};
+
+static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int ds) {
+    const int nk = ks->D * ks->S;
     const float work = static_cast<float>(ks->run_w.size()) + 1.4f * ks->layout.n_runs + 5.0f * nk;
     const float rounded = static_cast<float>((ks->D + ds - 1) / ds * ds) / ks->D;
-    return 1e-3f * kTileCost[c].base_us + 1e-6f * kTileCost[c].ns_per_work * work * rounded;
+    return 1e-3f * cost.base_us + 1e-6f * cost.ns_per_work * work * rounded;
 }
+
+static float estimated_tile_ms(const lpaici_kernelset *ks, int c) { return estimated_ms(ks, kTileCost[c], groups_of(c)); }
 
 // CTAs per SM of configuration c for ks on device dev (cached; 0 when it does not fit).
 static int cached_bps(const lpaici_kernelset *ks, int dev, int c, int max_optin) {
@@ -98,33 +104,40 @@ static double mixed_makespan(long n_big, double big_t, long n_small, double t, i
 
 // What a plan is chosen with: the tile times of a kernel set on the current device.
 struct PlanCosts {
-    int sms = 0;
-    bool forced = false;
+    int sms = 0, max_smem = 0;
+    bool forced = false, tuned = false;
     int forced_config = 0;
     float tile_ms[LPAICI_NUM_TILE_CONFIGS];  // <= 0: does not fit
     int bps[LPAICI_NUM_TILE_CONFIGS];
 };
 
 static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
-    int dev = 0, max_optin = 0;
+    int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    std::vector<float> tuned;
+    bool known = false;  // CTAs per SM of every configuration
     {
         std::lock_guard<std::mutex> lock(ks->mu);
         const bool have = dev < static_cast<int>(ks->tuned_config.size()) && ks->tuned_config[dev] >= 0;
-        const bool timed = dev < static_cast<int>(ks->tuned_tile_ms.size()) && !ks->tuned_tile_ms[dev].empty();
-        if (have && !timed) {  // forced by lpaici_set_tile_config
+        pc->tuned = dev < static_cast<int>(ks->tuned_tile_ms.size()) && !ks->tuned_tile_ms[dev].empty();
+        if (have && !pc->tuned) {  // forced by lpaici_set_tile_config
             pc->forced = true;
             pc->forced_config = ks->tuned_config[dev];
             return true;
         }
-        if (timed) tuned = ks->tuned_tile_ms[dev];
+        if (pc->tuned) std::copy_n(ks->tuned_tile_ms[dev].begin(), LPAICI_NUM_TILE_CONFIGS, pc->tile_ms);
+        if (dev < static_cast<int>(ks->blocks_per_sm.size()) && !ks->blocks_per_sm[dev].empty()) {
+            std::copy_n(ks->blocks_per_sm[dev].begin(), LPAICI_NUM_TILE_CONFIGS, pc->bps);
+            known = std::all_of(pc->bps, pc->bps + LPAICI_NUM_TILE_CONFIGS, [](int b) { return b >= 0; });
+        }
     }
     cudaDeviceGetAttribute(&pc->sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&pc->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        pc->bps[c] = cached_bps(ks, dev, c, max_optin);
-        pc->tile_ms[c] = pc->bps[c] <= 0 ? 0.0f : tuned.empty() ? estimated_tile_ms(ks, c) : tuned[c];
+        if (!known) pc->bps[c] = cached_bps(ks, dev, c, pc->max_smem);
+        if (pc->bps[c] <= 0)
+            pc->tile_ms[c] = 0.0f;
+        else if (!pc->tuned)
+            pc->tile_ms[c] = estimated_tile_ms(ks, c);
     }
     return true;
 }
@@ -164,6 +177,22 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
         plan.config = default_config(ks);
         return plan;
     }
+    // one image of a few tiles: clusters, as long as they all run at once
+    if (by_rows && n == 1 && !pc.tuned) {
+        for (int c = 0; c < LPAICI_NUM_CLUSTERS; c++) {
+            int tw = 1, th = 1, ctas = 1, groups = 1;
+            size_t smem = 0;
+            cluster_config(c, ks->radius, ks->layout.total_words, ks->D * ks->S, &tw, &th, &ctas, &groups, &smem);
+            const long tiles = static_cast<long>((widths[0] + tw - 1) / tw) * ((rows[0] + th - 1) / th);
+            const long slots = (pc.sms - 4 - 3 * ctas) / ctas;  // a cluster's CTAs run in one GPC
+            const double est = estimated_ms(ks, kClusterCost[c], groups);
+            if (tiles <= slots && smem <= static_cast<size_t>(pc.max_smem) && est < best_ms) {
+                best_ms = est;
+                plan = TilePlan{};
+                plan.cluster = c;
+            }
+        }
+    }
     // a mix: whole waves of big tiles, or one wave fewer, the rest in small ones
     for (const auto &mix : kMixes) {
         const int a = mix[0], b = mix[1];
@@ -183,7 +212,7 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
             const double est = mixed_makespan(big, pc.tile_ms[a], small, pc.tile_ms[b], pc.sms);
             if (est < best_ms) {
                 best_ms = est;
-                plan = TilePlan{a, b, big_rows};
+                plan = TilePlan{a, b, big_rows, -1};
             }
         };
         const long row = by_rows ? static_cast<long>(widths[0] / aw) * n : 1;  // big tiles of one tile row
@@ -196,6 +225,7 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
 }
 
 TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n) {
+    if (n == 1) return choose_plan(ks, &width, &rows, 1, true);
     const std::vector<int> w(n, width), h(n, rows);
     return choose_plan(ks, w.data(), h.data(), n, true);
 }
@@ -488,7 +518,7 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
             rc = cuda_error(e, "lpaici_denoise_host: upload");
             break;
         }
-        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.rest, (r1 - r0) / big_h} : TilePlan{low_config, -1, 0};
+        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.rest, (r1 - r0) / big_h, -1} : TilePlan{low_config, -1, 0, -1};
         rc = forward_common(ks, b.in, width, width, height, r0, r1 - r0, b.out + static_cast<size_t>(r0) * width, width,
                             nullptr, sigma, gamma, nullptr, sc, &band);
         if (rc != LPAICI_OK) break;
@@ -625,7 +655,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
     int best = -1;
     std::vector<float> config_ms(LPAICI_NUM_TILE_CONFIGS, -1.0f);
     for (int c = 0; rc == LPAICI_OK && c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        int crc = launch_forward(img, tab, TilePlan{c, -1, 0}, stream);  // warm-up
+        int crc = launch_forward(img, tab, TilePlan{c, -1, 0, -1}, stream);  // warm-up
         if (crc != LPAICI_OK) {
             if (ms_out) ms_out[c] = -1.0f;
             if (crc == LPAICI_ERR_UNSUPPORTED) continue;  // this tile does not fit for this kernel set
@@ -633,7 +663,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
             break;
         }
         cudaEventRecord(e0, stream);
-        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(img, tab, TilePlan{c, -1, 0}, stream);
+        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(img, tab, TilePlan{c, -1, 0, -1}, stream);
         cudaEventRecord(e1, stream);
         e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) {

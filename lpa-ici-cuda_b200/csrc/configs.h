@@ -31,6 +31,14 @@
     X(5, 1, 1, 8, 16)
 #define LPAICI_TILE_MIXES {{0, 4}, {0, 5}, {1, 5}, {3, 5}}
 
+// Tiles that the C CTAs of a cluster share (images of a few tiles; lpaici_forward_cluster_kernel): each CTA has
+// DS direction groups.
+// X(index, WX, WY, Q, DS, C)
+#define LPAICI_CLUSTERS(X) \
+    X(0, 1, 1, 4, 4, 4)    \
+    X(1, 1, 1, 8, 4, 4)
+#define LPAICI_NUM_CLUSTERS 2
+
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.
 #define LPAICI_TILE_PREFERENCE {0, 8, 1, 3, 2, 4, 9, 5, 10, 6, 7}

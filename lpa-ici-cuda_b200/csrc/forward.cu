@@ -114,7 +114,56 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// An image of a few tiles: C CTAs of a cluster share each tile's directions, as the groups of a CTA do.  Each
+// stages only the runs of its directions if one round covers them all.  97 x 64, 16 x 7 symmetric set: 36.9 us
+// with one CTA per 16 x 16 tile, 22.6 us with four.
+template <int WX, int WY, int Q, int DS, int C, bool Fused>
+__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
+    lpaici_forward_cluster_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
+    extern __shared__ __align__(16) int smem[];
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const int nk = tab.D * tab.S, tile = blockIdx.x / C, rank = blockIdx.x % C;
+    const int across = (img.W + Shape::kTileW - 1) / Shape::kTileW;
+    const int x0 = (tile % across) * Shape::kTileW, y0 = (tile / across) * Shape::kTileH;
+    const SweepCta<WX, WY, Q, DS> cta(smem, tab.blob_words, nk, tab.R);
+    load_tile(cta.tile, img, x0, y0, cta.g);
+    int from = 0, to = 1 << 30;
+    if (tab.D <= DS * C) {
+        from = __ldg(tab.blob + min(tab.D, rank * DS) * tab.S);
+        to = __ldg(tab.blob + min(tab.D, (rank + 1) * DS) * tab.S);
+    }
+    stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.mask_word, tab.stream_word, cta.g.pitch2, from, to);
+    stage_tables(cta.tab, tab.var, tab.thr, nk);
+    tile_wait();
+    __syncthreads();
+    sweep_tile<WX, WY, Q, DS, Fused, C>(img, x0, y0, tab.D, tab.S, cta.g, cta.blob, cta.tab, cta.tile, cta.xch,
+                                        tab.neg_zero);
+}
+
 namespace {
+
+template <int WX, int WY, int Q, int DS, int C, bool Fused>
+int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t stream) {
+    using Shape = TileShape<WX, WY, Q, DS>;
+    const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
+    auto kern = lpaici_forward_cluster_kernel<WX, WY, Q, DS, C, Fused>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, clusters)");
+    const int tiles = ((img.W + Shape::kTileW - 1) / Shape::kTileW) * ((img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = C;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles) * C);
+    cfg.blockDim = dim3(Shape::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, img, tab);
+    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "forward launch (clusters)");
+}
 
 // across x down tiles from the image's origin (0: as many as cover it)
 template <int WX, int WY, int Q, int DS>
@@ -290,6 +339,31 @@ static int launch_rest_config(const ImageArgs &img, const KernelTables &tab, con
 #undef LPAICI_REST_CASE
 }
 
+static int launch_cluster_config(const ImageArgs &img, const KernelTables &tab, int index, bool fused, cudaStream_t stream) {
+#define LPAICI_CLUSTER_CASE(idx, WX, WY, Q, DS, C)                                        \
+    case idx:                                                                             \
+        return fused ? launch_cluster<WX, WY, Q, DS, C, true>(img, tab, stream)           \
+                     : launch_cluster<WX, WY, Q, DS, C, false>(img, tab, stream);
+    switch (index) {
+        LPAICI_CLUSTERS(LPAICI_CLUSTER_CASE)
+        default: return set_error(LPAICI_ERR_INVALID_ARG, "cluster configuration %d out of range", index);
+    }
+#undef LPAICI_CLUSTER_CASE
+}
+
+void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, int *tile_h, int *ctas, int *groups, size_t *smem) {
+#define LPAICI_CLUSTER_CASE(idx, WX, WY, Q, DS, C)                                 \
+    case idx:                                                                      \
+        *tile_w = 4 * (Q) * (WX);                                                  \
+        *tile_h = 16 * (WY);                                                       \
+        *ctas = C;                                                                 \
+        *groups = (DS) * (C);                                                      \
+        *smem = sweep_smem<TileShape<WX, WY, Q, DS>, Q>(blob_words, nk, radius);   \
+        return;
+    switch (index) { LPAICI_CLUSTERS(LPAICI_CLUSTER_CASE) }
+#undef LPAICI_CLUSTER_CASE
+}
+
 // The strips of a plan's mix, for images of img's size.
 static MixGrid mix_grid(const ImageArgs &img, const TilePlan &plan, int n, int *across) {
     int tw = 1, th = 1;
@@ -326,6 +400,7 @@ int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan
                          kMaxScales);
     int rc = check_forward_limit(tab);
     if (rc != LPAICI_OK) return rc;
+    if (plan.cluster >= 0) return launch_cluster_config(img, tab, plan.cluster, fused, stream);
     if (plan.rest < 0) return launch_config(img, tab, plan.config, 0, 0, fused, stream);
     int across = 0;
     const MixGrid g = mix_grid(img, plan, 1, &across);

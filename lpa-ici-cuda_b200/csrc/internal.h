@@ -80,6 +80,7 @@ struct KernelTables {
 struct TilePlan {
     int config = 0;
     int rest = -1, big_rows = 0;
+    int cluster = -1;  // >= 0: tiles shared by clusters, entry of LPAICI_CLUSTERS (one image, instead of config)
 };
 
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
@@ -166,6 +167,8 @@ TilePlan plan_for_images(const lpaici_kernelset *ks, const int *widths, const in
 int check_forward_limit(const KernelTables &tab);
 // CTAs of the forward kernel of `config` that fit on one SM with `smem` bytes of shared memory.
 int config_blocks_per_sm(int config, size_t smem);
+// Tile, CTAs, direction groups (of all CTAs) and shared memory per CTA of entry `index` of LPAICI_CLUSTERS.
+void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, int *tile_h, int *ctas, int *groups, size_t *smem);
 // Tile width and height of a configuration.
 void config_tile(int config, int *tile_w, int *tile_h);
 // One image of a batch plan (batched.cu): out may be null (no estimate), smap and rden optional.

@@ -144,6 +144,22 @@ __device__ __forceinline__ void copy_or_zero(unsigned dst, const float *src, boo
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 
+// Every thread of the cluster's CTAs; shared memory written before it is visible to the others after it.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Shared address a as CTA `rank` of the cluster has it, and a load from there.
+__device__ __forceinline__ unsigned cluster_addr(unsigned a, unsigned rank) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(a), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ float cluster_lds1(unsigned remote) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
 // Smallest odd pitch (in float2) >= need.
 __host__ __device__ inline int tile_pitch2(int need) { return need | 1; }
 
@@ -268,27 +284,28 @@ __device__ __forceinline__ void conv_taps(float2 (&acc)[Q], unsigned lane_base, 
 
 // Copies the forward blob to shared memory and resolves it for this tile: kernel table entries become
 // shared addresses, run descriptors {dy, dx0, L % 4, L / 4} the offsets and addresses that conv_taps reads.
+// Only the stream's bytes [from, to) are copied (a CTA that sweeps some directions).
 template <int Q>
 __device__ __forceinline__ void stage_blob(int *dst, const int *__restrict__ src, int words, int mask_word, int stream_word,
-                                           int pitch2) {
+                                           int pitch2, int from = 0, int to = 1 << 30) {
     const int4 *s = reinterpret_cast<const int4 *>(src);
     int4 *d = reinterpret_cast<int4 *>(dst);
     const int m0 = mask_word >> 2, s0 = stream_word >> 2;
     const int stream = static_cast<int>(smem_addr(dst + stream_word));
     constexpr int kAhead = 4;  // groups and mask words loaded before the first is used
-    const int n = words >> 2, step = blockDim.x;
-    for (int i0 = threadIdx.x; i0 < n; i0 += kAhead * step) {
+    const int n = min(words, stream_word + (to >> 2)) >> 2, step = blockDim.x, skip = from >> 4;
+    for (int i0 = threadIdx.x; i0 < n - skip; i0 += kAhead * step) {
         int4 v[kAhead];
         int m[kAhead];
 #pragma unroll
         for (int e = 0; e < kAhead; e++) {
-            const int i = i0 + e * step, j = i - s0;
+            const int i = i0 + e * step + (i0 + e * step >= s0 ? skip : 0), j = i - s0;
             v[e] = i < n ? __ldg(s + i) : make_int4(0, 0, 0, 0);
             m[e] = i < n && j >= 0 ? __ldg(src + mask_word + (j >> 5)) >> (j & 31) : 0;
         }
 #pragma unroll
         for (int e = 0; e < kAhead; e++) {
-            const int i = i0 + e * step, j = i - s0;
+            const int i = i0 + e * step + (i0 + e * step >= s0 ? skip : 0), j = i - s0;
             int4 r = v[e];
             if (i < m0) {
                 r = make_int4(stream + r.x, stream + r.y, stream + r.z, stream + r.w);
@@ -420,11 +437,18 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
 // us before, 36 us as 16 x 16 tiles of 8 groups; 512^2: 268 us before, 135 us as 64 x 32 tiles of 4).  It
 // costs halo and a barrier per round: at 4096^2 the tiles of 2, 4, 8 and 16 groups take 7.3, 7.3, 7.8 and
 // 8.3 ms against 6.84 ms.
-template <int WX, int WY, int Q, int DS, bool Fused>
+//
+// C > 1: the CTAs of a cluster share the tile in the same way, CTA `rank` with the directions
+// round * DS * C + rank * DS + group; the estimates meet through distributed shared memory.
+template <int WX, int WY, int Q, int DS, bool Fused, int C = 1>
 __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0, int D, int S, const TileGeom &g,
                                            const int *s_blob, const float *s_tab, const float2 *s_tile, float *s_xch,
                                            float neg_zero) {
     using Shape = TileShape<WX, WY, Q, DS>;
+    static_assert(C == 1 || DS > 1, "a cluster's CTAs have the exchange of direction groups");
+    constexpr int kGroups = DS * C;
+    unsigned rank = 0;
+    if constexpr (C > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     // first output row and column of a thread's pixels (see the thread mapping above), from its index: formed
     // again where results are written (`again` is opaque), so that the sweep does not carry them
     auto place = [&](int t, int *oy, int *ox) {
@@ -460,7 +484,8 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
     const float2 nz = make_float2(neg_zero, neg_zero);
 
     // the pixels whose num and den this thread sums: all 2Q (DS = 1), else kOwn of them
-    constexpr int kOwn = DS == 1 ? 2 * Q : (2 * Q >= DS ? 2 * Q / DS : 1);
+    constexpr int kOwn = DS == 1 ? 2 * Q : (2 * Q >= kGroups ? 2 * Q / kGroups : 1);
+    const int owner = static_cast<int>(rank) * DS + group;  // among all groups
     float2 num[Q], den[Q];
     float onum[kOwn], oden[kOwn];
     if constexpr (DS == 1) {
@@ -472,9 +497,14 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
     }
 
 #pragma unroll 1
-    for (int d0 = 0; d0 < D; d0 += DS) {
-        const int d = d0 + group;
-        if (DS > 1 && d0 > 0) __syncthreads();  // the previous round's estimates have been added
+    for (int d0 = 0; d0 < D; d0 += kGroups) {
+        const int d = d0 + owner;
+        if (DS > 1 && d0 > 0) {  // the previous round's estimates have been added
+            if constexpr (C > 1)
+                cluster_barrier();
+            else
+                __syncthreads();
+        }
         if (d < D && work) {
             float2 best[Q];
             unsigned sidx[Q / 4];
@@ -522,28 +552,38 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
             }
         }
         if constexpr (DS > 1) {
-            __syncthreads();
-            if (group * kOwn < 2 * Q && work) {
-                const float *x = s_xch + group * kOwn * Shape::kRegion + threadIdx.x % Shape::kRegion;
+            if constexpr (C > 1)
+                cluster_barrier();
+            else
+                __syncthreads();
+            if (owner * kOwn < 2 * Q && work) {
+                const float *x = s_xch + owner * kOwn * Shape::kRegion + threadIdx.x % Shape::kRegion;
 #pragma unroll
-                for (int e = 0; e < DS; e++) {
+                for (int e = 0; e < kGroups; e++) {
                     if (d0 + e >= D) break;
 #pragma unroll
                     for (int i = 0; i < kOwn; i++) {
-                        const float *p = x + (e * 2 * Q + i) * Shape::kRegion;
-                        onum[i] = __fadd_rn(onum[i], p[0]);
-                        oden[i] = __fadd_rn(oden[i], p[DS * 2 * Q * Shape::kRegion]);
+                        const float *p = x + (e % DS * 2 * Q + i) * Shape::kRegion;
+                        if constexpr (C > 1) {
+                            const unsigned at = cluster_addr(smem_addr(p), e / DS);
+                            onum[i] = __fadd_rn(onum[i], cluster_lds1(at));
+                            oden[i] = __fadd_rn(oden[i], cluster_lds1(at + sizeof(float) * DS * 2 * Q * Shape::kRegion));
+                        } else {
+                            onum[i] = __fadd_rn(onum[i], p[0]);
+                            oden[i] = __fadd_rn(oden[i], p[DS * 2 * Q * Shape::kRegion]);
+                        }
                     }
                 }
             }
         }
     }
-    if (DS > 1 && group * kOwn >= 2 * Q) return;
+    if constexpr (C > 1) cluster_barrier();  // a CTA's shared memory stays until every other one has read it
+    if (DS > 1 && owner * kOwn >= 2 * Q) return;
     int oy, ox;
     place(again(), &oy, &ox);
 #pragma unroll
     for (int j = 0; j < kOwn; j++) {
-        const int i = DS == 1 ? j : group * kOwn + j;
+        const int i = DS == 1 ? j : owner * kOwn + j;
         if (!(valid & (1u << i))) continue;
         const float nu = DS == 1 ? pick<Q>(num, j) : onum[j], de = DS == 1 ? pick<Q>(den, j) : oden[j];
         const int y = oy + g.half * (i & 1), x = ox + (i >> 1);

@@ -78,3 +78,32 @@ def test_non_finite_pixels_reach_the_same_outputs():
         assert np.array_equal(np.nan_to_num(out, nan=7.5).view(np.uint32),
                               np.nan_to_num(ref[0], nan=7.5).view(np.uint32)), config
         assert np.array_equal(smap, ref[1]), config
+
+
+@pytest.mark.parametrize("D,S", [(3, 4), (16, 2), (17, 2)])
+def test_few_tiles_shared_by_clusters(D, S):
+    """Kernels of a few hundred taps on images of a few tiles: clusters of CTAs split the directions, with
+    fewer directions than a round takes, as many, and one more."""
+    import torch
+
+    rng = np.random.default_rng(D)
+    n = 25
+    w = rng.uniform(0.0, 1.0, (D * S, n, n)).astype(np.float32)
+    w[:, :, 0] = 0.0
+    w[rng.random((D * S, n, n)) < 0.1] = 0.0
+    w /= w.sum((1, 2), keepdims=True)
+    off = np.arange(D * S, dtype=np.int32) * n * n
+    rows = np.full(D * S, n, np.int32)
+    ks = lpaici.KernelSet.from_dense(w.ravel(), off, rows, rows, D, S)
+    ko = ob.DenseKernels(D, S, w.ravel(), off, rows, rows)
+    var = ks.variances(0.1)
+    for W, H in ((1, 1), (16, 16), (17, 33), (97, 64), (130, 127)):
+        x = rng.uniform(0.0, 1.0, (H, W)).astype(np.float32)
+        t = torch.from_numpy(x).cuda()
+        out, smap = lpaici.forward(ks, t, 0.1, 0.6, scale_map=True)
+        ref, rmap, _ = ob.oracle_forward_f32(x, ko, var, 0.6, want_map=True)
+        assert np.array_equal(smap.cpu().numpy(), rmap), (W, H)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32)), (W, H)
+        # through a state as well: 1 / den of the same sums
+        state_out, _ = lpaici.forward_state(ks, t, 0.1, 0.6)
+        assert torch.equal(state_out.view(torch.int32), out.view(torch.int32))
