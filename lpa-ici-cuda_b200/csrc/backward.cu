@@ -17,11 +17,11 @@
 //      turns the sum over scales into
 //          sum_s D_s (*) (c_d [s* >= s]):
 //      the field is zeroed in place where s* < s, scale after scale (only where the next kernel
-//      reaches), and never rebuilt.  Two groups of warps take every other run of each kernel over the same
+//      reaches), and never rebuilt.  Two groups of warps take every other unit of each kernel over the same
 //      outputs.  Every output is written once: no atomics, deterministic.
 //
 // Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
-// zero (its runs in order), the chunks' sums are added in order, and group 1's total is added to group 0's.
+// zero (its units in order), the chunks' sums are added in order, and group 1's total is added to group 0's.
 // A tile is gathered by one CTA or by a cluster of kGatherChunks or half as many CTAs (the tiles after the last
 // whole wave, gather_plan) that share the chunks
 // and add the same sums in the same order through distributed shared memory, so the gradient does not depend on
@@ -54,8 +54,8 @@ namespace {
 // against 2.4 to 3.4 with three register pairs (measured in chains).  It costs the taps where only one of
 // two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.
 // Q = 16 spreads a run's descriptor, branches and window over 32 outputs.
-// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 475 us now (313 us of it the runs: 254 cycles
-// a run of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 47 us, masking 60 us); tapered
+// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 471 us now (300 us of it the units: 250 cycles
+// a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 63 us); tapered
 // set 964 and 705 us; 384 x 320 (15 tiles) 571 and 70 us.
 constexpr int kGatherQ = 16;
 constexpr int kGatherGroups = 2;
@@ -116,18 +116,16 @@ struct GatherSmem {
     }
 };
 
-// The first H = L % 4 taps of a run: H + 15 field values, H weight pairs; leaves the next tap's window.
+// The first H = L % 4 taps of a unit; the next tap's window is loaded already, src points at its first value.
 template <int H>
-__device__ __forceinline__ void gather_head(float2 (&acc)[kGatherQ], float (&win)[kGatherQ], unsigned &src, unsigned &wp) {
+__device__ __forceinline__ void gather_head(float2 (&acc)[kGatherQ], const float (&win)[kGatherQ], unsigned src, unsigned &at) {
     constexpr int Q = kGatherQ;
-    float lead[H > 0 ? H : 1];  // the H columns before the next tap's window
-    float2 w[H > 0 ? H : 1];
+    float lead[H];  // the H columns before the window
+    float2 w[H];
 #pragma unroll
-    for (int j = 0; j < H; j++) w[j] = lds2(wp + 8 * j);
+    for (int j = 0; j < H; j++) w[j] = lds2(at + 8 * j);
 #pragma unroll
-    for (int j = 0; j < H; j++) lead[j] = lds1(src + 4 * j);
-#pragma unroll
-    for (int i = 0; i < Q - 1; i++) win[i] = lds1(src + 4 * (H + i));
+    for (int j = 0; j < H; j++) lead[j] = lds1(src + 4 * j - 4 * H);
 #pragma unroll
     for (int j = 0; j < H; j++)
 #pragma unroll
@@ -135,8 +133,7 @@ __device__ __forceinline__ void gather_head(float2 (&acc)[kGatherQ], float (&win
             const float x = j + m < H ? lead[j + m < H ? j + m : 0] : win[j + m < H ? 0 : j + m - H];
             acc[m] = fma2(w[j], make_float2(x, x), acc[m]);
         }
-    src += 4 * (H + Q - 1);
-    wp += 8 * H;
+    at += 8 * H;
 }
 
 // Four taps; the window slots have been rotated by 4 * P taps.
@@ -157,35 +154,41 @@ __device__ __forceinline__ void gather_block(float2 (&acc)[kGatherQ], float (&wi
     }
 }
 
-// acc[m] += {w0_t, w1_t} * field[src + m + t] over a run of 4n + h taps.
-__device__ __forceinline__ void gather_run(float2 (&acc)[kGatherQ], unsigned src, unsigned wp, int h, int n) {
+// acc[m] += {w0_t, w1_t} * field[m + t] over a unit of h + 4n taps whose L weight pairs are at [at, end); src: the
+// field value of tap h.  The window is loaded before the dispatch on h: loaded in each head it costs register moves
+// where the heads meet.
+__device__ __forceinline__ void gather_unit(float2 (&acc)[kGatherQ], unsigned src, unsigned h, unsigned at, unsigned end) {
     float win[kGatherQ];
-    if (h < 2) {
-        if (h == 0)
-            gather_head<0>(acc, win, src, wp);
+#pragma unroll
+    for (int i = 0; i < kGatherQ - 1; i++) win[i] = lds1(src + 4 * i);
+    if (h > 0) {
+        if (h == 1)
+            gather_head<1>(acc, win, src, at);
+        else if (h == 2)
+            gather_head<2>(acc, win, src, at);
         else
-            gather_head<1>(acc, win, src, wp);
-    } else {
-        if (h == 2)
-            gather_head<2>(acc, win, src, wp);
-        else
-            gather_head<3>(acc, win, src, wp);
+            gather_head<3>(acc, win, src, at);
     }
-    if (n == 0) return;
+    if (at == end) return;
+    src += 4 * (kGatherQ - 1);
 #pragma unroll 1
     while (true) {
-        gather_block<0>(acc, win, src, wp);
-        src += 16; wp += 32;
-        if (--n == 0) break;
-        gather_block<1>(acc, win, src, wp);
-        src += 16; wp += 32;
-        if (--n == 0) break;
-        gather_block<2>(acc, win, src, wp);
-        src += 16; wp += 32;
-        if (--n == 0) break;
-        gather_block<3>(acc, win, src, wp);
-        src += 16; wp += 32;
-        if (--n == 0) break;
+        gather_block<0>(acc, win, src, at);
+        src += 16;
+        at += 32;
+        if (at == end) break;
+        gather_block<1>(acc, win, src, at);
+        src += 16;
+        at += 32;
+        if (at == end) break;
+        gather_block<2>(acc, win, src, at);
+        src += 16;
+        at += 32;
+        if (at == end) break;
+        gather_block<3>(acc, win, src, at);
+        src += 16;
+        at += 32;
+        if (at == end) break;
     }
 }
 
@@ -203,20 +206,35 @@ __device__ __noinline__ void gather_run_skipping(float2 *acc, unsigned src, unsi
     }
 }
 
-// A byte or a float from global memory, 0 (and no read) unless ok: predicated, no branch around every load.
+// The byte or float `Off` elements past p in global memory, 0 (and no read) unless ok: predicated, no branch around
+// every load, and the offset is the instruction's own.
+template <int Off>
 __device__ __forceinline__ unsigned ldg_u8_if(const uint8_t *p, bool ok) {
     unsigned v;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.nc.u8 %0, [%1];\n\t}"
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.nc.u8 %0, [%1 + %3];\n\t}"
                  : "=r"(v)
-                 : "l"(p), "r"(static_cast<int>(ok)));
+                 : "l"(p), "r"(static_cast<int>(ok)), "n"(Off));
     return v;
 }
+template <int Off>
 __device__ __forceinline__ float ldg_if(const float *p, bool ok) {
     float v;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1 + %3];\n\t}"
                  : "=f"(v)
-                 : "l"(p), "r"(static_cast<int>(ok)));
+                 : "l"(p), "r"(static_cast<int>(ok)), "n"(4 * Off));
     return v;
+}
+// Pieces I .. N - 1 of one row, 32 columns apart: in the image for first <= piece < past.
+template <bool UReady, int I, int N>
+__device__ __forceinline__ void load_pieces(unsigned (&sc)[N], float (&u)[N], const uint8_t *map, const float *den, const float *g,
+                                            int first, int past) {
+    if constexpr (I < N) {
+        const bool in = I >= first && I < past;
+        sc[I] = ldg_u8_if<32 * I>(map, in);
+        u[I] = ldg_if<32 * I>(den, in);
+        if (!UReady) u[I] = ldg_if<32 * I>(g, in) * u[I];
+        load_pieces<UReady, I + 1, N>(sc, u, map, den, g, first, past);
+    }
 }
 
 // s*(d, .) and c_d = u / v_{d, s*}, u = g / den (0 outside the image), for the field rows [dr.x, dr.y) and
@@ -226,49 +244,43 @@ __device__ __forceinline__ float ldg_if(const float *p, bool ok) {
 // loads in flight: between the barriers around it the build is bound by the loads' latency and the index
 // arithmetic, not by the bytes.  Returns whether a value of this thread is infinite or NaN.
 template <bool UReady, bool Inside>
-__device__ __forceinline__ bool build_field(float *s_f, uint8_t *s_s, const float *rv_d, const GatherImage &im,
+__device__ __forceinline__ bool build_field(unsigned s_f, unsigned s_s, unsigned rv, const GatherImage &im,
                                             const uint8_t *map, const int4 dr, int gx0, int gy0, int pitch, int plane,
                                             int warp, int nwarps, int lane) {
     constexpr int kRows = 2, kAcross = 5;
     bool bad = false;
-    const unsigned rv = smem_addr(rv_d);
     for (int c0 = dr.z; c0 < dr.w; c0 += 32 * kAcross) {
         const int c = c0 + lane, gx = gx0 + c;
         // columns c + 32 i: stored for i < stored, read from the image for first <= i < past
         const int stored = (dr.w - c + 31) >> 5, first = gx >= 0 ? 0 : (-gx + 31) >> 5, past = min(stored, (im.W - gx + 31) >> 5);
+        // of field row 0 (outside the image possibly: only rows and columns inside are read)
+        const long long px0 = static_cast<long long>(gy0) * im.W + gx;
+        const uint8_t *pm0 = map + px0;
+        const float *pd0 = im.rden + px0, *pg0 = im.g + static_cast<long long>(gy0) * im.g_pitch + gx;
         for (int r0 = dr.x + warp; r0 < dr.y; r0 += kRows * nwarps) {
             float u[kRows][kAcross];
             unsigned sc[kRows][kAcross];
 #pragma unroll
             for (int j = 0; j < kRows; j++) {
-                const int r = r0 + j * nwarps, gy = gy0 + r;
-                const bool ok = r < dr.y && (Inside || (gy >= 0 && gy < im.H));
-                const ptrdiff_t px = static_cast<ptrdiff_t>(ok ? gy : 0) * im.W + gx;
-                const uint8_t *pm = map + px;
-                const float *pd = im.rden + px, *pg = im.g + static_cast<ptrdiff_t>(ok ? gy : 0) * im.g_pitch + gx;
-                const int f = Inside ? 0 : first, e = ok ? (Inside ? stored : past) : 0;
-#pragma unroll
-                for (int i = 0; i < kAcross; i++) {
-                    const bool in = (Inside || i >= f) && i < e;
-                    sc[j][i] = ldg_u8_if(pm + 32 * i, in);
-                    u[j][i] = ldg_if(pd + 32 * i, in);
-                    if (!UReady) u[j][i] = ldg_if(pg + 32 * i, in) * u[j][i];
-                }
+                const int r = r0 + j * nwarps;
+                const bool ok = r < dr.y && (Inside || static_cast<unsigned>(gy0 + r) < static_cast<unsigned>(im.H));
+                const long long px = static_cast<long long>(r) * im.W;
+                load_pieces<UReady, 0>(sc[j], u[j], pm0 + px, pd0 + px, pg0 + static_cast<long long>(r) * im.g_pitch,
+                                       Inside ? 0 : first, ok ? (Inside ? stored : past) : 0);
             }
 #pragma unroll
             for (int j = 0; j < kRows; j++) {
                 const int r = r0 + j * nwarps;
                 if (r >= dr.y) break;
-                const int at = (r & 1) * plane + (r >> 1) * pitch + c;
-                float *pf = s_f + at;
-                uint8_t *ps = s_s + at;
+                const unsigned at = (r & 1) * plane + (r >> 1) * pitch + c;
+                const unsigned pf = s_f + 4 * at, ps = s_s + at;
 #pragma unroll
                 for (int i = 0; i < kAcross; i++) {
                     const float v = u[j][i] * lds1(rv + 4 * sc[j][i]);
                     bad |= !(fabsf(v) <= FLT_MAX);
                     if (i < stored) {
-                        ps[32 * i] = static_cast<uint8_t>(sc[j][i]);
-                        pf[32 * i] = v;
+                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(ps + 32 * i), "r"(sc[j][i]) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(pf + 128 * i), "f"(v) : "memory");
                     }
                 }
             }
@@ -290,39 +302,44 @@ __device__ __forceinline__ unsigned spread_top_bit(unsigned v) {
 // those rows are masked too: zeroing a cell with s* < s anywhere keeps the field c_d [s* >= s]).  Per byte,
 // (s* | 0x80) - s keeps its top bit exactly where s* >= s (scales are below 0x80) and borrows from no other
 // byte; cells outside this direction's region hold stale bytes, which no correlation reads.
-__device__ __forceinline__ void mask_words(float *s_f, const uint8_t *s_s, int first, int end, unsigned below, int nthreads) {
+// `at`, `end`: shared addresses of this thread's first word of selected scales and of the range's end; f4 its cells.
+template <int Threads>
+__device__ __forceinline__ void mask_words(unsigned at, unsigned end, unsigned f4, unsigned below) {
     constexpr int kWords = 4;  // loaded before the first is used
-    const unsigned *sw = reinterpret_cast<const unsigned *>(s_s);
-    float4 *f4 = reinterpret_cast<float4 *>(s_f);
-    for (int w = first; w < end; w += kWords * nthreads) {
+    for (; at < end; at += 4 * kWords * Threads, f4 += 16 * kWords * Threads) {
         unsigned v[kWords];
 #pragma unroll
-        for (int j = 0; j < kWords; j++) v[j] = w + j * nthreads < end ? sw[w + j * nthreads] : 0xffffffffu;
+        for (int j = 0; j < kWords; j++) {
+            v[j] = 0xffffffffu;
+            if (at + 4 * Threads * j < end) v[j] = lds_u1(at + 4 * Threads * j);
+        }
 #pragma unroll
         for (int j = 0; j < kWords; j++) {
             const unsigned ge = ((v[j] | 0x80808080u) - below) & 0x80808080u;
             if (ge != 0x80808080u) {  // a cell of the word has s* < s: keep the others
-                float4 f = f4[w + j * nthreads];
-                f.x = __uint_as_float(__float_as_uint(f.x) & spread_top_bit<0>(ge));
-                f.y = __uint_as_float(__float_as_uint(f.y) & spread_top_bit<1>(ge));
-                f.z = __uint_as_float(__float_as_uint(f.z) & spread_top_bit<2>(ge));
-                f.w = __uint_as_float(__float_as_uint(f.w) & spread_top_bit<3>(ge));
-                f4[w + j * nthreads] = f;
+                const float4 f = lds4(f4 + 16 * Threads * j);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(f4 + 16 * Threads * j),
+                             "r"(__float_as_uint(f.x) & spread_top_bit<0>(ge)), "r"(__float_as_uint(f.y) & spread_top_bit<1>(ge)),
+                             "r"(__float_as_uint(f.z) & spread_top_bit<2>(ge)), "r"(__float_as_uint(f.w) & spread_top_bit<3>(ge))
+                             : "memory");
             }
         }
     }
 }
-__device__ __forceinline__ void mask_field(float *s_f, const uint8_t *s_s, const int4 rc, unsigned s, int pitch, int plane,
-                                           int tid, int nthreads) {
+template <int Threads>
+__device__ __forceinline__ void mask_field(unsigned s_f, unsigned s_s, const int4 rc, unsigned s, int pitch, int plane, int tid) {
     const unsigned below = 0x01010101u * s;
     // even rows (rc.x + 1) / 2 .. (rc.y + 1) / 2 of plane 0, odd rows rc.x / 2 .. rc.y / 2 of plane 1; the odd
     // rows go to the threads from the last one on, which the even rows' last step leaves idle
     const int e0 = (rc.x + 1) >> 1, e1 = (rc.y + 1) >> 1, o0 = rc.x >> 1, o1 = rc.y >> 1;
-    if (e1 > e0)
-        mask_words(s_f, s_s, ((e0 * pitch + rc.z) >> 2) + tid, ((e1 - 1) * pitch + rc.w + 3) >> 2, below, nthreads);
-    if (o1 > o0)
-        mask_words(s_f, s_s, ((plane + o0 * pitch + rc.z) >> 2) + (nthreads - 1 - tid), (plane + (o1 - 1) * pitch + rc.w + 3) >> 2,
-                   below, nthreads);
+    if (e1 > e0) {
+        const int w = ((e0 * pitch + rc.z) >> 2) + tid, end = ((e1 - 1) * pitch + rc.w + 3) >> 2;
+        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, below);
+    }
+    if (o1 > o0) {
+        const int w = ((plane + o0 * pitch + rc.z) >> 2) + (Threads - 1 - tid), end = (plane + (o1 - 1) * pitch + rc.w + 3) >> 2;
+        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, below);
+    }
 }
 
 // The float2 at shared address a of CTA `rank` of the cluster.
@@ -344,8 +361,9 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     uint2 *s_tab = reinterpret_cast<uint2 *>(base);
     float *s_rv = reinterpret_cast<float *>(base + lay.rv);
     int *s_flag = reinterpret_cast<int *>(base + lay.flag);
-    float *s_f = reinterpret_cast<float *>(base + lay.field);  // the field of the current direction
-    uint8_t *s_s = reinterpret_cast<uint8_t *>(base + lay.smap);  // s*(d, .) on the halo'd tile
+    // the field of the current direction and s*(d, .) on the halo'd tile, as shared addresses (loads and stores
+    // through pointers cost an address computation each)
+    const unsigned s_f = smem_addr(base + lay.field), s_s = smem_addr(base + lay.smap);
     // the rest's CTAs may start once every CTA of this launch has (they depend on nothing of it)
     if (a.rest_follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int rank = a.cluster > 1 ? static_cast<int>(blockIdx.x % a.cluster) : 0;
@@ -367,7 +385,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     const int gtid = tid % Shape::kRegion;
     const int gwarp = gtid >> 5;
     const int ty = (gwarp / WX) * 32 + 2 * (lane & 15), tx = (gwarp % WX) * 32 + (lane >> 4) * Q;
-    const unsigned lane_base = smem_addr(s_f + (ty >> 1) * a.pitch + tx);
+    const unsigned lane_base = s_f + 4 * ((ty >> 1) * a.pitch + tx);
     const unsigned blocks = smem_addr(base + lay.block);
 
     for (int i = tid; i <= nk; i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
@@ -409,7 +427,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
         for (; d < d_stop; d++) {
             __syncthreads();  // the previous direction's correlations are done with the field
             const uint8_t *map = im.smap + static_cast<size_t>(d) * im.H * im.W;
-            const float *rv_d = s_rv + d * a.S;
+            const unsigned rv_d = smem_addr(s_rv + d * a.S);
             const int4 dr = a.drect[d];
             const bool inside = gx0 + dr.z >= 0 && gx0 + dr.w <= im.W && gy0 + dr.x >= 0 && gy0 + dr.y <= im.H;
             bool bad;
@@ -427,30 +445,33 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                     stage(k + 1);
                 else
                     asm volatile("cp.async.commit_group;" ::: "memory");
-                if (s > 0) mask_field(s_f, s_s, a.rect[k], static_cast<unsigned>(s), a.pitch, a.plane, tid, nthreads);
+                if (s > 0) mask_field<nthreads>(s_f, s_s, a.rect[k], static_cast<unsigned>(s), a.pitch, a.plane, tid);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // this kernel's block has landed
                 __syncthreads();
                 const bool finite = s_flag[d & 1] == 0;
                 if (s == 0 && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
                 const unsigned block = blocks + (k & 1) * a.block_bytes;
-                const unsigned n_units = s_tab[k].y;
-                // units group, group + 2, ... of the kernel: {field byte offset | taps % 4, taps / 4 | weights << 8}
-                unsigned up = block + 8 * group;
-                const unsigned uend = block + 8 * n_units;
+                // the group's units: one stream, the next unit behind the weights of the one before
+                const unsigned ends = s_tab[k].y;
+                unsigned at = block + (group == 0 ? 0 : 8 * (ends & 0xffffu));
+                const unsigned last = block + 8 * (group == 0 ? ends & 0xffffu : ends >> 16);
                 if (finite) {
 #pragma unroll 1
-                    for (; up < uend; up += 8 * kGatherGroups) {
-                        const uint2 u = lds_u2(up);
-                        gather_run(acc, lane_base + (u.x & ~3u), block + 8 * (u.y >> 8), u.x & 3, u.y & 255);
+                    while (at != last) {
+                        const uint2 u = lds_u2(at);
+                        const unsigned h = u.y & 3u, end = at + u.y - h;
+                        gather_unit(acc, lane_base + u.x, h, at + 8, end);
+                        at = end;
                     }
                 } else {
                     float2 tmp[Q];
 #pragma unroll
                     for (int i = 0; i < Q; i++) tmp[i] = acc[i];
 #pragma unroll 1
-                    for (; up < uend; up += 8 * kGatherGroups) {
-                        const uint2 u = lds_u2(up);
-                        gather_run_skipping(tmp, lane_base + (u.x & ~3u), block + 8 * (u.y >> 8), 4 * (u.y & 255) + (u.x & 3));
+                    while (at != last) {
+                        const uint2 u = lds_u2(at);
+                        gather_run_skipping(tmp, lane_base + u.x - 4 * (u.y & 3u), at + 8, (u.y - 8) / 8);
+                        at += u.y & ~3u;
                     }
 #pragma unroll
                     for (int i = 0; i < Q; i++) acc[i] = tmp[i];

@@ -166,18 +166,27 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
     blob.reserve(limit_words + limit_words / 4);
     blob.assign((2 * (static_cast<size_t>(nk) + 1) + 3) & ~size_t(3), 0);
     for (int k = 0; k < nk; k++) {
-        blob[2 * k] = static_cast<int>(4 * blob.size());
-        blob[2 * k + 1] = static_cast<int>(units[k].size());
-        int at = static_cast<int>(units[k].size());  // in 8-byte pairs from the block's start
-        for (const Unit &u : units[k]) {
-            const int row = R + u.row;
-            blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col) | (u.len % 4));
-            blob.push_back(u.len / 4 | at << 8);
-            at += u.len;
+        const size_t start = blob.size();
+        size_t ends[2];  // of the two groups' streams, in 8-byte pairs: every other unit each
+        for (int g = 0; g < 2; g++) {
+            size_t w = 0;
+            for (size_t i = 0; i < units[k].size(); i++) {
+                const Unit &u = units[k][i];
+                if (static_cast<int>(i % 2) == g) {
+                    const int row = R + u.row;
+                    blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col + u.len % 4));
+                    blob.push_back((8 + 8 * u.len) | (u.len % 4));
+                    const size_t n = blob.size();
+                    blob.resize(n + 2 * u.len);
+                    std::memcpy(blob.data() + n, pairs[k].data() + w, 8 * static_cast<size_t>(u.len));
+                }
+                w += 2 * static_cast<size_t>(u.len);
+            }
+            ends[g] = (blob.size() - start) / 2;
         }
-        const size_t n = blob.size();
-        blob.resize((n + pairs[k].size() + 3) & ~size_t(3), 0);
-        std::memcpy(blob.data() + n, pairs[k].data(), 4 * pairs[k].size());
+        blob[2 * k] = static_cast<int>(4 * start);
+        blob[2 * k + 1] = static_cast<int32_t>(ends[0] | ends[1] << 16);  // (a kernel has at most 127 x 255 taps)
+        blob.resize((blob.size() + 3) & ~size_t(3), 0);
     }
     blob[2 * nk] = static_cast<int>(4 * blob.size());
     blob.resize(std::max<size_t>(blob.size(), limit_words), 0);
