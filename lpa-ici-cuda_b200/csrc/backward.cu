@@ -6,11 +6,10 @@
 //     c_d(p) = g(p) / den(p) / v_{d, s*(d,p)},
 //     dL/dx(q) = sum_d sum_s sum_t h'_{d,s}(t) [s*(d, q + t) = s] c_d(q + t)       (zero padding)
 // where h' is h mirrored through its centre: for every direction and scale, a correlation of the field
-// masked to the pixels that selected that scale.  Three launches:
+// masked to the pixels that selected that scale.  Two passes:
 //   A. selection: the forward's exact tile sweep recomputes s*(d,p) (one byte per direction and
-//      pixel) and 1/den(p) into a transient workspace -- the forward stores nothing for the adjoint;
-//   u: u = g / den over the workspace's 1/den (an elementwise pass; from a kept state the gather forms
-//      the product itself);
+//      pixel) and writes u = g * (1/den) beside it, into a transient workspace -- the forward stores
+//      nothing for the adjoint (a kept state holds 1/den, and the gather forms the product itself);
 //   B. gather: 128 x 64 output tiles.  Per direction it reads s*(d,.) and u on the tile plus its R-pixel
 //      halo (from L2) and forms the field c_d = u / v_{d,s*} in shared memory.
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
@@ -71,12 +70,12 @@ struct GatherShape {
 struct GatherImage {
     const float *g;        // cotangent, pitch g_pitch
     const uint8_t *smap;   // D x H x W selected scales (pass A)
-    const float *rden;     // H x W, pitch W: 1 / den, den = sum_d 1/v_d (pass A); u = g / den when u_ready
+    const float *rden;     // H x W, pitch W: 1 / den, den = sum_d 1/v_d (pass A); u = g * (1/den) when u_ready
     float *grad;           // result, pitch grad_pitch
     const float *rvar;     // 1 / v_k of this image (batched plans; one image: GatherArgs::rvar)
     int g_pitch, grad_pitch, W, H;
     int tiles_x;
-    int u_ready;           // rden holds u = g * (1 / den) already (lpaici_adjoint_u_kernel)
+    int u_ready;           // rden holds u = g * (1 / den) already (pass A)
 };
 
 struct GatherArgs {
@@ -540,33 +539,6 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// u = g * (1 / den) written over 1 / den, once per image between the two passes of the recomputing
-// adjoints (the 1/den map is their own workspace there), so that the gather's per-direction field builds
-// read one map instead of two.  The product is the one the gather forms otherwise.  Images blockIdx.y,
-// blockIdx.y + gridDim.y, ... of a batched plan (images: n descriptors), else the single one.
-__global__ void lpaici_adjoint_u_kernel(const GatherImage *images, const GatherImage single, int n) {
-    for (int i = blockIdx.y; i < n; i += gridDim.y) {
-        const GatherImage im = images ? images[i] : single;
-        float *u = const_cast<float *>(im.rden);
-        for (int y = blockIdx.x; y < im.H; y += gridDim.x) {
-            const float *grow = im.g + static_cast<size_t>(y) * im.g_pitch;
-            float *urow = u + static_cast<size_t>(y) * im.W;
-            for (int x = threadIdx.x; x < im.W; x += blockDim.x) urow[x] = grow[x] * urow[x];
-        }
-    }
-}
-
-int u_launch(const GatherImage *images, const GatherImage &single, int n, int max_h, cudaStream_t stream) {
-    const dim3 grid(static_cast<unsigned>(std::min(max_h, 1184)), static_cast<unsigned>(std::min(n, 65535)));
-    lpaici_adjoint_u_kernel<<<grid, 256, 0, stream>>>(images, single, n);
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "adjoint u launch");
-}
-
-}  // namespace
-
-namespace {
-
 const void *gather_fn(const AdjointLayout &L) {
     return L.wx == 4 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2>)
                      : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1>);
@@ -722,6 +694,8 @@ int adjoint_passes(const lpaici_kernelset *ks, const int *blob, const int *adj_b
     img.out = nullptr;
     img.smap = smap;
     img.rden = rden;
+    img.g = d_grad_out;
+    img.g_pitch = gout_pitch;
     img.W = width;
     img.in_h = height;
     img.in_pitch = noisy_pitch;
@@ -733,11 +707,6 @@ int adjoint_passes(const lpaici_kernelset *ks, const int *blob, const int *adj_b
     tab.blob = blob;
     int rc = launch_forward(img, tab, plan_for(ks, width, height), stream);
     if (rc != LPAICI_OK) return rc;
-    // u = g / den over the workspace's 1/den
-    rc = u_launch(nullptr, GatherImage{d_grad_out, smap, rden, d_grad_in, nullptr, gout_pitch, gin_pitch, width, height, 0, 0},
-                  1, height, stream);
-    if (rc != LPAICI_OK) return rc;
-
     // B. gather
     return gather_pass(ks, adj_blob, smap, rden, d_grad_out, gout_pitch, d_grad_in, gin_pitch, width, height, sigma,
                        true, stream);
@@ -881,7 +850,6 @@ struct lpaici_backward_batch {
     size_t smem = 0;
     AdjointLayout layout;
     GatherPlan plan;
-    int n = 0, max_h = 0;  // images; the tallest one's rows (the u launch)
     bool use_graph = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -891,8 +859,6 @@ namespace {
 
 int backward_batch_enqueue(lpaici_backward_batch *b, cudaStream_t stream) {
     int rc = batch_plan_enqueue(b->select, stream);
-    if (rc != LPAICI_OK) return rc;
-    rc = u_launch(b->ga.images, GatherImage{}, b->n, b->max_h, stream);
     if (rc != LPAICI_OK) return rc;
     return gather_launch(b->layout, b->ga, b->plan, b->smem, stream);
 }
@@ -983,12 +949,11 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
         desc[i] = GatherImage{im.grad_out, smap, rden, im.grad_in,
                               reinterpret_cast<const float *>(base + rvar_off) + static_cast<size_t>(i) * nk,
                               im.gout_pitch, im.gin_pitch, im.width, im.height, tiles_x[i], 1};
-        b->max_h = std::max(b->max_h, im.height);
         int tx = 0;
         const long t = gather_tiles(ks->adj_layout, im.width, im.height, &tx);
         for (long j = 0; j < t; j++) items.push_back(make_int2(i, static_cast<int>(j)));
         specs[i] = BatchSpec{im.noisy, nullptr, smap, rden, im.width, im.height, im.noisy_pitch, im.width, im.sigma,
-                             im.gamma};
+                             im.gamma, im.grad_out, im.gout_pitch};
     }
     e = cudaMemcpy(base + desc_off, desc.data(), sizeof(GatherImage) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(base + rvar_off, rvar.data(), sizeof(float) * rvar.size(), cudaMemcpyHostToDevice);
@@ -1004,7 +969,6 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
         backward_batch_free(b);
         return rc;
     }
-    b->n = n;
 
     const int config = opts ? opts->tile_config : -1;
     rc = batch_plan_create(ks, specs.data(), n, config, false, stream, &b->select);

@@ -28,9 +28,9 @@ struct BatchImage {
     float *out;       // null: no estimate (the adjoint's selection pass)
     uint8_t *smap;
     float *rden;      // optional 1/den map (the adjoint's selection pass)
-    int W, H, in_pitch, out_pitch;
+    const float *g;   // optional cotangent: rden is g / den
+    int W, H, in_pitch, out_pitch, g_pitch;
     int tab_offset;  // float index of var[nk] (thr[nk] follows) in the plan's table array
-    int pad;
 };
 
 struct BatchArgs {
@@ -77,6 +77,8 @@ __device__ __forceinline__ void batched_image(const BatchArgs &a, int image, Ima
         img.out = bi.out;
         img.smap = bi.smap;
         img.rden = bi.rden;
+        img.g = bi.g;
+        img.g_pitch = bi.g_pitch;
         img.W = bi.W;
         img.in_h = bi.H;
         img.in_pitch = bi.in_pitch;
@@ -224,7 +226,8 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         one_size = ai.width == a0.width && ai.height == a0.height && ai.noisy_pitch == a0.noisy_pitch &&
                    ai.out_pitch == a0.out_pitch && ai.sigma == a0.sigma && ai.gamma == a0.gamma &&
                    (ai.out == nullptr) == (a0.out == nullptr) && (ai.smap == nullptr) == (a0.smap == nullptr) &&
-                   (ai.rden == nullptr) == (a0.rden == nullptr);
+                   (ai.rden == nullptr) == (a0.rden == nullptr) && (ai.g == nullptr) == (a0.g == nullptr) &&
+                   ai.g_pitch == a0.g_pitch;
     }
     if (config >= 0) {
         b->plan.config = config;
@@ -267,8 +270,8 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         fill_tables(ks, nullptr, im.sigma, im.gamma, &t);
         std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk], t.var, sizeof(float) * nk);
         std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk + nk], t.thr, sizeof(float) * nk);
-        imgs[i] = BatchImage{im.noisy, im.out, im.smap, im.rden, im.width, im.height, im.noisy_pitch, im.out_pitch,
-                             i * 2 * nk, 0};
+        imgs[i] = BatchImage{im.noisy, im.out, im.smap, im.rden, im.g, im.width, im.height, im.noisy_pitch, im.out_pitch,
+                             im.g_pitch, i * 2 * nk};
         for (int y = 0; y < im.height; y += b->info.tile_h)
             for (int x = 0; x < im.width; x += b->info.tile_w) push(items, i, x, y, b->info.tile_w, b->info.tile_h);
     }
@@ -360,11 +363,14 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
             b->mi.out[i] = specs[i].out;
             b->mi.smap[i] = specs[i].smap;
             b->mi.rden[i] = specs[i].rden;
+            b->mi.g[i] = specs[i].g;
         }
         b->img.in = im.noisy;
         b->img.out = im.out;
         b->img.smap = im.smap;
         b->img.rden = im.rden;
+        b->img.g = im.g;
+        b->img.g_pitch = im.g_pitch;
         b->img.W = im.width;
         b->img.in_h = im.height;
         b->img.in_pitch = im.noisy_pitch;

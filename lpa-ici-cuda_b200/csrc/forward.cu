@@ -54,6 +54,7 @@ struct SharedImage {
                 im.out = mi.out[z];
                 im.smap = mi.smap[z];
                 im.rden = mi.rden[z];
+                im.g = mi.g[z];
             }
         }
         __syncthreads();

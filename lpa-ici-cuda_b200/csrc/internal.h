@@ -59,7 +59,8 @@ struct ImageArgs {
     float *out;       // optional output rows [0, rows_out), pitch out_pitch
     uint8_t *smap;    // optional D x rows_out x W scale map
     float *rden;      // optional rows_out x W map of 1 / sum_d 1/v_d (pitch W; the adjoint's selection pass)
-    int W, in_h, in_pitch, out_pitch;
+    const float *g;   // optional, with rden: the map is g * (1 / sum_d 1/v_d) (pitch g_pitch)
+    int W, in_h, in_pitch, out_pitch, g_pitch;
     int row_begin;    // output row r is input row row_begin + r
     int rows_out;
     int step = 1;     // floats between neighbouring pixels of a row, in and out (channels of an interleaved image)
@@ -85,13 +86,14 @@ struct TilePlan {
 };
 
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
-// output, scale maps and 1/den (the last three may be null, as in ImageArgs).
+// output, scale maps, 1/den and cotangent (the last four may be null, as in ImageArgs).
 constexpr int kMaxMultiImages = 64;
 struct MultiImages {
     const float *in[kMaxMultiImages];
     float *out[kMaxMultiImages];
     uint8_t *smap[kMaxMultiImages];
     float *rden[kMaxMultiImages];
+    const float *g[kMaxMultiImages];
 };
 
 int set_error(int code, const char *fmt, ...);
@@ -172,7 +174,7 @@ int config_blocks_per_sm(int config, size_t smem);
 void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, int *tile_h, int *ctas, int *groups, size_t *smem);
 // Tile width and height of a configuration.
 void config_tile(int config, int *tile_w, int *tile_h);
-// One image of a batch plan (batched.cu): out may be null (no estimate), smap and rden optional.
+// One image of a batch plan (batched.cu): out may be null (no estimate), smap, rden and g optional.
 struct BatchSpec {
     const float *noisy;
     float *out;
@@ -180,6 +182,8 @@ struct BatchSpec {
     float *rden;
     int width, height, noisy_pitch, out_pitch;
     float sigma, gamma;
+    const float *g = nullptr;  // with rden: the map is g / den
+    int g_pitch = 0;
 };
 // config < 0: chosen for the images (plan_for, plan_for_images).
 int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n, int config, bool use_graph,

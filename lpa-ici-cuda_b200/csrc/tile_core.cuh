@@ -589,7 +589,10 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
         const int y = oy + g.half * (i & 1), x = ox + (i >> 1);
         if (img.out)
             img.out[static_cast<size_t>(y) * img.out_pitch + static_cast<size_t>(x) * img.step] = __fdiv_rn(nu, de);
-        if (img.rden) img.rden[static_cast<size_t>(y) * img.W + x] = __frcp_rn(de);
+        if (img.rden) {
+            const float r = __frcp_rn(de);
+            img.rden[static_cast<size_t>(y) * img.W + x] = img.g ? __ldg(img.g + static_cast<size_t>(y) * img.g_pitch + x) * r : r;
+        }
     }
 }
 
