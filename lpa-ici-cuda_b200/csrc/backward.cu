@@ -15,8 +15,7 @@
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
 //      turns the sum over scales into
 //          sum_s D_s (*) (c_d [s* >= s]):
-//      the field is zeroed in place where s* < s, scale after scale (only where the next kernel
-//      reaches), and never rebuilt.  Two groups of warps take every other unit of each kernel over the same
+//      the field is zeroed in place where s* < s, scale after scale, and never rebuilt.  Two groups of warps take every other unit of each kernel over the same
 //      outputs.  Every output is written once: no atomics, deterministic.
 //
 // Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
@@ -53,9 +52,9 @@ namespace {
 // against 2.4 to 3.4 with three register pairs (measured in chains).  It costs the taps where only one of
 // two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.
 // Q = 16 spreads a run's descriptor, branches and window over 32 outputs.
-// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 471 us now (300 us of it the units: 250 cycles
-// a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 63 us); tapered
-// set 964 and 705 us; 384 x 320 (15 tiles) 571 and 70 us.
+// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 464 us now (300 us of it the units: 250 cycles
+// a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 56 us); tapered
+// set 964 and 699 us; 384 x 320 (15 tiles) 571 and 69 us.
 constexpr int kGatherQ = 16;
 constexpr int kGatherGroups = 2;
 constexpr int kGatherChunks = 8;
@@ -90,9 +89,7 @@ struct GatherArgs {
     int first_tile;        // this launch's tiles start here
     int rest_follows;      // a launch over the tiles after this one's follows
     float rvar[kMaxKernels];  // 1 / v_k of the one image
-    // per kernel: the field cells its correlation reads, rows [x, y), columns [z, w); per direction: the
-    // union over its scales (the cells its field needs)
-    int4 rect[kMaxKernels];
+    // per direction: the field cells its kernels read, rows [x, y), columns [z, w)
     int4 drect[kMaxKernels];
 };
 
@@ -205,33 +202,27 @@ __device__ __noinline__ void gather_run_skipping(float2 *acc, unsigned src, unsi
     }
 }
 
-// The byte or float `Off` elements past p in global memory, 0 (and no read) unless ok: predicated, no branch around
-// every load, and the offset is the instruction's own.
-template <int Off>
-__device__ __forceinline__ unsigned ldg_u8_if(const uint8_t *p, bool ok) {
-    unsigned v;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.nc.u8 %0, [%1 + %3];\n\t}"
-                 : "=r"(v)
-                 : "l"(p), "r"(static_cast<int>(ok)), "n"(Off));
-    return v;
-}
-template <int Off>
-__device__ __forceinline__ float ldg_if(const float *p, bool ok) {
-    float v;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1 + %3];\n\t}"
-                 : "=f"(v)
-                 : "l"(p), "r"(static_cast<int>(ok)), "n"(4 * Off));
-    return v;
-}
-// Pieces I .. N - 1 of one row, 32 columns apart: in the image for first <= piece < past.
+// Pieces I .. N - 1 of one row, 32 columns apart: selected scale and u of the lane's column, zero (and no read) unless
+// first <= piece < past.  One predicate for both loads, no branch around them, offsets in the instructions.
 template <bool UReady, int I, int N>
 __device__ __forceinline__ void load_pieces(unsigned (&sc)[N], float (&u)[N], const uint8_t *map, const float *den, const float *g,
                                             int first, int past) {
     if constexpr (I < N) {
-        const bool in = I >= first && I < past;
-        sc[I] = ldg_u8_if<32 * I>(map, in);
-        u[I] = ldg_if<32 * I>(den, in);
-        if (!UReady) u[I] = ldg_if<32 * I>(g, in) * u[I];
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.le.s32 p, %4, %6;\n\tsetp.gt.and.s32 q, %5, %6, p;\n\t"
+            "mov.u32 %0, 0;\n\tmov.f32 %1, 0f00000000;\n\t"
+            "@q ld.global.nc.u8 %0, [%2 + %7];\n\t@q ld.global.nc.f32 %1, [%3 + %8];\n\t}"
+            : "=r"(sc[I]), "=f"(u[I])
+            : "l"(map), "l"(den), "r"(first), "r"(past), "n"(I), "n"(32 * I), "n"(128 * I));
+        if constexpr (!UReady) {
+            float x;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\tsetp.le.s32 p, %2, %4;\n\tsetp.gt.and.s32 q, %3, %4, p;\n\t"
+                "mov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1 + %5];\n\t}"
+                : "=f"(x)
+                : "l"(g), "r"(first), "r"(past), "n"(I), "n"(128 * I));
+            u[I] = x * u[I];
+        }
         load_pieces<UReady, I + 1, N>(sc, u, map, den, g, first, past);
     }
 }
@@ -288,22 +279,16 @@ __device__ __forceinline__ bool build_field(unsigned s_f, unsigned s_s, unsigned
     return bad;
 }
 
-// All ones where the top bit of byte B is set, else 0 (prmt's sign replication).
-template <int B>
-__device__ __forceinline__ unsigned spread_top_bit(unsigned v) {
-    unsigned r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(0x8888 + 0x1111 * B));
-    return r;
-}
-
-// Zeroes the field where s* < s, in the rows and columns of rc: every 4-cell word from the rectangle's first
-// cell to its last in each row plane, as one flat range over all threads (the cells beside the rectangle in
-// those rows are masked too: zeroing a cell with s* < s anywhere keeps the field c_d [s* >= s]).  Per byte,
-// (s* | 0x80) - s keeps its top bit exactly where s* >= s (scales are below 0x80) and borrows from no other
-// byte; cells outside this direction's region hold stale bytes, which no correlation reads.
-// `at`, `end`: shared addresses of this thread's first word of selected scales and of the range's end; f4 its cells.
+// Zeroes the direction's field where s* = s - 1 (smaller scales are zero since their own pass): the cells of every
+// 4-cell word from the rectangle's first cell to its last in each row plane, as one flat range over all threads.  Only
+// the excluded cells are stored to: reading and writing back whole words (16 bytes of 4 cells) costs 8 shared-memory
+// wavefronts a warp where these stores cost one or two each, although it can skip the cells a scale's kernel does not
+// reach (1024^2: 471 us so, 464 us now).  The cells beside the rectangle in those rows and those outside this
+// direction's region hold stale values, which no correlation reads.
+// `at`, `end`: shared addresses of this thread's first word of selected scales and of the range's end; f4 its cells;
+// excluded: the scale that is masked now, s - 1, in every byte.
 template <int Threads>
-__device__ __forceinline__ void mask_words(unsigned at, unsigned end, unsigned f4, unsigned below) {
+__device__ __forceinline__ void mask_words(unsigned at, unsigned end, unsigned f4, unsigned excluded) {
     constexpr int kWords = 4;  // loaded before the first is used
     for (; at < end; at += 4 * kWords * Threads, f4 += 16 * kWords * Threads) {
         unsigned v[kWords];
@@ -314,30 +299,32 @@ __device__ __forceinline__ void mask_words(unsigned at, unsigned end, unsigned f
         }
 #pragma unroll
         for (int j = 0; j < kWords; j++) {
-            const unsigned ge = ((v[j] | 0x80808080u) - below) & 0x80808080u;
-            if (ge != 0x80808080u) {  // a cell of the word has s* < s: keep the others
-                const float4 f = lds4(f4 + 16 * Threads * j);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(f4 + 16 * Threads * j),
-                             "r"(__float_as_uint(f.x) & spread_top_bit<0>(ge)), "r"(__float_as_uint(f.y) & spread_top_bit<1>(ge)),
-                             "r"(__float_as_uint(f.z) & spread_top_bit<2>(ge)), "r"(__float_as_uint(f.w) & spread_top_bit<3>(ge))
-                             : "memory");
-            }
+            // a byte's top bit stays exactly where it differs from `excluded` (scales are below 0x80)
+            const unsigned keep = ((v[j] ^ excluded) | 0x80808080u) - 0x01010101u;
+            asm volatile(
+                "{\n\t.reg .pred p0, p1, p2, p3;\n\t.reg .b32 t0, t1, t2, t3;\n\t"
+                "and.b32 t0, %1, 0x80;\n\tand.b32 t1, %1, 0x8000;\n\tand.b32 t2, %1, 0x800000;\n\tand.b32 t3, %1, 0x80000000;\n\t"
+                "setp.eq.u32 p0, t0, 0;\n\tsetp.eq.u32 p1, t1, 0;\n\tsetp.eq.u32 p2, t2, 0;\n\tsetp.eq.u32 p3, t3, 0;\n\t"
+                "@p0 st.shared.b32 [%0], 0;\n\t@p1 st.shared.b32 [%0 + 4], 0;\n\t@p2 st.shared.b32 [%0 + 8], 0;\n\t"
+                "@p3 st.shared.b32 [%0 + 12], 0;\n\t}" ::"r"(f4 + 16 * Threads * j),
+                "r"(keep)
+                : "memory");
         }
     }
 }
 template <int Threads>
 __device__ __forceinline__ void mask_field(unsigned s_f, unsigned s_s, const int4 rc, unsigned s, int pitch, int plane, int tid) {
-    const unsigned below = 0x01010101u * s;
+    const unsigned excluded = 0x01010101u * (s - 1);
     // even rows (rc.x + 1) / 2 .. (rc.y + 1) / 2 of plane 0, odd rows rc.x / 2 .. rc.y / 2 of plane 1; the odd
     // rows go to the threads from the last one on, which the even rows' last step leaves idle
     const int e0 = (rc.x + 1) >> 1, e1 = (rc.y + 1) >> 1, o0 = rc.x >> 1, o1 = rc.y >> 1;
     if (e1 > e0) {
         const int w = ((e0 * pitch + rc.z) >> 2) + tid, end = ((e1 - 1) * pitch + rc.w + 3) >> 2;
-        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, below);
+        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, excluded);
     }
     if (o1 > o0) {
         const int w = ((plane + o0 * pitch + rc.z) >> 2) + (Threads - 1 - tid), end = (plane + (o1 - 1) * pitch + rc.w + 3) >> 2;
-        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, below);
+        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, excluded);
     }
 }
 
@@ -444,7 +431,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                     stage(k + 1);
                 else
                     asm volatile("cp.async.commit_group;" ::: "memory");
-                if (s > 0) mask_field<nthreads>(s_f, s_s, a.rect[k], static_cast<unsigned>(s), a.pitch, a.plane, tid);
+                if (s > 0) mask_field<nthreads>(s_f, s_s, a.drect[d], static_cast<unsigned>(s), a.pitch, a.plane, tid);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // this kernel's block has landed
                 __syncthreads();
                 const bool finite = s_flag[d & 1] == 0;
@@ -587,7 +574,7 @@ int gather_launch(const AdjointLayout &L, const GatherArgs &args, const GatherPl
     return LPAICI_OK;
 }
 
-// Fills the geometry and the per-kernel rectangles of the in-place masking; smem receives the dynamic shared
+// Fills the geometry and the directions' rectangles of the field; smem receives the dynamic shared
 // memory of one CTA per tile, checked against the device.
 int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga, size_t *smem) {
     const AdjointLayout &L = ks->adj_layout;
@@ -611,25 +598,17 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
         return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d", *smem,
                          max_optin);
     const int rows = th + 2 * ga->R;
-    for (int k = 0; k < nk; k++) {
+    for (int d = 0; d < ks->D; d++) {
         // a lane reads rows ty + R + j for field rows j of its two output rows (ty + 1 < th) and columns
         // tx + R + dx + [0, Q) (tx + Q <= tile width): rows [R + dy_min, R + th + dy_max), columns
         // [R + dx_min, R + tile width + dx_max)
-        const int4 box = make_int4(L.box[4 * k], L.box[4 * k + 1], L.box[4 * k + 2], L.box[4 * k + 3]);
-        ga->rect[k] = box.y < box.x ? make_int4(0, 0, 0, 0)
-                                    : make_int4(std::max(0, ga->R + box.x), std::min(rows, ga->R + th + box.y),
-                                                std::max(0, ga->R + box.z), std::min(ga->pitch, ga->R + tw + box.w));
-    }
-    for (int d = 0; d < ks->D; d++) {
         int4 u = make_int4(0, 0, 0, 0);
         for (int s = 0; s < ks->S; s++) {
-            const int4 r = ga->rect[d * ks->S + s];
-            if (r.y <= r.x || r.w <= r.z) continue;
-            if (u.y <= u.x) {
-                u = r;
-            } else {
-                u = make_int4(std::min(u.x, r.x), std::max(u.y, r.y), std::min(u.z, r.z), std::max(u.w, r.w));
-            }
+            const int *box = &L.box[4 * (static_cast<size_t>(d) * ks->S + s)];
+            if (box[1] < box[0]) continue;
+            const int4 r = make_int4(std::max(0, ga->R + box[0]), std::min(rows, ga->R + th + box[1]),
+                                     std::max(0, ga->R + box[2]), std::min(ga->pitch, ga->R + tw + box[3]));
+            u = u.y <= u.x ? r : make_int4(std::min(u.x, r.x), std::max(u.y, r.y), std::min(u.z, r.z), std::max(u.w, r.w));
         }
         ga->drect[d] = u;
     }
