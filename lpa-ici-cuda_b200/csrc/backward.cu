@@ -52,9 +52,9 @@ namespace {
 // against 2.4 to 3.4 with three register pairs (measured in chains).  It costs the taps where only one of
 // two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.
 // Q = 16 spreads a run's descriptor, branches and window over 32 outputs.
-// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 464 us now (300 us of it the units: 250 cycles
-// a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 56 us); tapered
-// set 964 and 699 us; 384 x 320 (15 tiles) 571 and 69 us.
+// From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 452 us now (300 us of it the units: 250 cycles
+// a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 45 us); tapered
+// set 964 and 685 us; 384 x 320 (15 tiles) 571 and 66 us.
 constexpr int kGatherQ = 16;
 constexpr int kGatherGroups = 2;
 constexpr int kGatherChunks = 8;
@@ -279,53 +279,75 @@ __device__ __forceinline__ bool build_field(unsigned s_f, unsigned s_s, unsigned
     return bad;
 }
 
-// Zeroes the direction's field where s* = s - 1 (smaller scales are zero since their own pass): the cells of every
-// 4-cell word from the rectangle's first cell to its last in each row plane, as one flat range over all threads.  Only
-// the excluded cells are stored to: reading and writing back whole words (16 bytes of 4 cells) costs 8 shared-memory
-// wavefronts a warp where these stores cost one or two each, although it can skip the cells a scale's kernel does not
-// reach (1024^2: 471 us so, 464 us now).  The cells beside the rectangle in those rows and those outside this
-// direction's region hold stale values, which no correlation reads.
-// `at`, `end`: shared addresses of this thread's first word of selected scales and of the range's end; f4 its cells;
-// excluded: the scale that is masked now, s - 1, in every byte.
-template <int Threads>
-__device__ __forceinline__ void mask_words(unsigned at, unsigned end, unsigned f4, unsigned excluded) {
-    constexpr int kWords = 4;  // loaded before the first is used
-    for (; at < end; at += 4 * kWords * Threads, f4 += 16 * kWords * Threads) {
-        unsigned v[kWords];
-#pragma unroll
-        for (int j = 0; j < kWords; j++) {
-            v[j] = 0xffffffffu;
-            if (at + 4 * Threads * j < end) v[j] = lds_u1(at + 4 * Threads * j);
-        }
-#pragma unroll
-        for (int j = 0; j < kWords; j++) {
-            // a byte's top bit stays exactly where it differs from `excluded` (scales are below 0x80)
-            const unsigned keep = ((v[j] ^ excluded) | 0x80808080u) - 0x01010101u;
-            asm volatile(
-                "{\n\t.reg .pred p0, p1, p2, p3;\n\t.reg .b32 t0, t1, t2, t3;\n\t"
-                "and.b32 t0, %1, 0x80;\n\tand.b32 t1, %1, 0x8000;\n\tand.b32 t2, %1, 0x800000;\n\tand.b32 t3, %1, 0x80000000;\n\t"
-                "setp.eq.u32 p0, t0, 0;\n\tsetp.eq.u32 p1, t1, 0;\n\tsetp.eq.u32 p2, t2, 0;\n\tsetp.eq.u32 p3, t3, 0;\n\t"
-                "@p0 st.shared.b32 [%0], 0;\n\t@p1 st.shared.b32 [%0 + 4], 0;\n\t@p2 st.shared.b32 [%0 + 8], 0;\n\t"
-                "@p3 st.shared.b32 [%0 + 12], 0;\n\t}" ::"r"(f4 + 16 * Threads * j),
-                "r"(keep)
-                : "memory");
-        }
+// Masking zeroes the direction's field where s* = s - 1 (smaller scales are zero since their own pass): the cells of
+// every 4-cell word from the rectangle's first cell to its last in each row plane, as one flat range over all threads.
+// Only the excluded cells are stored to: reading and writing back whole words (16 bytes of 4 cells) costs 8
+// shared-memory wavefronts a warp where these stores cost one or two each, although it can skip the cells a scale's
+// kernel does not reach (1024^2: 471 us so, 464 us with stores alone).  The cells beside the rectangle in those rows
+// and those outside this direction's region hold stale values, which no correlation reads.
+struct MaskRange {
+    int w0[2], w1[2];  // words [w0, w1) of the even and the odd plane
+    __device__ __forceinline__ MaskRange(const int4 dr, int pitch, int plane) {
+        const int e0 = (dr.x + 1) >> 1, e1 = (dr.y + 1) >> 1, o0 = dr.x >> 1, o1 = dr.y >> 1;
+        w0[0] = (e0 * pitch + dr.z) >> 2;
+        w1[0] = e1 > e0 ? ((e1 - 1) * pitch + dr.w + 3) >> 2 : w0[0];
+        w0[1] = (plane + o0 * pitch + dr.z) >> 2;
+        w1[1] = o1 > o0 ? (plane + (o1 - 1) * pitch + dr.w + 3) >> 2 : w0[1];
     }
+};
+
+// Zeroes the cells (16 bytes at f4) of a word of selected scales v that equal the byte `excluded` repeats: a byte's
+// top bit stays exactly where it differs (scales are below 0x80).
+template <int Offset>
+__device__ __forceinline__ void mask_word(unsigned v, unsigned f4, unsigned excluded) {
+    const unsigned keep = ((v ^ excluded) | 0x80808080u) - 0x01010101u;
+    asm volatile(
+        "{\n\t.reg .pred p0, p1, p2, p3;\n\t.reg .b32 t0, t1, t2, t3;\n\t"
+        "and.b32 t0, %1, 0x80;\n\tand.b32 t1, %1, 0x8000;\n\tand.b32 t2, %1, 0x800000;\n\tand.b32 t3, %1, 0x80000000;\n\t"
+        "setp.eq.u32 p0, t0, 0;\n\tsetp.eq.u32 p1, t1, 0;\n\tsetp.eq.u32 p2, t2, 0;\n\tsetp.eq.u32 p3, t3, 0;\n\t"
+        "@p0 st.shared.b32 [%0 + %2], 0;\n\t@p1 st.shared.b32 [%0 + %2 + 4], 0;\n\t@p2 st.shared.b32 [%0 + %2 + 8], 0;\n\t"
+        "@p3 st.shared.b32 [%0 + %2 + 12], 0;\n\t}" ::"r"(f4),
+        "r"(keep), "n"(Offset)
+        : "memory");
 }
+
+// A thread's words of both planes, held in registers over a direction's scales where the range has no more than
+// kHeldWords a thread (sets of radius 31: 95 rows of 191 cells are 2,300 words a plane; 1024^2 464 us with the words
+// read again for every scale, 452 us so).
+constexpr int kHeldWords = 5;
 template <int Threads>
-__device__ __forceinline__ void mask_field(unsigned s_f, unsigned s_s, const int4 rc, unsigned s, int pitch, int plane, int tid) {
-    const unsigned excluded = 0x01010101u * (s - 1);
-    // even rows (rc.x + 1) / 2 .. (rc.y + 1) / 2 of plane 0, odd rows rc.x / 2 .. rc.y / 2 of plane 1; the odd
-    // rows go to the threads from the last one on, which the even rows' last step leaves idle
-    const int e0 = (rc.x + 1) >> 1, e1 = (rc.y + 1) >> 1, o0 = rc.x >> 1, o1 = rc.y >> 1;
-    if (e1 > e0) {
-        const int w = ((e0 * pitch + rc.z) >> 2) + tid, end = ((e1 - 1) * pitch + rc.w + 3) >> 2;
-        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, excluded);
+struct HeldWords {
+    unsigned v[2][kHeldWords];
+    static __device__ __forceinline__ bool fits(const MaskRange &m) {
+        return m.w1[0] - m.w0[0] <= kHeldWords * Threads && m.w1[1] - m.w0[1] <= kHeldWords * Threads;
     }
-    if (o1 > o0) {
-        const int w = ((plane + o0 * pitch + rc.z) >> 2) + (Threads - 1 - tid), end = (plane + (o1 - 1) * pitch + rc.w + 3) >> 2;
-        mask_words<Threads>(s_s + 4 * w, s_s + 4 * end, s_f + 16 * w, excluded);
+    __device__ __forceinline__ void load(const MaskRange &m, unsigned s_s, int tid) {
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int j = 0; j < kHeldWords; j++) {
+                v[p][j] = 0xffffffffu;  // no scale
+                const int w = m.w0[p] + tid + j * Threads;
+                if (w < m.w1[p]) v[p][j] = lds_u1(s_s + 4 * w);
+            }
     }
+    __device__ __forceinline__ void mask(const MaskRange &m, unsigned s_f, int tid, unsigned excluded) const {
+        static_assert(kHeldWords == 5, "one mask_word per word");
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            const unsigned f4 = s_f + 16 * (m.w0[p] + tid);
+            mask_word<0>(v[p][0], f4, excluded);
+            mask_word<16 * Threads>(v[p][1], f4, excluded);
+            mask_word<32 * Threads>(v[p][2], f4, excluded);
+            mask_word<48 * Threads>(v[p][3], f4, excluded);
+            mask_word<64 * Threads>(v[p][4], f4, excluded);
+        }
+    }
+};
+// Ranges of more words: read again for every scale.
+__device__ __forceinline__ void mask_read(const MaskRange &m, unsigned s_f, unsigned s_s, int tid, int nthreads, unsigned excluded) {
+    for (int p = 0; p < 2; p++)
+        for (int w = m.w0[p] + tid; w < m.w1[p]; w += nthreads) mask_word<0>(lds_u1(s_s + 4 * w), s_f + 16 * w, excluded);
 }
 
 // The float2 at shared address a of CTA `rank` of the cluster.
@@ -423,6 +445,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
             else
                 bad = build_field<false, false>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane);
             if (bad) s_flag[d & 1] = 1;
+            HeldWords<nthreads> held;
 #pragma unroll 1
             for (int s = 0; s < a.S; s++) {
                 const int k = d * a.S + s;
@@ -431,7 +454,16 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                     stage(k + 1);
                 else
                     asm volatile("cp.async.commit_group;" ::: "memory");
-                if (s > 0) mask_field<nthreads>(s_f, s_s, a.drect[d], static_cast<unsigned>(s), a.pitch, a.plane, tid);
+                if (s > 0) {
+                    const MaskRange range(dr, a.pitch, a.plane);
+                    const unsigned excluded = 0x01010101u * static_cast<unsigned>(s - 1);
+                    if (HeldWords<nthreads>::fits(range)) {
+                        if (s == 1) held.load(range, s_s, tid);
+                        held.mask(range, s_f, tid, excluded);
+                    } else {
+                        mask_read(range, s_f, s_s, tid, nthreads, excluded);
+                    }
+                }
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // this kernel's block has landed
                 __syncthreads();
                 const bool finite = s_flag[d & 1] == 0;

@@ -85,3 +85,31 @@ def test_non_finite_cotangents_reach_only_their_kernels():
     reach = reach[R:R + H, R:R + W]
     assert reach.any() and not reach.all()
     assert np.array_equal(~np.isfinite(got), reach)
+
+
+@pytest.mark.parametrize("R", [36, 40, 48, 55])
+@pytest.mark.parametrize("W,H", [(64, 32), (150, 141), (33, 200)])
+def test_gather_of_wide_kernels(R, W, H):
+    """Radii past the usual 31: fields of more words than a thread holds, and the 64 x 32 tile."""
+    import torch
+
+    D, S, n = 2, 3, 2 * R + 1
+    rng = np.random.default_rng(R)
+    w = np.zeros((D * S, n, n), np.float32)
+    for d in range(D):
+        for y in range(n):
+            m = int(rng.integers(1, 6))
+            x = int(rng.integers(0, n - m + 1))
+            w[d * S:(d + 1) * S, y, x:x + m] = rng.uniform(0.05, 1.0, (S, m))  # the scales' rows lie alike
+    w /= w.sum((1, 2), keepdims=True)
+    off = np.arange(D * S, dtype=np.int32) * n * n
+    rows = np.full(D * S, n, np.int32)
+    ks = lpaici.KernelSet.from_dense(w.ravel(), off, rows, rows, D, S)
+    ko = ob.DenseKernels(D, S, w.ravel(), off, rows, rows)
+    x = rng.uniform(0.0, 1.0, (H, W)).astype(np.float32)
+    g = rng.standard_normal((H, W)).astype(np.float32)
+    got = lpaici.backward(ks, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda(), 0.1, 1.7).cpu().numpy()
+    var = ks.variances(0.1)
+    _, smap, _ = ob.oracle_forward_f32(x, ko, var, 1.7, want_map=True)
+    ref = ob.oracle_adjoint_f64(ko, var, smap, g.astype(np.float64))
+    assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max() + 1e-6
