@@ -10,7 +10,7 @@
 //   A. selection: the forward's exact tile sweep recomputes s*(d,p) (one byte per direction and
 //      pixel) and writes u = g * (1/den) beside it, into a transient workspace -- the forward stores
 //      nothing for the adjoint (a kept state holds 1/den, and the gather forms the product itself);
-//   B. gather: 128 x 64 output tiles.  Per direction it reads s*(d,.) and u on the tile plus its R-pixel
+//   B. gather: 128 x 64 output tiles (128 x 32 or 64 x 32 for kernels that leave no room).  Per direction it reads s*(d,.) and u on the tile plus its R-pixel
 //      halo (from L2) and forms the field c_d = u / v_{d,s*} in shared memory.
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
 //      turns the sum over scales into
@@ -559,8 +559,9 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
 }
 
 const void *gather_fn(const AdjointLayout &L) {
-    return L.wx == 4 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2>)
-                     : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1>);
+    return L.wx == 2   ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1>)
+           : L.wy == 1 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 1>)
+                       : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2>);
 }
 
 int gather_threads(const AdjointLayout &L) { return kGatherGroups * 32 * L.wx * L.wy; }

@@ -104,7 +104,7 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
     L.limit_bytes = 4 * (static_cast<size_t>(limit_words) + ((nk + 3) & ~3)) + 4 * limit_cells + ((limit_cells + 4 + 15) & ~size_t(15));
 
     // units and weights of every kernel; the offsets of a unit's field rows need the tile's geometry, and the
-    // tile needs the largest block: 128 x 64 outputs if that fits on an SM, else 64 x 32
+    // tile needs the largest block: 128 x 64 outputs if that fits on an SM, else 128 x 32 or 64 x 32
     struct Unit {
         int row, col, len;
     };
@@ -134,19 +134,31 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
             int row_of[2] = {-1, -1};  // the runs of rows j and j - 1
             for (int q = r; q < begin[k + 1] && rdy[q] <= j; q++) row_of[rdy[q] == j ? 0 : 1] = q;
             if (row_of[0] < 0 && row_of[1] < 0) continue;
-            int c0 = 1 << 30, c1 = -(1 << 30);
-            for (const int q : row_of)
-                if (q >= 0) {
-                    c0 = std::min(c0, rdx[q]);
-                    c1 = std::max(c1, rdx[q] + rlen[q]);
-                }
-            units[k].push_back({j, c0, c1 - c0});
-            for (int c = c0; c < c1; c++)
-                for (const int q : row_of) {
-                    const bool tap = q >= 0 && c >= rdx[q] && c < rdx[q] + rlen[q];
-                    const float v = tap ? w[first_w[q - begin[k]] + c - rdx[q]] : 0.0f;
-                    pairs[k].push_back(tap ? (v == 0.0f ? 0.0f : v) : -0.0f);  // -0 marks padding only
-                }
+            // one unit over the columns of both rows, or (rows that hardly overlap) one for each row: a unit costs
+            // about as much as a tap and a half beside its taps
+            const auto first_col = [&](int q) { return rdx[q]; };
+            const auto past_col = [&](int q) { return rdx[q] + rlen[q]; };
+            const bool both = row_of[0] >= 0 && row_of[1] >= 0;
+            int hull = 0;
+            if (both)
+                hull = std::max(past_col(row_of[0]), past_col(row_of[1])) - std::min(first_col(row_of[0]), first_col(row_of[1]));
+            const bool apart = both && hull > rlen[row_of[0]] + rlen[row_of[1]] + 1;
+            for (int part = 0; part < (apart ? 2 : 1); part++) {
+                const int in_unit[2] = {apart && part == 1 ? -1 : row_of[0], apart && part == 0 ? -1 : row_of[1]};
+                int c0 = 1 << 30, c1 = -(1 << 30);
+                for (const int q : in_unit)
+                    if (q >= 0) {
+                        c0 = std::min(c0, first_col(q));
+                        c1 = std::max(c1, past_col(q));
+                    }
+                units[k].push_back({j, c0, c1 - c0});
+                for (int c = c0; c < c1; c++)
+                    for (const int q : in_unit) {
+                        const bool tap = q >= 0 && c >= rdx[q] && c < rdx[q] + rlen[q];
+                        const float v = tap ? w[first_w[q - begin[k]] + c - rdx[q]] : 0.0f;
+                        pairs[k].push_back(tap ? (v == 0.0f ? 0.0f : v) : -0.0f);  // -0 marks padding only
+                    }
+            }
         }
         const int bytes = static_cast<int>(8 * units[k].size() + 4 * pairs[k].size());
         L.block_bytes = std::max(L.block_bytes, (bytes + 15) & ~15);
@@ -154,9 +166,9 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         L.taps += static_cast<int>(pairs[k].size() / 2);
     }
     constexpr size_t kSharedPerCta = 232448;  // sm_100a
-    for (const int wide : {1, 0}) {
-        L.wx = wide ? 4 : 2;
-        L.wy = wide ? 2 : 1;
+    for (const int size : {2, 1, 0}) {
+        L.wx = size > 0 ? 4 : 2;
+        L.wy = size > 1 ? 2 : 1;
         L.pitch = (32 * L.wx + 2 * R) | 1;
         L.plane = ((32 * L.wy + 2 * R + 1) / 2 * L.pitch + 3) & ~3;
         const size_t sums = 8 * 16 * 2 * static_cast<size_t>(32 * L.wx * L.wy);
