@@ -36,9 +36,10 @@ int default_config(const lpaici_kernelset *ks) {
 // taps, a kernel's interval update about 5 (measured with synthetic kernel sets of one run length).
 struct TileCost {
     float base_us, ns_per_work;
+    int ctas = 1;  // CTAs per SM of the fit
 };
 static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{8.7f, 59.7f}, {8.1f, 31.2f}, {7.3f, 25.0f}, {4.2f, 15.8f},
-                                                            {2.9f, 8.35f}, {0.6f, 4.58f}, {1.2f, 2.60f}, {0.5f, 26.1f},
+                                                            {2.9f, 8.35f}, {0.6f, 4.58f}, {1.2f, 2.60f, 2}, {0.5f, 26.1f},
                                                             {9.0f, 47.3f}, {9.8f, 36.9f}, {4.8f, 19.5f}};
 
 static int groups_of(int c) {
@@ -52,8 +53,9 @@ static int groups_of(int c) {
 }
 
 // The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; 97 x 64 takes 22.6 us with the
-// symmetric set and 28.7 us with the tapered one, 128 x 128 28.7 and 36.9 us, of which a launch is 3.6 us).
-static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{10.0f, 1.05f}, {14.0f, 1.30f}};
+// symmetric set and 28.7 us with the tapered one, 128 x 128 28.7 and 36.9 us, 150 x 120 30.8 and 45.1 us, of which a
+// launch is 3.6 us).
+static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{10.0f, 1.05f}, {14.0f, 1.30f}, {9.5f, 2.2f}};
 
 static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int ds) {
     const int nk = ks->D * ks->S;
@@ -136,8 +138,8 @@ static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
         if (!known) pc->bps[c] = cached_bps(ks, dev, c, pc->max_smem);
         if (pc->bps[c] <= 0)
             pc->tile_ms[c] = 0.0f;
-        else if (!pc->tuned)
-            pc->tile_ms[c] = estimated_tile_ms(ks, c);
+        else if (!pc->tuned)  // (one CTA where the fit had two: 1.5 tile times, as for a lone one below)
+            pc->tile_ms[c] = estimated_tile_ms(ks, c) * (pc->bps[c] < kTileCost[c].ctas ? 1.5f : 1.0f);
     }
     return true;
 }

@@ -36,8 +36,9 @@
 // X(index, WX, WY, Q, DS, C)
 #define LPAICI_CLUSTERS(X) \
     X(0, 1, 1, 4, 4, 4)    \
-    X(1, 1, 1, 8, 4, 4)
-#define LPAICI_NUM_CLUSTERS 2
+    X(1, 1, 1, 8, 4, 4)    \
+    X(2, 1, 1, 8, 8, 2)
+#define LPAICI_NUM_CLUSTERS 3
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.
