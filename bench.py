@@ -60,10 +60,10 @@ SEED = 20250910
 SIZE = 4096
 # DRAM bytes of one forward launch on the 4096^2 workload, read + written, from the ncu capture in
 # profiles/forward_4096_sym.md (dram__bytes_read.sum + dram__bytes_write.sum; the halo re-reads are
-# served by L2), valid for the tile configurations listed (the two 768-thread shapes, which stage the
-# same halo'd tiles): reported only when the run uses one of them at that size.
-FORWARD_DRAM_BYTES = 95.0e6
-FORWARD_DRAM_CONFIGS = (9, 10)
+# served by L2), valid for the tile configurations listed: reported only when the run uses one of them at
+# that size.
+FORWARD_DRAM_BYTES = 92.4e6
+FORWARD_DRAM_CONFIGS = (0,)
 
 
 def kernel_path(name: str, tmp: str) -> str:
@@ -214,6 +214,33 @@ def time_launches(torch, fn, steps: int, warmup: int, flush) -> list[float]:
         e1.synchronize()
         ms.append(e0.elapsed_time(e1))
     return ms
+
+
+def launches_of(torch, fn) -> int:
+    """Kernels that one call of fn() launches: the nodes of the CUDA graph it is captured into (an image
+    whose last wave is taken by smaller tiles is two launches)."""
+    import ctypes
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    n = ctypes.c_size_t(0)
+    rc = ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None,
+                                                          ctypes.byref(n))
+    if rc != 0:
+        raise RuntimeError(f"cudaGraphGetNodes: error {rc}")
+    return n.value
+
+
+REFERENCE_MISSING = "oracle/_ref/libref_v1_0.so or libref_v0_0.so not built (no reference sources here)"
+
+
+def reference_built() -> bool:
+    """Whether the reference's CPU engines are compiled here (oracle/Makefile, from its sources)."""
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import oracle_bind as ob
+
+    return ob.ref_available("v1_0") and ob.ref_available("v0_0")
 
 
 def cpu_reference_sample(noisy: np.ndarray, crop: int, threads: int, sigma: float, gamma: float, seed: int = 0,
@@ -376,6 +403,9 @@ def host_threads() -> int:
 def run_reference(args, rank: int, world: int) -> None:
     if rank != 0:
         return
+    if not reference_built():
+        print(json.dumps({"impl": "reference", "unavailable": REFERENCE_MISSING}), flush=True)
+        return
     threads = host_threads()
     _, noisy = reference_bench_image(SIZE, SEED, SIGMA)
     for _ in range(args.warmup):
@@ -430,6 +460,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     del smap
 
     fwd = lambda: lpaici.forward(ks, x, SIGMA, GAMMA, out=out)  # noqa: E731
+    step_launches = launches_of(torch, fwd)
     clocks = Clocks(local_rank)
     clocks.start()
     for _ in range(args.warmup):
@@ -522,7 +553,9 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
         extra["reference_gpu_v4_1"] = ref_gpu
 
     cpu = parity = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not reference_built():
+        cpu = {"unavailable": REFERENCE_MISSING}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = host_threads()
         v, s, kept = cpu_reference_sample(noisy_h, 256, threads, SIGMA, GAMMA, keep=True)
         parity = crop_parity(out.cpu().numpy(), kept, ks.radius)
@@ -545,7 +578,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     tw, th, thr, ppt = lpaici.tile_configs()[best]
     traffic = FORWARD_DRAM_BYTES if (size == SIZE and best in FORWARD_DRAM_CONFIGS) else None
     traffic_note = ("bytes per launch, dram__bytes_read.sum + dram__bytes_write.sum: a constant from the ncu capture "
-                    "in profiles/forward_4096_sym.md (67.8 MB read + 27.2 MB written; algorithmic 134.2 MB: 4 B in "
+                    "in profiles/forward_4096_sym.md (67.4 MB read + 25.0 MB written; algorithmic 134.2 MB: 4 B in "
                     "+ 4 B out per pixel), not measured by this run")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -574,7 +607,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
         "cpu_baseline": cpu,
         "e2e": {"value": world * px / e2e_step / 1e6, "unit": UNIT, "h2d_bytes_per_step": px * 4,
                 "d2h_bytes_per_step": px * 4},
-        "gpu_launches": args.steps,
+        "gpu_launches": args.steps * step_launches,
         "clocks": clk,
         "parity": parity,
         "extra": extra,
@@ -712,7 +745,7 @@ def run_extras(torch, lpaici, ks, args, flush, peak) -> dict:
                     "value": m * 1024 * 1024 / (np.mean(ab_ms) * 1e-3) / 1e6,
                     "forward_same_images": m * 1024 * 1024 / (np.mean(fb_ms) * 1e-3) / 1e6,
                     "adjoint_over_forward_time": float(np.mean(ab_ms) / np.mean(fb_ms)),
-                    "how": "batched plans (selection, u = g/den and gather: one launch each; one forward "
+                    "how": "batched plans (selection with u = g/den, and gather; one forward "
                            "launch), CUDA graphs",
                     "bit_equal_to_single": bool(batched_same),
                     "single_image_calls": {"value": m * 1024 * 1024 / (np.mean(a_ms) * 1e-3) / 1e6,

@@ -181,7 +181,7 @@ int lpaici_forward_channels(const lpaici_kernelset *ks, const float *d_noisy, in
                             int out_pitch, int width, int height, int channels, float sigma, float gamma,
                             lpaici_stream_t stream);
 
-/* ---- batched forward: images of uneven sizes, sigmas and gammas in one launch ---------------- */
+/* ---- batched forward: images of uneven sizes, sigmas and gammas, planned together -------- */
 typedef struct {
     const float *noisy;  /* device, width x height, pitch noisy_pitch floats */
     float *denoised;     /* device, width x height, pitch out_pitch floats */
@@ -192,9 +192,9 @@ typedef struct {
 
 typedef struct {
     int use_graph;   /* nonzero: capture the launch sequence in a CUDA graph at plan time, replay on run */
-    int tile_config; /* -1: the configuration expected fastest for these images (per-tile times, autotuned
-                      * or built in, times the waves of the whole tile queue); else an index
-                      * < lpaici_num_tile_configs() */
+    int tile_config; /* -1: the configuration, or the mix of two, expected fastest for these images (from
+                      * per-tile times, autotuned or built in, and the waves of all images' tiles); else an
+                      * index < lpaici_num_tile_configs() */
 } lpaici_batch_options;
 
 typedef struct lpaici_batch lpaici_batch;
@@ -270,12 +270,11 @@ typedef struct {
 
 typedef struct lpaici_backward_batch lpaici_backward_batch;
 
-/* Plans the adjoint of many images: pass A (selection) as one launch over all images'
- * tiles (the forward batch kernel writing s* and 1/den into memory the plan owns, D+4 bytes per
- * pixel), u = g/den over the plan's 1/den maps as one elementwise launch, pass B (gather) as one launch
- * over all images' tiles; with use_graph all three are captured in one CUDA graph.  Gradients equal lpaici_backward's, image by image, bit for bit.  The pointers are
- * baked in: rerun when the contents change, re-plan when the pointers change.  No counterpart in the
- * reference. */
+/* Plans the adjoint of many images: pass A (selection) as the forward batch's launches over all images'
+ * tiles (writing s* and u = g/den into memory the plan owns, D+4 bytes per pixel), pass B (gather) as one
+ * launch over all images' tiles; with use_graph they are captured in one CUDA graph.  Gradients equal
+ * lpaici_backward's, image by image, bit for bit.  The pointers are baked in: rerun when the contents
+ * change, re-plan when the pointers change.  No counterpart in the reference. */
 int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lpaici_grad_image *images, int n,
                                  const lpaici_batch_options *opts, lpaici_stream_t stream,
                                  lpaici_backward_batch **out);

@@ -10,13 +10,15 @@
 //   A. selection: the forward's exact tile sweep recomputes s*(d,p) (one byte per direction and
 //      pixel) and writes u = g * (1/den) beside it, into a transient workspace -- the forward stores
 //      nothing for the adjoint (a kept state holds 1/den, and the gather forms the product itself);
-//   B. gather: 128 x 64 output tiles (128 x 32 or 64 x 32 for kernels that leave no room).  Per direction it reads s*(d,.) and u on the tile plus its R-pixel
-//      halo (from L2) and forms the field c_d = u / v_{d,s*} in shared memory.
+//   B. gather: 128 x 64 output tiles (128 x 32 or 64 x 32 for kernels that leave no room).  Per direction
+//      it reads s*(d,.) and u on the tile plus its R-pixel halo (from L2) and forms the field
+//      c_d = u / v_{d,s*} in shared memory.
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
 //      turns the sum over scales into
 //          sum_s D_s (*) (c_d [s* >= s]):
-//      the field is zeroed in place where s* < s, scale after scale, and never rebuilt.  Two groups of warps take every other unit of each kernel over the same
-//      outputs.  Every output is written once: no atomics, deterministic.
+//      the field is zeroed in place where s* < s, scale after scale, and never rebuilt.  Two groups of
+//      warps take every other unit of each kernel over the same outputs.  Every output is written once: no
+//      atomics, deterministic.
 //
 // Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
 // zero (its units in order), the chunks' sums are added in order, and group 1's total is added to group 0's.

@@ -1,16 +1,17 @@
-// batched.cu -- many images of uneven sizes, sigmas and gammas in one launch.
+// batched.cu -- many images of uneven sizes, sigmas and gammas, planned together.
 //
-// The plan cuts every image into the tiles of one tile configuration and orders the tiles into a
-// single work queue, full tiles of the largest images first and partial edge tiles last, so the
-// cheap ragged tiles fill the tail.  The launch has one CTA per queue item: the hardware dispatches
-// blocks in index order as SMs free up, so the queue order is the execution order without a
-// persistent loop (measured: a persistent grid pulling items from an atomic counter kept its
-// 768-thread instances at the 80-register limit and ran 2-2.5 % slower).  There is no inter-CTA
-// waiting of any kind.  With use_graph the launch is captured once into a CUDA graph and replayed
-// by lpaici_batch_run.  A plan of one image launches the single-image kernel instead (image and tables
-// as launch parameters): there are no small-image tails to fill, and the queue decode would cost a
-// little per CTA.  A plan of up to kMaxMultiImages images of one size, pitch, sigma and gamma launches
-// that kernel once with a grid layer per image (lpaici_forward_multi_kernel).
+// The plan (plan_for_images) takes one tile configuration, or a mix: big tiles where whole ones fit, in
+// whole waves, and small tiles for the rest, as a second launch that starts while the first one's last
+// tiles run (programmatic dependent launch; the two write different tiles).  Each launch has one CTA per
+// item {image, x0, y0}, full tiles of the largest images first and partial edge tiles last: the hardware
+// dispatches blocks in index order as SMs free up, so the queue order is the execution order without a
+// persistent loop (a persistent grid pulling items from an atomic counter ran 2-2.5 % slower).  Ten mixed
+// images of 4.9 Mpx in all: one configuration 2.51 ms, both tiles in one kernel 2.19, two launches 2.12.
+// No CTA waits for another.  With use_graph the launches are captured once into a CUDA graph and replayed
+// by lpaici_batch_run.  A plan of one image launches the single-image kernel instead (image and tables as
+// launch parameters): there are no small-image tails to fill, and the item's decode would cost a little
+// per CTA.  A plan of up to kMaxMultiImages images of one size, pitch, sigma and gamma launches that
+// kernel with a grid layer per image (lpaici_forward_multi_kernel).
 // No reference counterpart: the reference denoises one image per process
 // (src/v4_1_lpa_ici_2D_sparse_shared.cu:365-530).
 #include <algorithm>

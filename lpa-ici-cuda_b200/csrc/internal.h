@@ -188,7 +188,7 @@ struct BatchSpec {
 // config < 0: chosen for the images (plan_for, plan_for_images).
 int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n, int config, bool use_graph,
                       cudaStream_t stream, lpaici_batch **out);
-int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream);  // queue reset + persistent launch
+int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream);  // the launch, or the launch and the rest's
 void batch_plan_free(lpaici_batch *b);
 
 // The adjoint's two passes over storage the caller provides: device copies of ks->blob and ks->adj_blob,

@@ -33,9 +33,10 @@
 //   - shared memory is read by 32-bit shared addresses (ld.shared in PTX): generic pointers cost a third
 //     of the uniform instructions per run.
 // 4096^2, 16 x 7 symmetric kernels: 8.15 ms before (Q = 4, 64 x 96 tiles, 103 warp instructions per run of
-// a 256-pixel warp), 6.84 ms now (128 x 64 tiles, 144 per run of a 512-pixel warp; with descriptors and weights
-// behind pointers of their own 7.04 ms); the packed arithmetic alone would take 5.3 ms.  Per tile of 8,192 pixels and 16 warps: 32 cycles a tap (the packed arithmetic's
-// own), about 45 a run and 150 an interval update.
+// a 256-pixel warp), 6.84 ms now (128 x 64 tiles, 144 per run of a 512-pixel warp; with descriptors and
+// weights behind pointers of their own 7.04 ms); the packed arithmetic alone would take 5.3 ms.  Per tile of
+// 8,192 pixels and 16 warps: 32 cycles a tap (the packed arithmetic's own), about 45 a run and 150 an
+// interval update.
 //
 // Arithmetic (bit-identical to src/v1_0_lpa_ici_2D_fused.cpp:803-930 for finite inputs):
 //   conv  = sum over the kernel's taps in row-major order of w*x (rounded), added one by one with

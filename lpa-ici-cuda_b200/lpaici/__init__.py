@@ -433,7 +433,7 @@ def backward(ks: KernelSet, noisy, grad_out, sigma: float, gamma: float, grad_in
 
 
 class Batch:
-    """A planned batch of images (lpaici_batch): one persistent launch over a shared tile queue,
+    """A planned batch of images (lpaici_batch): one or two launches over all images' tiles,
     optionally replayed from a CUDA graph."""
 
     def __init__(self, ks: KernelSet, noisy: Sequence, outs: Sequence, sigmas: Sequence[float],
@@ -477,8 +477,8 @@ class Batch:
 
 
 class BackwardBatch:
-    """A planned batched adjoint (lpaici_backward_batch): selection of all images in one persistent
-    launch, gather of all images' tiles in one launch, optionally replayed from a CUDA graph."""
+    """A planned batched adjoint (lpaici_backward_batch): selection of all images in one or two
+    launches, gather of all images' tiles in one launch, optionally replayed from a CUDA graph."""
 
     def __init__(self, ks: KernelSet, noisy: Sequence, grad_out: Sequence, grad_in: Sequence,
                  sigmas: Sequence[float], gammas: Sequence[float], use_graph: bool = True, tile_config: int = -1):
