@@ -332,22 +332,29 @@ __device__ __forceinline__ void stage_tables(float *s_tab, const float *var, con
 // (gy0 + j + TH/2, gx0 + c), gy0 = y0 + row_begin - R, gx0 = x0 - R.  Asynchronous 4-byte copies straight
 // into the interleaved pairs (no alignment asked of the image, zeros where it ends): no load latency is
 // waited for until tile_wait, and the kernel set is staged meanwhile (16 x 16 tiles: 22.4 us a tile, 24.0
-// with plain loads; 128 x 64: 503 us, 508).
+// with plain loads; 128 x 64: 503 us, 508).  A lane keeps its column and walks down the rows, four rows of
+// copies at a time: with few warps on an SM the copies' addresses, not the memory, are what takes time (97 x
+// 64 in clusters 20.6 us with a row's pointers formed per copy, 18.9 us so; 1535 x 1021 691 and 683 us).
 __device__ __forceinline__ void load_tile(float2 *s_tile, const ImageArgs &img, int x0, int y0, const TileGeom &g) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int gy0 = y0 + img.row_begin - g.R, gx0 = x0 - g.R;
-    for (int j = warp; j < g.pairs; j += nwarps) {
-        const int ga = gy0 + j, gb = ga + g.half;
-        const bool ok_a = ga >= 0 && ga < img.in_h, ok_b = gb >= 0 && gb < img.in_h;
-        const float *ra = img.in + static_cast<size_t>(ok_a ? ga : 0) * img.in_pitch;
-        const float *rb = img.in + static_cast<size_t>(ok_b ? gb : 0) * img.in_pitch;
-        const unsigned dst = smem_addr(s_tile + j * g.pitch2);
-        for (int c = lane; c < g.pitch2; c += 32) {
-            const int gx = gx0 + c;
-            const bool ok_x = gx >= 0 && gx < img.W;
-            const size_t at = static_cast<size_t>(ok_x ? gx : 0) * img.step;
-            copy_or_zero(dst + 8 * c, ra + at, ok_a && ok_x);
-            copy_or_zero(dst + 8 * c + 4, rb + at, ok_b && ok_x);
+    const ptrdiff_t down = static_cast<ptrdiff_t>(g.half) * img.in_pitch, next = static_cast<ptrdiff_t>(nwarps) * img.in_pitch;
+    for (int c = lane; c < g.pitch2; c += 32) {
+        const int gx = gx0 + c;
+        const bool ok_x = gx >= 0 && gx < img.W;
+        const int in_h = ok_x ? img.in_h : 0;
+        int row = gy0 + warp;
+        const float *src = img.in + static_cast<ptrdiff_t>(row) * img.in_pitch + static_cast<ptrdiff_t>(gx) * img.step;
+        unsigned dst = smem_addr(s_tile + warp * g.pitch2 + c);
+#pragma unroll 4
+        for (int j = warp; j < g.pairs; j += nwarps) {
+            const bool ok_a = static_cast<unsigned>(row) < static_cast<unsigned>(in_h);
+            const bool ok_b = static_cast<unsigned>(row + g.half) < static_cast<unsigned>(in_h);
+            copy_or_zero(dst, ok_a ? src : img.in, ok_a);
+            copy_or_zero(dst + 4, ok_b ? src + down : img.in, ok_b);
+            row += nwarps;
+            src += next;
+            dst += 8 * nwarps * g.pitch2;
         }
     }
 }
