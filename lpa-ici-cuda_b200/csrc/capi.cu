@@ -52,10 +52,9 @@ static int groups_of(int c) {
 #undef LPAICI_GROUPS_CASE
 }
 
-// The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; 97 x 64 takes 22.6 us with the
-// symmetric set and 28.7 us with the tapered one, 128 x 128 28.7 and 36.9 us, 150 x 120 30.8 and 45.1 us, of which a
-// launch is 3.6 us).
-static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{10.0f, 1.05f}, {14.0f, 1.30f}, {9.5f, 2.2f}};
+// The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; back to back 97 x 64 takes 12.8 us
+// with the symmetric set and 17.3 us with the tapered one, 128 x 128 17.0 and 24.1 us, 150 x 120 22.7 and 36.2 us).
+static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{5.3f, 0.72f}, {6.4f, 1.12f}, {4.2f, 2.1f}};
 
 static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int ds) {
     const int nk = ks->D * ks->S;

@@ -116,10 +116,11 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
 }
 
 // An image of a few tiles: C CTAs of a cluster share each tile's directions, as the groups of a CTA do.  Each
-// stages only the runs of its directions if one round covers them all.  97 x 64, 16 x 7 symmetric set: 36.9 us
-// with one CTA per 16 x 16 tile, 22.6 us with four.
+// stages only the runs of its directions if one round covers them all.  A group is one warp and its helper
+// (SweepSplit).  97 x 64, 16 x 7 symmetric set: 36.9 us with one CTA per 16 x 16 tile, 22.6 us with four, 15.0 us
+// with helpers.
 template <int WX, int WY, int Q, int DS, int C, bool Fused>
-__global__ void __launch_bounds__(32 * WX * WY * DS, 1)
+__global__ void __launch_bounds__(2 * 32 * WX * WY * DS, 1)
     lpaici_forward_cluster_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
     extern __shared__ __align__(16) int smem[];
     using Shape = TileShape<WX, WY, Q, DS>;
@@ -127,12 +128,12 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
     const int across = (img.W + Shape::kTileW - 1) / Shape::kTileW;
     const int x0 = (tile % across) * Shape::kTileW, y0 = (tile / across) * Shape::kTileH;
     const SweepCta<WX, WY, Q, DS> cta(smem, tab.blob_words, nk, tab.R);
-    load_tile(cta.tile, img, x0, y0, cta.g);
     int from = 0, to = 1 << 30;
     if (tab.D <= DS * C) {
         from = __ldg(tab.blob + min(tab.D, rank * DS) * tab.S);
         to = __ldg(tab.blob + min(tab.D, (rank + 1) * DS) * tab.S);
     }
+    load_tile(cta.tile, img, x0, y0, cta.g);
     stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.mask_word, tab.stream_word, cta.g.pitch2, from, to);
     stage_tables(cta.tab, tab.var, tab.thr, nk);
     tile_wait();
@@ -143,10 +144,16 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
 
 namespace {
 
+template <class Shape, int Q, int DS>
+size_t cluster_smem(int blob_words, int nk, int radius) {
+    return sweep_smem<Shape, Q>(blob_words, nk, radius) + sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS;
+}
+
 template <int WX, int WY, int Q, int DS, int C, bool Fused>
 int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t stream) {
     using Shape = TileShape<WX, WY, Q, DS>;
-    const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
+    static_assert(Shape::kRegion == 32, "a group is one warp and its helper");
+    const size_t smem = cluster_smem<Shape, Q, DS>(tab.blob_words, tab.D * tab.S, tab.R);
     auto kern = lpaici_forward_cluster_kernel<WX, WY, Q, DS, C, Fused>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, clusters)");
@@ -157,7 +164,7 @@ int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t s
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles) * C);
-    cfg.blockDim = dim3(Shape::kThreads);
+    cfg.blockDim = dim3(2 * Shape::kThreads);  // every warp has a helper
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
@@ -359,7 +366,7 @@ void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, 
         *tile_h = 16 * (WY);                                                       \
         *ctas = C;                                                                 \
         *groups = (DS) * (C);                                                      \
-        *smem = sweep_smem<TileShape<WX, WY, Q, DS>, Q>(blob_words, nk, radius);   \
+        *smem = cluster_smem<TileShape<WX, WY, Q, DS>, Q, DS>(blob_words, nk, radius); \
         return;
     switch (index) { LPAICI_CLUSTERS(LPAICI_CLUSTER_CASE) }
 #undef LPAICI_CLUSTER_CASE

@@ -365,16 +365,41 @@ __device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_all;" 
 template <int Q>
 __device__ __forceinline__ float pick(const float2 (&v)[Q], int i) { return (i & 1) ? v[i >> 1].y : v[i >> 1].x; }
 
+// Two warps share a direction of a cluster's tile (SweepSplit): the second one, its helper, convolves the scales
+// from `first` on (the last one or two) while the other sweeps those before it, and hands the sums over in
+// shared memory.  There is one warp to a scheduler otherwise, which waits for its own results most of the time
+// (26,800 cycles for the slowest direction of 97 x 64, 6,000 of them packed arithmetic), and the largest scales
+// are half of a direction's work.  97 x 64 18.9 -> 12.8 us, 128 x 128 23.6 -> 17.0, 150 x 120 27.2 -> 22.7; tapered
+// set 25.0 -> 17.3, 32.9 -> 24.1, 41.9 -> 36.2 (with the exchange's loads ahead of its sums).
+constexpr int kHelperScales = 2;
+struct SweepSplit {
+    int first;      // scale; S: no helper
+    unsigned sums;  // shared address of the lane's first pair; a pair of the next column is kRegion pairs on
+    unsigned pair;  // named barrier of the two warps
+};
+// The first scale of direction d's helper: both warps' parts of the stream as equal as they get.
+__device__ __forceinline__ int helper_first(unsigned kernel_table, int d, int S) {
+    if (S < 2) return S;
+    const unsigned at = kernel_table + 4 * d * S;
+    const unsigned begin = lds_u1(at), end = lds_u1(at + 4 * S), last = lds_u1(at + 4 * (S - 1));
+    if (S == 2) return 1;
+    const unsigned before = lds_u1(at + 4 * (S - 2));
+    return max(before - begin, end - before) < max(last - begin, end - last) ? S - 2 : S - 1;
+}
+__device__ __forceinline__ void pair_arrive(unsigned id) { asm volatile("barrier.cta.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void pair_wait(unsigned id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
+
 // The ICI scale sweep of direction d for the thread's 2Q pixels (mask `valid`): per pixel the estimate
 // of the last accepted scale (best) and that scale's index (4 bits per pixel in sidx, 8 pixels a word).
 // The intersection [lo, hi] only shrinks, so once it is empty no later scale can be accepted: a stopped
 // pixel needs no mask, its updates simply never accept again; a pixel outside the image starts with an
 // empty intersection.  Scale 0 is always accepted (lo = -inf, hi = +inf before it), so the index is the
 // count of accepted scales after it.  Warp-uniform scale loop; it ends when no pixel of the warp accepts.
-template <int Q, class Tap>
+template <int Q, bool Split, class Tap>
 __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, unsigned lane_base, unsigned kernel_table,
                                                 unsigned thr_addr, const Tap &tap, float2 (&best)[Q],
-                                                unsigned (&sidx)[Q / 4]) {
+                                                unsigned (&sidx)[Q / 4], const SweepSplit &split = {}) {
+    [[maybe_unused]] bool waited = false;
     float lo[2 * Q], hi[2 * Q];
     unsigned next = kernel_table + 4 * d * S;
     unsigned thr_at = thr_addr + 4 * d * S;
@@ -386,12 +411,19 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
         float2 acc[Q];
 #pragma unroll
         for (int m = 0; m < Q; m++) acc[m] = make_float2(0.0f, 0.0f);
-        next += 4;
-        const unsigned end = lds_u1(next);
-        if (at != end) {
+        if (!Split || s < split.first) {
+            next += 4;
+            const unsigned end = lds_u1(next);
+            if (at != end) {
 #pragma unroll 1
-            do conv_taps<Q>(acc, lane_base, at, tap);
-            while (at != end);
+                do conv_taps<Q>(acc, lane_base, at, tap);
+                while (at != end);
+            }
+        } else {
+            if (!waited) pair_wait(split.pair);
+            waited = true;
+#pragma unroll
+            for (int m = 0; m < Q; m++) acc[m] = lds2(split.sums + 8 * 32 * ((s - split.first) * Q + m));
         }
         const float thr = lds1(thr_at);
         thr_at += 4;
@@ -432,6 +464,35 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
         for (int i = 0; i < Q / 4; i++) changed |= was[i] ^ sidx[i];
         if (!__any_sync(0xffffffffu, changed != 0)) break;  // every pixel of the warp has stopped
     }
+    if constexpr (Split)
+        if (!waited) pair_wait(split.pair);
+}
+
+// The helper's part: the sums of the scales from split.first on.
+template <int Q, class Tap>
+__device__ __forceinline__ void helper_sweep(int d, int S, unsigned lane_base, unsigned kernel_table, const Tap &tap,
+                                             const SweepSplit &split) {
+    unsigned next = kernel_table + 4 * (d * S + split.first);
+    unsigned at = lds_u1(next), to = split.sums;
+#pragma unroll 1
+    for (int s = split.first; s < S; s++) {
+        float2 acc[Q];
+#pragma unroll
+        for (int m = 0; m < Q; m++) acc[m] = make_float2(0.0f, 0.0f);
+        next += 4;
+        const unsigned end = lds_u1(next);
+        if (at != end) {
+#pragma unroll 1
+            do conv_taps<Q>(acc, lane_base, at, tap);
+            while (at != end);
+        }
+#pragma unroll
+        for (int m = 0; m < Q; m++) {
+            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(acc[m].x), "f"(acc[m].y) : "memory");
+            to += 8 * 32;
+        }
+    }
+    pair_arrive(split.pair);
 }
 
 // The forward sweep of one tile (blob, tables and tile in shared memory, block-synchronised).
@@ -472,7 +533,9 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
     };
     // the group is the same in every lane of a warp: reduced, the compiler knows it warp-uniform, so the run
     // loops branch without reconvergence bookkeeping
-    const int group = DS == 1 ? 0 : static_cast<int>(__reduce_max_sync(0xffffffffu, threadIdx.x / Shape::kRegion));
+    const int groups_warp = DS == 1 ? 0 : static_cast<int>(__reduce_max_sync(0xffffffffu, threadIdx.x / Shape::kRegion));
+    const bool helper = C > 1 && groups_warp >= DS;
+    const int group = helper ? groups_warp - DS : groups_warp;
     const int nk = D * S;
     unsigned valid = 0, lane_base;
     {
@@ -513,13 +576,29 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
             else
                 __syncthreads();
         }
-        if (d < D && work) {
+        if (helper && d < D && work) {
+            const SweepSplit split{helper_first(kernel_table, d, S),
+                                   smem_addr(s_xch) + static_cast<unsigned>(Shape::kXchBytes) +
+                                       8 * (group * kHelperScales * Q * 32 + threadIdx.x % 32),
+                                   1u + group};
+            if constexpr (Fused)
+                helper_sweep<Q>(d, S, lane_base, kernel_table, FmaTap{}, split);
+            else
+                helper_sweep<Q>(d, S, lane_base, kernel_table, ExactTap{nz}, split);
+        } else if (d < D && work) {
             float2 best[Q];
             unsigned sidx[Q / 4];
+            SweepSplit split{};
+            if constexpr (C > 1) {
+                split.first = helper_first(kernel_table, d, S);
+                split.sums = smem_addr(s_xch) + static_cast<unsigned>(Shape::kXchBytes) +
+                             8 * (group * kHelperScales * Q * 32 + threadIdx.x % 32);
+                split.pair = 1 + group;
+            }
             if constexpr (Fused)
-                direction_sweep<Q>(d, S, valid, lane_base, kernel_table, thr_addr, FmaTap{}, best, sidx);
+                direction_sweep<Q, (C > 1)>(d, S, valid, lane_base, kernel_table, thr_addr, FmaTap{}, best, sidx, split);
             else
-                direction_sweep<Q>(d, S, valid, lane_base, kernel_table, thr_addr, ExactTap{nz}, best, sidx);
+                direction_sweep<Q, (C > 1)>(d, S, valid, lane_base, kernel_table, thr_addr, ExactTap{nz}, best, sidx, split);
             const unsigned rd = rvar_addr + 4 * d * S;
 #pragma unroll
             for (int m = 0; m < Q; m++) {
@@ -564,29 +643,37 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
                 cluster_barrier();
             else
                 __syncthreads();
-            if (owner * kOwn < 2 * Q && work) {
+            if (owner * kOwn < 2 * Q && work && !helper) {
                 const float *x = s_xch + owner * kOwn * Shape::kRegion + threadIdx.x % Shape::kRegion;
+                // all loads before the first sum: one latency a round instead of one per group
+                float nu[kGroups][kOwn], de[kGroups][kOwn];
 #pragma unroll
-                for (int e = 0; e < kGroups; e++) {
-                    if (d0 + e >= D) break;
+                for (int e = 0; e < kGroups; e++)
 #pragma unroll
                     for (int i = 0; i < kOwn; i++) {
                         const float *p = x + (e % DS * 2 * Q + i) * Shape::kRegion;
                         if constexpr (C > 1) {
                             const unsigned at = cluster_addr(smem_addr(p), e / DS);
-                            onum[i] = __fadd_rn(onum[i], cluster_lds1(at));
-                            oden[i] = __fadd_rn(oden[i], cluster_lds1(at + sizeof(float) * DS * 2 * Q * Shape::kRegion));
+                            nu[e][i] = cluster_lds1(at);
+                            de[e][i] = cluster_lds1(at + sizeof(float) * DS * 2 * Q * Shape::kRegion);
                         } else {
-                            onum[i] = __fadd_rn(onum[i], p[0]);
-                            oden[i] = __fadd_rn(oden[i], p[DS * 2 * Q * Shape::kRegion]);
+                            nu[e][i] = p[0];
+                            de[e][i] = p[DS * 2 * Q * Shape::kRegion];
                         }
                     }
-                }
+#pragma unroll
+                for (int e = 0; e < kGroups; e++)
+                    if (d0 + e < D)
+#pragma unroll
+                        for (int i = 0; i < kOwn; i++) {
+                            onum[i] = __fadd_rn(onum[i], nu[e][i]);
+                            oden[i] = __fadd_rn(oden[i], de[e][i]);
+                        }
             }
         }
     }
     if constexpr (C > 1) cluster_barrier();  // a CTA's shared memory stays until every other one has read it
-    if (DS > 1 && owner * kOwn >= 2 * Q) return;
+    if (DS > 1 && (owner * kOwn >= 2 * Q || helper)) return;
     int oy, ox;
     place(again(), &oy, &ox);
 #pragma unroll

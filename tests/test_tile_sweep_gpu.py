@@ -107,3 +107,35 @@ def test_few_tiles_shared_by_clusters(D, S):
         # through a state as well: 1 / den of the same sums
         state_out, _ = lpaici.forward_state(ks, t, 0.1, 0.6)
         assert torch.equal(state_out.view(torch.int32), out.view(torch.int32))
+
+
+@pytest.mark.parametrize("D,sizes", [(5, (25,)), (18, (9, 25)), (4, (5, 21, 25)), (5, (3, 3, 27, 25, 23)), (16, (21, 9, 3))])
+def test_cluster_helpers(D, sizes):
+    """The last one or two scales of a direction swept by a second warp: one scale (none to hand over), two,
+    the split before the last scale and before the last two, scales that shrink, more than one round of directions,
+    and images whose warps partly lie outside."""
+    rng = np.random.default_rng(D)
+    S = len(sizes)
+    rows = np.tile(np.array(sizes, np.int32), D)
+    off = (np.cumsum(rows * rows) - rows * rows).astype(np.int32)
+    w = []
+    for n in rows:
+        k = rng.uniform(0.1, 1.0, (n, n)).astype(np.float32)
+        w.append((k / k.sum()).ravel())
+    w = np.concatenate(w).astype(np.float32)
+    ks = lpaici.KernelSet.from_dense(w, off, rows, rows, D, S)
+    ko = ob.DenseKernels(D, S, w, off, rows, rows)
+    var = ks.variances(0.1)
+    for W, H in ((1, 1), (19, 33), (90, 64), (127, 70), (150, 120)):
+        x = rng.uniform(0.0, 1.0, (H, W)).astype(np.float32)
+        for gamma in (0.4, 3.0):
+            out, smap = lpaici.forward(ks, torch_image(x), 0.1, gamma, scale_map=True)
+            ref, rmap, _ = ob.oracle_forward_f32(x, ko, var, gamma, want_map=True)
+            assert np.array_equal(smap.cpu().numpy(), rmap), (W, H, gamma)
+            assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32)), (W, H, gamma)
+
+
+def torch_image(x):
+    import torch
+
+    return torch.from_numpy(x).cuda()
