@@ -53,8 +53,9 @@ static int groups_of(int c) {
 }
 
 // The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; back to back 97 x 64 takes 12.8 us
-// with the symmetric set and 17.3 us with the tapered one, 128 x 128 17.0 and 24.1 us, 150 x 120 22.7 and 36.2 us).
-static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{5.3f, 0.72f}, {6.4f, 1.12f}, {4.2f, 2.1f}};
+// with the symmetric set and 17.3 us with the tapered one, 128 x 128 17.0 and 24.1 us, 150 x 120 22.7 and 36.2 us,
+// 200 x 150 25.1 and 40.7 us).
+static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{5.3f, 0.72f}, {6.4f, 1.12f}, {4.2f, 2.1f}, {3.8f, 2.45f}};
 
 static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int ds) {
     const int nk = ks->D * ks->S;
@@ -185,7 +186,7 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
             size_t smem = 0;
             cluster_config(c, ks->radius, ks->layout.total_words, ks->D * ks->S, &tw, &th, &ctas, &groups, &smem);
             const long tiles = static_cast<long>((widths[0] + tw - 1) / tw) * ((rows[0] + th - 1) / th);
-            const long slots = (pc.sms - 4 - 3 * ctas) / ctas;  // a cluster's CTAs run in one GPC
+            const long slots = ctas == 1 ? pc.sms : (pc.sms - 4 - 3 * ctas) / ctas;  // a cluster's CTAs run in one GPC
             const double est = estimated_ms(ks, kClusterCost[c], groups);
             if (tiles <= slots && smem <= static_cast<size_t>(pc.max_smem) && est < best_ms) {
                 best_ms = est;

@@ -32,13 +32,16 @@
 #define LPAICI_TILE_MIXES {{0, 4}, {0, 5}, {1, 5}, {3, 5}}
 
 // Tiles that the C CTAs of a cluster share (images of a few tiles; lpaici_forward_cluster_kernel): each CTA has
-// DS direction groups.
+// DS direction groups.  C = 1 takes the images that have more tiles than pairs of CTAs run at once, but no more
+// than there are SMs: a tile's 16 directions in one round (200 x 150: 33.5 us as entry 6 above, 25.1 us so; tapered
+// set 51.4 and 40.7 us).
 // X(index, WX, WY, Q, DS, C)
 #define LPAICI_CLUSTERS(X) \
     X(0, 1, 1, 4, 4, 4)    \
     X(1, 1, 1, 8, 4, 4)    \
-    X(2, 1, 1, 8, 8, 2)
-#define LPAICI_NUM_CLUSTERS 3
+    X(2, 1, 1, 8, 8, 2)    \
+    X(3, 1, 1, 4, 16, 1)
+#define LPAICI_NUM_CLUSTERS 4
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.

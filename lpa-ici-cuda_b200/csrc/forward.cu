@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
 // (SweepSplit).  97 x 64, 16 x 7 symmetric set: 36.9 us with one CTA per 16 x 16 tile, 22.6 us with four, 15.0 us
 // with helpers.
 template <int WX, int WY, int Q, int DS, int C, bool Fused>
-__global__ void __launch_bounds__(2 * 32 * WX * WY * DS, 1)
+__global__ void __launch_bounds__((C > 1 ? 2 : 1) * 32 * WX * WY * DS, 1)
     lpaici_forward_cluster_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
     extern __shared__ __align__(16) int smem[];
     using Shape = TileShape<WX, WY, Q, DS>;
@@ -164,7 +164,7 @@ int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t s
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>(tiles) * C);
-    cfg.blockDim = dim3(2 * Shape::kThreads);  // every warp has a helper
+    cfg.blockDim = dim3((C > 1 ? 2 : 1) * Shape::kThreads);  // every warp has a helper
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;

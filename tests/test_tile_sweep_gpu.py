@@ -6,6 +6,7 @@ import pytest
 
 import lpaici
 import oracle_bind as ob
+from conftest import SYM, kernel_file
 
 pytestmark = pytest.mark.gpu
 
@@ -139,3 +140,19 @@ def torch_image(x):
     import torch
 
     return torch.from_numpy(x).cuda()
+
+
+@pytest.mark.parametrize("W,H", [(200, 150), (180, 190), (592, 64), (16, 2368), (145, 255), (593, 64)])
+def test_one_round_per_tile(W, H):
+    """Images of up to as many 16 x 16 tiles as there are SMs, ragged ones, and one tile column more."""
+    import torch
+
+    ks = lpaici.KernelSet.load(kernel_file(SYM))
+    x = torch_image(np.random.default_rng(W).uniform(0.0, 1.0, (H, W)).astype(np.float32))
+    out, smap = lpaici.forward(ks, x, 0.08, 2.0, scale_map=True)
+    fused = lpaici.forward(ks, x, 0.08, 2.0, ffma=True)
+    ks.set_tile_config(0)
+    ref, rmap = lpaici.forward(ks, x, 0.08, 2.0, scale_map=True)
+    fref = lpaici.forward(ks, x, 0.08, 2.0, ffma=True)
+    assert torch.equal(out.view(torch.int32), ref.view(torch.int32)) and torch.equal(smap, rmap)
+    assert torch.equal(fused.view(torch.int32), fref.view(torch.int32))
