@@ -203,12 +203,113 @@ void batch_plan_free(lpaici_batch *b) {
     delete b;
 }
 
+// The tile configurations of a plan that is not a cluster's, and whether they fit.
+static int check_tiles(lpaici_batch *b, const KernelTables &tab) {
+    int rc = get_info(b->plan.config, tab, &b->info);
+    if (rc == LPAICI_OK && b->plan.rest >= 0) rc = get_info(b->plan.rest, tab, &b->rest);
+    if (rc != LPAICI_OK) return rc;
+    int max_optin = 0;
+    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    if (b->info.smem > static_cast<size_t>(max_optin))
+        return set_error(LPAICI_ERR_UNSUPPORTED, "batched tile needs %zu B of shared memory, device allows %d",
+                         b->info.smem, max_optin);
+    return LPAICI_OK;
+}
+
+// The queue of a plan over images of several sizes, sigmas or gammas: descriptors, tables and ordered items in
+// device memory.
+static int build_queue(lpaici_batch *b, const lpaici_kernelset *ks, const BatchSpec *specs, int n, const KernelTables &tab) {
+    const int nk = ks->D * ks->S;
+    std::vector<BatchImage> imgs(n);
+    std::vector<float> tables(static_cast<size_t>(n) * 2 * nk);
+    struct Item {
+        int image, x, y;
+        long key;
+    };
+    std::vector<Item> items, small;
+    auto push = [&](std::vector<Item> &to, int i, int x, int y, int tw, int th) {
+        const int w = std::min(tw, specs[i].width - x), h = std::min(th, specs[i].height - y);
+        // full tiles first, then by image size (largest first), then raster order
+        const long area = static_cast<long>(specs[i].width) * specs[i].height;
+        if (w > 0 && h > 0) to.push_back({i, x, y, static_cast<long>(w) * h * (1L << 40) + area});
+    };
+    for (int i = 0; i < n; i++) {
+        const BatchSpec &im = specs[i];
+        KernelTables t;
+        fill_tables(ks, nullptr, im.sigma, im.gamma, &t);
+        std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk], t.var, sizeof(float) * nk);
+        std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk + nk], t.thr, sizeof(float) * nk);
+        imgs[i] = BatchImage{im.noisy, im.out, im.smap, im.rden, im.g, im.width, im.height, im.noisy_pitch, im.out_pitch,
+                             im.g_pitch, i * 2 * nk};
+        for (int y = 0; y < im.height; y += b->info.tile_h)
+            for (int x = 0; x < im.width; x += b->info.tile_w) push(items, i, x, y, b->info.tile_w, b->info.tile_h);
+    }
+    const auto by_key = [](const Item &p, const Item &q) { return p.key > q.key; };
+    std::stable_sort(items.begin(), items.end(), by_key);
+    if (b->plan.rest >= 0) {  // all tiles past the plan's big ones are cut small
+        const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_rows));
+        for (size_t j = big; j < items.size(); j++)
+            for (int y = 0; y < b->info.tile_h; y += b->rest.tile_h)
+                for (int x = 0; x < b->info.tile_w; x += b->rest.tile_w)
+                    push(small, items[j].image, items[j].x + x, items[j].y + y, b->rest.tile_w, b->rest.tile_h);
+        items.resize(big);
+        std::stable_sort(small.begin(), small.end(), by_key);
+    }
+    std::vector<int4> qitems;
+    qitems.reserve(items.size() + small.size());
+    for (const Item &it : items) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
+    for (const Item &it : small) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
+
+    const size_t img_bytes = sizeof(BatchImage) * n;
+    const size_t tab_off = (img_bytes + 255) & ~size_t(255);
+    const size_t tab_bytes = sizeof(float) * tables.size();
+    const size_t item_off = (tab_off + tab_bytes + 255) & ~size_t(255);
+    const size_t item_bytes = sizeof(int4) * qitems.size();
+    cudaError_t e = cudaMalloc(&b->dev_mem, item_off + item_bytes);
+    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc(batch plan)");
+    char *base = static_cast<char *>(b->dev_mem);
+    e = cudaMemcpy(base, imgs.data(), img_bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + tab_off, tables.data(), tab_bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(base + item_off, qitems.data(), item_bytes, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_error(e, "cudaMemcpy(batch plan)");
+    b->args.images = reinterpret_cast<const BatchImage *>(base);
+    b->args.tables = reinterpret_cast<const float *>(base + tab_off);
+    b->args.items = reinterpret_cast<const int4 *>(base + item_off);
+    b->args.D = ks->D;
+    b->args.S = ks->S;
+    b->args.R = ks->radius;
+    b->args.blob = tab.blob;
+    b->args.blob_words = tab.blob_words;
+    b->args.mask_word = tab.mask_word;
+    b->args.stream_word = tab.stream_word;
+    b->args.neg_zero = -0.0f;
+    bool same = true;
+    for (int i = 1; i < n; i++) same = same && specs[i].sigma == specs[0].sigma && specs[i].gamma == specs[0].gamma;
+    b->args.shared_tables = same ? 1 : 0;
+    if (same) {
+        std::memcpy(b->args.var, tables.data(), sizeof(float) * nk);
+        std::memcpy(b->args.thr, tables.data() + nk, sizeof(float) * nk);
+    }
+    b->grid = static_cast<int>(items.size());  // one CTA per queue item
+    b->rest_grid = static_cast<int>(small.size());
+    b->args.rest_follows = b->rest_grid > 0 ? 1 : 0;
+
+    int per_sm = 0;
+    e = cudaFuncSetAttribute(b->info.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->info.smem));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->info.fn, b->info.threads, b->info.smem);
+    if (e != cudaSuccess) return cuda_error(e, "batched occupancy");
+    if (per_sm <= 0) return set_error(LPAICI_ERR_UNSUPPORTED, "batched kernel does not fit on an SM");
+    if (b->rest_grid > 0)
+        e = cudaFuncSetAttribute(b->rest.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->rest.smem));
+    return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "batched attributes");
+}
+
 // The plan of lpaici_batch_create for already validated images (specs); the adjoint's batched
 // selection pass uses it with out = null and smap/rden set.
 int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n, int config, bool use_graph,
                       cudaStream_t stream, lpaici_batch **out) {
     *out = nullptr;
-    const int nk = ks->D * ks->S;
     if (ks->S > kMaxScales)
         return set_error(LPAICI_ERR_UNSUPPORTED, "%d scales per direction; the kernels support at most %d", ks->S,
                          kMaxScales);
@@ -242,117 +343,12 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         }
         b->plan = plan_for_images(ks, w.data(), h.data(), n);
     }
-    const bool mixed = b->plan.rest >= 0;
     rc = check_forward_limit(tab);
-    if (rc == LPAICI_OK) rc = get_info(b->plan.config, tab, &b->info);
-    if (rc == LPAICI_OK && mixed) rc = get_info(b->plan.rest, tab, &b->rest);
+    if (rc == LPAICI_OK && b->plan.cluster < 0) rc = check_tiles(b, tab);  // (clusters are chosen among those that fit)
+    if (rc == LPAICI_OK && n != 1 && !one_size) rc = build_queue(b, ks, specs, n, tab);
     if (rc != LPAICI_OK) {
         batch_plan_free(b);
         return rc;
-    }
-
-    // host images: descriptors, tables, and the ordered work queue
-    std::vector<BatchImage> imgs(n);
-    std::vector<float> tables(static_cast<size_t>(n) * 2 * nk);
-    struct Item {
-        int image, x, y;
-        long key;
-    };
-    std::vector<Item> items, small;
-    auto push = [&](std::vector<Item> &to, int i, int x, int y, int tw, int th) {
-        const int w = std::min(tw, specs[i].width - x), h = std::min(th, specs[i].height - y);
-        // full tiles first, then by image size (largest first), then raster order
-        const long area = static_cast<long>(specs[i].width) * specs[i].height;
-        if (w > 0 && h > 0) to.push_back({i, x, y, static_cast<long>(w) * h * (1L << 40) + area});
-    };
-    for (int i = 0; i < n; i++) {
-        const BatchSpec &im = specs[i];
-        KernelTables t;
-        fill_tables(ks, nullptr, im.sigma, im.gamma, &t);
-        std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk], t.var, sizeof(float) * nk);
-        std::memcpy(&tables[static_cast<size_t>(i) * 2 * nk + nk], t.thr, sizeof(float) * nk);
-        imgs[i] = BatchImage{im.noisy, im.out, im.smap, im.rden, im.g, im.width, im.height, im.noisy_pitch, im.out_pitch,
-                             im.g_pitch, i * 2 * nk};
-        for (int y = 0; y < im.height; y += b->info.tile_h)
-            for (int x = 0; x < im.width; x += b->info.tile_w) push(items, i, x, y, b->info.tile_w, b->info.tile_h);
-    }
-    const auto by_key = [](const Item &p, const Item &q) { return p.key > q.key; };
-    std::stable_sort(items.begin(), items.end(), by_key);
-    if (mixed && !(n == 1 || one_size)) {  // all tiles past the plan's big ones are cut small
-        const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_rows));
-        for (size_t j = big; j < items.size(); j++)
-            for (int y = 0; y < b->info.tile_h; y += b->rest.tile_h)
-                for (int x = 0; x < b->info.tile_w; x += b->rest.tile_w)
-                    push(small, items[j].image, items[j].x + x, items[j].y + y, b->rest.tile_w, b->rest.tile_h);
-        items.resize(big);
-        std::stable_sort(small.begin(), small.end(), by_key);
-    }
-    std::vector<int4> qitems;
-    qitems.reserve(items.size() + small.size());
-    for (const Item &it : items) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
-    for (const Item &it : small) qitems.push_back(make_int4(it.image, it.x, it.y, 0));
-
-    const size_t img_bytes = sizeof(BatchImage) * n;
-    const size_t tab_off = (img_bytes + 255) & ~size_t(255);
-    const size_t tab_bytes = sizeof(float) * tables.size();
-    const size_t item_off = (tab_off + tab_bytes + 255) & ~size_t(255);
-    const size_t item_bytes = sizeof(int4) * qitems.size();
-    const size_t total = item_off + item_bytes;
-    cudaError_t e = cudaMalloc(&b->dev_mem, total);
-    if (e != cudaSuccess) {
-        batch_plan_free(b);
-        return cuda_error(e, "cudaMalloc(batch plan)");
-    }
-    char *base = static_cast<char *>(b->dev_mem);
-    e = cudaMemcpy(base, imgs.data(), img_bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + tab_off, tables.data(), tab_bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + item_off, qitems.data(), item_bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        batch_plan_free(b);
-        return cuda_error(e, "cudaMemcpy(batch plan)");
-    }
-    b->args.images = reinterpret_cast<const BatchImage *>(base);
-    b->args.tables = reinterpret_cast<const float *>(base + tab_off);
-    b->args.items = reinterpret_cast<const int4 *>(base + item_off);
-    b->args.D = ks->D;
-    b->args.S = ks->S;
-    b->args.R = ks->radius;
-    b->args.blob = blob;
-    b->args.blob_words = tab.blob_words;
-    b->args.mask_word = tab.mask_word;
-    b->args.stream_word = tab.stream_word;
-    b->args.neg_zero = -0.0f;
-    bool same = true;
-    for (int i = 1; i < n; i++) same = same && specs[i].sigma == specs[0].sigma && specs[i].gamma == specs[0].gamma;
-    b->args.shared_tables = same ? 1 : 0;
-    if (same) {
-        std::memcpy(b->args.var, tables.data(), sizeof(float) * nk);
-        std::memcpy(b->args.thr, tables.data() + nk, sizeof(float) * nk);
-    }
-
-    int max_optin = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-    if (b->info.smem > static_cast<size_t>(max_optin)) {
-        batch_plan_free(b);
-        return set_error(LPAICI_ERR_UNSUPPORTED, "batched tile needs %zu B of shared memory, device allows %d",
-                         b->info.smem, max_optin);
-    }
-    e = cudaFuncSetAttribute(b->info.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->info.smem));
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->info.fn, b->info.threads, b->info.smem);
-    if (e != cudaSuccess || per_sm <= 0) {
-        batch_plan_free(b);
-        return e != cudaSuccess ? cuda_error(e, "batched occupancy")
-                                : set_error(LPAICI_ERR_UNSUPPORTED, "batched kernel does not fit on an SM");
-    }
-    b->grid = static_cast<int>(items.size());  // one CTA per queue item
-    b->rest_grid = static_cast<int>(small.size());
-    b->args.rest_follows = b->rest_grid > 0 ? 1 : 0;
-    if (e == cudaSuccess && b->rest_grid > 0)
-        e = cudaFuncSetAttribute(b->rest.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->rest.smem));
-    if (e != cudaSuccess) {
-        batch_plan_free(b);
-        return cuda_error(e, "batched attributes");
     }
     if (n == 1 || one_size) {
         const BatchSpec &im = specs[0];
@@ -385,7 +381,7 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
     b->use_graph = use_graph;
     if (b->use_graph) {
         cudaStream_t cap = nullptr;
-        e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+        cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             rc = batch_plan_enqueue(b, cap);

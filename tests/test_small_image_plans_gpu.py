@@ -1,0 +1,54 @@
+"""Plans and host arrays of one image of a few tiles, which clusters sweep, with kernel sets that the largest tile
+configuration does not fit: every entry point takes what lpaici_forward and lpaici_backward take, bit for bit."""
+import numpy as np
+import pytest
+
+import lpaici
+
+pytestmark = pytest.mark.gpu
+
+SIGMA, GAMMA = 0.08, 2.0
+# (directions, scales): radius 39 of sixteen directions, radius 47 of eight
+WIDE = [(16, (1, 2, 4, 8, 16, 24, 40)), (8, (1, 48))]
+
+
+def bits(t):
+    import torch
+
+    return t.view(torch.int32)
+
+
+def image(W, H, seed=0):
+    import torch
+
+    g = torch.Generator("cuda")
+    g.manual_seed(W * 8192 + H + seed)
+    return torch.rand(H, W, device="cuda", generator=g)
+
+
+@pytest.mark.parametrize("D,scales", WIDE)
+@pytest.mark.parametrize("W,H", [(64, 64), (97, 64), (150, 120), (200, 150)])
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_plan_of_one_small_image(D, scales, W, H, use_graph):
+    import torch
+
+    ks = lpaici.KernelSet.generate(D, list(scales), 1)
+    x, g = image(W, H), image(W, H, 1)
+    out, grad = torch.empty_like(x), torch.empty_like(x)
+    plan = lpaici.Batch(ks, [x], [out], [SIGMA], [GAMMA], use_graph=use_graph)
+    plan.run()
+    assert torch.equal(bits(out), bits(lpaici.forward(ks, x, SIGMA, GAMMA)))
+    plan.close()
+    plan = lpaici.BackwardBatch(ks, [x], [g], [grad], [SIGMA], [GAMMA], use_graph=use_graph)
+    plan.run()
+    assert torch.equal(bits(grad), bits(lpaici.backward(ks, x, g, SIGMA, GAMMA)))
+    plan.close()
+    assert torch.equal(bits(lpaici.forward_batched(ks, [x], [SIGMA], [GAMMA])[0]), bits(out))
+
+
+def test_forced_configuration_that_does_not_fit_is_refused():
+    ks = lpaici.KernelSet.generate(16, list(WIDE[0][1]), 1)
+    x = image(64, 64)
+    with pytest.raises(lpaici.LpaIciError) as e:
+        lpaici.Batch(ks, [x], [image(64, 64, 2)], [SIGMA], [GAMMA], tile_config=0)
+    assert e.value.code == lpaici.ERR_UNSUPPORTED
