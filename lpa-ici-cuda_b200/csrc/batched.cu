@@ -206,7 +206,7 @@ void batch_plan_free(lpaici_batch *b) {
 // The tile configurations of a plan that is not a cluster's, and whether they fit.
 static int check_tiles(lpaici_batch *b, const KernelTables &tab) {
     int rc = get_info(b->plan.config, tab, &b->info);
-    if (rc == LPAICI_OK && b->plan.rest >= 0) rc = get_info(b->plan.rest, tab, &b->rest);
+    if (rc == LPAICI_OK && b->plan.kind == TilePlan::kMix) rc = get_info(b->plan.rest, tab, &b->rest);
     if (rc != LPAICI_OK) return rc;
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
@@ -246,8 +246,8 @@ static int build_queue(lpaici_batch *b, const lpaici_kernelset *ks, const BatchS
     }
     const auto by_key = [](const Item &p, const Item &q) { return p.key > q.key; };
     std::stable_sort(items.begin(), items.end(), by_key);
-    if (b->plan.rest >= 0) {  // all tiles past the plan's big ones are cut small
-        const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_rows));
+    if (b->plan.kind == TilePlan::kMix) {  // all tiles past the plan's big ones are cut small
+        const size_t big = std::min(items.size(), static_cast<size_t>(b->plan.big_tiles));
         for (size_t j = big; j < items.size(); j++)
             for (int y = 0; y < b->info.tile_h; y += b->rest.tile_h)
                 for (int x = 0; x < b->info.tile_w; x += b->rest.tile_w)
@@ -332,7 +332,7 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
                    ai.g_pitch == a0.g_pitch;
     }
     if (config >= 0) {
-        b->plan.config = config;
+        b->plan = TilePlan::one(config);
     } else if (n == 1 || one_size) {
         b->plan = plan_for(ks, specs[0].width, specs[0].height, n);
     } else {
@@ -344,7 +344,7 @@ int batch_plan_create(const lpaici_kernelset *ks, const BatchSpec *specs, int n,
         b->plan = plan_for_images(ks, w.data(), h.data(), n);
     }
     rc = check_forward_limit(tab);
-    if (rc == LPAICI_OK && b->plan.cluster < 0) rc = check_tiles(b, tab);  // (clusters are chosen among those that fit)
+    if (rc == LPAICI_OK && b->plan.kind != TilePlan::kCluster) rc = check_tiles(b, tab);  // (clusters are chosen among those that fit)
     if (rc == LPAICI_OK && n != 1 && !one_size) rc = build_queue(b, ks, specs, n, tab);
     if (rc != LPAICI_OK) {
         batch_plan_free(b);

@@ -150,14 +150,8 @@ static constexpr int kMixes[][2] = LPAICI_TILE_MIXES;
 static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const int *rows, int n, bool by_rows) {
     TilePlan plan;
     PlanCosts pc;
-    if (!plan_costs(ks, &pc)) {
-        plan.config = default_config(ks);
-        return plan;
-    }
-    if (pc.forced) {
-        plan.config = pc.forced_config;
-        return plan;
-    }
+    if (!plan_costs(ks, &pc)) return TilePlan::one(default_config(ks));
+    if (pc.forced) return TilePlan::one(pc.forced_config);
     double best_ms = -1.0;
     for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
         const float tile_ms = pc.tile_ms[c];
@@ -171,14 +165,11 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
         const double waves = tiles <= pc.sms ? 0.5 * (1 + bps) / bps : static_cast<double>((tiles + slots - 1) / slots);
         const double est = tile_ms * bps * waves;
         if (best_ms < 0.0 || est < best_ms) {
-            plan.config = c;
+            plan = TilePlan::one(c);
             best_ms = est;
         }
     }
-    if (best_ms < 0.0) {
-        plan.config = default_config(ks);
-        return plan;
-    }
+    if (best_ms < 0.0) return TilePlan::one(default_config(ks));
     // one image of a few tiles: clusters, as long as they all run at once
     if (by_rows && n == 1 && !pc.tuned) {
         for (int c = 0; c < LPAICI_NUM_CLUSTERS; c++) {
@@ -190,8 +181,7 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
             const double est = estimated_ms(ks, kClusterCost[c], groups);
             if (tiles <= slots && smem <= static_cast<size_t>(pc.max_smem) && est < best_ms) {
                 best_ms = est;
-                plan = TilePlan{};
-                plan.cluster = c;
+                plan = TilePlan::clusters(c);
             }
         }
     }
@@ -208,20 +198,21 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
             all += static_cast<long>((widths[i] + bw - 1) / bw) * ((rows[i] + bh - 1) / bh);
         }
         const long per = static_cast<long>(aw / bw) * (ah / bh);
-        auto consider = [&](long big, int big_rows) {
+        const long row = by_rows ? static_cast<long>(widths[0] / aw) * n : 1;  // big tiles of one tile row
+        auto consider = [&](long rows_or_tiles) {
+            const long big = rows_or_tiles * row;
             const long small = all - big * per;
             if (big <= 0 || small <= 0) return;
             const double est = mixed_makespan(big, pc.tile_ms[a], small, pc.tile_ms[b], pc.sms);
             if (est < best_ms) {
                 best_ms = est;
-                plan = TilePlan{a, b, big_rows, -1};
+                plan = by_rows ? TilePlan::mix_rows(a, b, static_cast<int>(rows_or_tiles)) : TilePlan::mix_tiles(a, b, big);
             }
         };
-        const long row = by_rows ? static_cast<long>(widths[0] / aw) * n : 1;  // big tiles of one tile row
         if (row <= 0 || whole <= 0) continue;
         const long full = whole / row, w0 = whole / pc.sms;
         for (long r : {full, std::min(full, w0 * pc.sms / row), std::min(full, (w0 - 1) * pc.sms / row)})
-            consider(r * row, static_cast<int>(r));
+            consider(r);
     }
     return plan;
 }
@@ -464,19 +455,22 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
     // image's plan, big tiles in the upper bands and the plan's small ones in the lower (2048^2: 2.45 ms with
     // one configuration in ten bands on two streams, 1.95 ms so).  The first band is one tile row, so that the first forward
     // starts after a short upload, the last one at most two rows of small tiles, so that the download after the
-    // last forward is short; the bands between are about a sixth of the image.
+    // last forward is short; the bands between are about a sixth of the image.  An image that clusters sweep is
+    // one band: it has one wave of tiles, and its copies (under 150 KB each) take less than a band's launches.
     const TilePlan plan = plan_for(ks, width, height);
-    const bool mixed = plan.rest >= 0;
-    int big_h = 64, low_h = 64;
-    lpaici_tile_config_desc(plan.config, nullptr, &big_h, nullptr, nullptr);
+    const bool mixed = plan.kind == TilePlan::kMix;
     const int low_config = mixed ? plan.rest : plan.config;
-    lpaici_tile_config_desc(low_config, nullptr, &low_h, nullptr, nullptr);
+    int big_h = height, low_h = height;
+    if (plan.kind != TilePlan::kCluster) {
+        lpaici_tile_config_desc(plan.config, nullptr, &big_h, nullptr, nullptr);
+        lpaici_tile_config_desc(low_config, nullptr, &low_h, nullptr, nullptr);
+    }
     const int R = ks->radius;
     // band i covers rows [edge[i], edge[i + 1]); bands from `low` on use low_config
     int edge[kMaxBands + 1];
     int nb = 0, low = 0;
     edge[0] = 0;
-    if (height <= 3 * big_h) {
+    if (plan.kind == TilePlan::kCluster || height <= 3 * big_h) {
         edge[++nb] = height;
         low = nb;
     } else {
@@ -520,7 +514,8 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
             rc = cuda_error(e, "lpaici_denoise_host: upload");
             break;
         }
-        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan{plan.config, plan.rest, (r1 - r0) / big_h, -1} : TilePlan{low_config, -1, 0, -1};
+        const TilePlan band = nb == 1 ? plan : i < low ? TilePlan::mix_rows(plan.config, plan.rest, (r1 - r0) / big_h)
+                                               : TilePlan::one(low_config);
         rc = forward_common(ks, b.in, width, width, height, r0, r1 - r0, b.out + static_cast<size_t>(r0) * width, width,
                             nullptr, sigma, gamma, nullptr, sc, &band);
         if (rc != LPAICI_OK) break;
@@ -657,7 +652,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
     int best = -1;
     std::vector<float> config_ms(LPAICI_NUM_TILE_CONFIGS, -1.0f);
     for (int c = 0; rc == LPAICI_OK && c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        int crc = launch_forward(img, tab, TilePlan{c, -1, 0, -1}, stream);  // warm-up
+        int crc = launch_forward(img, tab, TilePlan::one(c), stream);  // warm-up
         if (crc != LPAICI_OK) {
             if (ms_out) ms_out[c] = -1.0f;
             if (crc == LPAICI_ERR_UNSUPPORTED) continue;  // this tile does not fit for this kernel set
@@ -665,7 +660,7 @@ extern "C" int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int 
             break;
         }
         cudaEventRecord(e0, stream);
-        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(img, tab, TilePlan{c, -1, 0, -1}, stream);
+        for (int r = 0; r < reps && crc == LPAICI_OK; r++) crc = launch_forward(img, tab, TilePlan::one(c), stream);
         cudaEventRecord(e1, stream);
         e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) {

@@ -393,7 +393,7 @@ int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const Mu
     if (rc != LPAICI_OK) return rc;
     if (n < 1 || n > kMaxMultiImages)
         return set_error(LPAICI_ERR_INVALID_ARG, "%d images in one launch; at most %d", n, kMaxMultiImages);
-    if (plan.rest < 0) return launch_multi_config(img, tab, mi, n, plan.config, 0, 0, stream);
+    if (plan.kind == TilePlan::kOne) return launch_multi_config(img, tab, mi, n, plan.config, 0, 0, stream);
     int across = 0;
     const MixGrid g = mix_grid(img, plan, n, &across);
     KernelTables first = tab;
@@ -408,8 +408,8 @@ int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan
                          kMaxScales);
     int rc = check_forward_limit(tab);
     if (rc != LPAICI_OK) return rc;
-    if (plan.cluster >= 0) return launch_cluster_config(img, tab, plan.cluster, fused, stream);
-    if (plan.rest < 0) return launch_config(img, tab, plan.config, 0, 0, fused, stream);
+    if (plan.kind == TilePlan::kCluster) return launch_cluster_config(img, tab, plan.cluster, fused, stream);
+    if (plan.kind == TilePlan::kOne) return launch_config(img, tab, plan.config, 0, 0, fused, stream);
     int across = 0;
     const MixGrid g = mix_grid(img, plan, 1, &across);
     KernelTables first = tab;

@@ -77,12 +77,21 @@ struct KernelTables {
     float thr[kMaxKernels];
 };
 
-// How a launch cuts its images into tiles: configuration `config` everywhere, or (rest >= 0) `config` over the
-// whole tile columns of the first big_rows tile rows and configuration `rest` over what they leave.
+// How a launch cuts its images into tiles.  Fields that a kind does not have are -1.
 struct TilePlan {
-    int config = 0;
-    int rest = -1, big_rows = 0;
-    int cluster = -1;  // >= 0: tiles shared by clusters, entry of LPAICI_CLUSTERS (one image, instead of config)
+    enum Kind {
+        kOne,      // configuration `config` everywhere
+        kMix,      // `config` over whole tiles, configuration `rest` over what they leave
+        kCluster,  // one image, its tiles shared by clusters: entry `cluster` of LPAICI_CLUSTERS
+    };
+    Kind kind = kOne;
+    int config = -1, rest = -1, cluster = -1;
+    int big_rows = -1;   // mix over images of one size: whole tile rows of `config`, over their whole tile columns
+    long big_tiles = -1; // mix over images of any sizes: whole tiles of `config`, largest images first
+    static TilePlan one(int config) { return TilePlan{kOne, config, -1, -1, -1, -1}; }
+    static TilePlan mix_rows(int config, int rest, int rows) { return TilePlan{kMix, config, rest, -1, rows, -1}; }
+    static TilePlan mix_tiles(int config, int rest, long tiles) { return TilePlan{kMix, config, rest, -1, -1, tiles}; }
+    static TilePlan clusters(int entry) { return TilePlan{kCluster, -1, -1, entry, -1, -1}; }
 };
 
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
@@ -162,7 +171,6 @@ int default_config(const lpaici_kernelset *ks);
 // else a B200 cost model) times the waves of CTAs the images need.  A forced configuration wins.
 TilePlan plan_for(const lpaici_kernelset *ks, int width, int rows, int n = 1);
 // The same for one launch over n images of any sizes (a batched plan's tile queue): the images' tiles add up.
-// big_rows stands for the number of big tiles.
 TilePlan plan_for_images(const lpaici_kernelset *ks, const int *widths, const int *rows, int n);
 // Kernel sets are supported up to what a 64 x 32 tile with 24 + 2R pair rows takes in shared memory beside
 // the set with duplicated weights: the bound on radius and taps that callers have always met, kept as it is

@@ -52,3 +52,14 @@ def test_forced_configuration_that_does_not_fit_is_refused():
     with pytest.raises(lpaici.LpaIciError) as e:
         lpaici.Batch(ks, [x], [image(64, 64, 2)], [SIGMA], [GAMMA], tile_config=0)
     assert e.value.code == lpaici.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("D,scales", WIDE + [(16, (1, 2, 4, 8, 16, 24, 32))])
+@pytest.mark.parametrize("W,H", [(96, 193), (110, 200), (128, 256), (150, 200), (64, 500), (16, 2000)])
+def test_host_array_of_a_few_tiles(D, scales, W, H):
+    """Taller than three rows of the largest tile, where larger images are cut into bands."""
+    ks = lpaici.KernelSet.generate(D, list(scales), 1)
+    x = image(W, H, 3)
+    ref = lpaici.forward(ks, x, SIGMA, GAMMA).cpu().numpy()
+    got = lpaici.denoise_host(ks, x.cpu().numpy(), SIGMA, GAMMA)
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
