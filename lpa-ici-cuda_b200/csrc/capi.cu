@@ -453,10 +453,13 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
     // idle), its download on s_out.  With pinned host buffers the copies overlap the kernels.
     // The bands' launches overlap, so the GPU sees one stream of tiles: they take the whole
     // image's plan, big tiles in the upper bands and the plan's small ones in the lower (2048^2: 2.45 ms with
-    // one configuration in ten bands on two streams, 1.95 ms so).  The first band is one tile row, so that the first forward
+    // one configuration in ten bands on two streams, 1.95 ms so).
+    // Bands hide the copies behind the kernels at about 6 us of host calls each: as many as make (copies / bands)
+    // + 6 us * bands least, six at most.  Six bands or more: the first is one tile row, so that the first forward
     // starts after a short upload, the last one at most two rows of small tiles, so that the download after the
-    // last forward is short; the bands between are about a sixth of the image.  An image that clusters sweep is
-    // one band: it has one wave of tiles, and its copies (under 150 KB each) take less than a band's launches.
+    // last forward is short.  us from pinned arrays, five to eleven bands at every size and so: 8 directions of one
+    // scale 200x150 58 and 37, 512^2 95 and 64; 16x7 symmetric set 256^2 132 and 73, 512^2 252 and 196; the same from
+    // about 1.35 Mpx on.  An image that clusters sweep is one band too (under 150 KB, one wave of tiles).
     const TilePlan plan = plan_for(ks, width, height);
     const bool mixed = plan.kind == TilePlan::kMix;
     const int low_config = mixed ? plan.rest : plan.config;
@@ -470,10 +473,15 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
     int edge[kMaxBands + 1];
     int nb = 0, low = 0;
     edge[0] = 0;
-    if (plan.kind == TilePlan::kCluster || height <= 3 * big_h) {
+    constexpr int kMostBands = 6;
+    const double copies_us = 2.0 * sizeof(float) * static_cast<double>(n) / 50e3;  // PCIe 5 x16, about 50 GB/s
+    const int bands = std::clamp(static_cast<int>(std::sqrt(copies_us / 6.0)), 1, kMostBands);
+    if (plan.kind == TilePlan::kCluster || bands == 1) {
         edge[++nb] = height;
         low = nb;
     } else {
+        const bool thin_ends = bands == kMostBands;
+        const int rows = (height + bands - 1) / bands;
         const int upper = mixed ? std::min(plan.big_rows * big_h, height) : 0;
         auto cut = [&](int to, int tile, int rows) {  // bands of about `rows` rows, whole tile rows, up to row `to`
             int band = std::max(1, (rows + tile - 1) / tile) * tile;
@@ -484,14 +492,18 @@ int lpaici_denoise_host(const lpaici_kernelset *ks, const float *host_noisy, flo
             if (edge[nb] < to) edge[++nb] = to;
         };
         if (upper > 0) {
-            cut(big_h, big_h, big_h);
-            cut(upper, big_h, (height + 5) / 6);
+            if (thin_ends) cut(big_h, big_h, big_h);
+            cut(upper, big_h, rows);
         }
         low = nb;
-        if (nb == 0) cut(low_h, low_h, low_h);
-        const int last = std::max(edge[nb], height - 2 * low_h - (height - edge[nb]) % low_h);
-        cut(last, low_h, (height + 5) / 6);
-        cut(height, height, height);
+        if (thin_ends) {
+            if (nb == 0) cut(low_h, low_h, low_h);
+            const int last = std::max(edge[nb], height - 2 * low_h - (height - edge[nb]) % low_h);
+            cut(last, low_h, rows);
+            cut(height, height, height);
+        } else {
+            cut(height, low_h, rows);
+        }
         if (!mixed) low = 0;
     }
     HostBuffers &b = t_bufs;

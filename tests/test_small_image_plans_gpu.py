@@ -63,3 +63,15 @@ def test_host_array_of_a_few_tiles(D, scales, W, H):
     ref = lpaici.forward(ks, x, SIGMA, GAMMA).cpu().numpy()
     got = lpaici.denoise_host(ks, x.cpu().numpy(), SIGMA, GAMMA)
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("D,scales", [(8, (1,)), (8, (1, 2, 4, 8)), (16, (1, 2, 4, 8, 16, 24, 32))])
+@pytest.mark.parametrize("W,H", [(200, 150), (275, 273), (390, 400), (1100, 130), (700, 500), (40, 9000), (900, 901), (1200, 1000),
+                                 (1500, 1000), (1, 100000)])
+def test_host_array_of_every_number_of_bands(D, scales, W, H):
+    """One to six bands, with one configuration and with mixes."""
+    ks = lpaici.KernelSet.generate(D, list(scales), 1)
+    x = image(W, H, 4)
+    ref = lpaici.forward(ks, x, SIGMA, GAMMA).cpu().numpy()
+    got = lpaici.denoise_host(ks, x.cpu().numpy(), SIGMA, GAMMA)
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
