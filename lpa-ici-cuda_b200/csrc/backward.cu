@@ -656,7 +656,7 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
 // fitted to the symmetric (475 us), tapered (706 us) and 8 x 4 (74 us) sets.
 // Measured (16 x 7 symmetric set, us for 1 / 4 / 8 CTAs per tile): 15 tiles 473 / 129 / 70, 32 tiles
 // 475 / 130 / 201, 40 tiles 475 / 254 / 203, 128 tiles 475 / 505 / 599, 160 tiles 947 / 629 / 732.
-int gather_plan(const lpaici_kernelset *ks, long tiles, size_t smem, GatherPlan *plan) {
+int gather_plan(const lpaici_kernelset *ks, long tiles, GatherPlan *plan) {
     const AdjointLayout &L = ks->adj_layout;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -679,7 +679,7 @@ int gather_plan(const lpaici_kernelset *ks, long tiles, size_t smem, GatherPlan 
             }
         }
     }
-    const cudaError_t e = cudaFuncSetAttribute(gather_fn(L), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = allow_shared_memory(gather_fn(L));
     return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "adjoint gather attributes");
 }
 
@@ -739,7 +739,7 @@ int gather_pass(const lpaici_kernelset *ks, const int *adj_blob, const uint8_t *
     const long tiles = gather_tiles(ks->adj_layout, width, height, &tiles_x);
     if (tiles > 0x7fffffffL) return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", width, height);
     GatherPlan plan;
-    rc = gather_plan(ks, tiles, smem, &plan);
+    rc = gather_plan(ks, tiles, &plan);
     if (rc != LPAICI_OK) return rc;
     KernelTables tab;
     fill_tables(ks, nullptr, sigma, 1.0f, &tab);
@@ -978,7 +978,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
     }
     b->ga.images = reinterpret_cast<const GatherImage *>(base + desc_off);
     b->ga.items = reinterpret_cast<const int2 *>(base + item_off);
-    rc = gather_plan(ks, total_tiles, b->smem, &b->plan);
+    rc = gather_plan(ks, total_tiles, &b->plan);
     if (rc != LPAICI_OK) {
         backward_batch_free(b);
         return rc;

@@ -295,13 +295,12 @@ static int build_queue(lpaici_batch *b, const lpaici_kernelset *ks, const BatchS
     b->args.rest_follows = b->rest_grid > 0 ? 1 : 0;
 
     int per_sm = 0;
-    e = cudaFuncSetAttribute(b->info.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->info.smem));
+    e = allow_shared_memory(b->info.fn, kStaticShared);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->info.fn, b->info.threads, b->info.smem);
     if (e != cudaSuccess) return cuda_error(e, "batched occupancy");
     if (per_sm <= 0) return set_error(LPAICI_ERR_UNSUPPORTED, "batched kernel does not fit on an SM");
-    if (b->rest_grid > 0)
-        e = cudaFuncSetAttribute(b->rest.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(b->rest.smem));
+    if (b->rest_grid > 0) e = allow_shared_memory(b->rest.fn, kStaticShared);
     return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "batched attributes");
 }
 

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
 // registers its pointers would stay live across the sweep (the single-image kernel reads its parameters).
 struct SharedImage {
     __align__(16) unsigned char raw[sizeof(ImageArgs)];
+    static_assert(sizeof(ImageArgs) + 16 <= kStaticShared, "static shared memory of the kernels that hold one");
     __device__ __forceinline__ const ImageArgs &fill(const ImageArgs &img, const MultiImages &mi, int images, int z) {
         ImageArgs &im = *reinterpret_cast<ImageArgs *>(raw);
         if (threadIdx.x == 0) {
@@ -155,7 +156,7 @@ int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t s
     static_assert(Shape::kRegion == 32, "a group is one warp and its helper");
     const size_t smem = cluster_smem<Shape, Q, DS>(tab.blob_words, tab.D * tab.S, tab.R);
     auto kern = lpaici_forward_cluster_kernel<WX, WY, Q, DS, C, Fused>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, clusters)");
     const int tiles = ((img.W + Shape::kTileW - 1) / Shape::kTileW) * ((img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
     cudaLaunchAttribute attr{};
@@ -186,7 +187,7 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
     if (smem > static_cast<size_t>(max_optin))
         return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d", smem,
                          max_optin);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern), kStaticShared);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, several images)");
     const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
                     across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH, n);
@@ -208,7 +209,7 @@ int launch_cfg(const ImageArgs &img, const KernelTables &tab, int across, int do
     if (smem > static_cast<size_t>(max_optin))
         return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d", smem,
                          max_optin);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward)");
     const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
                     across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
@@ -224,7 +225,7 @@ int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages
     using Shape = TileShape<WX, WY, Q, DS>;
     const size_t smem = sweep_smem<Shape, Q>(tab.blob_words, tab.D * tab.S, tab.R);
     auto kern = lpaici_forward_rest_kernel<WX, WY, Q, DS, Fused>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern), kStaticShared);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, rest)");
     MixGrid g = grid;
     g.right_x = (img.W - g.wb + Shape::kTileW - 1) / Shape::kTileW;
@@ -250,6 +251,14 @@ int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages
 
 }  // namespace
 
+cudaError_t allow_shared_memory(const void *fn, size_t static_bytes) {
+    int dev = 0, max_optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin - static_cast<int>(static_bytes));
+}
+
 #define LPAICI_FWD_CASE(idx, WX, WY, Q, DS)                                      \
     case idx:                                                                    \
         return fused ? launch_cfg<WX, WY, Q, DS, true>(img, tab, across, down, stream) \
@@ -258,7 +267,7 @@ int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages
 template <int WX, int WY, int Q, int DS>
 int blocks_per_sm(size_t smem) {
     auto kern = lpaici_forward_kernel<WX, WY, Q, DS, false>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess) {
+    if (allow_shared_memory(reinterpret_cast<const void *>(kern)) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }

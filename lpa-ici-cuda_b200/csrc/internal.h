@@ -163,6 +163,12 @@ int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan
 // n images of img's size, pitches and tables (tab) in one launch, their buffers in mi.
 int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, const TilePlan &plan,
                          cudaStream_t stream);
+// Static shared memory of the kernels over several images and of the rest (their image arguments), rounded up.
+constexpr size_t kStaticShared = 128;
+// Lets kernel fn launch with all the dynamic shared memory that the current device has beside `static_bytes`.  The
+// value never depends on the kernel set: the attribute belongs to the function, so that a smaller set's size would be
+// in the way of a plan made before with a larger one, and of another thread's launch.
+cudaError_t allow_shared_memory(const void *fn, size_t static_bytes = 0);
 // Bytes of shared memory tile configuration `config` needs for a kernel set.
 size_t config_smem(int config, int blob_words, int nk, int R);
 // The autotuned configuration of ks on the current device, else the first one that fits.

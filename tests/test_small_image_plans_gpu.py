@@ -75,3 +75,68 @@ def test_host_array_of_every_number_of_bands(D, scales, W, H):
     ref = lpaici.forward(ks, x, SIGMA, GAMMA).cpu().numpy()
     got = lpaici.denoise_host(ks, x.cpu().numpy(), SIGMA, GAMMA)
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+def small_and_large_sets():
+    return (lpaici.KernelSet.generate(16, [1, 2, 4, 8, 16, 24, 32], 1), lpaici.KernelSet.generate(8, [1, 2, 4], 1))
+
+
+def test_plans_of_a_large_and_a_small_set_in_turn():
+    """A plan keeps working after another set's plans, launches and adjoints have used the same kernels with less
+    shared memory."""
+    import torch
+
+    sets = small_and_large_sets()
+    xs = [image(300, 200), image(150, 260, 1), image(64, 64, 2)]
+    gs = [image(300, 200, 5), image(150, 260, 6), image(64, 64, 7)]
+    sig = [SIGMA, SIGMA + 0.01, SIGMA]
+    for config in (-1, 0, 4):
+        plans = []
+        for ks in sets:
+            outs, grads = [torch.empty_like(x) for x in xs], [torch.empty_like(x) for x in xs]
+            plans.append((ks, outs, grads, lpaici.Batch(ks, xs, outs, sig, [GAMMA] * 3, use_graph=False, tile_config=config),
+                          lpaici.BackwardBatch(ks, xs, gs, grads, sig, [GAMMA] * 3, use_graph=False, tile_config=config)))
+        for _ in range(2):
+            for ks, outs, grads, fwd, bwd in plans:
+                fwd.run()
+                bwd.run()
+                for x, g, s, o, d in zip(xs, gs, sig, outs, grads):
+                    assert torch.equal(bits(o), bits(lpaici.forward(ks, x, s, GAMMA)))
+                    assert torch.equal(bits(d), bits(lpaici.backward(ks, x, g, s, GAMMA)))
+        for _, _, _, fwd, bwd in plans:
+            fwd.close()
+            bwd.close()
+
+
+def test_threads_with_a_large_and_a_small_set():
+    """Two host threads launch the same kernels with different sets, each on a stream of its own."""
+    import threading
+
+    import torch
+
+    x = image(128, 128)
+    sets = small_and_large_sets()
+    refs = []
+    for ks in sets:
+        ks.set_tile_config(3)
+        refs.append(lpaici.forward(ks, x, SIGMA, GAMMA))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(ks, ref):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(300):
+                    out = lpaici.forward(ks, x, SIGMA, GAMMA)
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(bits(out), bits(ref)):
+                    wrong.append("bits")
+        except lpaici.LpaIciError as e:
+            wrong.append(str(e))
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(sets, refs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
