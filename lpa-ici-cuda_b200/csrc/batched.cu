@@ -210,9 +210,9 @@ static int check_tiles(lpaici_batch *b, const KernelTables &tab) {
     if (rc != LPAICI_OK) return rc;
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-    if (b->info.smem > static_cast<size_t>(max_optin))
+    if (b->info.smem + kStaticShared > static_cast<size_t>(max_optin))
         return set_error(LPAICI_ERR_UNSUPPORTED, "batched tile needs %zu B of shared memory, device allows %d",
-                         b->info.smem, max_optin);
+                         b->info.smem + kStaticShared, max_optin);
     return LPAICI_OK;
 }
 

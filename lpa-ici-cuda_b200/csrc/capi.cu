@@ -24,7 +24,7 @@ int default_config(const lpaici_kernelset *ks) {
     static const int order[] = LPAICI_TILE_PREFERENCE;
     static_assert(sizeof(order) / sizeof(order[0]) == LPAICI_NUM_TILE_CONFIGS, "one preference per configuration");
     for (const int c : order)
-        if (config_smem(c, ks->layout.total_words, ks->D * ks->S, ks->radius) <= static_cast<size_t>(max_optin))
+        if (config_smem(c, ks->layout.total_words, ks->D * ks->S, ks->radius) + kStaticShared <= static_cast<size_t>(max_optin))
             return c;
     return LPAICI_DEFAULT_TILE_CONFIG;  // nothing fits: the launch reports LPAICI_ERR_UNSUPPORTED
 }
@@ -66,7 +66,7 @@ static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int 
 
 static float estimated_tile_ms(const lpaici_kernelset *ks, int c) { return estimated_ms(ks, kTileCost[c], groups_of(c)); }
 
-// CTAs per SM of configuration c for ks on device dev (cached; 0 when it does not fit).
+// CTAs per SM of configuration c for ks on device dev (cached; 0 when it does not fit every kernel of it).
 static int cached_bps(const lpaici_kernelset *ks, int dev, int c, int max_optin) {
     {
         std::lock_guard<std::mutex> lock(ks->mu);
@@ -75,7 +75,7 @@ static int cached_bps(const lpaici_kernelset *ks, int dev, int c, int max_optin)
             return ks->blocks_per_sm[dev][c];
     }
     const size_t smem = config_smem(c, ks->layout.total_words, ks->D * ks->S, ks->radius);
-    const int n = smem <= static_cast<size_t>(max_optin) ? config_blocks_per_sm(c, smem) : 0;
+    const int n = smem + kStaticShared <= static_cast<size_t>(max_optin) ? config_blocks_per_sm(c, smem) : 0;
     std::lock_guard<std::mutex> lock(ks->mu);
     if (static_cast<int>(ks->blocks_per_sm.size()) <= dev) ks->blocks_per_sm.resize(dev + 1);
     if (ks->blocks_per_sm[dev].empty()) ks->blocks_per_sm[dev].assign(LPAICI_NUM_TILE_CONFIGS, -1);

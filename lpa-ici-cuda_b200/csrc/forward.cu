@@ -184,9 +184,9 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
     int dev = 0, max_optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (smem > static_cast<size_t>(max_optin))
-        return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d", smem,
-                         max_optin);
+    if (smem + kStaticShared > static_cast<size_t>(max_optin))
+        return set_error(LPAICI_ERR_UNSUPPORTED, "forward tile needs %zu B of shared memory, device allows %d",
+                         smem + kStaticShared, max_optin);
     cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern), kStaticShared);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, several images)");
     const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,

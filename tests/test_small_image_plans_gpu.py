@@ -140,3 +140,44 @@ def test_threads_with_a_large_and_a_small_set():
     for t in threads:
         t.join()
     assert not wrong, wrong
+
+
+def set_filling_shared_memory(spare):
+    """28 kernels of radius 31 whose set leaves `spare` bytes of an SM's 232,448 beside the 128 x 64 tile: rows of eight
+    taps, the last ones of four (a row is a group of 16 bytes and one per four taps, a bit of the mask per group)."""
+    D, S, n = 7, 4, 63
+    tile = ((128 + 62 + 8) | 1) * (32 + 62) * 8
+    words = (232448 - spare - tile) // 4 - ((3 * D * S + 3) & ~3) - ((D * S + 4) & ~3)
+    groups = words // 4
+    while groups + (((groups + 31) // 32 + 3) // 4) > words // 4:
+        groups -= 1
+    rows = (groups + 2) // 3
+    short = 3 * rows - groups
+    assert rows <= D * S * n
+    w = np.zeros((D * S, n, n), np.float32)
+    for r in range(rows):
+        w[r // n, r % n, (r * 7) % 40:(r * 7) % 40 + (4 if r >= rows - short else 8)] = 1.0 + r % 5
+    w /= np.maximum(w.sum((1, 2), keepdims=True), 1e-6)  # (the last kernel may be empty)
+    off = np.arange(D * S, dtype=np.int32) * n * n
+    rows_ = np.full(D * S, n, np.int32)
+    return lpaici.KernelSet.from_dense(w.ravel(), off, rows_, rows_, D, S)
+
+
+@pytest.mark.parametrize("spare", [0, 16, 32, 48, 64, 80, 96, 128, 144])
+def test_tile_that_leaves_no_room_for_the_image_arguments(spare):
+    """Plans of several images keep their arguments in static shared memory beside the tile."""
+    import torch
+
+    ks = set_filling_shared_memory(spare)
+    xs = [image(900, 640), image(700, 500, 1)]
+    outs = [torch.empty_like(x) for x in xs]
+    plan = lpaici.Batch(ks, xs, outs, [SIGMA, SIGMA], [GAMMA, GAMMA], use_graph=False)
+    plan.run()
+    one = [torch.empty_like(xs[0]) for _ in range(3)]
+    same = lpaici.Batch(ks, [xs[0]] * 3, one, [SIGMA] * 3, [GAMMA] * 3, use_graph=False)
+    same.run()
+    ks.set_tile_config(7)
+    for x, o in zip(xs + [xs[0]], outs + [one[2]]):
+        assert torch.equal(bits(o), bits(lpaici.forward(ks, x, SIGMA, GAMMA)))
+    plan.close()
+    same.close()
