@@ -25,10 +25,13 @@
 #define LPAICI_DEFAULT_TILE_CONFIG 0
 
 // The configurations that can take what whole waves of bigger tiles leave of an image (launch_rest in
-// forward.cu), and the mixes {big, rest} that a plan considers.
+// forward.cu), the mixes {big, rest} that a plan considers, and, in order of preference, the configurations for
+// images of more tile rows than a grid has (the last one fits every supported kernel set).
 #define LPAICI_REST_CONFIGS(X) \
     X(4, 1, 2, 8, 8)           \
-    X(5, 1, 1, 8, 16)
+    X(5, 1, 1, 8, 16)          \
+    X(7, 4, 2, 4, 1)
+#define LPAICI_TALL_CONFIGS {4, 7}
 #define LPAICI_TILE_MIXES {{0, 4}, {0, 5}, {1, 5}, {3, 5}}
 
 // Tiles that the C CTAs of a cluster share (images of a few tiles; lpaici_forward_cluster_kernel): each CTA has

@@ -191,7 +191,6 @@ int launch_multi_cfg(const ImageArgs &img, const KernelTables &tab, const MultiI
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, several images)");
     const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
                     across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH, n);
-    if (grid.y > 65535u) return set_error(LPAICI_ERR_UNSUPPORTED, "image too tall: %d rows", img.rows_out);
     kern<<<grid, Shape::kThreads, smem, stream>>>(img, tab, mi);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "forward launch (several images)");
@@ -213,7 +212,6 @@ int launch_cfg(const ImageArgs &img, const KernelTables &tab, int across, int do
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward)");
     const dim3 grid(across > 0 ? across : (img.W + Shape::kTileW - 1) / Shape::kTileW,
                     across > 0 ? down : (img.rows_out + Shape::kTileH - 1) / Shape::kTileH);
-    if (grid.y > 65535u) return set_error(LPAICI_ERR_UNSUPPORTED, "image too tall: %d rows", img.rows_out);
     kern<<<grid, Shape::kThreads, smem, stream>>>(img, tab);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(e, "forward launch");
@@ -235,6 +233,7 @@ int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages
     const long ctas = static_cast<long>(g.images) * g.n_small;
     if (ctas > 0x7fffffffL) return set_error(LPAICI_ERR_UNSUPPORTED, "image too large: %d x %d", img.W, img.rows_out);
     if (ctas == 0) return LPAICI_OK;
+    const bool follows = g.wb > 0 && g.hb > 0;  // a launch over the big tiles; else this one has the whole image
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -244,7 +243,7 @@ int launch_rest(const ImageArgs &img, const KernelTables &tab, const MultiImages
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = follows ? 1 : 0;
     e = cudaLaunchKernelEx(&cfg, kern, img, tab, mi, g);
     return e == cudaSuccess ? LPAICI_OK : cuda_error(e, "forward launch (rest)");
 }
@@ -381,6 +380,33 @@ void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, 
 #undef LPAICI_CLUSTER_CASE
 }
 
+// Images of more tile rows than a grid has (16-row tiles: 1,048,560 rows) are swept as a rest without big tiles,
+// whose tiles are all in blockIdx.x; taller than 65,535 of the tallest tiles there have been (128 rows), they are
+// refused.  64-row tiles in grid layers were possible too, but the layer's row cost the other images 1.4 to 2.7 % (768
+// x 513 x 3 channels 527 us and 541).
+constexpr int kMaxGridRows = 65535;
+constexpr int kMaxRows = 128 * kMaxGridRows;
+static bool too_tall(const ImageArgs &img, const TilePlan &plan) {
+    int tw = 1, th = 1;
+    if (plan.kind == TilePlan::kCluster) return false;
+    config_tile(plan.config, &tw, &th);
+    return (plan.kind == TilePlan::kMix ? plan.big_rows : (img.rows_out + th - 1) / th) > kMaxGridRows;
+}
+static int launch_tall(const ImageArgs &img, const KernelTables &tab, const MultiImages &mi, int n, bool fused,
+                       cudaStream_t stream) {
+    if (img.rows_out > kMaxRows) return set_error(LPAICI_ERR_UNSUPPORTED, "image too tall: %d rows", img.rows_out);
+    int dev = 0, max_optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    MixGrid g{};
+    g.images = n;
+    static const int order[] = LPAICI_TALL_CONFIGS;
+    for (const int c : order)
+        if (config_smem(c, tab.blob_words, tab.D * tab.S, tab.R) + kStaticShared <= static_cast<size_t>(max_optin))
+            return launch_rest_config(img, tab, mi, g, c, fused, stream);
+    return set_error(LPAICI_ERR_UNSUPPORTED, "no tile for images of %d rows fits", img.rows_out);
+}
+
 // The strips of a plan's mix, for images of img's size.
 static MixGrid mix_grid(const ImageArgs &img, const TilePlan &plan, int n, int *across) {
     int tw = 1, th = 1;
@@ -402,6 +428,7 @@ int launch_forward_multi(const ImageArgs &img, const KernelTables &tab, const Mu
     if (rc != LPAICI_OK) return rc;
     if (n < 1 || n > kMaxMultiImages)
         return set_error(LPAICI_ERR_INVALID_ARG, "%d images in one launch; at most %d", n, kMaxMultiImages);
+    if (too_tall(img, plan)) return launch_tall(img, tab, mi, n, false, stream);
     if (plan.kind == TilePlan::kOne) return launch_multi_config(img, tab, mi, n, plan.config, 0, 0, stream);
     int across = 0;
     const MixGrid g = mix_grid(img, plan, n, &across);
@@ -417,6 +444,7 @@ int launch_forward(const ImageArgs &img, const KernelTables &tab, const TilePlan
                          kMaxScales);
     int rc = check_forward_limit(tab);
     if (rc != LPAICI_OK) return rc;
+    if (too_tall(img, plan)) return launch_tall(img, tab, MultiImages{}, 1, fused, stream);
     if (plan.kind == TilePlan::kCluster) return launch_cluster_config(img, tab, plan.cluster, fused, stream);
     if (plan.kind == TilePlan::kOne) return launch_config(img, tab, plan.config, 0, 0, fused, stream);
     int across = 0;

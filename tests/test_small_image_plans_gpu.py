@@ -181,3 +181,42 @@ def test_tile_that_leaves_no_room_for_the_image_arguments(spare):
         assert torch.equal(bits(o), bits(lpaici.forward(ks, x, SIGMA, GAMMA)))
     plan.close()
     same.close()
+
+
+def check_rows(ks, x, out):
+    """out against bands of x: its first and last rows, and those around the 65,535th 16-, 32- and 64-row tile."""
+    import torch
+
+    H, R = x.shape[0], ks.radius
+    for at in (0, H - 100, 16 * 65535 - 50, 32 * 65535 - 50, 64 * 65535 - 50):
+        if not 0 <= at <= H - 100:
+            continue
+        lo, hi = max(0, at - R), min(H, at + 100 + R)
+        ref = lpaici.forward_rows(ks, x[lo:hi], at - lo, 100, SIGMA, GAMMA)
+        assert torch.equal(bits(out[at:at + 100]), bits(ref)), at
+
+
+@pytest.mark.parametrize("W,H", [(1, 1048561), (5, 1048700), (16, 2097121), (33, 2100000), (64, 4194241), (3, 8388480)])
+def test_images_of_more_tile_rows_than_a_grid(W, H):
+    import torch
+
+    ks = lpaici.KernelSet.generate(8, [1, 2, 4], 1)
+    x = image(W, H)
+    check_rows(ks, x, lpaici.forward(ks, x, SIGMA, GAMMA))
+    if W * H < 40_000_000:
+        outs = [torch.empty_like(x) for _ in range(3)]
+        xs = [x, image(W, H, 1), image(W, H, 2)]
+        plan = lpaici.Batch(ks, xs, outs, [SIGMA] * 3, [GAMMA] * 3)
+        plan.run()
+        for a, o in zip(xs, outs):
+            check_rows(ks, a, o)
+        plan.close()
+    ks.set_tile_config(6)
+    check_rows(ks, x, lpaici.forward(ks, x, SIGMA, GAMMA))
+
+
+def test_images_past_the_tallest_are_refused():
+    ks = lpaici.KernelSet.generate(8, [1, 2, 4], 1)
+    with pytest.raises(lpaici.LpaIciError) as e:
+        lpaici.forward(ks, image(1, 8388481), SIGMA, GAMMA)
+    assert e.value.code == lpaici.ERR_UNSUPPORTED and "too tall" in str(e.value)
