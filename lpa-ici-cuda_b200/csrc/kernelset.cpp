@@ -234,7 +234,8 @@ static int finish_kernelset(lpaici_kernelset *ks) {
             }
             if (any == 0) continue;
             int first = 0, last = Cc - 1;
-            while (row[first] == 0.0f) first++;
+            while (first < Cc && row[first] == 0.0f) first++;
+            if (first == Cc) continue;  // subnormal weights only, on a thread that takes them as zero
             while (row[last] == 0.0f) last--;
             for (int c = first; c <= last; c++) {
                 nsq += row[c] * row[c];  // compute_kernel_variances order; the zero taps left out would add +0
