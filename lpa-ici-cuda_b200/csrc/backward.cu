@@ -85,7 +85,8 @@ struct GatherArgs {
     const int2 *items;           // batched: (image, tile) of every tile
     int D, S, R;
     const int *blob;       // mirrored kernels (lpaici_kernelset::adj_blob, AdjointLayout)
-    int block_bytes;       // shared memory for one kernel's block
+    int pieces;
+    int block_bytes;       // shared memory for one piece's block
     int pitch, plane;      // field geometry (AdjointLayout)
     int cluster;           // CTAs per tile: 1, kGatherChunks / 2 or kGatherChunks
     int first_tile;        // this launch's tiles start here
@@ -93,17 +94,18 @@ struct GatherArgs {
     float rvar[kMaxKernels];  // 1 / v_k of the one image
     // per direction: the field cells its kernels read, rows [x, y), columns [z, w)
     int4 drect[kMaxKernels];
+    int first_piece[kMaxKernels + 1];  // per direction, and past the last one
 };
 
-// Shared memory: kernel table | 1/v table | non-finite flags | two kernel blocks | field | selected scales |
+// Shared memory: piece table | 1/v table | non-finite flags | two blocks | field | selected scales |
 // the groups' sums over the chunks (touched once per chunk: in registers they would cost the run loop its own).
 // The field is stored as two planes of even and odd rows (field row r: plane r & 1, row r >> 1): the 16 row
 // pairs of a warp start on rows of one parity, so with an odd pitch its 32 scalar loads hit 32 banks.
 struct GatherSmem {
     int rv, flag, block, field, smap, sums, total;  // byte offsets
-    __host__ __device__ static GatherSmem make(int nk, int block_bytes, int plane, int region) {
+    __host__ __device__ static GatherSmem make(int nk, int pieces, int block_bytes, int plane, int region) {
         GatherSmem m;
-        m.rv = (8 * (nk + 1) + 15) & ~15;
+        m.rv = (8 * (pieces + 1) + 15) & ~15;
         m.flag = m.rv + ((4 * nk + 15) & ~15);
         m.block = m.flag + 16;
         m.field = m.block + 2 * block_bytes;
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     constexpr int Q = kGatherQ, nthreads = Shape::kThreads;
     extern __shared__ __align__(16) int smem[];
     const int nk = a.D * a.S;
-    const GatherSmem lay = GatherSmem::make(nk, a.block_bytes, a.plane, Shape::kRegion);
+    const GatherSmem lay = GatherSmem::make(nk, a.pieces, a.block_bytes, a.plane, Shape::kRegion);
     char *base = reinterpret_cast<char *>(smem);
     uint2 *s_tab = reinterpret_cast<uint2 *>(base);
     float *s_rv = reinterpret_cast<float *>(base + lay.rv);
@@ -398,14 +400,14 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     const unsigned lane_base = s_f + 4 * ((ty >> 1) * a.pitch + tx);
     const unsigned blocks = smem_addr(base + lay.block);
 
-    for (int i = tid; i <= nk; i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
+    for (int i = tid; i <= a.pieces; i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
     for (int k = tid; k < nk; k += nthreads) s_rv[k] = rvar_k[k];
     if (tid < 2) s_flag[tid] = 0;
     __syncthreads();
-    // kernel k's block to shared memory, asynchronously, into block buffer k & 1
-    auto stage = [&](int k) {
-        const unsigned from = s_tab[k].x, bytes = s_tab[k + 1].x - from;
-        const unsigned dst = blocks + (k & 1) * a.block_bytes;
+    // piece q's block to shared memory, asynchronously, into block buffer q & 1
+    auto stage = [&](int q) {
+        const unsigned from = s_tab[q].x & ~15u, bytes = (s_tab[q + 1].x & ~15u) - from;
+        const unsigned dst = blocks + (q & 1) * a.block_bytes;
         const char *src = reinterpret_cast<const char *>(a.blob) + from;
         for (unsigned o = 16 * tid; o < bytes; o += 16 * nthreads)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + o), "l"(src + o) : "memory");
@@ -415,8 +417,8 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     const int per_chunk = (a.D + kGatherChunks - 1) / kGatherChunks;
     const int chunks = kGatherChunks / a.cluster;  // of this CTA
     const int d_begin = min(a.D, rank * chunks * per_chunk), d_end = min(a.D, (rank + 1) * chunks * per_chunk);
-    const int k_end = d_end * a.S;
-    if (d_begin < d_end) stage(d_begin * a.S);
+    const int q_end = a.first_piece[d_end];
+    if (d_begin < d_end) stage(a.first_piece[d_begin]);
 
     float2 acc[Q];
     // sums of this thread's outputs, pair i at [i * kRegion]: over all chunks (one CTA per tile), else the
@@ -448,12 +450,14 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                 bad = build_field<false, false>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane);
             if (bad) s_flag[d & 1] = 1;
             HeldWords<nthreads> held;
+            const int q_begin = a.first_piece[d], q_stop = a.first_piece[d + 1];
 #pragma unroll 1
-            for (int s = 0; s < a.S; s++) {
-                const int k = d * a.S + s;
-                if (s > 0) __syncthreads();  // every correlation of the previous scale is done with the field
-                if (k + 1 < k_end)
-                    stage(k + 1);
+            for (int q = q_begin; q < q_stop; q++) {
+                // (a scale of several pieces is masked again for each, which changes nothing)
+                const int s = static_cast<int>(s_tab[q].x & 15u);
+                if (q > q_begin) __syncthreads();  // every correlation of the previous piece is done with the field
+                if (q + 1 < q_end)
+                    stage(q + 1);
                 else
                     asm volatile("cp.async.commit_group;" ::: "memory");
                 if (s > 0) {
@@ -466,13 +470,13 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                         mask_read(range, s_f, s_s, tid, nthreads, excluded);
                     }
                 }
-                asm volatile("cp.async.wait_group 1;" ::: "memory");  // this kernel's block has landed
+                asm volatile("cp.async.wait_group 1;" ::: "memory");  // this piece's block has landed
                 __syncthreads();
                 const bool finite = s_flag[d & 1] == 0;
-                if (s == 0 && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
-                const unsigned block = blocks + (k & 1) * a.block_bytes;
+                if (q == q_begin && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
+                const unsigned block = blocks + (q & 1) * a.block_bytes;
                 // the group's units: one stream, the next unit behind the weights of the one before
-                const unsigned ends = s_tab[k].y;
+                const unsigned ends = s_tab[q].y;
                 unsigned at = block + (group == 0 ? 0 : 8 * (ends & 0xffffu));
                 const unsigned last = block + 8 * (group == 0 ? ends & 0xffffu : ends >> 16);
                 if (finite) {
@@ -624,10 +628,12 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
     ga->S = ks->S;
     ga->R = ks->radius;
     ga->blob = adj_blob;
+    ga->pieces = L.pieces;
+    std::copy(L.first_piece.begin(), L.first_piece.end(), ga->first_piece);
     ga->block_bytes = L.block_bytes;
     ga->pitch = L.pitch;
     ga->plane = L.plane;
-    const GatherSmem m = GatherSmem::make(nk, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    const GatherSmem m = GatherSmem::make(nk, L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy);
     *smem = m.total;
     if (*smem > static_cast<size_t>(max_optin))
         return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d", *smem,
@@ -664,7 +670,7 @@ int gather_plan(const lpaici_kernelset *ks, long tiles, GatherPlan *plan) {
     *plan = GatherPlan{tiles, tiles, 1};
     const double tile_us = ks->D * (1.8 + 1.27 * ks->S) + 0.0354 * L.taps + 0.046 * L.units;
     double best = static_cast<double>((tiles + sms - 1) / sms);
-    const GatherSmem m = GatherSmem::make(ks->D * ks->S, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    const GatherSmem m = GatherSmem::make(ks->D * ks->S, L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy);
     for (const int c : {kGatherChunks / 2, kGatherChunks}) {
         // the second chunk's sums of half as many CTAs lie over everything before the first one's
         if (c < kGatherChunks && m.sums < m.total - m.sums) continue;

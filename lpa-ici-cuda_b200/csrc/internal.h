@@ -36,10 +36,11 @@ struct BlobLayout {
 
 // Device image of the adjoint's kernels (mirrored and telescoped, kernelset.cpp) for the gather's tile of
 // 32*wx x 32*wy outputs and its field of two row planes (backward.cu), in bytes:
-//   [0, 8*(nk+1))  per kernel {its block's byte offset, ends of its two streams in 8-byte pairs from the block's
-//                  start, 16 bits each}; kernel k's block ends where k + 1's begins
+//   [0, 8*(pieces+1))  per piece {its block's byte offset | its scale, ends of its two streams in 8-byte pairs from the
+//                  block's start, 16 bits each}; a block ends where the next one begins
 //   blocks, 16-byte aligned: the stream of the first group of warps (units 0, 2, ...), then the second's; a unit is
 //                  {field byte offset, its bytes | L % 4} and L weight pairs
+// A piece is a kernel, or some units of one whose block is too large for two of them in shared memory.
 // A unit is a field row j of a kernel and the columns [a, a + L) where kernel row j (the tap of the lane's first
 // output row) or kernel row j - 1 (of its second) has taps.  The field offset is that of (row R + j, column
 // R + a + L % 4); the pairs are {D(j, t), D(j - 1, t)}, -0 where a row has no tap.
@@ -47,6 +48,8 @@ struct AdjointLayout {
     int wx = 0, wy = 0;       // warps of one group across and down a tile
     int pitch = 0, plane = 0; // floats of a field row and of a row plane
     int block_bytes = 0;      // the largest block
+    int pieces = 0;
+    std::vector<int> first_piece;  // per direction, and past the last one
     int units = 0, taps = 0;  // of all kernels (weight pairs)
     size_t limit_bytes = 0;   // shared memory the support limit counts (gather_setup)
     std::vector<int> box;     // per kernel: first and last row, first and last column of its taps (empty: 0, -1)

@@ -104,7 +104,8 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
     L.limit_bytes = 4 * (static_cast<size_t>(limit_words) + ((nk + 3) & ~3)) + 4 * limit_cells + ((limit_cells + 4 + 15) & ~size_t(15));
 
     // units and weights of every kernel; the offsets of a unit's field rows need the tile's geometry, and the
-    // tile needs the largest block: 128 x 64 outputs if that fits on an SM, else 128 x 32 or 64 x 32
+    // tile needs the largest block: 128 x 64 outputs if two of them fit on an SM beside it, else 128 x 32 or 64 x 32,
+    // or (kernels of thousands of taps) 64 x 32 with blocks cut into pieces of which two fit
     struct Unit {
         int row, col, len;
     };
@@ -166,25 +167,54 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         L.taps += static_cast<int>(pairs[k].size() / 2);
     }
     constexpr size_t kSharedPerCta = 232448;  // sm_100a
+    size_t piece_bytes = L.block_bytes;
     for (const int size : {2, 1, 0}) {
         L.wx = size > 0 ? 4 : 2;
         L.wy = size > 1 ? 2 : 1;
         L.pitch = (32 * L.wx + 2 * R) | 1;
         L.plane = ((32 * L.wy + 2 * R + 1) / 2 * L.pitch + 3) & ~3;
         const size_t sums = 8 * 16 * 2 * static_cast<size_t>(32 * L.wx * L.wy);
-        if (10 * static_cast<size_t>(L.plane) + 2 * L.block_bytes + 12 * (nk + 1) + 64 + sums <= kSharedPerCta) break;
+        const size_t fixed = 10 * static_cast<size_t>(L.plane) + 12 * (nk + 1) + 64 + sums;
+        if (fixed + 2 * L.block_bytes <= kSharedPerCta) break;
+        constexpr size_t kMoreTable = 1024;  // table entries of the pieces; 4096: more than the longest unit
+        if (size == 0) piece_bytes = std::max<size_t>(4096, kSharedPerCta - std::min(kSharedPerCta, fixed + kMoreTable)) / 2;
     }
+    // the units of piece i: [cut[i], cut[i + 1]) of kernel piece_kernel[i]
+    std::vector<int> piece_kernel, cut;
+    L.first_piece.clear();
+    L.block_bytes = 0;
+    for (int k = 0; k < nk; k++) {
+        if (k % S == 0) L.first_piece.push_back(static_cast<int>(piece_kernel.size()));
+        size_t bytes = 0;
+        for (size_t i = 0; i <= units[k].size(); i++) {
+            const size_t unit = i < units[k].size() ? 8 + 8 * static_cast<size_t>(units[k][i].len) : 0;
+            if (i == 0 || ((bytes + unit + 15) & ~size_t(15)) > piece_bytes) {
+                piece_kernel.push_back(k);
+                cut.push_back(static_cast<int>(i));
+                bytes = 0;
+            }
+            bytes += unit;
+            L.block_bytes = std::max(L.block_bytes, static_cast<int>((bytes + 15) & ~size_t(15)));
+        }
+    }
+    L.pieces = static_cast<int>(piece_kernel.size());
+    L.first_piece.push_back(L.pieces);
+    piece_kernel.push_back(nk);
+    cut.push_back(0);
     std::vector<int32_t> &blob = ks->adj_blob;
     blob.reserve(limit_words + limit_words / 4);
-    blob.assign((2 * (static_cast<size_t>(nk) + 1) + 3) & ~size_t(3), 0);
-    for (int k = 0; k < nk; k++) {
+    blob.assign((2 * (static_cast<size_t>(L.pieces) + 1) + 3) & ~size_t(3), 0);
+    size_t w_kernel = 0;  // floats of the kernel's units before the piece
+    for (int p = 0; p < L.pieces; p++) {
+        const int k = piece_kernel[p], past = piece_kernel[p + 1] == k ? cut[p + 1] : static_cast<int>(units[k].size());
+        if (cut[p] == 0) w_kernel = 0;
         const size_t start = blob.size();
-        size_t ends[2];  // of the two groups' streams, in 8-byte pairs: every other unit each
+        size_t ends[2], w = 0;  // ends of the two groups' streams, in 8-byte pairs: every other unit each
         for (int g = 0; g < 2; g++) {
-            size_t w = 0;
-            for (size_t i = 0; i < units[k].size(); i++) {
+            w = w_kernel;
+            for (int i = cut[p]; i < past; i++) {
                 const Unit &u = units[k][i];
-                if (static_cast<int>(i % 2) == g) {
+                if (i % 2 == g) {
                     const int row = R + u.row;
                     blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col + u.len % 4));
                     blob.push_back((8 + 8 * u.len) | (u.len % 4));
@@ -196,11 +226,12 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
             }
             ends[g] = (blob.size() - start) / 2;
         }
-        blob[2 * k] = static_cast<int>(4 * start);
-        blob[2 * k + 1] = static_cast<int32_t>(ends[0] | ends[1] << 16);  // (a kernel has at most 127 x 255 taps)
+        w_kernel = w;
+        blob[2 * p] = static_cast<int>(4 * start) | (k % S & 15);
+        blob[2 * p + 1] = static_cast<int32_t>(ends[0] | ends[1] << 16);  // (a piece is less than 232,448 bytes)
         blob.resize((blob.size() + 3) & ~size_t(3), 0);
     }
-    blob[2 * nk] = static_cast<int>(4 * blob.size());
+    blob[2 * L.pieces] = static_cast<int>(4 * blob.size());
     blob.resize(std::max<size_t>(blob.size(), limit_words), 0);
     return LPAICI_OK;
 }
