@@ -145,16 +145,17 @@ __global__ void __launch_bounds__((C > 1 ? 2 : 1) * 32 * WX * WY * DS, 1)
 
 namespace {
 
-template <class Shape, int Q, int DS>
+// The helpers' sums follow the exchange; a cluster of one CTA has no helpers.
+template <class Shape, int Q, int DS, int C>
 size_t cluster_smem(int blob_words, int nk, int radius) {
-    return sweep_smem<Shape, Q>(blob_words, nk, radius) + sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS;
+    return sweep_smem<Shape, Q>(blob_words, nk, radius) + (C > 1 ? sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS : 0);
 }
 
 template <int WX, int WY, int Q, int DS, int C, bool Fused>
 int launch_cluster(const ImageArgs &img, const KernelTables &tab, cudaStream_t stream) {
     using Shape = TileShape<WX, WY, Q, DS>;
     static_assert(Shape::kRegion == 32, "a group is one warp and its helper");
-    const size_t smem = cluster_smem<Shape, Q, DS>(tab.blob_words, tab.D * tab.S, tab.R);
+    const size_t smem = cluster_smem<Shape, Q, DS, C>(tab.blob_words, tab.D * tab.S, tab.R);
     auto kern = lpaici_forward_cluster_kernel<WX, WY, Q, DS, C, Fused>;
     cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kern));
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(forward, clusters)");
@@ -374,7 +375,7 @@ void cluster_config(int index, int radius, int blob_words, int nk, int *tile_w, 
         *tile_h = 16 * (WY);                                                       \
         *ctas = C;                                                                 \
         *groups = (DS) * (C);                                                      \
-        *smem = cluster_smem<TileShape<WX, WY, Q, DS>, Q, DS>(blob_words, nk, radius); \
+        *smem = cluster_smem<TileShape<WX, WY, Q, DS>, Q, DS, C>(blob_words, nk, radius); \
         return;
     switch (index) { LPAICI_CLUSTERS(LPAICI_CLUSTER_CASE) }
 #undef LPAICI_CLUSTER_CASE
