@@ -134,6 +134,9 @@ __global__ void __launch_bounds__((C > 1 ? 2 : 1) * 32 * WX * WY * DS, 1)
         from = __ldg(tab.blob + min(tab.D, rank * DS) * tab.S);
         to = __ldg(tab.blob + min(tab.D, (rank + 1) * DS) * tab.S);
     }
+    if (C > 1 && threadIdx.x < DS)  // no direction stopped yet
+        reinterpret_cast<unsigned *>(reinterpret_cast<char *>(cta.xch) + Shape::kXchBytes +
+                                     sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS)[threadIdx.x] = 0;
     load_tile(cta.tile, img, x0, y0, cta.g);
     stage_blob<Q>(cta.blob, tab.blob, tab.blob_words, tab.mask_word, tab.stream_word, cta.g.pitch2, from, to);
     stage_tables(cta.tab, tab.var, tab.thr, nk);
@@ -145,10 +148,11 @@ __global__ void __launch_bounds__((C > 1 ? 2 : 1) * 32 * WX * WY * DS, 1)
 
 namespace {
 
-// The helpers' sums follow the exchange; a cluster of one CTA has no helpers.
+// The helpers' sums and stop words follow the exchange; a cluster of one CTA has no helpers.
 template <class Shape, int Q, int DS, int C>
 size_t cluster_smem(int blob_words, int nk, int radius) {
-    return sweep_smem<Shape, Q>(blob_words, nk, radius) + (C > 1 ? sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS : 0);
+    constexpr size_t helpers = sizeof(float2) * kHelperScales * Q * Shape::kRegion * DS + sizeof(int) * DS;
+    return sweep_smem<Shape, Q>(blob_words, nk, radius) + (C > 1 ? helpers : 0);
 }
 
 template <int WX, int WY, int Q, int DS, int C, bool Fused>

@@ -376,6 +376,7 @@ struct SweepSplit {
     int first;      // scale; S: no helper
     unsigned sums;  // shared address of the lane's first pair; a pair of the next column is kRegion pairs on
     unsigned pair;  // named barrier of the two warps
+    unsigned stop;  // shared address of the number of the direction (+ 1) whose remaining scales nobody needs
 };
 // The first scale of direction d's helper: both warps' parts of the stream as equal as they get.
 __device__ __forceinline__ int helper_first(unsigned kernel_table, int d, int S) {
@@ -465,10 +466,16 @@ __device__ __forceinline__ void direction_sweep(int d, int S, unsigned valid, un
         if (!__any_sync(0xffffffffu, changed != 0)) break;  // every pixel of the warp has stopped
     }
     if constexpr (Split)
-        if (!waited) pair_wait(split.pair);
+        if (!waited) {
+            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(split.stop), "r"(d + 1) : "memory");
+            pair_wait(split.pair);
+        }
 }
 
-// The helper's part: the sums of the scales from split.first on.
+// The helper's part: the sums of the scales from split.first on.  Between runs it looks whether the other warp has
+// stopped before them (volatile: an ordinary shared load is hoisted out of the loop), so that a tile whose pixels all
+// stop early ends early: one direction of scales 1 to 42, 33 x 17 flat 116 us without and 39 us so, 16 x 7 symmetric
+// set 97 x 64 14.5 us either way.
 template <int Q, class Tap>
 __device__ __forceinline__ void helper_sweep(int d, int S, unsigned lane_base, unsigned kernel_table, const Tap &tap,
                                              const SweepSplit &split) {
@@ -481,11 +488,17 @@ __device__ __forceinline__ void helper_sweep(int d, int S, unsigned lane_base, u
         for (int m = 0; m < Q; m++) acc[m] = make_float2(0.0f, 0.0f);
         next += 4;
         const unsigned end = lds_u1(next);
+        bool stopped = false;
         if (at != end) {
 #pragma unroll 1
-            do conv_taps<Q>(acc, lane_base, at, tap);
-            while (at != end);
+            do {
+                unsigned word;
+                asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(word) : "r"(split.stop) : "memory");
+                conv_taps<Q>(acc, lane_base, at, tap);
+                stopped = __any_sync(0xffffffffu, word == static_cast<unsigned>(d + 1));
+            } while (at != end && !stopped);
         }
+        if (stopped) break;
 #pragma unroll
         for (int m = 0; m < Q; m++) {
             asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(acc[m].x), "f"(acc[m].y) : "memory");
@@ -554,6 +567,9 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
     asm volatile("mov.b32 %0, %0;" : "+f"(neg_zero));
     const float2 nz = make_float2(neg_zero, neg_zero);
 
+    auto stop_word = [&](int g) {
+        return smem_addr(s_xch) + static_cast<unsigned>(Shape::kXchBytes) + 8 * DS * kHelperScales * Q * 32 + 4 * g;
+    };
     // the pixels whose num and den this thread sums: all 2Q (DS = 1), else kOwn of them
     constexpr int kOwn = DS == 1 ? 2 * Q : (2 * Q >= kGroups ? 2 * Q / kGroups : 1);
     const int owner = static_cast<int>(rank) * DS + group;  // among all groups
@@ -580,7 +596,7 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
             const SweepSplit split{helper_first(kernel_table, d, S),
                                    smem_addr(s_xch) + static_cast<unsigned>(Shape::kXchBytes) +
                                        8 * (group * kHelperScales * Q * 32 + threadIdx.x % 32),
-                                   1u + group};
+                                   1u + group, stop_word(group)};
             if constexpr (Fused)
                 helper_sweep<Q>(d, S, lane_base, kernel_table, FmaTap{}, split);
             else
@@ -594,6 +610,7 @@ __device__ __forceinline__ void sweep_tile(const ImageArgs &img, int x0, int y0,
                 split.sums = smem_addr(s_xch) + static_cast<unsigned>(Shape::kXchBytes) +
                              8 * (group * kHelperScales * Q * 32 + threadIdx.x % 32);
                 split.pair = 1 + group;
+                split.stop = stop_word(group);
             }
             if constexpr (Fused)
                 direction_sweep<Q, (C > 1)>(d, S, valid, lane_base, kernel_table, thr_addr, FmaTap{}, best, sidx, split);
