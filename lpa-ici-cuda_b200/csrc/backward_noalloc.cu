@@ -18,8 +18,13 @@ using namespace lpaici;
 
 namespace {
 
+// Which images fit is counted with the mirrored kernels as the support limit counts them
+// (AdjointLayout::limit_words), so that it does not depend on their layout.  The blob can be larger than that: of
+// kernels whose neighbouring rows do not overlap, every tap is in two weight pairs, at most twice the limit's 8
+// bytes (under 232,448 bytes in all) and a few per unit.  The array has that much more room.
 constexpr size_t kScratchBytes = LPAICI_NOALLOC_SCRATCH_BYTES;
-__device__ __align__(256) unsigned char g_adjoint_scratch[kScratchBytes];
+constexpr size_t kLargerBlob = size_t(512) << 10;
+__device__ __align__(256) unsigned char g_adjoint_scratch[kScratchBytes + kLargerBlob];
 
 size_t round256(size_t n) { return (n + 255) & ~size_t(255); }
 
@@ -52,8 +57,9 @@ extern "C" int lpaici_backward_noalloc(const lpaici_kernelset *ks, const float *
     const size_t blob_bytes = round256(sizeof(int) * ks->blob.size());
     const size_t adj_bytes = round256(sizeof(int) * ks->adj_blob.size());
     const size_t smap_bytes = round256(static_cast<size_t>(ks->D) * npx);
-    const size_t need = blob_bytes + adj_bytes + smap_bytes + sizeof(float) * npx;
-    if (need > kScratchBytes)
+    const size_t fixed = blob_bytes + smap_bytes + sizeof(float) * npx;
+    const size_t need = fixed + round256(sizeof(int) * ks->adj_layout.limit_words);
+    if (need > kScratchBytes || fixed + adj_bytes > sizeof(g_adjoint_scratch))
         return set_error(LPAICI_ERR_UNSUPPORTED,
                          "lpaici_backward_noalloc: a %dx%d image with %d directions needs %zu bytes of scratch, the "
                          "static scratch holds %zu (LPAICI_NOALLOC_SCRATCH_BYTES); use lpaici_backward",

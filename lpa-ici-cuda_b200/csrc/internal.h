@@ -52,6 +52,7 @@ struct AdjointLayout {
     std::vector<int> first_piece;  // per direction, and past the last one
     int units = 0, taps = 0;  // of all kernels (weight pairs)
     size_t limit_bytes = 0;   // shared memory the support limit counts (gather_setup)
+    size_t limit_words = 0;   // of these the kernels, every weight stored twice; also the least size of the blob
     std::vector<int> box;     // per kernel: first and last row, first and last column of its taps (empty: 0, -1)
 };
 

@@ -101,6 +101,7 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
     const int limit_words = (((nk + 1 + 3) & ~3) + 4 * n_runs + 2 * n2 + 3) & ~3;
     const size_t limit_cells = (static_cast<size_t>(16 + 2 * R) * (((128 + 2 * R + 14) & ~7) + 1) + 3) & ~size_t(3);
     AdjointLayout &L = ks->adj_layout;
+    L.limit_words = limit_words;
     L.limit_bytes = 4 * (static_cast<size_t>(limit_words) + ((nk + 3) & ~3)) + 4 * limit_cells + ((limit_cells + 4 + 15) & ~size_t(15));
 
     // units and weights of every kernel; the offsets of a unit's field rows need the tile's geometry, and the
