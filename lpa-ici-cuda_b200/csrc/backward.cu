@@ -16,12 +16,12 @@
 //      The kernels are telescoped, D_s = h'_s - h'_{s-1} (D_0 = h'_0, built by kernelset.cpp), which
 //      turns the sum over scales into
 //          sum_s D_s (*) (c_d [s* >= s]):
-//      the field is zeroed in place where s* < s, scale after scale, and never rebuilt.  Two groups of
-//      warps take every other unit of each kernel over the same outputs.  Every output is written once: no
-//      atomics, deterministic.
+//      the field is zeroed in place where s* < s, scale after scale, and never rebuilt.  Two (or four)
+//      groups of warps take every second (fourth) unit of each kernel over the same outputs.  Every output is
+//      written once: no atomics, deterministic.
 //
 // Order of the sums.  The directions are cut into kGatherChunks chunks; each group sums every chunk from
-// zero (its units in order), the chunks' sums are added in order, and group 1's total is added to group 0's.
+// zero (its units in order), the chunks' sums are added in order, and the groups' totals are added in order.
 // A tile is gathered by one CTA or by a cluster of kGatherChunks or half as many CTAs (the tiles after the last
 // whole wave, gather_plan) that share the chunks
 // and add the same sums in the same order through distributed shared memory, so the gradient does not depend on
@@ -43,7 +43,7 @@ namespace {
 
 // Gather tile geometry.  A lane owns output rows ty, ty + 1 (ty even) at Q = 16 consecutive columns; a warp
 // covers 32 rows x 32 columns (lane l: row pair l & 15, column group l >> 4), WX x WY warps make a group,
-// two groups a CTA.
+// two or four groups a CTA (AdjointLayout::groups).
 //
 // Why row pairs one row apart: field row j meets output row y in kernel row j - y and output row y + 1 in
 // kernel row j - y - 1, so one window of field values serves both output rows, and the packed FMA takes
@@ -52,19 +52,22 @@ namespace {
 // wavefronts a run of 5.7 taps against 8 x 5.7 packed FMAs at 16 outputs a lane), and the packed FMA itself
 // issues faster: 2.0 to 2.2 cycles with one 64-bit operand reused, one broadcast and the accumulator,
 // against 2.4 to 3.4 with three register pairs (measured in chains).  It costs the taps where only one of
-// two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.
+// two neighbouring kernel rows has one: 18 % more for the 16 x 7 sets, 10 % for the tapered ones.  Sets with much
+// more of them have units of single weights and windows of both field rows (single_unit): twice the shared loads, 3 %
+// more for a packed FMA, twice the time before a unit's first tap, no padding (kernelset.cpp has the rule).
 // Q = 16 spreads a run's descriptor, branches and window over 32 outputs.
 // From kept state, 16 x 7 symmetric set: 1024^2 573 us before, 452 us now (300 us of it the units: 250 cycles
 // a unit of 6.0 taps and 32 outputs a lane, 191 of them the packed FMAs; builds 44 us, masking 45 us); tapered
 // set 964 and 685 us; 384 x 320 (15 tiles) 571 and 66 us.
 constexpr int kGatherQ = 16;
-constexpr int kGatherGroups = 2;
 constexpr int kGatherChunks = 8;
-template <int WX, int WY>
+template <int WX, int WY, bool Single>
 struct GatherShape {
     static constexpr int kTW = 32 * WX, kTH = 32 * WY;
+    static constexpr int kGroups = AdjointLayout::groups(WX, WY, Single);
+    static constexpr int kEntry = AdjointLayout::entry_words(kGroups);
     static constexpr int kRegion = 32 * WX * WY;
-    static constexpr int kThreads = kGatherGroups * kRegion;
+    static constexpr int kThreads = kGroups * kRegion;
 };
 
 // One image of the gather: pass A's outputs and the caller's buffers.
@@ -103,15 +106,15 @@ struct GatherArgs {
 // pairs of a warp start on rows of one parity, so with an odd pitch its 32 scalar loads hit 32 banks.
 struct GatherSmem {
     int rv, flag, block, field, smap, sums, total;  // byte offsets
-    __host__ __device__ static GatherSmem make(int nk, int pieces, int block_bytes, int plane, int region) {
+    __host__ __device__ static GatherSmem make(int nk, int entry_words, int pieces, int block_bytes, int plane, int region, int groups) {
         GatherSmem m;
-        m.rv = (8 * (pieces + 1) + 15) & ~15;
+        m.rv = (4 * entry_words * (pieces + 1) + 15) & ~15;
         m.flag = m.rv + ((4 * nk + 15) & ~15);
         m.block = m.flag + 16;
         m.field = m.block + 2 * block_bytes;
         m.smap = m.field + 4 * 2 * plane;
         m.sums = m.smap + ((2 * plane + 15) & ~15);
-        m.total = m.sums + static_cast<int>(sizeof(float2)) * kGatherQ * region * kGatherGroups;
+        m.total = m.sums + static_cast<int>(sizeof(float2)) * kGatherQ * region * groups;
         return m;
     }
 };
@@ -192,7 +195,73 @@ __device__ __forceinline__ void gather_unit(float2 (&acc)[kGatherQ], unsigned sr
     }
 }
 
-// The same for a field with infinities or NaNs: the padding weights (-0, where only the other output row has
+// A unit of single weights (AdjointLayout::single): acc[m] += w_t * {field row r, field row r + 1}[m + t].  The window
+// holds both rows; a and b: their values of tap h.
+template <int H>
+__device__ __forceinline__ void single_head(float2 (&acc)[kGatherQ], const float2 (&win)[kGatherQ], unsigned a, unsigned b,
+                                            unsigned &at) {
+    constexpr int Q = kGatherQ;
+    float2 lead[H];
+    float w[4] = {};
+    const float2 v = lds2(at);
+    w[0] = v.x, w[1] = v.y;
+    if constexpr (H == 3) w[2] = lds1(at + 8);
+#pragma unroll
+    for (int j = 0; j < H; j++) lead[j] = make_float2(lds1(a + 4 * j - 4 * H), lds1(b + 4 * j - 4 * H));
+#pragma unroll
+    for (int j = 0; j < H; j++)
+#pragma unroll
+        for (int m = 0; m < Q; m++)
+            acc[m] = fma2(make_float2(w[j], w[j]), j + m < H ? lead[j + m < H ? j + m : 0] : win[j + m < H ? 0 : j + m - H], acc[m]);
+    at += H == 3 ? 16 : 8;
+}
+template <int P>
+__device__ __forceinline__ void single_block(float2 (&acc)[kGatherQ], float2 (&win)[kGatherQ], unsigned a, unsigned b, unsigned wp) {
+    constexpr int Q = kGatherQ;
+    const float2 w01 = lds2(wp), w23 = lds2(wp + 8);
+    const float w[4] = {w01.x, w01.y, w23.x, w23.y};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        win[(4 * P + j + Q - 1) % Q] = make_float2(lds1(a + 4 * j), lds1(b + 4 * j));
+#pragma unroll
+        for (int m = 0; m < Q; m++) acc[m] = fma2(make_float2(w[j], w[j]), win[(4 * P + j + m) % Q], acc[m]);
+    }
+}
+__device__ __forceinline__ void single_unit(float2 (&acc)[kGatherQ], unsigned a, unsigned b, unsigned h, unsigned at, unsigned end) {
+    float2 win[kGatherQ];
+#pragma unroll
+    for (int i = 0; i < kGatherQ - 1; i++) win[i] = make_float2(lds1(a + 4 * i), lds1(b + 4 * i));
+    if (h > 0) {
+        if (h == 1)
+            single_head<1>(acc, win, a, b, at);
+        else if (h == 2)
+            single_head<2>(acc, win, a, b, at);
+        else
+            single_head<3>(acc, win, a, b, at);
+    }
+    if (at == end) return;
+    a += 4 * (kGatherQ - 1);
+    b += 4 * (kGatherQ - 1);
+#pragma unroll 1
+    while (true) {
+        single_block<0>(acc, win, a, b, at);
+        at += 16;
+        if (at == end) break;
+        single_block<1>(acc, win, a + 16, b + 16, at);
+        at += 16;
+        if (at == end) break;
+        single_block<2>(acc, win, a + 32, b + 32, at);
+        at += 16;
+        if (at == end) break;
+        single_block<3>(acc, win, a + 48, b + 48, at);
+        at += 16;
+        if (at == end) break;
+        a += 64;
+        b += 64;
+    }
+}
+
+// The same as gather_unit for a field with infinities or NaNs: the padding weights (-0, where only the other output row has
 // a tap) are skipped, so that only the pixels whose kernels reach such a value see it.
 __device__ __noinline__ void gather_run_skipping(float2 *acc, unsigned src, unsigned wp, int len) {
     for (int t = 0; t < len; t++) {
@@ -361,14 +430,14 @@ __device__ __forceinline__ float2 cluster_lds2(unsigned a, unsigned rank) {
     return v;
 }
 
-template <int WX, int WY>
-__global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
+template <int WX, int WY, bool Single>
+__global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
     lpaici_adjoint_gather_kernel(const __grid_constant__ GatherArgs a) {
-    using Shape = GatherShape<WX, WY>;
-    constexpr int Q = kGatherQ, nthreads = Shape::kThreads;
+    using Shape = GatherShape<WX, WY, Single>;
+    constexpr int Q = kGatherQ, nthreads = Shape::kThreads, kGroups = Shape::kGroups, kEntry = Shape::kEntry;
     extern __shared__ __align__(16) int smem[];
     const int nk = a.D * a.S;
-    const GatherSmem lay = GatherSmem::make(nk, a.pieces, a.block_bytes, a.plane, Shape::kRegion);
+    const GatherSmem lay = GatherSmem::make(nk, kEntry, a.pieces, a.block_bytes, a.plane, Shape::kRegion, kGroups);
     char *base = reinterpret_cast<char *>(smem);
     uint2 *s_tab = reinterpret_cast<uint2 *>(base);
     float *s_rv = reinterpret_cast<float *>(base + lay.rv);
@@ -398,15 +467,17 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     const int gwarp = gtid >> 5;
     const int ty = (gwarp / WX) * 32 + 2 * (lane & 15), tx = (gwarp % WX) * 32 + (lane >> 4) * Q;
     const unsigned lane_base = s_f + 4 * ((ty >> 1) * a.pitch + tx);
+    // from a cell to the one a row down, from the even and from the odd rows' plane
+    [[maybe_unused]] const int to_odd = 4 * a.plane, to_even = 4 * (a.pitch - a.plane);
     const unsigned blocks = smem_addr(base + lay.block);
 
-    for (int i = tid; i <= a.pieces; i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
+    for (int i = tid; i < kEntry / 2 * (a.pieces + 1); i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
     for (int k = tid; k < nk; k += nthreads) s_rv[k] = rvar_k[k];
     if (tid < 2) s_flag[tid] = 0;
     __syncthreads();
     // piece q's block to shared memory, asynchronously, into block buffer q & 1
     auto stage = [&](int q) {
-        const unsigned from = s_tab[q].x & ~15u, bytes = (s_tab[q + 1].x & ~15u) - from;
+        const unsigned from = s_tab[kEntry / 2 * q].x & ~15u, bytes = (s_tab[kEntry / 2 * (q + 1)].x & ~15u) - from;
         const unsigned dst = blocks + (q & 1) * a.block_bytes;
         const char *src = reinterpret_cast<const char *>(a.blob) + from;
         for (unsigned o = 16 * tid; o < bytes; o += 16 * nthreads)
@@ -454,7 +525,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
 #pragma unroll 1
             for (int q = q_begin; q < q_stop; q++) {
                 // (a scale of several pieces is masked again for each, which changes nothing)
-                const int s = static_cast<int>(s_tab[q].x & 15u);
+                const int s = static_cast<int>(s_tab[kEntry / 2 * q].x & 15u);
                 if (q > q_begin) __syncthreads();  // every correlation of the previous piece is done with the field
                 if (q + 1 < q_end)
                     stage(q + 1);
@@ -476,10 +547,26 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
                 if (q == q_begin && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
                 const unsigned block = blocks + (q & 1) * a.block_bytes;
                 // the group's units: one stream, the next unit behind the weights of the one before
-                const unsigned ends = s_tab[q].y;
-                unsigned at = block + (group == 0 ? 0 : 8 * (ends & 0xffffu));
-                const unsigned last = block + 8 * (group == 0 ? ends & 0xffffu : ends >> 16);
-                if (finite) {
+                const unsigned ends = s_tab[kEntry / 2 * q].y;
+                unsigned at, last;
+                if constexpr (kGroups == 2) {
+                    at = block + (group == 0 ? 0 : 8 * (ends & 0xffffu));
+                    last = block + 8 * (group == 0 ? ends & 0xffffu : ends >> 16);
+                } else {
+                    const unsigned more = s_tab[kEntry / 2 * q + 1].x;
+                    const unsigned e0 = ends & 0xffffu, e1 = ends >> 16, e2 = more & 0xffffu, e3 = more >> 16;
+                    at = block + 8 * (group < 2 ? (group == 0 ? 0 : e0) : (group == 2 ? e1 : e2));
+                    last = block + 8 * (group < 2 ? (group == 0 ? e0 : e1) : (group == 2 ? e2 : e3));
+                }
+                if constexpr (Single) {  // no padding taps: infinities and NaNs need no other loop
+#pragma unroll 1
+                    while (at != last) {
+                        const uint2 u = lds_u2(at);
+                        const unsigned h = u.y & 3u, end = at + (u.y & ~7u), row = lane_base + u.x;
+                        single_unit(acc, row, row + ((u.y & 4u) ? to_even : to_odd), h, at + 8, end);
+                        at = end;
+                    }
+                } else if (finite) {
 #pragma unroll 1
                     while (at != last) {
                         const uint2 u = lds_u2(at);
@@ -516,8 +603,13 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
         if (group == 0) {
 #pragma unroll
             for (int i = 0; i < Q; i++) {
-                const float2 t = s_sum[i * Shape::kRegion], other = s_sum[slot + i * Shape::kRegion];
-                acc[i] = make_float2(t.x + other.x, t.y + other.y);
+                float2 t = s_sum[i * Shape::kRegion];
+#pragma unroll
+                for (int g = 1; g < kGroups; g++) {
+                    const float2 other = s_sum[g * slot + i * Shape::kRegion];
+                    t = make_float2(t.x + other.x, t.y + other.y);
+                }
+                acc[i] = t;
             }
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -542,21 +634,23 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     const int share = slot / a.cluster;
     const unsigned part[2] = {smem_addr(base + lay.sums), smem_addr(s_second)};
     for (int e = rank * share + tid; e < (rank + 1) * share; e += nthreads) {
-        float2 sum[kGatherGroups];
+        float2 sum[kGroups];
 #pragma unroll
-        for (int g = 0; g < kGatherGroups; g++) {
+        for (int g = 0; g < kGroups; g++) {
             sum[g] = make_float2(0.0f, 0.0f);
             for (int c = 0; c < kGatherChunks; c++) {
                 const float2 v = cluster_lds2(part[c % chunks] + 8 * (g * slot + e), c / chunks);
                 sum[g] = make_float2(sum[g].x + v.x, sum[g].y + v.y);
             }
         }
+#pragma unroll
+        for (int g = 1; g < kGroups; g++) sum[0] = make_float2(sum[0].x + sum[g].x, sum[0].y + sum[g].y);
         const int t = e % Shape::kRegion, m = e / Shape::kRegion, w = t >> 5, l = t & 31;
         const int ox = x0 + (w % WX) * 32 + (l >> 4) * Q + m, oy = y0 + (w / WX) * 32 + 2 * (l & 15);
         if (ox < im.W && oy < im.H) {
             float *o = im.grad + static_cast<size_t>(oy) * im.grad_pitch + ox;
-            o[0] = sum[0].x + sum[1].x;
-            if (oy + 1 < im.H) o[im.grad_pitch] = sum[0].y + sum[1].y;
+            o[0] = sum[0].x;
+            if (oy + 1 < im.H) o[im.grad_pitch] = sum[0].y;
         }
     }
     cluster_barrier();  // a CTA's shared memory stays until every other one has read it
@@ -564,13 +658,16 @@ __global__ void __launch_bounds__(GatherShape<WX, WY>::kThreads, 1)
     if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-const void *gather_fn(const AdjointLayout &L) {
-    return L.wx == 2   ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1>)
-           : L.wy == 1 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 1>)
-                       : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2>);
+template <bool Single>
+const void *gather_fn_of(const AdjointLayout &L) {
+    return L.wx == 2   ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<2, 1, Single>)
+           : L.wy == 1 ? reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 1, Single>)
+                       : reinterpret_cast<const void *>(lpaici_adjoint_gather_kernel<4, 2, Single>);
 }
+const void *gather_fn(const AdjointLayout &L) { return L.single ? gather_fn_of<true>(L) : gather_fn_of<false>(L); }
 
-int gather_threads(const AdjointLayout &L) { return kGatherGroups * 32 * L.wx * L.wy; }
+int gather_groups(const AdjointLayout &L) { return AdjointLayout::groups(L.wx, L.wy, L.single); }
+int gather_threads(const AdjointLayout &L) { return gather_groups(L) * 32 * L.wx * L.wy; }
 
 // How a launch's tiles are gathered: the first n_single by one CTA each, the others by clusters of `cluster`.
 struct GatherPlan {
@@ -633,7 +730,7 @@ int gather_setup(const lpaici_kernelset *ks, const int *adj_blob, GatherArgs *ga
     ga->block_bytes = L.block_bytes;
     ga->pitch = L.pitch;
     ga->plane = L.plane;
-    const GatherSmem m = GatherSmem::make(nk, L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    const GatherSmem m = GatherSmem::make(nk, AdjointLayout::entry_words(gather_groups(L)), L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy, gather_groups(L));
     *smem = m.total;
     if (*smem > static_cast<size_t>(max_optin))
         return set_error(LPAICI_ERR_UNSUPPORTED, "adjoint tile needs %zu B of shared memory, device allows %d", *smem,
@@ -668,9 +765,9 @@ int gather_plan(const lpaici_kernelset *ks, long tiles, GatherPlan *plan) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     *plan = GatherPlan{tiles, tiles, 1};
-    const double tile_us = ks->D * (1.8 + 1.27 * ks->S) + 0.0354 * L.taps + 0.046 * L.units;
+    const double tile_us = ks->D * (1.8 + 1.27 * ks->S) + (L.single ? 0.037 * L.taps + 0.1 * L.units : 0.0354 * L.taps + 0.046 * L.units);
     double best = static_cast<double>((tiles + sms - 1) / sms);
-    const GatherSmem m = GatherSmem::make(ks->D * ks->S, L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy);
+    const GatherSmem m = GatherSmem::make(ks->D * ks->S, AdjointLayout::entry_words(gather_groups(L)), L.pieces, L.block_bytes, L.plane, 32 * L.wx * L.wy, gather_groups(L));
     for (const int c : {kGatherChunks / 2, kGatherChunks}) {
         // the second chunk's sums of half as many CTAs lie over everything before the first one's
         if (c < kGatherChunks && m.sums < m.total - m.sums) continue;

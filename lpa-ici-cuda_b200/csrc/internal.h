@@ -36,21 +36,31 @@ struct BlobLayout {
 
 // Device image of the adjoint's kernels (mirrored and telescoped, kernelset.cpp) for the gather's tile of
 // 32*wx x 32*wy outputs and its field of two row planes (backward.cu), in bytes:
-//   [0, 8*(pieces+1))  per piece {its block's byte offset | its scale, ends of its two streams in 8-byte pairs from the
-//                  block's start, 16 bits each}; a block ends where the next one begins
-//   blocks, 16-byte aligned: the stream of the first group of warps (units 0, 2, ...), then the second's; a unit is
-//                  {field byte offset, its bytes | L % 4} and L weight pairs
-// A piece is a kernel, or some units of one whose block is too large for two of them in shared memory.
-// A unit is a field row j of a kernel and the columns [a, a + L) where kernel row j (the tap of the lane's first
-// output row) or kernel row j - 1 (of its second) has taps.  The field offset is that of (row R + j, column
-// R + a + L % 4); the pairs are {D(j, t), D(j - 1, t)}, -0 where a row has no tap.
+//   table          per piece entry_words(groups) words: {its block's byte offset | its scale, then 16 bits for each group's
+//                  end of its stream, in 8-byte pairs from the block's start}, and one more entry; a block ends where the
+//                  next one begins
+//   blocks, 16-byte aligned: the stream of the first group of warps (every groups-th unit), then the next group's
+// A piece is a kernel, or some units of one whose block is too large for two of them in shared memory.  A unit is
+// {field byte offset, its bytes | flags | L % 4} and the weights of L taps, in one of two forms (a set has one):
+//   pairs   a field row j of a kernel and the columns [a, a + L) where kernel row j (the tap of the lane's first output
+//           row) or kernel row j - 1 (of its second) has taps; the weights are {D(j, t), D(j - 1, t)}, -0 where a row has
+//           no tap;
+//   single  a row j of a kernel, which the lane's second output row meets a field row further down; the weights are
+//           D(j, t), the first L % 4 padded to an even number; flag 4: field row R + j is odd.
+// The field offset is that of (row R + j, column R + a + L % 4).
 struct AdjointLayout {
     int wx = 0, wy = 0;       // warps of one group across and down a tile
+    bool single = false;      // the units' form
+    // Groups of warps that share a tile's units.  Four where two are few warps for an SM (64 x 32 tiles: one to a
+    // scheduler; 1024^2 from kept state, a 75 x 75 kernel in three scales 488 and 394 us), but not for 128 x 32 tiles of
+    // pairs, which the two more groups' sums would leave no room (4 x 4 kernels of radius 45 529 and 642 us).
+    static constexpr int groups(int wx, int wy, bool single) { return wx == 2 || (single && wy == 1) ? 4 : 2; }
+    static constexpr int entry_words(int groups) { return groups > 2 ? 4 : 2; }
     int pitch = 0, plane = 0; // floats of a field row and of a row plane
     int block_bytes = 0;      // the largest block
     int pieces = 0;
     std::vector<int> first_piece;  // per direction, and past the last one
-    int units = 0, taps = 0;  // of all kernels (weight pairs)
+    int units = 0, taps = 0;  // of all kernels (weight pairs, or single weights)
     size_t limit_bytes = 0;   // shared memory the support limit counts (gather_setup)
     size_t limit_words = 0;   // of these the kernels, every weight stored twice; also the least size of the blob
     std::vector<int> box;     // per kernel: first and last row, first and last column of its taps (empty: 0, -1)

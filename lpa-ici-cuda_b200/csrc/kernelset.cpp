@@ -42,7 +42,8 @@ int cuda_error(cudaError_t e, const char *what) {
 // so the gather masks one field in place, scale after scale, instead of building a field per scale.
 // The difference is formed in double over the union of the two kernels' boxes (centres aligned) and
 // rounded once.  A lane of the gather owns two neighbouring output rows, so every field row of a kernel
-// becomes a unit of weight pairs {D(j, t), D(j - 1, t)} over the columns of either row (AdjointLayout).
+// becomes a unit of weight pairs {D(j, t), D(j - 1, t)} over the columns of either row, or, in sets whose neighbouring
+// rows hardly overlap, every kernel row a unit of single weights (AdjointLayout).
 // ---------------------------------------------------------------------------------------------
 static int build_adjoint_blob(lpaici_kernelset *ks) {
     const int D = ks->D, S = ks->S, nk = D * S;
@@ -162,10 +163,35 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
                     }
             }
         }
-        const int bytes = static_cast<int>(8 * units[k].size() + 4 * pairs[k].size());
-        L.block_bytes = std::max(L.block_bytes, (bytes + 15) & ~15);
         L.units += static_cast<int>(units[k].size());
         L.taps += static_cast<int>(pairs[k].size() / 2);
+    }
+    // Single weights where the pairs have too much padding.  A tile of 128 x 64 outputs takes 0.037 us a pair and 0.023 a
+    // unit of pairs, 0.038 us a single weight and 0.076 its unit, beside what both take (fitted to 2048^2 with 14 sets,
+    // from lines to dense squares: the fit misses 6 us of a tile at most).  1024^2 from kept state, pairs and single: 16 x
+    // 7 symmetric set (18 % padding) 455 and 477 us, lines of 16 directions 268 and 285; 8 x 3 random rows 454 and 368,
+    // rows of alternating halves 258 and 158.
+    L.single = 0.038 * w.size() + 0.076 * n_runs < 0.037 * L.taps + 0.023 * L.units;
+    if (L.single) {
+        L.units = n_runs;
+        L.taps = static_cast<int>(w.size());
+        auto at = w.begin();
+        for (int k = 0; k < nk; k++) {
+            units[k].clear();
+            pairs[k].clear();
+            for (int r = begin[k]; r < begin[k + 1]; r++) {
+                units[k].push_back({rdy[r], rdx[r], rlen[r]});
+                pairs[k].insert(pairs[k].end(), at, at + rlen[r]);
+                at += rlen[r];
+            }
+        }
+    }
+    const int per_tap = L.single ? 1 : 2;  // weights
+    const auto unit_bytes = [&](const Unit &u) { return 8 + 4 * static_cast<size_t>((per_tap * u.len + 1) & ~1); };
+    for (int k = 0; k < nk; k++) {
+        size_t bytes = 0;
+        for (const Unit &u : units[k]) bytes += unit_bytes(u);
+        L.block_bytes = std::max(L.block_bytes, static_cast<int>((bytes + 15) & ~size_t(15)));
     }
     constexpr size_t kSharedPerCta = 232448;  // sm_100a
     size_t piece_bytes = L.block_bytes;
@@ -174,10 +200,11 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         L.wy = size > 1 ? 2 : 1;
         L.pitch = (32 * L.wx + 2 * R) | 1;
         L.plane = ((32 * L.wy + 2 * R + 1) / 2 * L.pitch + 3) & ~3;
-        const size_t sums = 8 * 16 * 2 * static_cast<size_t>(32 * L.wx * L.wy);
-        const size_t fixed = 10 * static_cast<size_t>(L.plane) + 12 * (nk + 1) + 64 + sums;
+        const int groups = AdjointLayout::groups(L.wx, L.wy, L.single);
+        const size_t sums = 8 * 16 * groups * static_cast<size_t>(32 * L.wx * L.wy);
+        const size_t fixed = 10 * static_cast<size_t>(L.plane) + (4 + 4 * AdjointLayout::entry_words(groups)) * (nk + 1) + 64 + sums;
         if (fixed + 2 * L.block_bytes <= kSharedPerCta) break;
-        constexpr size_t kMoreTable = 1024;  // table entries of the pieces; 4096: more than the longest unit
+        constexpr size_t kMoreTable = 2048;  // 128 pieces; 4096: more than the longest unit
         if (size == 0) piece_bytes = std::max<size_t>(4096, kSharedPerCta - std::min(kSharedPerCta, fixed + kMoreTable)) / 2;
     }
     // the units of piece i: [cut[i], cut[i + 1]) of kernel piece_kernel[i]
@@ -188,7 +215,7 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         if (k % S == 0) L.first_piece.push_back(static_cast<int>(piece_kernel.size()));
         size_t bytes = 0;
         for (size_t i = 0; i <= units[k].size(); i++) {
-            const size_t unit = i < units[k].size() ? 8 + 8 * static_cast<size_t>(units[k][i].len) : 0;
+            const size_t unit = i < units[k].size() ? unit_bytes(units[k][i]) : 0;
             if (i == 0 || ((bytes + unit + 15) & ~size_t(15)) > piece_bytes) {
                 piece_kernel.push_back(k);
                 cut.push_back(static_cast<int>(i));
@@ -204,35 +231,40 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
     cut.push_back(0);
     std::vector<int32_t> &blob = ks->adj_blob;
     blob.reserve(limit_words + limit_words / 4);
-    blob.assign((2 * (static_cast<size_t>(L.pieces) + 1) + 3) & ~size_t(3), 0);
+    const int groups = AdjointLayout::groups(L.wx, L.wy, L.single), entry = AdjointLayout::entry_words(groups);
+    blob.assign((entry * (static_cast<size_t>(L.pieces) + 1) + 3) & ~size_t(3), 0);
     size_t w_kernel = 0;  // floats of the kernel's units before the piece
     for (int p = 0; p < L.pieces; p++) {
         const int k = piece_kernel[p], past = piece_kernel[p + 1] == k ? cut[p + 1] : static_cast<int>(units[k].size());
         if (cut[p] == 0) w_kernel = 0;
         const size_t start = blob.size();
-        size_t ends[2], w = 0;  // ends of the two groups' streams, in 8-byte pairs: every other unit each
-        for (int g = 0; g < 2; g++) {
+        size_t w = 0;
+        for (int g = 0; g < groups; g++) {
             w = w_kernel;
             for (int i = cut[p]; i < past; i++) {
                 const Unit &u = units[k][i];
-                if (i % 2 == g) {
-                    const int row = R + u.row;
-                    blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col + u.len % 4));
-                    blob.push_back((8 + 8 * u.len) | (u.len % 4));
-                    const size_t n = blob.size();
-                    blob.resize(n + 2 * u.len);
-                    std::memcpy(blob.data() + n, pairs[k].data() + w, 8 * static_cast<size_t>(u.len));
+                if (i % groups == g) {
+                    const int row = R + u.row, head = u.len % 4;
+                    blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col + head));
+                    blob.push_back(static_cast<int32_t>(unit_bytes(u)) | (L.single ? (row & 1) << 2 : 0) | head);
+                    const auto put = [&](size_t from, int n) {
+                        blob.resize(blob.size() + n);
+                        std::memcpy(blob.data() + blob.size() - n, pairs[k].data() + from, 4 * static_cast<size_t>(n));
+                    };
+                    put(w, per_tap * head);
+                    if (blob.size() % 2) blob.push_back(0);
+                    put(w + per_tap * head, per_tap * (u.len - head));
                 }
-                w += 2 * static_cast<size_t>(u.len);
+                w += per_tap * static_cast<size_t>(u.len);
             }
-            ends[g] = (blob.size() - start) / 2;
+            // the stream's end in 8-byte pairs, 16 bits (a piece is less than 232,448 bytes)
+            blob[entry * p + 1 + g / 2] |= static_cast<int32_t>((blob.size() - start) / 2 << 16 * (g % 2));
         }
         w_kernel = w;
-        blob[2 * p] = static_cast<int>(4 * start) | (k % S & 15);
-        blob[2 * p + 1] = static_cast<int32_t>(ends[0] | ends[1] << 16);  // (a piece is less than 232,448 bytes)
+        blob[entry * p] = static_cast<int>(4 * start) | (k % S & 15);
         blob.resize((blob.size() + 3) & ~size_t(3), 0);
     }
-    blob[2 * L.pieces] = static_cast<int>(4 * blob.size());
+    blob[entry * L.pieces] = static_cast<int>(4 * blob.size());
     blob.resize(std::max<size_t>(blob.size(), limit_words), 0);
     return LPAICI_OK;
 }
