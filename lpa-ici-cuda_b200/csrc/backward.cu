@@ -68,6 +68,9 @@ struct GatherShape {
     static constexpr int kEntry = AdjointLayout::entry_words(kGroups);
     static constexpr int kRegion = 32 * WX * WY;
     static constexpr int kThreads = kGroups * kRegion;
+    // Kernels in pieces have the smallest tile (build_adjoint_blob); elsewhere a piece is a kernel, and looking pieces up
+    // would cost (64 directions of two scales, 2048^2 from kept state: 2,152 us with lookups, 2,119 us so).
+    static constexpr bool kPieces = WX == 2;
 };
 
 // One image of the gather: pass A's outputs and the caller's buffers.
@@ -437,7 +440,8 @@ __global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
     constexpr int Q = kGatherQ, nthreads = Shape::kThreads, kGroups = Shape::kGroups, kEntry = Shape::kEntry;
     extern __shared__ __align__(16) int smem[];
     const int nk = a.D * a.S;
-    const GatherSmem lay = GatherSmem::make(nk, kEntry, a.pieces, a.block_bytes, a.plane, Shape::kRegion, kGroups);
+    const int pieces = Shape::kPieces ? a.pieces : nk;
+    const GatherSmem lay = GatherSmem::make(nk, kEntry, pieces, a.block_bytes, a.plane, Shape::kRegion, kGroups);
     char *base = reinterpret_cast<char *>(smem);
     uint2 *s_tab = reinterpret_cast<uint2 *>(base);
     float *s_rv = reinterpret_cast<float *>(base + lay.rv);
@@ -471,7 +475,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
     [[maybe_unused]] const int to_odd = 4 * a.plane, to_even = 4 * (a.pitch - a.plane);
     const unsigned blocks = smem_addr(base + lay.block);
 
-    for (int i = tid; i < kEntry / 2 * (a.pieces + 1); i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
+    for (int i = tid; i < kEntry / 2 * (pieces + 1); i += nthreads) s_tab[i] = __ldg(reinterpret_cast<const uint2 *>(a.blob) + i);
     for (int k = tid; k < nk; k += nthreads) s_rv[k] = rvar_k[k];
     if (tid < 2) s_flag[tid] = 0;
     __syncthreads();
@@ -488,8 +492,9 @@ __global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
     const int per_chunk = (a.D + kGatherChunks - 1) / kGatherChunks;
     const int chunks = kGatherChunks / a.cluster;  // of this CTA
     const int d_begin = min(a.D, rank * chunks * per_chunk), d_end = min(a.D, (rank + 1) * chunks * per_chunk);
-    const int q_end = a.first_piece[d_end];
-    if (d_begin < d_end) stage(a.first_piece[d_begin]);
+    const auto first_piece = [&](int d) { return Shape::kPieces ? a.first_piece[d] : d * a.S; };
+    const int q_end = first_piece(d_end);
+    if (d_begin < d_end) stage(first_piece(d_begin));
 
     float2 acc[Q];
     // sums of this thread's outputs, pair i at [i * kRegion]: over all chunks (one CTA per tile), else the
@@ -521,12 +526,12 @@ __global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
                 bad = build_field<false, false>(s_f, s_s, rv_d, im, map, dr, gx0, gy0, a.pitch, a.plane, warp, nwarps, lane);
             if (bad) s_flag[d & 1] = 1;
             HeldWords<nthreads> held;
-            const int q_begin = a.first_piece[d], q_stop = a.first_piece[d + 1];
+            const int q_begin = first_piece(d), n = Shape::kPieces ? first_piece(d + 1) - q_begin : a.S;
 #pragma unroll 1
-            for (int q = q_begin; q < q_stop; q++) {
+            for (int i = 0; i < n; i++) {
                 // (a scale of several pieces is masked again for each, which changes nothing)
-                const int s = static_cast<int>(s_tab[kEntry / 2 * q].x & 15u);
-                if (q > q_begin) __syncthreads();  // every correlation of the previous piece is done with the field
+                const int q = q_begin + i, s = Shape::kPieces ? static_cast<int>(s_tab[kEntry / 2 * q].x & 15u) : i;
+                if (i > 0) __syncthreads();  // every correlation of the previous piece is done with the field
                 if (q + 1 < q_end)
                     stage(q + 1);
                 else
@@ -544,7 +549,7 @@ __global__ void __launch_bounds__(GatherShape<WX, WY, Single>::kThreads, 1)
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // this piece's block has landed
                 __syncthreads();
                 const bool finite = s_flag[d & 1] == 0;
-                if (q == q_begin && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
+                if (i == 0 && tid == 0) s_flag[(d + 1) & 1] = 0;  // last read before this direction's first barrier
                 const unsigned block = blocks + (q & 1) * a.block_bytes;
                 // the group's units: one stream, the next unit behind the weights of the one before
                 const unsigned ends = s_tab[kEntry / 2 * q].y;
