@@ -64,7 +64,10 @@ static float estimated_ms(const lpaici_kernelset *ks, const TileCost &cost, int 
     return 1e-3f * cost.base_us + 1e-6f * cost.ns_per_work * work * rounded;
 }
 
-static float estimated_tile_ms(const lpaici_kernelset *ks, int c) { return estimated_ms(ks, kTileCost[c], groups_of(c)); }
+// (one CTA an SM where the fit had two: 1.5 tile times, as for a lone one in choose_plan)
+static float estimated_tile_ms(const lpaici_kernelset *ks, int c, int bps) {
+    return estimated_ms(ks, kTileCost[c], groups_of(c)) * (bps < kTileCost[c].ctas ? 1.5f : 1.0f);
+}
 
 // CTAs per SM of configuration c for ks on device dev (cached; 0 when it does not fit every kernel of it).
 static int cached_bps(const lpaici_kernelset *ks, int dev, int c, int max_optin) {
@@ -138,8 +141,8 @@ static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
         if (!known) pc->bps[c] = cached_bps(ks, dev, c, pc->max_smem);
         if (pc->bps[c] <= 0)
             pc->tile_ms[c] = 0.0f;
-        else if (!pc->tuned)  // (one CTA where the fit had two: 1.5 tile times, as for a lone one below)
-            pc->tile_ms[c] = estimated_tile_ms(ks, c) * (pc->bps[c] < kTileCost[c].ctas ? 1.5f : 1.0f);
+        else if (!pc->tuned)
+            pc->tile_ms[c] = estimated_tile_ms(ks, c, pc->bps[c]);
     }
     return true;
 }
@@ -170,15 +173,19 @@ static TilePlan choose_plan(const lpaici_kernelset *ks, const int *widths, const
         }
     }
     if (best_ms < 0.0) return TilePlan::one(default_config(ks));
-    // one image of a few tiles: clusters, as long as they all run at once
-    if (by_rows && n == 1 && !pc.tuned) {
+    // one image of a few tiles: clusters, as long as they all run at once.  The autotuner times no clusters: of a tuned
+    // set they are taken to be off their estimates as the one configuration of the same tile is (33 x 20 and 97 x 64 take
+    // 2.4 and 2.3 times as long without, 200 x 150 1.3 times).
+    if (by_rows && n == 1) {
         for (int c = 0; c < LPAICI_NUM_CLUSTERS; c++) {
             int tw = 1, th = 1, ctas = 1, groups = 1;
             size_t smem = 0;
             cluster_config(c, ks->radius, ks->layout.total_words, ks->D * ks->S, &tw, &th, &ctas, &groups, &smem);
             const long tiles = static_cast<long>((widths[0] + tw - 1) / tw) * ((rows[0] + th - 1) / th);
             const long slots = ctas == 1 ? pc.sms : (pc.sms - 4 - 3 * ctas) / ctas;  // a cluster's CTAs run in one GPC
-            const double est = estimated_ms(ks, kClusterCost[c], groups);
+            double est = estimated_ms(ks, kClusterCost[c], groups);
+            const int like = tw == 16 ? 6 : 5;
+            if (pc.tuned && pc.tile_ms[like] > 0.0f) est *= pc.tile_ms[like] / estimated_tile_ms(ks, like, pc.bps[like]);
             if (tiles <= slots && smem <= static_cast<size_t>(pc.max_smem) && est < best_ms) {
                 best_ms = est;
                 plan = TilePlan::clusters(c);
