@@ -33,14 +33,16 @@ int default_config(const lpaici_kernelset *ks) {
 //   base + per_work * W * (directions a round takes, rounded up) / D,   W = taps + 1.4 runs + 5 kernels,
 // fitted to 4096^2 launches (time / waves) of the 16 x 7 symmetric set (W = 8,041) and the 8 x 4 set
 // (W = 545); the tapered set (W = 14,552) is 4 % above its estimate.  A run costs about 1.4 taps beside its
-// taps, a kernel's interval update about 5 (measured with synthetic kernel sets of one run length).
+// taps, a kernel's interval update about 5 (measured with synthetic kernel sets of one run length).  The last entry (64 x
+// 16) stands to the 64 x 32 one a little above their measured times (61 x 61 64 and 89 us, 85 x 85 119 and 164; both are
+// sets of one direction, whose 64 x 32 tiles take less than this table says).
 struct TileCost {
     float base_us, ns_per_work;
     int ctas = 1;  // CTAs per SM of the fit
 };
 static const TileCost kTileCost[LPAICI_NUM_TILE_CONFIGS] = {{8.7f, 59.7f}, {8.1f, 31.2f}, {7.3f, 25.0f}, {4.2f, 15.8f},
                                                             {2.9f, 8.35f}, {0.6f, 4.58f}, {1.2f, 2.60f, 2}, {0.5f, 26.1f},
-                                                            {9.0f, 47.3f}, {9.8f, 36.9f}, {4.8f, 19.5f}};
+                                                            {9.0f, 47.3f}, {9.8f, 36.9f}, {4.8f, 19.5f}, {0.5f, 22.0f}};
 
 static int groups_of(int c) {
 #define LPAICI_GROUPS_CASE(idx, WX, WY, Q, DS) \

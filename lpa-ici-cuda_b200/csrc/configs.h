@@ -4,7 +4,9 @@
 // share the tile and split the directions (sweep_tile in tile_core.cuh).  Each launch takes the
 // configuration with the least estimated time for its image (plan_for in capi.cu); configurations whose
 // shared memory does not fit a kernel set are skipped.  The adjoint's selection pass runs the configuration
-// the forward uses.
+// the forward uses.  The last one is for sets of one or two directions, which groups do not divide, on images of few
+// rows or few tiles: half of a 64 x 32 tile's time (85 x 85 in three scales, us: 4000 x 16 164 as 64 x 32 tiles, 118 as
+// 64 x 16; 200 x 150 164 and 119).
 #pragma once
 
 // X(index, WX, WY, Q, DS)
@@ -19,9 +21,10 @@
     X(7, 4, 2, 4, 1)           \
     X(8, 3, 4, 8, 1)           \
     X(9, 2, 4, 8, 1)           \
-    X(10, 2, 4, 4, 2)
+    X(10, 2, 4, 4, 2)          \
+    X(11, 4, 1, 4, 1)
 
-#define LPAICI_NUM_TILE_CONFIGS 11
+#define LPAICI_NUM_TILE_CONFIGS 12
 #define LPAICI_DEFAULT_TILE_CONFIG 0
 
 // The configurations that can take what whole waves of bigger tiles leave of an image (launch_rest in
@@ -48,4 +51,4 @@
 
 // Without a device to estimate on, the first of these whose shared memory fits is used: the configurations
 // in order of their B200 time on the 4096^2 benchmark image (16x7 symmetric kernels), fastest first.
-#define LPAICI_TILE_PREFERENCE {0, 8, 1, 3, 2, 4, 9, 5, 10, 6, 7}
+#define LPAICI_TILE_PREFERENCE {0, 8, 1, 3, 2, 4, 9, 5, 10, 6, 7, 11}
