@@ -221,7 +221,8 @@ int lpaici_tile_config_desc(int index, int *tile_w, int *tile_h, int *threads, i
 /* Autotuner: times every tile configuration (one warm-up and `reps` timed launches each, CUDA
  * events on `stream`) on the device image d_sample (width x height, pitch floats) -- or, when
  * d_sample is NULL, on a built-in synthetic image of that size -- and makes the fastest the
- * default of this kernel set on the current device.  Per-configuration milliseconds go to
+ * default of this kernel set on the current device: other image sizes take the plan that the measured
+ * times per tile make fastest.  Per-configuration milliseconds go to
  * ms_out[lpaici_num_tile_configs()] when not NULL.  Synchronises `stream`. */
 int lpaici_autotune(lpaici_kernelset *ks, const float *d_sample, int width, int height, int pitch, float sigma,
                     float gamma, int reps, int *best_config, float *ms_out, lpaici_stream_t stream);
@@ -295,14 +296,15 @@ int lpaici_trim_workspace(void);
  * pools.  No counterpart in the reference.
  *   - Size limit: 256-byte-rounded (blob + mirrored blob + D*width*height bytes) + 4*width*height bytes
  *     must fit the scratch (with 16 directions about 3.3 Mpx, e.g. 1920 x 1080); larger images return
- *     LPAICI_ERR_UNSUPPORTED before any CUDA call.
+ *     LPAICI_ERR_UNSUPPORTED before any CUDA call.  The mirrored blob counts with 16 bytes a run and 8 a tap, at
+ *     most lpaici_kernelset_info_t's adjoint_blob_bytes.
  *   - Nothing has to start at zero: every call copies the blobs in (host to device on `stream`) and
  *     the selection sweep writes every byte the gather reads.
  *   - Every call looks up the array's address with cudaGetSymbolAddress; the first call on a device
  *     can load the module holding it, so a caller that captures streams makes that first call before.
- *   - Under CUDA's default lazy module loading, the 64 MiB are reserved on a device only once a process
+ *   - Under CUDA's default lazy module loading, the scratch (and 512 KB) is reserved on a device only once a process
  *     calls this entry point there; with CUDA_MODULE_LOADING=EAGER every process that loads the
- *     library reserves them on every device it uses, forward-only and command-line users included.
+ *     library reserves it on every device it uses, forward-only and command-line users included.
  *   - One scratch per device: calls that overlap on one device (different streams or threads with
  *     work in flight at once) race on it.  Serialise them, e.g. on one stream. */
 int lpaici_backward_noalloc(const lpaici_kernelset *ks, const float *d_noisy, int noisy_pitch,
@@ -314,7 +316,7 @@ int lpaici_backward_noalloc(const lpaici_kernelset *ks, const float *d_noisy, in
 /* The reference engine's own signature and ownership (anisotropic_lpa_ici_gpu_fused,
  * src/v4_1_lpa_ici_2D_sparse_shared.cu:1122-1244): host input and output buffers, the dense
  * kernels and the caller's variances; copies in, denoises on the current device, copies out,
- * synchronously.  channels: 1, or up to 64 interleaved channels denoised one by one (the reference
+ * synchronously.  channels: 1, or up to 64 interleaved channels, each denoised on its own (the reference
  * implements one; lpaici_forward_channels); host_global_weights_buffer is unused (may be NULL), as on the
  * reference's GPU path.  *seconds, if not NULL, receives the reference's timing window: from
  * after the uploads to after the copy of the result back to the host (:1216-1240).

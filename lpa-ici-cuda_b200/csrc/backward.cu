@@ -943,7 +943,7 @@ extern "C" int lpaici_backward(const lpaici_kernelset *ks, const float *d_noisy,
     if (rc == LPAICI_OK) rc = device_adj_blob(ks, &adj);
     if (rc != LPAICI_OK) return rc;
 
-    // transient workspace: D selection planes (bytes) and 1/den (floats)
+    // transient workspace: D selection planes (bytes) and g/den (floats)
     cudaMemPool_t pool = nullptr;
     rc = workspace_pool(&pool);
     if (rc != LPAICI_OK) return rc;
@@ -966,8 +966,8 @@ extern "C" int lpaici_backward(const lpaici_kernelset *ks, const float *d_noisy,
 // ---------------------------------------------------------------------------------------------
 struct lpaici_backward_batch {
     int device = -1;
-    lpaici_batch *select = nullptr;  // pass A: the forward batch plan (out = null, s* and 1/den on)
-    void *dev_mem = nullptr;         // s* planes | 1/den maps | GatherImage[n] | 1/v tables | items
+    lpaici_batch *select = nullptr;  // pass A: the forward batch plan (out = null, s* and g/den on)
+    void *dev_mem = nullptr;         // s* planes | g/den maps | GatherImage[n] | 1/v tables | items
     GatherArgs ga{};
     size_t smem = 0;
     AdjointLayout layout;
@@ -1025,7 +1025,7 @@ extern "C" int lpaici_backward_batch_create(const lpaici_kernelset *ks, const lp
         return rc;
     }
 
-    // plan memory: per image s* planes and 1/den, then the gather's descriptors, tables and items
+    // plan memory: per image s* planes and g/den, then the gather's descriptors, tables and items
     const int nk = ks->D * ks->S;
     std::vector<size_t> smap_off(n), rden_off(n);
     std::vector<int> tiles_x(n);

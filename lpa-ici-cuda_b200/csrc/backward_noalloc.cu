@@ -3,12 +3,12 @@
 // cudaMalloc, cudaMallocAsync or memory pool; no torch).
 //
 // Scratch layout (each part starts on a 256-byte boundary):
-//   [forward kernel blob | mirrored kernel blob | D*W*H selection bytes | W*H floats of 1/den]
+//   [forward kernel blob | mirrored kernel blob | D*W*H selection bytes | W*H floats of g/den]
 // Nothing in it needs to start at zero: the two blobs are copied in by every call, pass A writes every
-// selection byte and 1/den value that pass B reads.
+// selection byte and g/den value that pass B reads.
 //
 // The array lives in its own translation unit.  Under CUDA's default lazy module loading the module that
-// holds it is loaded, and its 64 MiB reserved on a device, only when a process calls this entry point on
+// holds it is loaded, and its 64.5 MiB reserved on a device, only when a process calls this entry point on
 // that device; with CUDA_MODULE_LOADING=EAGER every process that loads the library reserves it on every
 // device it uses.  No counterpart in the reference.
 

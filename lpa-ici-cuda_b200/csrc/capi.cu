@@ -54,7 +54,7 @@ static int groups_of(int c) {
 #undef LPAICI_GROUPS_CASE
 }
 
-// The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; back to back 97 x 64 takes 12.8 us
+// The same for a tile that a cluster shares, alone on its SMs (LPAICI_CLUSTERS; back to back in a graph 97 x 64 takes 12.8 us
 // with the symmetric set and 17.3 us with the tapered one, 128 x 128 17.0 and 24.1 us, 150 x 120 22.7 and 36.2 us,
 // 200 x 150 25.1 and 40.7 us).
 static const TileCost kClusterCost[LPAICI_NUM_CLUSTERS] = {{5.3f, 0.72f}, {6.4f, 1.12f}, {4.2f, 2.1f}, {3.8f, 2.45f}};
@@ -377,7 +377,6 @@ int lpaici_tile_config_desc(int index, int *tile_w, int *tile_h, int *threads, i
 // ---- host-pointer engines ---------------------------------------------------------------------
 
 namespace {
-// Device buffers of lpaici_denoise_host, per thread and device.
 // Device buffers and the copy/compute pipeline of lpaici_denoise_host, per host thread and device.
 constexpr int kMaxBands = 64;
 // Bands in flight: one of fewer tiles than SMs would otherwise hold back the next one on its stream for a tile's time.

@@ -1,5 +1,6 @@
-// forward.cu -- single-image LPA-ICI forward: one launch, one CTA per output tile, all directions
-// and scales of the tile inside the CTA, aggregation in registers.
+// forward.cu -- LPA-ICI forward of one image, or of several of one size: a CTA (a cluster of CTAs for images of a few
+// tiles) sweeps all directions and scales of an output tile and aggregates them; one launch, or two for images whose
+// last wave small tiles take (launch_rest).
 //
 // Replaces the directional loop of anisotropic_lpa_ici_gpu_fused
 // (src/v4_1_lpa_ici_2D_sparse_shared.cu:1216-1235), i.e. 16 launches of
@@ -118,8 +119,8 @@ __global__ void __launch_bounds__(32 * WX * WY * DS, 1)
 
 // An image of a few tiles: C CTAs of a cluster share each tile's directions, as the groups of a CTA do.  Each
 // stages only the runs of its directions if one round covers them all.  A group is one warp and its helper
-// (SweepSplit).  97 x 64, 16 x 7 symmetric set: 36.9 us with one CTA per 16 x 16 tile, 22.6 us with four, 15.0 us
-// with helpers.
+// (SweepSplit).  97 x 64, 16 x 7 symmetric set, calls in a stream one after the other: 36.9 us with one CTA per 16 x 16
+// tile, 22.6 us with four, 14.4 us with helpers (12.9 us of it the kernel, back to back in a graph).
 template <int WX, int WY, int Q, int DS, int C, bool Fused>
 __global__ void __launch_bounds__((C > 1 ? 2 : 1) * 32 * WX * WY * DS, 1)
     lpaici_forward_cluster_kernel(const __grid_constant__ ImageArgs img, const __grid_constant__ KernelTables tab) {
@@ -306,7 +307,7 @@ void config_tile(int config, int *tile_w, int *tile_h) {
 #undef LPAICI_TILE_CASE
 }
 
-// Shared memory a tile configuration needs for a kernel set: blob + tables + the T8 tile.
+// Shared memory a tile configuration needs for a kernel set: blob + tables + the tile + the exchange.
 size_t config_smem(int config, int blob_words, int nk, int R) {
 #define LPAICI_SMEM_CASE(idx, WX, WY, Q, DS)                                                   \
     case idx:                                             \

@@ -109,7 +109,7 @@ struct TilePlan {
 };
 
 // Buffers of the images of a one-size batched plan (lpaici_forward_multi_kernel): image z's input,
-// output, scale maps, 1/den and cotangent (the last four may be null, as in ImageArgs).
+// output, scale maps, 1/den (with a cotangent g/den) and cotangent (the last four may be null, as in ImageArgs).
 constexpr int kMaxMultiImages = 64;
 struct MultiImages {
     const float *in[kMaxMultiImages];
@@ -154,7 +154,7 @@ struct lpaici_kernelset {
     mutable std::vector<int *> dev_adj_blob;
     mutable std::vector<int> tuned_config;  // per device, -1 = not tuned
     // per device: ms one SM spends on one tile of each configuration, from lpaici_autotune (empty: not
-    // tuned, or a configuration forced by lpaici_set_tile_config); and CTAs per SM of each (0: unknown)
+    // tuned, or a configuration forced by lpaici_set_tile_config); and CTAs per SM of each (-1: unknown)
     mutable std::vector<std::vector<float>> tuned_tile_ms;
     mutable std::vector<std::vector<int>> blocks_per_sm;
 };
@@ -220,7 +220,7 @@ int batch_plan_enqueue(lpaici_batch *b, cudaStream_t stream);  // the launch, or
 void batch_plan_free(lpaici_batch *b);
 
 // The adjoint's two passes over storage the caller provides: device copies of ks->blob and ks->adj_blob,
-// D*width*height selection bytes and width*height floats of 1/den.  Allocates nothing.
+// D*width*height selection bytes and width*height floats of g/den.  Allocates nothing.
 int adjoint_passes(const lpaici_kernelset *ks, const int *blob, const int *adj_blob, uint8_t *smap, float *rden,
                    const float *d_noisy, int noisy_pitch, const float *d_grad_out, int gout_pitch, float *d_grad_in,
                    int gin_pitch, int width, int height, float sigma, float gamma, cudaStream_t stream);

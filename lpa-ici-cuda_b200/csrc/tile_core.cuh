@@ -369,7 +369,7 @@ __device__ __forceinline__ float pick(const float2 (&v)[Q], int i) { return (i &
 // from `first` on (the last one or two) while the other sweeps those before it, and hands the sums over in
 // shared memory.  There is one warp to a scheduler otherwise, which waits for its own results most of the time
 // (26,800 cycles for the slowest direction of 97 x 64, 6,000 of them packed arithmetic), and the largest scales
-// are half of a direction's work.  97 x 64 18.9 -> 12.8 us, 128 x 128 23.6 -> 17.0, 150 x 120 27.2 -> 22.7; tapered
+// are half of a direction's work.  Back to back in a graph, us: 97 x 64 18.9 -> 12.8 us, 128 x 128 23.6 -> 17.0, 150 x 120 27.2 -> 22.7; tapered
 // set 25.0 -> 17.3, 32.9 -> 24.1, 41.9 -> 36.2 (with the exchange's loads ahead of its sums).
 constexpr int kHelperScales = 2;
 struct SweepSplit {
