@@ -19,9 +19,9 @@ using namespace lpaici;
 namespace {
 
 // Which images fit is counted with the mirrored kernels as the support limit counts them
-// (AdjointLayout::limit_words), so that it does not depend on their layout.  The blob can be larger than that: of
-// kernels whose neighbouring rows do not overlap, every tap is in two weight pairs, at most twice the limit's 8
-// bytes (under 232,448 bytes in all) and a few per unit.  The array has that much more room.
+// (AdjointLayout::limit_words), so that it does not depend on their layout.  The blob can be larger than that: a tap
+// of a kernel whose neighbouring rows do not overlap is in two weight pairs, at most twice the limit's 8 bytes (under
+// 232,448 bytes in all), beside a few per unit.  The array has that much more room.
 constexpr size_t kScratchBytes = LPAICI_NOALLOC_SCRATCH_BYTES;
 constexpr size_t kLargerBlob = size_t(512) << 10;
 __device__ __align__(256) unsigned char g_adjoint_scratch[kScratchBytes + kLargerBlob];

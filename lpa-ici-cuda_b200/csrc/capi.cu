@@ -121,6 +121,10 @@ struct PlanCosts {
 static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    // the last configuration is for sets of one or two directions: others need not ask what fits of it (3 us of a new
+    // set's first call)
+    const int n = ks->D > 2 ? LPAICI_NUM_TILE_CONFIGS - 1 : LPAICI_NUM_TILE_CONFIGS;
+    pc->bps[LPAICI_NUM_TILE_CONFIGS - 1] = 0;
     bool known = false;  // CTAs per SM of every configuration
     {
         std::lock_guard<std::mutex> lock(ks->mu);
@@ -133,14 +137,14 @@ static bool plan_costs(const lpaici_kernelset *ks, PlanCosts *pc) {
         }
         if (pc->tuned) std::copy_n(ks->tuned_tile_ms[dev].begin(), LPAICI_NUM_TILE_CONFIGS, pc->tile_ms);
         if (dev < static_cast<int>(ks->blocks_per_sm.size()) && !ks->blocks_per_sm[dev].empty()) {
-            std::copy_n(ks->blocks_per_sm[dev].begin(), LPAICI_NUM_TILE_CONFIGS, pc->bps);
-            known = std::all_of(pc->bps, pc->bps + LPAICI_NUM_TILE_CONFIGS, [](int b) { return b >= 0; });
+            std::copy_n(ks->blocks_per_sm[dev].begin(), n, pc->bps);
+            known = std::all_of(pc->bps, pc->bps + n, [](int b) { return b >= 0; });
         }
     }
     cudaDeviceGetAttribute(&pc->sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&pc->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     for (int c = 0; c < LPAICI_NUM_TILE_CONFIGS; c++) {
-        if (!known) pc->bps[c] = cached_bps(ks, dev, c, pc->max_smem);
+        if (!known && c < n) pc->bps[c] = cached_bps(ks, dev, c, pc->max_smem);
         if (pc->bps[c] <= 0)
             pc->tile_ms[c] = 0.0f;
         else if (!pc->tuned)
