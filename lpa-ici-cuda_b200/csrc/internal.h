@@ -39,7 +39,7 @@ struct BlobLayout {
 //   table          per piece entry_words(groups) words: {its block's byte offset | its scale, then 16 bits for each group's
 //                  end of its stream, in 8-byte pairs from the block's start}, and one more entry; a block ends where the
 //                  next one begins
-//   blocks, 16-byte aligned: the stream of the first group of warps (every groups-th unit), then the next group's
+//   blocks, 16-byte aligned: the stream of the first group of warps (every groups-th unit), then the next one's
 // A piece is a kernel, or some units of one whose block is too large for two of them in shared memory.  A unit is
 // {field byte offset, its bytes | flags | L % 4} and the weights of L taps, in one of two forms (a set has one):
 //   pairs   a field row j of a kernel and the columns [a, a + L) where kernel row j (the tap of the lane's first output

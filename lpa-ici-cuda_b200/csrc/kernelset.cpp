@@ -238,12 +238,17 @@ static int build_adjoint_blob(lpaici_kernelset *ks) {
         const int k = piece_kernel[p], past = piece_kernel[p + 1] == k ? cut[p + 1] : static_cast<int>(units[k].size());
         if (cut[p] == 0) w_kernel = 0;
         const size_t start = blob.size();
+        // which group takes a unit: counted from the centre row for single weights, so that a row's weights of one scale
+        // and what the next scale takes back of them meet in one sum (8 x 3 random rows of radius 20, 200 x 130: error
+        // against 64 bits 3.3e-7 of the gradient's rms counted from the first row, 2.1e-7 so; pairs 2.7e-7)
+        int centre = 0;
+        while (L.single && centre < static_cast<int>(units[k].size()) && units[k][centre].row < 0) centre++;
         size_t w = 0;
         for (int g = 0; g < groups; g++) {
             w = w_kernel;
             for (int i = cut[p]; i < past; i++) {
                 const Unit &u = units[k][i];
-                if (i % groups == g) {
+                if ((i + centre * (groups - 1)) % groups == g) {
                     const int row = R + u.row, head = u.len % 4;
                     blob.push_back(4 * ((row & 1) * L.plane + (row >> 1) * L.pitch + R + u.col + head));
                     blob.push_back(static_cast<int32_t>(unit_bytes(u)) | (L.single ? (row & 1) << 2 : 0) | head);
